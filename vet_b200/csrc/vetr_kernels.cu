@@ -1055,87 +1055,135 @@ struct CamAcc
     }
 };
 
-// Sums the accumulators over the CTA and adds the totals to the outputs of `view`: one atomic per value and
-// (CTA, view) instead of one per fragment.
-template <bool kIntr>
-__device__ void reduce_cam(const Frame& f, const BackPtrs& bp, CamAcc<kIntr>& acc, int view, double (*red)[8])
+// Sum over the lanes of a warp of N values per lane, N a power of two: at every step a lane hands the half of its values
+// that the other half-warp is going to own to its partner, so N = 8 takes 9 shuffles instead of 40.  Afterwards v[0] of
+// lane l is the total of value warp_sum_slot<N>(l).
+template <int N>
+__device__ __forceinline__ void warp_sum(double (&v)[N])
 {
-    constexpr int kN = kIntr ? 21 : 7;
+    const int lane = threadIdx.x & 31;
+    int bit = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h /= 2, bit /= 2)
+    {
+        const bool up = lane & bit;
+#pragma unroll
+        for (int i = 0; i < h; ++i)
+        {
+            const double send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+    }
+    for (; bit >= 1; bit /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+}
+template <int N>
+__device__ __forceinline__ int warp_sum_slot(int lane)
+{
+    int slot = 0, bit = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h /= 2, bit /= 2) slot += lane & bit ? h : 0;
+    return slot;
+}
+
+// Sums the accumulators over the CTA and adds the totals to the outputs of `view`: one atomic per value and
+// (CTA, view) instead of one per fragment.  `red`: one row per warp.
+constexpr int kCamValues = 24;  // 8 (pose, its count, one unused) + 16 (intrinsics, their count, two unused)
+template <bool kIntr>
+__device__ void reduce_cam(const Frame& f, const BackPtrs& bp, CamAcc<kIntr>& acc, int view, double (*red)[kCamValues])
+{
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const ViewDev& vw = f.views[view];
-    for (int base = 0; base < kN; base += 8)
+    __syncthreads();  // the previous view's totals have been read
     {
-        __syncthreads();
-        for (int k = base; k < min(base + 8, kN); ++k)
+        double v[8] = {acc.pose[0], acc.pose[1], acc.pose[2], acc.pose[3], acc.pose[4], acc.pose[5], (double)acc.pose_count, 0.0};
+        warp_sum<8>(v);
+        if ((lane & 3) == 0) red[warp][warp_sum_slot<8>(lane)] = v[0];
+    }
+    if constexpr (kIntr)
+    {
+        double v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = k < 14 ? (double)acc.intr[k < 14 ? k : 0] : 0.0;
+        warp_sum<16>(v);
+        if ((lane & 1) == 0) red[warp][8 + warp_sum_slot<16>(lane)] = v[0];
+    }
+    __syncthreads();
+    const int k = threadIdx.x;
+    if (k < (kIntr ? 22 : 7) && k != 7)
+    {
+        double x = 0.0;
+        for (int w = 0; w < (int)blockDim.x / 32; ++w) x += red[w][k];
+        if (x != 0.0)
         {
-            double x = k < 6 ? acc.pose[k] : (k == 6 ? (double)acc.pose_count : (double)acc.intr[kIntr ? k - 7 : 0]);
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (lane == 0) red[warp][k - base] = x;
-        }
-        __syncthreads();
-        const int k = base + threadIdx.x;
-        if (threadIdx.x < 8 && k < kN)
-        {
-            double x = 0.0;
-            for (int w = 0; w < (int)blockDim.x / 32; ++w) x += red[w][threadIdx.x];
-            if (x != 0.0)
+            if (k < 6)
             {
-                if (k < 6)
-                    atomicAdd(bp.g_pose + 6 * vw.image_index + k, x);
-                else if (k == 6)
-                    atomicAdd(bp.g_pose_count + vw.image_index, (float)x);
-                else if (k < 20)
-                    atomicAdd(bp.g_intr + 13 * vw.camera_index + (k - 7), (float)x);
-                else
-                    atomicAdd(bp.g_intr_count + vw.camera_index, (float)x);
+                if (bp.g_pose) atomicAdd(bp.g_pose + 6 * vw.image_index + k, x);
             }
+            else if (k == 6)
+            {
+                if (bp.g_pose) atomicAdd(bp.g_pose_count + vw.image_index, (float)x);
+            }
+            else if (k < 21)
+                atomicAdd(bp.g_intr + 13 * vw.camera_index + (k - 8), (float)x);
+            else
+                atomicAdd(bp.g_intr_count + vw.camera_index, (float)x);
         }
     }
     acc.clear();
 }
 
-// Spatial gradient of one fragment: image-space gradient dR -> point, pose and intrinsics gradients
-// (RenderBackward.cu:1380-1460 and :3097-3180).
-template <bool kIntr>
-__device__ __forceinline__ void spatial_terms(const Frame& f, const BackPtrs& bp, const Camera& cam, int level,
-                                              const PointJac& jac, float2 dR, CamAcc<kIntr>& acc, BackOut& bo)
+// Image-space gradient of all fragments of a point in one view, brought to level 0.  The chain of Jacobians behind it is
+// linear and differs between the levels only by the factor 0.5^level of the crop matrix (a power of two: exact), so the
+// camera gradients, sums over many points, take it once per point and view instead of once per fragment.
+struct PointGrad
 {
-    float scale = 1.f;
-    for (int l = 0; l < level; ++l) scale *= 0.5f;
-    float crop2[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) crop2[k] = cam.crop[k] * scale;  // IntrinsicsPinhole::scale
-    project_backward_apply(jac, dR, cam, crop2, kIntr, bo);
-    if (bp.g_pose)
+    float x, y;
+    int hits;
+    __device__ __forceinline__ void clear() { x = y = 0.f, hits = 0; }
+    __device__ __forceinline__ void add(float2 g, int level)
     {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) acc.pose[k] += (double)bo.g_pose[k];
-        // RenderBackward.cu:379 (mode 0) and :3144 (mode 3) count 1 per hit, :993 and :1425 (modes 2, 1) count 1/1024
-        acc.pose_count += (f.mode == VETR_MODE_BILINEAR_BLEND || f.mode == VETR_MODE_FUZZY_DT) ? 1.f : (1.f / 1024.f);
+        const float scale = level_scale(level);
+        x += g.x * scale, y += g.y * scale, ++hits;
     }
-    if (kIntr)
-    {
-        bo.g_k[4] *= 0.f;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) acc.intr[k] += f.k_grad_factor * bo.g_k[k];
-        bo.g_dis[2] *= 0.25f;
-#pragma unroll
-        for (int k = 3; k < 8; ++k) bo.g_dis[k] *= 0.1f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc.intr[5 + k] += f.dist_grad_factor * bo.g_dis[k];
-        acc.intr[kIntr ? 13 : 0] += 1.f / 1024.f;
-    }
+    static __device__ __forceinline__ float level_scale(int level) { return __int_as_float((127 - level) << 23); }
+};
+
+// Point gradient of one fragment (RenderBackward.cu:1380-1400): gp.xyz += J^T dR.
+__device__ __forceinline__ void point_terms(const Camera& cam, const PointJac& jac, float2 dR, int level, float4& gp)
+{
+    const float scale = PointGrad::level_scale(level);
+    const float crop2[5] = {cam.crop[0] * scale, cam.crop[1] * scale, 0.f, 0.f, cam.crop[4] * scale};  // IntrinsicsPinhole::scale
+    float g[3];
+    project_backward_point(cam, project_backward_view(jac, dR, cam, crop2), g);
+    gp.x += g[0], gp.y += g[1], gp.z += g[2], gp.w += 1.f;
 }
 
+// Pose and intrinsics gradients of one point in one view (RenderBackward.cu:1400-1460 and :3130-3180).
 template <bool kIntr>
-__device__ __forceinline__ void spatial_backward(const Frame& f, const BackPtrs& bp, const Camera& cam, const PixInfo& px,
-                                                 int pid, float4 pos, float2 dR, CamAcc<kIntr>& acc)
+__device__ __forceinline__ void camera_terms(const Frame& f, const Camera& cam, const PointJac& jac, const PointGrad& g,
+                                             CamAcc<kIntr>& acc)
 {
-    PointJac jac;
-    if (!project_backward_prepare(pos, cam, f.dist_cutoff, kIntr, jac)) return;
-    BackOut bo;
-    spatial_terms<kIntr>(f, bp, cam, px.level, jac, dR, acc, bo);
-    if (bp.g_points) red_add_v4(bp.g_points + pid, make_float4(bo.g_point[0], bo.g_point[1], bo.g_point[2], 1.f));
+    const ViewGrad v = project_backward_view(jac, make_float2(g.x, g.y), cam, cam.crop);
+    float g_pose[6];
+    project_backward_pose(jac, v, g_pose);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc.pose[k] += (double)g_pose[k];
+    // RenderBackward.cu:379 (mode 0) and :3144 (mode 3) count 1 per hit, :993 and :1425 (modes 2, 1) count 1/1024
+    acc.pose_count += (f.mode == VETR_MODE_BILINEAR_BLEND || f.mode == VETR_MODE_FUZZY_DT) ? (float)g.hits : (float)g.hits * (1.f / 1024.f);
+    if (kIntr)
+    {
+        float g_k[5], g_dis[8];
+        project_backward_intrinsics(jac, v, cam, f.dist_cutoff, g_k, g_dis);
+        g_k[4] *= 0.f;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) acc.intr[k] += f.k_grad_factor * g_k[k];
+        g_dis[2] *= 0.25f;
+#pragma unroll
+        for (int k = 3; k < 8; ++k) g_dis[k] *= 0.1f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc.intr[5 + k] += f.dist_grad_factor * g_dis[k];
+        acc.intr[kIntr ? 13 : 0] += (float)g.hits * (1.f / 1024.f);
+    }
 }
 
 // Modes 1 and 2: approximate image-space gradient of a fragment from the neighbouring pixels
@@ -1693,77 +1741,67 @@ __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __g
 // ---------------------------------------------------------------------------------------------------------
 // Position, pose and intrinsics gradients (and the confidence gradient of mode 3), one pass over the points.
 //
-// Modes 1 and 2: every fragment's term is ProjectPointPinholeBackward of the image-space gradient that stage A parked
-// for it.  Mode 3: the fragment's alpha gradient was parked under (view, level, point, corner); here the point is
-// projected once per view exactly as the forward pass did (same bits), which gives the corner weights and their
-// Jacobians (compute_blending_fac) of all its fragments: confidence gradient += w * g_alpha, image-space gradient =
-// J_uv * confidence * g_alpha (RenderBackward.cu:3076-3180).  In every mode a fragment's term is evaluated with the
-// arithmetic of the per-fragment form (each addend has the reference's bits); a point's terms are summed in registers
-// in a fixed order and added to g_points by the one thread that owns the point.  Positions, masks and parked values are
-// read coalesced; camera gradients are summed per thread block and view.
+// Modes 1 and 2: ProjectPointPinholeBackward of the image-space gradients that stage A parked for the point's fragments.
+// Mode 3: the fragments' alpha gradients were parked under (view, level, point, corner); here the point is projected once
+// per view exactly as the forward pass did (same bits), which gives the corner weights and their Jacobians
+// (compute_blending_fac) of all its fragments: confidence gradient += w * g_alpha, image-space gradient =
+// J_uv * confidence * g_alpha (RenderBackward.cu:3076-3180).  Every fragment's position term is formed on its own and has the
+// bits of the per-fragment form; the camera gradients take the image-space gradient of a point and view summed over levels
+// and corners (PointGrad).  Positions, masks and parked values are read coalesced; a point's gradient is added to g_points
+// by the one thread that owns the point.
+//
+// Bound by instruction issue.  A CTA owns `tiles` runs of 256 points and takes them view by view, so that the camera
+// sums - 21 doubles over the CTA - are formed once per (CTA, view); the points' sums stay in shared memory meanwhile.
+// 8 M points x 4 views with pose and intrinsics gradients: 1638 us with one reduction per 512 points and the camera chain per
+// fragment, 600 us like this; mode 3, 3 M points x 2 views: 1587 -> 326 us.
+constexpr int kPointTilesMax = 8;
 
-#ifndef VETR_POINT_BACK_POINTS
-#    define VETR_POINT_BACK_POINTS 2
-#endif
-constexpr int kPointBackPoints = VETR_POINT_BACK_POINTS;
-
-#ifndef VETR_POINT_BACK_CTAS
-#    define VETR_POINT_BACK_CTAS 4
-#endif
 template <bool kIntr, bool kBilinear>
-__global__ void __launch_bounds__(kProjThreads, VETR_POINT_BACK_CTAS) point_backward_kernel(const __grid_constant__ Frame f,
-                                                                      const __grid_constant__ BackPtrs bp)
+__global__ void __launch_bounds__(kProjThreads, kIntr || kBilinear ? 3 : 4)
+    point_backward_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp, int tiles)
 {
+    extern __shared__ __align__(16) float4 s_gp[];  // [tiles][kProjThreads], every thread its own column
     __shared__ Camera s_cam[VETR_MAX_VIEWS];
-    __shared__ double s_red[kProjThreads / 32][8];
+    __shared__ double s_red[kProjThreads / 32][kCamValues];
     if (f.status[1] != 0) return;  // overflow / skipped list: some fragments never parked a value
     if (threadIdx.x < f.n_views) s_cam[threadIdx.x] = load_camera(f, threadIdx.x);
     __syncthreads();
-    const int first     = blockIdx.x * (kProjThreads * kPointBackPoints) + threadIdx.x;
+    const int first     = blockIdx.x * (kProjThreads * tiles) + threadIdx.x;
     const bool want_cam = bp.g_pose != nullptr || kIntr;
     const bool spatial  = f.need_point_grad != 0;
-    float4 pos[kPointBackPoints], gp[kPointBackPoints];
-#pragma unroll
-    for (int it = 0; it < kPointBackPoints; ++it)
-    {
-        const int pid = first + it * kProjThreads;
-        pos[it]       = pid < f.n ? __ldg(f.position + pid) : make_float4(0.f, 0.f, 0.f, 0.f);
-        gp[it]        = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    for (int it = 0; it < tiles; ++it) s_gp[it * kProjThreads + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int b = 0; b < f.n_views; ++b)
     {
         CamAcc<kIntr> acc;
         acc.clear();
-        unsigned mask[kPointBackPoints];
-#pragma unroll
-        for (int it = 0; it < kPointBackPoints; ++it)
-        {
-            const int pid = first + it * kProjThreads;
-            mask[it]      = pid < f.n ? f.level_mask[(size_t)b * f.n + pid] : 0u;
-        }
         bool any = false;
-#pragma unroll
-        for (int it = 0; it < kPointBackPoints; ++it)
+        const unsigned char* masks = f.level_mask + (size_t)b * f.n;
+        unsigned next_mask         = first < f.n ? masks[first] : 0u;  // requested one tile ahead
+        for (int it = 0; it < tiles; ++it)
         {
-            const int pid = first + it * kProjThreads;
-            if (!mask[it]) continue;
+            const int pid       = first + it * kProjThreads;
+            const unsigned mask = next_mask;
+            next_mask           = it + 1 < tiles && pid + kProjThreads < f.n ? masks[pid + kProjThreads] : 0u;
+            if (!mask) continue;
+            const float4 pos = __ldg(f.position + pid);
+            float4 gp        = s_gp[it * kProjThreads + threadIdx.x];
+            PointGrad g;
+            g.clear();
+            PointJac jac;
             if constexpr (!kBilinear)
             {
                 float2 dR[VETR_MAX_LAYERS];
 #pragma unroll
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l)
-                    if (mask[it] >> l & 1u) dR[l] = f.point_grad[((size_t)b * f.L + l) * f.n + pid];
-                PointJac jac;
-                if (!project_backward_prepare(pos[it], s_cam[b], f.dist_cutoff, kIntr, jac)) continue;
+                    if (mask >> l & 1u) dR[l] = f.point_grad[((size_t)b * f.L + l) * f.n + pid];
+                if (!project_backward_prepare(pos, s_cam[b], f.dist_cutoff, jac)) continue;
 #pragma unroll
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l)
-                {
-                    if (!(mask[it] >> l & 1u) || __float_as_int(dR[l].x) == kNoGradientBits) continue;
-                    BackOut bo;
-                    spatial_terms<kIntr>(f, bp, s_cam[b], l, jac, dR[l], acc, bo);
-                    gp[it].x += bo.g_point[0], gp[it].y += bo.g_point[1], gp[it].z += bo.g_point[2], gp[it].w += 1.f;
-                    any = true;
-                }
+                    if ((mask >> l & 1u) && __float_as_int(dR[l].x) != kNoGradientBits)
+                    {
+                        g.add(dR[l], l);
+                        point_terms(s_cam[b], jac, dR[l], l, gp);
+                    }
             }
             else
             {
@@ -1771,18 +1809,17 @@ __global__ void __launch_bounds__(kProjThreads, VETR_POINT_BACK_CTAS) point_back
                 float4 ga[VETR_MAX_LAYERS];  // the four corners' alpha gradients of every level
 #pragma unroll
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l)
-                    if (mask[it] >> l & 1u) ga[l] = *reinterpret_cast<const float4*>(parked + ((((size_t)b * f.L + l) * f.n + pid) << 2));
-                const int tex    = __ldg(f.index + pid);
-                const float conf = __ldg(f.confidence + tex);
-                const Projected pr = project_point(pos[it], s_cam[b], f.dist_cutoff);
-                PointJac jac;
-                const bool jac_ok = spatial && project_backward_prepare(pos[it], s_cam[b], f.dist_cutoff, kIntr, jac);
+                    if (mask >> l & 1u) ga[l] = *reinterpret_cast<const float4*>(parked + ((((size_t)b * f.L + l) * f.n + pid) << 2));
+                const int tex      = __ldg(f.index + pid);
+                const float conf   = __ldg(f.confidence + tex);
+                const Projected pr = project_point(pos, s_cam[b], f.dist_cutoff);
+                const bool jac_ok  = spatial && project_backward_prepare(pos, s_cam[b], f.dist_cutoff, jac);
                 float2 ip   = pr.ip;
                 float gconf = 0.f;
 #pragma unroll
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l, ip.x *= 0.5f, ip.y *= 0.5f)
                 {
-                    if (!(mask[it] >> l & 1u)) continue;
+                    if (!(mask >> l & 1u)) continue;
                     const int bx = round_down(ip.x), by = round_down(ip.y);
                     const float gl[4] = {ga[l].x, ga[l].y, ga[l].z, ga[l].w};
 #pragma unroll
@@ -1797,31 +1834,34 @@ __global__ void __launch_bounds__(kProjThreads, VETR_POINT_BACK_CTAS) point_back
                         gconf += w * gl[c];  // RenderBackward.cu:3076-3079
                         if (!jac_ok) continue;
                         const float single = conf * gl[c];
-                        BackOut bo;
-                        spatial_terms<kIntr>(f, bp, s_cam[b], l, jac, make_float2(jx * single, jy * single), acc, bo);
-                        gp[it].x += bo.g_point[0], gp[it].y += bo.g_point[1], gp[it].z += bo.g_point[2], gp[it].w += 1.f;
-                        any = true;
+                        const float2 dR    = make_float2(jx * single, jy * single);
+                        g.add(dR, l);
+                        point_terms(s_cam[b], jac, dR, l, gp);
                     }
                 }
                 if (gconf != 0.f) red_add(bp.g_conf + tex, gconf);
+            }
+            s_gp[it * kProjThreads + threadIdx.x] = gp;
+            if (want_cam && g.hits)
+            {
+                camera_terms<kIntr>(f, s_cam[b], jac, g, acc);
+                any = true;
             }
         }
         if (want_cam && __syncthreads_or(any)) reduce_cam<kIntr>(f, bp, acc, b, s_red);
     }
     if (bp.g_points)
-    {
-#pragma unroll
-        for (int it = 0; it < kPointBackPoints; ++it)
+        for (int it = 0; it < tiles; ++it)
         {
-            const int pid = first + it * kProjThreads;
-            if (pid < f.n && gp[it].w != 0.f)
+            const int pid   = first + it * kProjThreads;
+            const float4 gp = s_gp[it * kProjThreads + threadIdx.x];
+            if (pid < f.n && gp.w != 0.f)
             {
                 float4 cur = bp.g_points[pid];
-                cur.x += gp[it].x, cur.y += gp[it].y, cur.z += gp[it].z, cur.w += gp[it].w;
+                cur.x += gp.x, cur.y += gp.y, cur.z += gp.z, cur.w += gp.w;
                 bp.g_points[pid] = cur;
             }
         }
-    }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -1993,7 +2033,7 @@ __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_backward_kernel(const _
                                                                          const __grid_constant__ BackPtrs bp)
 {
     __shared__ Camera s_cam;
-    __shared__ double s_red[kProjThreads / 32][8];
+    __shared__ double s_red[kProjThreads / 32][kCamValues];
     const int b = blockIdx.y;
     if (threadIdx.x == 0) s_cam = load_camera(f, b);
     __syncthreads();
@@ -2002,12 +2042,16 @@ __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_backward_kernel(const _
     const int pid     = blockIdx.x * kProjThreads + threadIdx.x;
     CamAcc<kIntr> acc;
     acc.clear();
+    PointGrad grad;
+    grad.clear();
+    float4 gp = make_float4(0.f, 0.f, 0.f, 0.f);
     if (pid < f.n)
     {
         const bool drop_out = f.dropout && f.dropout[(size_t)b * f.n + pid] == 1.f;
         const float4 pos    = __ldg(f.position + pid);
         const Projected pr  = project_point(pos, cam, f.dist_cutoff, false);
-        if (pr.z != 0.f)
+        PointJac jac;
+        if (pr.z != 0.f && project_backward_prepare(pos, cam, f.dist_cutoff, jac))  // (z > 0: never declines)
         {
             const int tex = __ldg(f.index + pid);
             float2 ip     = pr.ip;
@@ -2033,7 +2077,14 @@ __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_backward_kernel(const _
                 }
                 const bool point_grad = (f.ghost && drop_out) | (!f.ghost && !drop_out);
                 if (!(point_grad && px.interior)) continue;
-                spatial_backward<kIntr>(f, bp, cam, px, pid, pos, neighbour_gradient_planar(f, bp, px, load_descriptor(f, tex)), acc);
+                const float2 dR = neighbour_gradient_planar(f, bp, px, load_descriptor(f, tex));
+                grad.add(dR, l);
+                point_terms(cam, jac, dR, l, gp);
+            }
+            if (grad.hits)
+            {
+                camera_terms<kIntr>(f, cam, jac, grad, acc);
+                if (bp.g_points) red_add_v4(bp.g_points + pid, gp);
             }
         }
     }
@@ -3017,21 +3068,24 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
     if ((phases & VETR_BACKWARD_POINTS) && point_pass && f.n > 0)
     {
         PassScope t(ctx, VETR_T_POINT_BACKWARD, 1);
-        const int ctas = (f.n + kProjThreads * kPointBackPoints - 1) / (kProjThreads * kPointBackPoints);
+        // several runs of 256 points per CTA share one camera reduction, as long as that leaves four CTAs per SM
+        const int tiles   = std::max(1, std::min(kPointTilesMax, f.n / (kProjThreads * ctx->sm_count * 4)));
+        const int ctas    = (f.n + kProjThreads * tiles - 1) / (kProjThreads * tiles);
+        const size_t smem = (size_t)tiles * kProjThreads * sizeof(float4);
         cudaStream_t st = ctx->stream;
         if (bilinear)
         {
             if (g_intr)
-                point_backward_kernel<true, true><<<ctas, kProjThreads, 0, st>>>(f, bp);
+                point_backward_kernel<true, true><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
             else
-                point_backward_kernel<false, true><<<ctas, kProjThreads, 0, st>>>(f, bp);
+                point_backward_kernel<false, true><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
         }
         else
         {
             if (g_intr)
-                point_backward_kernel<true, false><<<ctas, kProjThreads, 0, st>>>(f, bp);
+                point_backward_kernel<true, false><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
             else
-                point_backward_kernel<false, false><<<ctas, kProjThreads, 0, st>>>(f, bp);
+                point_backward_kernel<false, false><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
         }
     }
     VETR_CUDA(ctx, cudaGetLastError());

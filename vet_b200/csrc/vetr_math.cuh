@@ -117,6 +117,21 @@ __device__ __forceinline__ float2 distort(float2 p, const float* d, float cutoff
     return out;
 }
 
+// The same Jacobian with respect to the coefficients where all of them are zero (the model is then the identity, num = den =
+// radial = 1): the same bits as distort<true> without its divisions.
+__device__ __forceinline__ void distort_jacobian_at_zero(float2 p, float* J_d)
+{
+    const float x = p.x, y = p.y;
+    const float x2 = VM(x, x), y2 = VM(y, y), xy = VM(x, y);
+    const float r2 = VA(x2, y2), r4 = VM(r2, r2), r6 = VM(r4, r2);
+    J_d[0] = x * r2, J_d[1] = x * r4, J_d[2] = x * r6;
+    J_d[3] = -J_d[0], J_d[4] = -J_d[1], J_d[5] = -J_d[2];
+    J_d[6] = 2.f * xy, J_d[7] = r2 + 2.f * x2;
+    J_d[8] = y * r2, J_d[9] = y * r4, J_d[10] = y * r6;
+    J_d[11] = -J_d[8], J_d[12] = -J_d[9], J_d[13] = -J_d[10];
+    J_d[14] = r2 + 2.f * y2, J_d[15] = 2.f * xy;
+}
+
 // STRICT.  IntrinsicsPinhole::normalizedToImage, coefficient order fx fy cx cy s.
 __device__ __forceinline__ float2 k_apply(const float* K, float2 p)
 {
@@ -198,76 +213,88 @@ __device__ __forceinline__ float blending_fac(float2 uv, int bi, float* Jx, floa
 __device__ __forceinline__ float vetr_blend(float T, float a, float c, float dst) { return __fmaf_rn(VM(T, a), c, dst); }
 __device__ __forceinline__ float vetr_new_T(float T, float a) { return VM(VS(1.f, a), T); }
 
-struct BackOut
-{
-    float g_point[3], g_pose[6], g_k[5], g_dis[8];
-};
-
-// ProjectPointPinholeBackward, PointRendererHelper.h:317-372, in two steps: what depends on the point and the camera
-// only (computed once per point and view), and the chain of transposed Jacobians applied to one image-space gradient.
-// `cropK` is crop_transform.scale(0.5^level).
+// ProjectPointPinholeBackward, PointRendererHelper.h:317-372, in steps: what depends on the point and the camera only
+// (computed once per point and view), the chain of transposed Jacobians from one image-space gradient down to the view-space
+// point (project_backward_view), and what hangs on it.  Products with the structural zeros of the Jacobians are left out;
+// the remaining sums are in the reference's order.  `cropK` is crop_transform.scale(0.5^level).
 struct PointJac
 {
     float3 vp;
     float iz, gzx, gzy;  // 1/z and the z column of the division's Jacobian
-    float2 dp;
-    float Jpd[4], Jdd[16];
+    float Jpd[4];        // Jacobian of the distortion; read only if the camera has one
 };
 
-__device__ __forceinline__ bool project_backward_prepare(const float4 pos, const Camera& cam, float dist_cutoff,
-                                                         bool want_intrinsics, PointJac& j)
+__device__ __forceinline__ bool project_backward_prepare(const float4 pos, const Camera& cam, float dist_cutoff, PointJac& j)
 {
     j.vp = transform_point(cam.V, make_float3(pos.x, pos.y, pos.z));
     if (!(j.vp.z > 0)) return false;
     j.iz = 1.f / j.vp.z;
-    float2 np = make_float2(j.vp.x / j.vp.z, j.vp.y / j.vp.z);
     j.Jpd[0] = 1.f, j.Jpd[1] = 0.f, j.Jpd[2] = 0.f, j.Jpd[3] = 1.f;
-    j.dp = np;
-    if (cam.has_dist || want_intrinsics) j.dp = distort<true>(np, cam.dist, dist_cutoff, j.Jpd, j.Jdd);
+    if (cam.has_dist)
+    {
+        float Jdd[16];
+        distort<true>(make_float2(j.vp.x / j.vp.z, j.vp.y / j.vp.z), cam.dist, dist_cutoff, j.Jpd, Jdd);
+    }
     j.gzx = -j.vp.x * j.iz * j.iz;
     j.gzy = -j.vp.y * j.iz * j.iz;
     return true;
 }
 
-__device__ __forceinline__ void project_backward_apply(const PointJac& j, float2 grad, const Camera& cam, const float cropK[5],
-                                                       bool want_intrinsics, BackOut& o)
+// Gradients of the image-space position after K (g_k1: before K's matrix, g_k2: before the crop's) and of the view-space point.
+struct ViewGrad
 {
-    const float* R = cam.R;
-    const float3 vp = j.vp;
+    float2 g_k1, g_k2;
+    float gv[3];
+};
+
+__device__ __forceinline__ ViewGrad project_backward_view(const PointJac& j, float2 grad, const Camera& cam, const float cropK[5])
+{
+    ViewGrad o;
     // grad_p_rot = rot^T grad ; grad_p_k2 = J_p_K2^T grad_p_rot ; then J_p_K1^T, J_p_dis^T, J_div^T
-    float2 g_rot = make_float2(cam.rot[0] * grad.x + cam.rot[2] * grad.y, cam.rot[1] * grad.x + cam.rot[3] * grad.y);
-    float2 g_k2  = make_float2(cropK[0] * g_rot.x + 0.f * g_rot.y, cropK[4] * g_rot.x + cropK[1] * g_rot.y);
-    float2 g_k1  = make_float2(cam.K[0] * g_k2.x + 0.f * g_k2.y, cam.K[4] * g_k2.x + cam.K[1] * g_k2.y);
-    float2 g_dis = make_float2(j.Jpd[0] * g_k1.x + j.Jpd[2] * g_k1.y, j.Jpd[1] * g_k1.x + j.Jpd[3] * g_k1.y);
-    float gv0 = j.iz * g_dis.x + 0.f * g_dis.y;
-    float gv1 = 0.f * g_dis.x + j.iz * g_dis.y;
-    float gv2 = j.gzx * g_dis.x + j.gzy * g_dis.y;
-    for (int k = 0; k < 3; ++k) o.g_point[k] = R[0 + k] * gv0 + R[3 + k] * gv1 + R[6 + k] * gv2;
-    // J_pose = [ I | -skew(vp) ]
-    o.g_pose[0] = gv0;
-    o.g_pose[1] = gv1;
-    o.g_pose[2] = gv2;
-    o.g_pose[3] = 0.f * gv0 + (-vp.z) * gv1 + vp.y * gv2;
-    o.g_pose[4] = vp.z * gv0 + 0.f * gv1 + (-vp.x) * gv2;
-    o.g_pose[5] = (-vp.y) * gv0 + vp.x * gv1 + 0.f * gv2;
-    if (want_intrinsics)
-    {
-        o.g_k[0] = j.dp.x * g_k2.x;
-        o.g_k[1] = j.dp.y * g_k2.y;
-        o.g_k[2] = g_k2.x;
-        o.g_k[3] = g_k2.y;
-        o.g_k[4] = j.dp.y * g_k2.x;
-        for (int k = 0; k < 8; ++k) o.g_dis[k] = j.Jdd[k] * g_k1.x + j.Jdd[8 + k] * g_k1.y;
-    }
+    const float2 g_rot = make_float2(cam.rot[0] * grad.x + cam.rot[2] * grad.y, cam.rot[1] * grad.x + cam.rot[3] * grad.y);
+    o.g_k2 = make_float2(cropK[0] * g_rot.x, cropK[4] * g_rot.x + cropK[1] * g_rot.y);
+    o.g_k1 = make_float2(cam.K[0] * o.g_k2.x, cam.K[4] * o.g_k2.x + cam.K[1] * o.g_k2.y);
+    float2 g_dis = o.g_k1;
+    if (cam.has_dist)
+        g_dis = make_float2(j.Jpd[0] * o.g_k1.x + j.Jpd[2] * o.g_k1.y, j.Jpd[1] * o.g_k1.x + j.Jpd[3] * o.g_k1.y);
+    o.gv[0] = j.iz * g_dis.x;
+    o.gv[1] = j.iz * g_dis.y;
+    o.gv[2] = j.gzx * g_dis.x + j.gzy * g_dis.y;
+    return o;
 }
 
-__device__ __forceinline__ bool project_backward(const float4 pos, float2 grad, const Camera& cam, const float cropK[5],
-                                                 float dist_cutoff, bool want_intrinsics, BackOut& o)
+__device__ __forceinline__ void project_backward_point(const Camera& cam, const ViewGrad& g, float g_point[3])
 {
-    PointJac j;
-    if (!project_backward_prepare(pos, cam, dist_cutoff, want_intrinsics, j)) return false;
-    project_backward_apply(j, grad, cam, cropK, want_intrinsics, o);
-    return true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) g_point[k] = cam.R[0 + k] * g.gv[0] + cam.R[3 + k] * g.gv[1] + cam.R[6 + k] * g.gv[2];
+}
+
+__device__ __forceinline__ void project_backward_pose(const PointJac& j, const ViewGrad& g, float g_pose[6])
+{
+    // J_pose = [ I | -skew(vp) ]
+    const float3 vp = j.vp;
+    g_pose[0] = g.gv[0], g_pose[1] = g.gv[1], g_pose[2] = g.gv[2];
+    g_pose[3] = (-vp.z) * g.gv[1] + vp.y * g.gv[2];
+    g_pose[4] = vp.z * g.gv[0] + (-vp.x) * g.gv[2];
+    g_pose[5] = (-vp.y) * g.gv[0] + vp.x * g.gv[1];
+}
+
+__device__ __forceinline__ void project_backward_intrinsics(const PointJac& j, const ViewGrad& g, const Camera& cam, float dist_cutoff,
+                                                            float g_k[5], float g_dis[8])
+{
+    float2 p = make_float2(j.vp.x / j.vp.z, j.vp.y / j.vp.z);
+    float Jdd[16], Jpd[4];
+    if (cam.has_dist)
+        p = distort<true>(p, cam.dist, dist_cutoff, Jpd, Jdd);
+    else
+        distort_jacobian_at_zero(p, Jdd);  // (a point beyond the cutoff has no fragments)
+    g_k[0] = p.x * g.g_k2.x;
+    g_k[1] = p.y * g.g_k2.y;
+    g_k[2] = g.g_k2.x;
+    g_k[3] = g.g_k2.y;
+    g_k[4] = p.y * g.g_k2.x;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) g_dis[k] = Jdd[k] * g.g_k1.x + Jdd[8 + k] * g.g_k1.y;
 }
 
 }  // namespace vetr
