@@ -1,0 +1,50 @@
+"""Sizes at which a kernel takes another path than in the other parity tests: ends of tiles, remainders, the cells of the
+error grid that leave the row form.  Against the CPU oracle, with the bounds of the tests of the same function."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests import util
+from vet_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+# ---- error grid: rows of cells, rows and cells that go through the per-pixel test
+
+
+def _grid(cells, box):
+    a = np.arange(cells, dtype=np.float32) * np.float32(2 * box / cells) - np.float32(box)
+    m = np.stack(np.meshgrid(a, a, a, indexing="ij"), -1).reshape(-1, 3)
+    return np.ascontiguousarray(m), np.full_like(m, np.float32(2 * box / cells))
+
+
+@pytest.mark.parametrize("case", ["inside", "aligned", "distorted", "non_finite", "flat_boxes", "one_cell"])
+def test_grid_loss_paths(rasterizer, case):
+    """Coverage is exact whatever path a cell takes; values are sums of non-negative fp32 terms (1e-5)."""
+    import torch
+
+    w, h = 333, 251
+    sc = scenes.config_planar(64, w, h, 200.0, n_views=1, seed=3)
+    bb_min, bb_len = _grid(21, 10.0)  # the camera stands inside the grid: cells of a few pixels and of the whole image
+    rng = np.random.default_rng(1)
+    loss = rng.standard_normal((3, h, w)).astype(np.float32)
+    if case == "aligned":  # edges on pixel rows and columns, faces seen edge-on
+        sc.poses = np.array([[0, 0, 0, 1, 0, 0, 0, 0]], np.float64)
+        bb_min, bb_len = _grid(16, 8.0)
+    elif case == "distorted":
+        sc.intrinsics[0, 5:] = (0.05, -0.02, 0.001, 0.01, 0.0, 0.0, 0.001, -0.002)
+    elif case == "non_finite":
+        loss[0, 100, 60], loss[1, 120, 200] = np.inf, np.nan
+    elif case == "flat_boxes":
+        bb_len = bb_len * rng.choice(np.array([0.0, 1e-4, 1.0], np.float32), size=bb_len.shape)
+    elif case == "one_cell":
+        bb_min, bb_len = np.array([[-1.0, -1.0, -1.0]], np.float32), np.array([[2.0, 2.0, 2.0]], np.float32)
+    n = bb_min.shape[0]
+    ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    assert ref_c.sum() > 0
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+    np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0, equal_nan=True)

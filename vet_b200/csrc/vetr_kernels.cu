@@ -2353,177 +2353,6 @@ __global__ void __launch_bounds__(32 * kExchangeWarps) exchange_finalize_kernel(
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Error-grid rasterisation (FillSceneGridWithLossRasterize, RenderForward.cu:639-791): the step between a training
-// epoch and the point spawning.  One warp per grid cell: eight lanes project the corners of the cell's box, all lanes
-// walk the pixels of its screen rectangle (32-pixel border excluded), test them against the twelve triangles of the
-// box and add up the L1 loss.  The reference issues two global atomics per covered pixel; here a lane sums in
-// registers and the warp adds once per cell.
-
-struct GridArgs
-{
-    const float* bb_min;
-    const float* bb_len;
-    const float* loss;
-    float* value;
-    int* count;
-    int n_cells, channels, h, w, view;
-};
-
-__device__ __forceinline__ float tri_sign(float2 p1, float2 p2, float2 p3)
-{
-    return VS(VM(VS(p1.x, p3.x), VS(p2.y, p3.y)), VM(VS(p2.x, p3.x), VS(p1.y, p3.y)));
-}
-__device__ __forceinline__ bool point_in_triangle(float2 pt, float2 v1, float2 v2, float2 v3)
-{
-    const float d1 = tri_sign(pt, v1, v2), d2 = tri_sign(pt, v2, v3), d3 = tri_sign(pt, v3, v1);
-    const bool has_neg = (d1 < 0) || (d2 < 0) || (d3 < 0);
-    const bool has_pos = (d1 > 0) || (d2 > 0) || (d3 > 0);
-    return !(has_neg && has_pos);
-}
-
-constexpr int kGridWarps = 4;
-constexpr int kGridChunk = 4096;             // pixels of a cell's screen rectangle one warp walks
-constexpr int kGridQueueCap = 4 * 1024 * 1024;  // (cell, chunk) pairs handed to the second kernel
-
-// Screen rectangle of a cell: the eight projected corners (left in pp[]) and the clamped bounding rectangle.
-// Returns the number of pixels to test (0: cell ignored).  Called by a whole warp; s_pp is the warp's staging row.
-__device__ __forceinline__ long long grid_cell_rectangle(const Frame& f, const GridArgs& a, const Camera& cam, int c, int lane,
-                                                         float2* s_pp, float2 pp[8], float2& mn, int& x_size)
-{
-    const float border = 32.f;
-    bool behind = false;
-    if (lane < 8)
-    {
-        // corner order of the reference: (0,0,0) (1,0,0) (0,1,0) (0,0,1) (1,1,0) (1,0,1) (0,1,1) (1,1,1)
-        const float fx = (lane == 1 || lane == 4 || lane == 5 || lane == 7) ? 1.f : 0.f;
-        const float fy = (lane == 2 || lane == 4 || lane == 6 || lane == 7) ? 1.f : 0.f;
-        const float fz = (lane == 3 || lane == 5 || lane == 6 || lane == 7) ? 1.f : 0.f;
-        const float4 pos = make_float4(VA(a.bb_min[3 * c], VM(a.bb_len[3 * c], fx)), VA(a.bb_min[3 * c + 1], VM(a.bb_len[3 * c + 1], fy)),
-                                       VA(a.bb_min[3 * c + 2], VM(a.bb_len[3 * c + 2], fz)), 0.f);
-        const Projected pr = project_point(pos, cam, f.dist_cutoff);
-        behind      = pr.z <= 0.f;  // one corner behind the camera: the whole cell is ignored
-        s_pp[lane]  = pr.ip;
-    }
-    behind = __any_sync(0xffffffffu, behind);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) pp[i] = s_pp[i];
-    __syncwarp();  // the staging row is free for the warp's next cell
-    if (behind) return 0;
-    float2 mx = make_float2(-10000000.f, -10000000.f);
-    mn        = make_float2(10000000.f, 10000000.f);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-    {
-        mx.x = fmaxf(pp[i].x, mx.x), mx.y = fmaxf(pp[i].y, mx.y);
-        mn.x = fminf(pp[i].x, mn.x), mn.y = fminf(pp[i].y, mn.y);
-    }
-    const float W = (float)a.w, H = (float)a.h;
-    if (mx.x < border || mn.x >= VS(W, border) || mx.y < border || mn.y >= VS(H, border)) return 0;
-    mn.x = fmaxf(mn.x, border), mn.y = fmaxf(mn.y, border);
-    mx.x = fminf(mx.x, VS(W, border)), mx.y = fminf(mx.y, VS(H, border));
-    const int y_size = (int)VS(mx.y, mn.y);
-    x_size           = (int)VS(mx.x, mn.x);
-    return (long long)y_size * x_size;
-}
-
-// Pixels [first, last) of a cell's rectangle, one per lane and step; adds the warp's totals to the cell.
-__device__ __forceinline__ void grid_cell_pixels(const GridArgs& a, int c, int lane, const float2 pp[8], float2 mn, int x_size,
-                                                 long long first, long long last)
-{
-    float sum = 0.f;
-    int hits  = 0;
-    for (long long xy = first + lane; xy < last; xy += 32)
-    {
-        const int x_c = (int)VA((float)(int)(xy % x_size), mn.x);
-        const int y_c = (int)VA((float)(int)(xy / x_size), mn.y);
-        const float2 pt = make_float2((float)x_c, (float)y_c);
-        bool in = false;
-        // faces of the box as pairs of triangles (RenderForward.cu:676-677)
-        in |= point_in_triangle(pt, pp[0], pp[1], pp[4]) || point_in_triangle(pt, pp[0], pp[4], pp[2]);
-        in |= point_in_triangle(pt, pp[1], pp[5], pp[7]) || point_in_triangle(pt, pp[1], pp[7], pp[4]);
-        in |= point_in_triangle(pt, pp[5], pp[3], pp[6]) || point_in_triangle(pt, pp[5], pp[6], pp[7]);
-        in |= point_in_triangle(pt, pp[3], pp[0], pp[6]) || point_in_triangle(pt, pp[0], pp[6], pp[2]);
-        in |= point_in_triangle(pt, pp[3], pp[0], pp[5]) || point_in_triangle(pt, pp[0], pp[5], pp[1]);
-        in |= point_in_triangle(pt, pp[2], pp[4], pp[6]) || point_in_triangle(pt, pp[4], pp[6], pp[7]);
-        if (!in) continue;
-        float g = 0.f;
-        for (int i = 0; i < a.channels; ++i) g += fabsf(__ldg(a.loss + ((long long)i * a.h + y_c) * a.w + x_c));
-        sum += g;
-        ++hits;
-    }
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        sum += __shfl_down_sync(0xffffffffu, sum, o);
-        hits += __shfl_down_sync(0xffffffffu, hits, o);
-    }
-    if (lane == 0 && hits > 0)
-    {
-        atomicAdd(a.value + c, sum);
-        atomicAdd(a.count + c, hits);
-    }
-}
-
-// First kernel: one warp per cell.  Rectangles of up to kGridChunk pixels are walked right away; larger ones (a cell next
-// to the camera covers 10^5 pixels, a distant one 10) are cut into chunks that go to a queue, so that the second kernel
-// can spread them over all SMs.  If the queue is full the warp walks the whole rectangle itself.
-__global__ void __launch_bounds__(32 * kGridWarps) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
-                                                                     int2* queue, int* queue_count)
-{
-    __shared__ Camera s_cam;
-    __shared__ float2 s_pp[kGridWarps][8];
-    if (threadIdx.x == 0) s_cam = load_camera(f, a.view);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = blockIdx.x * kGridWarps + warp; c < a.n_cells; c += gridDim.x * kGridWarps)
-    {
-        float2 pp[8], mn;
-        int x_size;
-        const long long total = grid_cell_rectangle(f, a, s_cam, c, lane, s_pp[warp], pp, mn, x_size);
-        if (total <= 0) continue;
-        if (total > kGridChunk)
-        {
-            const int chunks = (int)((total + kGridChunk - 1) / kGridChunk);
-            int base = 0;
-            if (lane == 0) base = atomicAdd(queue_count, chunks);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + chunks <= kGridQueueCap)
-            {
-                for (int k = lane; k < chunks; k += 32) queue[base + k] = make_int2(c, k);
-                continue;
-            }
-            // no room for all chunks: whatever part of the reservation lies inside the queue is marked unused, and the warp
-            // walks the whole rectangle itself
-            for (int k = lane; k < chunks && base + k < kGridQueueCap; k += 32) queue[base + k] = make_int2(-1, 0);
-        }
-        grid_cell_pixels(a, c, lane, pp, mn, x_size, 0, total);
-    }
-}
-
-// Second kernel: one warp per queued (cell, chunk).
-__global__ void __launch_bounds__(32 * kGridWarps) grid_loss_chunk_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
-                                                                           const int2* queue, const int* queue_count)
-{
-    __shared__ Camera s_cam;
-    __shared__ float2 s_pp[kGridWarps][8];
-    if (threadIdx.x == 0) s_cam = load_camera(f, a.view);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // reservations past the capacity were never written: those cells were walked by the first kernel
-    const int n = min(*queue_count, kGridQueueCap);
-    for (int e = blockIdx.x * kGridWarps + warp; e < n; e += gridDim.x * kGridWarps)
-    {
-        const int2 q = queue[e];
-        if (q.x < 0) continue;
-        float2 pp[8], mn;
-        int x_size;
-        const long long total = grid_cell_rectangle(f, a, s_cam, q.x, lane, s_pp[warp], pp, mn, x_size);
-        const long long first = (long long)q.y * kGridChunk;
-        grid_cell_pixels(a, q.x, lane, pp, mn, x_size, first, min(first + kGridChunk, total));
-    }
-}
-
-// ---------------------------------------------------------------------------------------------------------
 // L1 loss of the whole output pyramid against a target pyramid and its gradient, in one launch (what a training step
 // does between the forward and the backward pass; with library element-wise kernels it is seven launches per level).
 
@@ -2592,6 +2421,7 @@ __global__ void __launch_bounds__(256) l1_loss_grad_kernel(const __grid_constant
 }  // namespace vetr
 
 #include "vetr_envmap.cuh"
+#include "vetr_grid.cuh"
 #include "vetr_knn.cuh"
 #include "vetr_points.cuh"
 
@@ -2609,7 +2439,9 @@ struct vetr_ctx
     long long* tile_sums = nullptr;  // scan scratch
     long long tile_cap   = 0;
     int2* grid_queue     = nullptr;  // (cell, chunk) queue of vetr_grid_loss, allocated by its first call
-    int* grid_queue_count = nullptr;
+    int* grid_queue_count = nullptr;  // {queue length, non-finite loss seen}
+    double* grid_prefix  = nullptr;  // running sums of the loss image's rows, grown on demand
+    long long grid_prefix_cap = 0;
     // scratch of vetr_knn_radius, grown on demand: per point (sorted copy, cell, queue) and per cell (starts, ends)
     float4* knn_sorted   = nullptr;
     int* knn_point_cell  = nullptr;
@@ -2799,6 +2631,7 @@ extern "C" void vetr_destroy(vetr_ctx* ctx)
     cudaSetDevice(ctx->device);
     if (ctx->tile_sums) cudaFree(ctx->tile_sums);
     if (ctx->grid_queue) cudaFree(ctx->grid_queue);
+    cudaFree(ctx->grid_prefix);
     cudaFree(ctx->knn_sorted), cudaFree(ctx->knn_point_cell), cudaFree(ctx->knn_queue);
     cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends), cudaFree(ctx->knn_tile_sums), cudaFree(ctx->points_flags);
     for (int i = 0; i < VETR_T_N; ++i)
@@ -3196,9 +3029,20 @@ extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vet
             VETR_CUDA(ctx, cudaMalloc(&ctx->grid_queue, (size_t)kGridQueueCap * sizeof(int2) + 256));
             ctx->grid_queue_count = reinterpret_cast<int*>(ctx->grid_queue + kGridQueueCap);
         }
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, sizeof(int), ctx->stream));
-        ctx->launches += 2;
-        const int ctas = min((n_cells + kGridWarps - 1) / kGridWarps, ctx->sm_count * 16);
+        const long long sums = (long long)view->h * (view->w + 1);
+        if (sums > ctx->grid_prefix_cap)
+        {
+            cudaFree(ctx->grid_prefix);
+            ctx->grid_prefix = nullptr, ctx->grid_prefix_cap = 0;
+            VETR_CUDA(ctx, cudaMalloc(&ctx->grid_prefix, (size_t)sums * sizeof(double)));
+            ctx->grid_prefix_cap = sums;
+        }
+        a.prefix = ctx->grid_prefix, a.non_finite = ctx->grid_queue_count + 1;
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, 2 * sizeof(int), ctx->stream));
+        ctx->launches += 3;
+        grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
+        const int groups = (n_cells + kGridGroup - 1) / kGridGroup;
+        const int ctas   = std::min((groups + kGridWarps - 1) / kGridWarps, ctx->sm_count * 12);
         grid_loss_kernel<<<ctas, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
         grid_loss_chunk_kernel<<<ctx->sm_count * 16, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
     }
