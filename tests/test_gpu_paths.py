@@ -6,6 +6,7 @@ import pytest
 from oracle import oracle as O
 from tests import util
 from vet_b200 import scenes
+from vet_b200.render import default_params
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +49,33 @@ def test_grid_loss_paths(rasterizer, case):
     assert ref_c.sum() > 0
     np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0, equal_nan=True)
+
+
+# ---- lists of more than 256 fragments: their sort (runs of 32, merges, up to 2048 in shared memory), their fold (blocks of
+# 1024), their sweeps (blocks of 768; mode 2: up to 1024, up to 4096)
+
+
+@pytest.mark.parametrize("mode, opacity", [(1, 0.005), (3, 0.005), (3, 0.1), (2, 0.005)])
+def test_long_list_lengths(rasterizer, mode, opacity):
+    lengths = (1, 255, 256, 257, 319, 511, 513, 767, 768, 769, 1023, 1024, 1025, 1537, 2047, 2048, 2049)
+    w, h, f = 64, 48, 50.0
+    n = sum(lengths)
+    sc = scenes.tiny_scene(n=n, w=w, h=h, n_views=1, seed=9)
+    rng = np.random.default_rng(4)
+    sc.poses = np.array([[0, 0, 0, 1, 0, 0, 0, 0]], np.float64)
+    sc.intrinsics[0] = 0
+    sc.intrinsics[0, :4] = f, f, w / 2, h / 2
+    pixel = np.repeat(np.arange(len(lengths)), lengths)  # a list each, in columns of 16 x 2 pixels; mode 3: 2 x 2 lists
+    u, v = 4 + 3 * (pixel % 16) + 0.2, 10 + 20 * (pixel // 16) + 0.3
+    z = rng.integers(512, 1536, n).astype(np.float32) / 256  # with points at equal depth: the point index decides
+    sc.position[:, 0], sc.position[:, 1], sc.position[:, 2] = (u - w / 2) / f * z, (v - h / 2) / f * z, z
+    sc.position[:] = sc.position[rng.permutation(n)]
+    sc.confidence[:] = (opacity * rng.random(sc.confidence.shape)).astype(np.float32)
+    params = default_params(render_mode=mode, drop_out_points_by_radius=0, num_layers=1)
+    ora = util.run_oracle(sc, params)
+    grads = util.random_grads(ora["fwd"]["color"], seed=3)
+    ora = util.run_oracle(sc, params, grads=grads)
+    gpu = util.run_gpu(rasterizer, sc, params, grads=grads)
+    assert gpu["longest"] == max(lengths)
+    util.compare_forward(gpu, ora, exact_images=True)
+    util.compare_backward(gpu["bwd_raw"], ora, sc.channels)
