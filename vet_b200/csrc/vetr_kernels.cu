@@ -3333,8 +3333,18 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     float cell = ext > 0.f ? ext / 32.f : 1.f;
     int d[3];
     long long cells = dims_for(cell, d);
+    bool counted = false;  // knn_starts and knn_point_cell hold the counts and cells of the current cell size
     for (int iter = 0; iter < 24 && ext > 0.f; ++iter)
     {
+        int d2[3];
+        const long long finer = dims_for(cell * 0.5f, d2);
+        // fewer cells than n / 8: more than 8 points in an occupied cell, whatever the counts are
+        if ((double)n / (double)cells > 8.0 && finer <= kKnnMaxCells)
+        {
+            cell *= 0.5f, cells = finer;
+            d[0] = d2[0], d[1] = d2[1], d[2] = d2[2];
+            continue;
+        }
         if (cells > ctx->knn_cap_cells)
         {
             cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends);
@@ -3347,34 +3357,39 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
         VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_starts, 0, (size_t)cells * sizeof(int), st));
         VETR_CUDA(ctx, cudaMemsetAsync(d_occ, 0, sizeof(unsigned long long), st));
-        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, nullptr);
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, ctx->knn_point_cell);
         knn_occupied_kernel<<<(int)std::min<long long>((cells + 255) / 256, ctx->sm_count * 16), 256, 0, st>>>(ctx->knn_starts, cells, d_occ);
         unsigned long long occupied = 0;
         VETR_CUDA(ctx, cudaMemcpyAsync(&occupied, d_occ, sizeof(occupied), cudaMemcpyDeviceToHost, st));
         VETR_CUDA(ctx, cudaStreamSynchronize(st));
         ctx->launches += 2;
+        counted = true;
         if (occupied == 0 || (double)n / (double)occupied <= 8.0) break;
-        int d2[3];
-        const long long finer = dims_for(cell * 0.5f, d2);
         if (finer > kKnnMaxCells) break;
+        counted = false;
         cell *= 0.5f, cells = finer;
         d[0] = d2[0], d[1] = d2[1], d[2] = d2[2];
     }
-    if (cells > ctx->knn_cap_cells)  // only when all points coincide (no iteration ran)
+    if (cells > ctx->knn_cap_cells)  // no iteration counted, as when all points coincide
     {
         cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends);
         ctx->knn_starts = nullptr, ctx->knn_ends = nullptr, ctx->knn_cap_cells = 0;
-        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_starts, (size_t)(1ll << 20) * sizeof(int)));
-        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_ends, (size_t)(1ll << 20) * sizeof(int)));
-        ctx->knn_cap_cells = 1ll << 20;
+        const long long cap = std::max(cells, 1ll << 20);
+        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_starts, (size_t)cap * sizeof(int)));
+        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_ends, (size_t)cap * sizeof(int)));
+        ctx->knn_cap_cells = cap;
     }
     g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
 
     // counting sort into the chosen grid
     const int n_tiles = (int)((cells + kKnnScanTile - 1) / kKnnScanTile);
-    VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_starts, 0, (size_t)cells * sizeof(int), st));
     VETR_CUDA(ctx, cudaMemsetAsync(d_queue_count, 0, sizeof(int), st));
-    knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, ctx->knn_point_cell);
+    if (!counted)
+    {
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_starts, 0, (size_t)cells * sizeof(int), st));
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, ctx->knn_point_cell);
+        ctx->launches += 1;
+    }
     knn_tile_sums_kernel<<<n_tiles, 256, 0, st>>>(ctx->knn_starts, cells, ctx->knn_tile_sums);
     knn_spine_kernel<<<1, 1024, 0, st>>>(ctx->knn_tile_sums, n_tiles);
     knn_apply_kernel<<<n_tiles, 256, 0, st>>>(ctx->knn_starts, cells, ctx->knn_tile_sums, ctx->knn_starts);
@@ -3393,7 +3408,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         a.dummies = 9 - k1, knn_launch_search<9>(ctx, a);
     else
         a.dummies = 17 - k1, knn_launch_search<17>(ctx, a);
-    ctx->launches += 8;
+    ctx->launches += 7;
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }

