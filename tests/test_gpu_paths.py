@@ -79,3 +79,23 @@ def test_long_list_lengths(rasterizer, mode, opacity):
     assert gpu["longest"] == max(lengths)
     util.compare_forward(gpu, ora, exact_images=True)
     util.compare_backward(gpu["bwd_raw"], ora, sc.channels)
+
+
+# ---- environment map: the backward kernel is compiled for up to four and for up to eight spheres
+
+
+@pytest.mark.parametrize("spheres", [2, 5, 8])
+def test_envmap_sphere_counts(rasterizer, spheres):
+    levels = 2
+    sc = util.env_scene(n_views=2, w=96, h=64, f=80.0)
+    rng = np.random.default_rng(spheres)
+    env = util.env_map(rng, S=spheres, R=32)
+    weight = util.env_weights(rng, sc, levels)
+    ref = O.envmap_forward(sc, sc.views, levels, env, weight)
+    gout = [rng.standard_normal(r.shape).astype(np.float32) for r in ref]
+    ref_d, ref_c, mag_d, mag_c = O.envmap_backward(sc, sc.views, levels, env, weight, gout)
+    out, g_density, g_color = util.env_gpu_run(sc, env, levels, weight, 0, gout)
+    tol = util.env_sample_tolerance(env)
+    assert all(np.abs(o - r).max() <= tol for o, r in zip(out, ref))
+    assert np.all(np.abs(g_density - ref_d) <= util.env_grad_tolerance(mag_d, env))
+    assert np.all(np.abs(g_color - ref_c) <= util.env_grad_tolerance(mag_c, env))

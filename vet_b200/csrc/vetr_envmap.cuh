@@ -134,20 +134,16 @@ struct EnvTap  // one sphere's sample: base texel and trilinear weights
 
 __device__ __forceinline__ float env_unnormalize(float c, int size) { return ((c + 1.f) / 2.f) * (float)(size - 1); }
 
-// CreateSampleUVMapAllSpheres for one sphere (EnvironmentMap.cu:620-682) + grid_sample's coordinate arithmetic.
-__device__ __forceinline__ EnvTap env_tap(const EnvArgs& a, const EnvRay& ray, int s)
+// CreateSampleUVMapAllSpheres for one sphere (EnvironmentMap.cu:620-682): texel coordinates of the ray's sample, false if
+// the ray misses the sphere.
+__device__ __forceinline__ bool env_coordinates(const EnvArgs& a, const EnvRay& ray, int s, float& ix, float& iy)
 {
-    EnvTap t;
-    t.hit = true;
-    t.x0 = t.y0 = t.z0 = 0;
-    t.wx[0] = t.wx[1] = t.wy[0] = t.wy[1] = t.wz[0] = t.wz[1] = 0.f;
     float3 sv = ray.d;
     if (s != a.S - 1)
     {
         const float r   = a.radii[s];
         const float det = ray.f + 2.f * ray.q2a * (r * r);
-        t.hit           = det >= 0.f;
-        if (!t.hit) return t;
+        if (!(det >= 0.f)) return false;
         const float res = (-ray.qb + sqrtf(det)) / ray.q2a;
         const float3 p  = make_float3(ray.o.x + res * ray.d.x, ray.o.y + res * ray.d.y, ray.o.z + res * ray.d.z);
         const float len = sqrtf(p.x * p.x + p.y * p.y + p.z * p.z);
@@ -162,8 +158,17 @@ __device__ __forceinline__ EnvTap env_tap(const EnvArgs& a, const EnvRay& ray, i
     const float lat = asinf(la), lon = atan2f(lb, lc);
     const float u = 2.f * (lon / 2.f / pi);
     const float v = 2.f * (lat / pi);
-    const float z = a.S == 1 ? 0.f : (float)s / (float)(a.S - 1) * 2.f - 1.f;
-    const float ix = env_unnormalize(u, a.R), iy = env_unnormalize(v, a.R), iz = env_unnormalize(z, a.S);
+    ix = env_unnormalize(u, a.R), iy = env_unnormalize(v, a.R);
+    return true;
+}
+
+// grid_sample's coordinate arithmetic for sphere s.
+__device__ __forceinline__ EnvTap env_tap_at(const EnvArgs& a, float ix, float iy, int s)
+{
+    EnvTap t;
+    t.hit = true;
+    const float z  = a.S == 1 ? 0.f : (float)s / (float)(a.S - 1) * 2.f - 1.f;
+    const float iz = env_unnormalize(z, a.S);
     const float fx = floorf(ix), fy = floorf(iy), fz = floorf(iz);
     // the base texel, kept inside [-2, size] so that the int conversion and the + 1 of the far corners are defined for
     // every float (anything out there is outside the texture and reads zero either way)
@@ -172,6 +177,17 @@ __device__ __forceinline__ EnvTap env_tap(const EnvArgs& a, const EnvRay& ray, i
     t.wx[1] = ix - fx, t.wx[0] = (fx + 1.f) - ix;
     t.wy[1] = iy - fy, t.wy[0] = (fy + 1.f) - iy;
     t.wz[1] = iz - fz, t.wz[0] = (fz + 1.f) - iz;
+    return t;
+}
+
+__device__ __forceinline__ EnvTap env_tap(const EnvArgs& a, const EnvRay& ray, int s)
+{
+    float ix, iy;
+    if (env_coordinates(a, ray, s, ix, iy)) return env_tap_at(a, ix, iy, s);
+    EnvTap t;
+    t.hit = false;
+    t.x0 = t.y0 = t.z0 = 0;
+    t.wx[0] = t.wx[1] = t.wy[0] = t.wy[1] = t.wz[0] = t.wz[1] = 0.f;
     return t;
 }
 
@@ -304,15 +320,21 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 //   d env / d colour_s = T_s alpha_s G,    d env / d alpha_s = T_s (D_s - rest_s),
 //   rest_s = sum over the spheres behind s of their contribution per unit of transmittance behind s
 //          = alpha_{s+1} D_{s+1} + (1 - alpha_{s+1}) rest_{s+1}
-// (no division by 1 - alpha, which a saturated sigmoid makes zero).  First sweep, front to back: sample, keep alpha,
-// sigmoid, D, T and the colours' signs.  Second sweep, back to front: the gradients of the sphere's samples, scattered
-// to the eight corners of its tap.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920 pixels
-// crosses a few hundred texels), so before the atomics the lanes of a warp that share a base texel, in runs of
-// consecutive lanes, are summed with a segmented shuffle reduction and the run's first lane issues one atomic per
-// corner and value.
+// (no division by 1 - alpha, which a saturated sigmoid makes zero).  First sweep, front to back: sample, keep alpha, D, T,
+// the texel coordinates and the colours' signs.  Second sweep, back to front: the gradients of the sphere's samples,
+// scattered to the eight corners of its tap.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920
+// pixels crosses a few hundred texels), so before the atomics the lanes of a warp that share a base texel, in runs of
+// consecutive lanes, are summed with a segmented shuffle reduction, as many steps as the warp's longest run takes, and the
+// run's first lane issues one atomic per corner and value.
+//
+// kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of
+// up to four spheres does not pay for eight, and has room for the coordinates (asin, atan2, two square roots) of the first
+// sweep.  Four spheres of 1024 x 1024, one 1920x1080 view: 1040 -> 965 us.  What is left does not follow the instruction
+// count any more: 30 M reductions of single floats.
 #ifndef VETR_ENV_BACK_CTAS
-#    define VETR_ENV_BACK_CTAS 3  // 80 registers with a few spills: 5.3 -> 4.1 ms on the benchmark row (2: 118 registers, 4: 64 registers, 4.5 ms)
+#    define VETR_ENV_BACK_CTAS 3
 #endif
+template <int kMaxSpheres>
 __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backward_kernel(const __grid_constant__ EnvArgs a)
 {
     __shared__ EnvCam s_cam[VETR_MAX_VIEWS];
@@ -343,27 +365,24 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 if (ch < a.C) G[ch] = g[ch * per_view];
             ray = env_ray(s_cam[p.b], a.lw[p.l], a.lh[p.l], a.scale[p.l], p.x, p.y);
         }
-        float alpha[kEnvMaxSpheres], sig[kEnvMaxSpheres], dot[kEnvMaxSpheres], Tin[kEnvMaxSpheres];
-        unsigned negative = 0;  // bit 4 s + ch: the raw colour sample is negative; bit 32.. not needed (S <= 8, C <= 4)
+        float alpha[kMaxSpheres], dot[kMaxSpheres], Tin[kMaxSpheres], ix[kMaxSpheres], iy[kMaxSpheres];
+        unsigned hits     = 0;  // bit s: the ray hits sphere s
+        unsigned negative = 0;  // bit 4 s + ch: the raw colour sample is negative (S <= 8, C <= 4)
         unsigned zero     = 0;  // the raw colour sample is exactly zero (abs has no gradient there)
         float T = env_start_T(wgt, a.flags);
 #pragma unroll
-        for (int s = 0; s < kEnvMaxSpheres; ++s)
+        for (int s = 0; s < kMaxSpheres; ++s)
         {
-            alpha[s] = 0.f, sig[s] = 0.f, dot[s] = 0.f, Tin[s] = T;
+            alpha[s] = 0.f, dot[s] = 0.f, Tin[s] = T, ix[s] = 0.f, iy[s] = 0.f;
             if (s < a.S && active)
             {
-                const EnvTap t = env_tap(a, ray, s);
-                if (t.hit)
+                if (env_coordinates(a, ray, s, ix[s], iy[s]))
                 {
+                    hits |= 1u << s;
                     EnvCorners c;
-                    env_corners(a, t, c);
+                    env_corners(a, env_tap_at(a, ix[s], iy[s], s), c);
                     alpha[s] = 1.f;
-                    if (s != a.S - 1)
-                    {
-                        sig[s]   = 1.f / (1.f + expf(-env_fetch(a.density, c)));
-                        alpha[s] = sig[s];
-                    }
+                    if (s != a.S - 1) alpha[s] = 1.f / (1.f + expf(-env_fetch(a.density, c)));
                     float d = 0.f;
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch)
@@ -385,23 +404,21 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
         }
         float rest = 0.f;
 #pragma unroll
-        for (int s = kEnvMaxSpheres - 1; s >= 0; --s)
+        for (int s = kMaxSpheres - 1; s >= 0; --s)
         {
             if (s >= a.S) continue;  // uniform over the grid
             const float g_alpha = Tin[s] * (dot[s] - rest);
             rest                = alpha[s] * dot[s] + (1.f - alpha[s]) * rest;
-            EnvTap t;
-            t.hit = false;
-            if (active) t = env_tap(a, ray, s);
-            const bool live = active && t.hit;
+            const bool live = hits >> s & 1;
             EnvCorners c;
             float gv[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // gradient of the density sample, then of the colour samples
             int key = -1 - lane;                      // never equal between lanes
             if (live)
             {
+                const EnvTap t = env_tap_at(a, ix[s], iy[s], s);
                 env_corners(a, t, c);
                 key   = (t.z0 * a.R + t.y0) * a.R + t.x0;
-                gv[0] = s == a.S - 1 ? 0.f : g_alpha * (sig[s] * (1.f - sig[s]));
+                gv[0] = s == a.S - 1 ? 0.f : g_alpha * (alpha[s] * (1.f - alpha[s]));  // alpha is the sigmoid
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch)
                     if (ch < a.C)
@@ -429,26 +446,35 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 const int other = __shfl_down_sync(0xffffffffu, seg, 1 << k);
                 if (lane + (1 << k) < 32 && other == seg) same |= 1u << k;
             }
+            const unsigned steps = __reduce_or_sync(0xffffffffu, same);  // bits 0 .. k: a run of more than 2^k lanes
 #pragma unroll
             for (int q = 0; q < 8; ++q)
             {
                 // a corner no lane of the warp uses (outside the texture, or the empty z slice of a tap that sits on a slice)
                 if (!__any_sync(0xffffffffu, c.off[q] >= 0 && c.w[q] != 0.f)) continue;
+                float x[5];
 #pragma unroll
-                for (int v = 0; v < 5; ++v)
+                for (int v = 0; v < 5; ++v) x[v] = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
+                // (one atomic per lane without this pre-sum was measured 3 % slower)
+#pragma unroll
+                for (int k = 0; k < 5; ++k)
                 {
-                    if (v > a.C) continue;
-                    if (v == 0 && s == a.S - 1) continue;  // the last sphere's alpha is the constant 1
-                    float x = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
-                    // (one atomic per lane without this pre-sum was measured 3 % slower)
+                    if (!(steps >> k & 1)) break;
 #pragma unroll
-                    for (int k = 0; k < 5; ++k)
+                    for (int v = 0; v < 5; ++v)
                     {
-                        const float y = __shfl_down_sync(0xffffffffu, x, 1 << k);
-                        if (same >> k & 1) x += y;
+                        if (v > a.C) continue;
+                        const float y = __shfl_down_sync(0xffffffffu, x[v], 1 << k);
+                        if (same >> k & 1) x[v] += y;
                     }
-                    if (head && c.off[q] >= 0 && x != 0.f)
-                        atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + c.off[q], x);
+                }
+                if (head && c.off[q] >= 0)
+                {
+#pragma unroll
+                    for (int v = 0; v < 5; ++v)
+                        // (value 0: the last sphere's alpha is a constant)
+                        if (v <= a.C && !(v == 0 && s == a.S - 1) && x[v] != 0.f)
+                            atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + c.off[q], x[v]);
                 }
             }
         }

@@ -3264,7 +3264,11 @@ extern "C" int vetr_envmap_backward(vetr_ctx* ctx, const vetr_cameras* cams, con
         a.g_density = g_density, a.g_color = g_color;
         const long long blocks = (a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads;
         ctx->launches += 1;
-        envmap_backward_kernel<<<(int)std::min<long long>(blocks, (long long)ctx->sm_count * 32), kEnvThreads, 0, ctx->stream>>>(a);
+        const int grid = (int)std::min<long long>(blocks, (long long)ctx->sm_count * 32);
+        if (a.S <= 4)
+            envmap_backward_kernel<4><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
+        else
+            envmap_backward_kernel<kEnvMaxSpheres><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
