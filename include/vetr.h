@@ -232,6 +232,11 @@ int vetr_finalize_gradients(vetr_ctx* ctx, int channels, int n_tex, const float*
                             float* g_points, float* g_points_count, int n_img, double* g_pose,
                             const float* g_pose_count, int n_cam, float* g_intr, const float* g_intr_count);
 
+/* Zero-fills up to VETR_MAX_ZERO device buffers in one launch on the context's stream (gradient buffers before
+ * vetr_backward; addresses and byte counts are multiples of 4). */
+#define VETR_MAX_ZERO 16
+int vetr_zero_buffers(vetr_ctx* ctx, void* const* buffers, const int64_t* bytes, int n);
+
 /* View-sharded training on several GPUs of one node (the reference is single-GPU; this has no counterpart there).
  * Every rank keeps its raw gradient sums of a step in ONE buffer, [descriptor gradient n_tex*4 | position gradient +
  * hit count n*4 | confidence gradient n_tex] floats (vetr_exchange_raw_floats), in memory its peers can address

@@ -99,3 +99,29 @@ def test_envmap_sphere_counts(rasterizer, spheres):
     assert all(np.abs(o - r).max() <= tol for o, r in zip(out, ref))
     assert np.all(np.abs(g_density - ref_d) <= util.env_grad_tolerance(mag_d, env))
     assert np.all(np.abs(g_color - ref_c) <= util.env_grad_tolerance(mag_c, env))
+
+
+# ---- zero fill of several buffers: partial last units, empty buffers, starts off a 16-byte boundary
+
+
+def test_zero_buffers(rasterizer):
+    import ctypes as C
+
+    import torch
+
+    from vet_b200 import _lib as L
+
+    sizes = [0, 1, 3, 4, 5, 4096, 4097, 100_003, 2, 7]
+    for shift in (0, 1):
+        whole = [torch.ones(n + 2, device=rasterizer.device) for n in sizes]
+        part = [t[shift:shift + n] for t, n in zip(whole, sizes)]
+        ptrs = (C.c_void_p * len(sizes))(*[t.data_ptr() for t in part])
+        nbytes = (C.c_int64 * len(sizes))(*[4 * n for n in sizes])
+        rasterizer._sync_stream()
+        assert L.lib().vetr_zero_buffers(rasterizer._ctx, ptrs, nbytes, len(sizes)) == L.OK
+        for t, n in zip(whole, sizes):
+            want = torch.ones_like(t)
+            want[shift:shift + n] = 0
+            assert torch.equal(t, want)
+    assert L.lib().vetr_zero_buffers(rasterizer._ctx, ptrs, (C.c_int64 * 1)(6), 1) == L.E_INVALID_ARG
+    assert L.lib().vetr_zero_buffers(rasterizer._ctx, None, None, 17) == L.E_INVALID_ARG

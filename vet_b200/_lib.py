@@ -79,6 +79,7 @@ EXPORTS = [
     "vetr_launch_count", "vetr_scan_counts_static", "vetr_exchange_raw_floats", "vetr_exchange_out_floats",
     "vetr_exchange_finalize", "vetr_grid_loss", "vetr_l1_loss_grad", "vetr_backward_phase", "vetr_exchange_finalize_part",
     "vetr_envmap_forward", "vetr_envmap_backward", "vetr_knn_radius", "vetr_remove_points_plan", "vetr_gather_points",
+    "vetr_zero_buffers",
 ]
 ENV_ADD, ENV_NOT_AT_POINTS, ENV_DEPTH_TEST_WEIGHT, ENV_NO_DISTORTION_CHECK = 1, 2, 4, 8
 BACKWARD_FRAGMENTS, BACKWARD_POINTS = 1, 2
@@ -126,6 +127,7 @@ def lib():
         L.vetr_finalize_gradients.argtypes = [vp, C.c_int, C.c_int, vp, vp, C.c_int, vp, vp, C.c_int, vp, vp, C.c_int,
                                               vp, vp]
         L.vetr_apply_tangent.argtypes = [vp, vp, vp, C.c_int]
+        L.vetr_zero_buffers.argtypes = [vp, vp, vp, C.c_int]
         L.vetr_read_status.argtypes = [vp, C.POINTER(Lists), C.POINTER(C.c_int64), C.POINTER(C.c_int32)]
         L.vetr_get_lists.argtypes = [vp, C.POINTER(Lists), C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp,
                                      C.POINTER(C.c_int64)]

@@ -2328,38 +2328,88 @@ __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_backward_kernel(const _
 // ---------------------------------------------------------------------------------------------------------
 // Epilogues.
 
-__global__ void transpose_desc_kernel(const float4* __restrict__ g_desc, float* __restrict__ g_texture, int n_tex, int C)
+// Epilogue of the gradients in one launch: descriptor gradient to the planar layout, point gradients divided by the hit
+// count (NormalizeGradient, PointRenderer.cu:1273-1280), rows of camera gradients divided by theirs
+// (NormalizeGradientDevTensor, :1092-1109).  Block ranges in this order; a part without blocks is not wanted.  Four launches
+// of this took 11 us for a scene of 5000 points, most of it start-up.
+struct FinalizeArgs
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_tex) return;
-    float4 v = g_desc[i];
-    g_texture[i] = v.x;
-    g_texture[(long long)n_tex + i] = v.y;
-    g_texture[2LL * n_tex + i] = v.z;
-    if (C > 3) g_texture[3LL * n_tex + i] = v.w;
-}
-
-// NormalizeGradient for points (PointRenderer.cu:1273-1280): divide by the hit count where it is positive.
-__global__ void normalize_points_kernel(float4* g_points, float* g_count, int n)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 v = g_points[i];
-    float c  = v.w;
-    if (g_count) g_count[i] = c;
-    if (c > 0) v.x = v.x / c, v.y = v.y / c, v.z = v.z / c;
-    v.w         = 0.f;
-    g_points[i] = v;
-}
+    const float4* g_desc;
+    float* g_texture;
+    float4* g_points;
+    float* g_points_count;
+    double* g_pose;
+    const float* g_pose_count;
+    float* g_intr;
+    const float* g_intr_count;
+    int C, n_tex, n, n_img, n_cam;
+    unsigned desc_end, points_end, pose_end;  // first block behind each part
+};
 
 template <typename T, int N>
-__global__ void normalize_rows_kernel(T* g, const float* count, int n)  // NormalizeGradientDevTensor, :1092-1109
+__device__ __forceinline__ void normalize_row(T* g, const float* count, int i, int n)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float c = count[i];
+    const float c = count[i];
     if (c > 0)
         for (int k = 0; k < N; ++k) g[(long long)i * N + k] = g[(long long)i * N + k] / c;
+}
+
+__global__ void __launch_bounds__(256) finalize_kernel(const __grid_constant__ FinalizeArgs a)
+{
+    const unsigned b = blockIdx.x;
+    if (b < a.desc_end)
+    {
+        const long long i = (long long)b * 256 + threadIdx.x;
+        if (i >= a.n_tex) return;
+        const float4 v = a.g_desc[i];
+        a.g_texture[i] = v.x;
+        a.g_texture[(long long)a.n_tex + i] = v.y;
+        a.g_texture[2LL * a.n_tex + i] = v.z;
+        if (a.C > 3) a.g_texture[3LL * a.n_tex + i] = v.w;
+    }
+    else if (b < a.points_end)
+    {
+        const long long i = (long long)(b - a.desc_end) * 256 + threadIdx.x;
+        if (i >= a.n) return;
+        float4 v = a.g_points[i];
+        const float c = v.w;
+        if (a.g_points_count) a.g_points_count[i] = c;
+        if (c > 0) v.x = v.x / c, v.y = v.y / c, v.z = v.z / c;
+        v.w           = 0.f;
+        a.g_points[i] = v;
+    }
+    else if (b < a.pose_end)
+        normalize_row<double, 6>(a.g_pose, a.g_pose_count, (int)((b - a.points_end) * 256 + threadIdx.x), a.n_img);
+    else
+        normalize_row<float, 13>(a.g_intr, a.g_intr_count, (int)((b - a.pose_end) * 256 + threadIdx.x), a.n_cam);
+}
+
+// Fills up to VETR_MAX_ZERO buffers with zeros in one launch: 16 bytes per thread and step where a buffer starts on such a
+// boundary.
+struct ZeroArgs
+{
+    unsigned* ptr[VETR_MAX_ZERO];
+    long long end[VETR_MAX_ZERO];  // running total of 16-byte units (the last one of a buffer may be partial)
+    int words[VETR_MAX_ZERO];      // 4-byte words in the last unit (1 to 4)
+    int n;
+};
+
+__global__ void __launch_bounds__(256) zero_buffers_kernel(const __grid_constant__ ZeroArgs a)
+{
+    const long long total = a.end[a.n - 1];
+    for (long long u = (long long)blockIdx.x * 256 + threadIdx.x; u < total; u += (long long)gridDim.x * 256)
+    {
+        int k = 0;
+        while (u >= a.end[k]) ++k;
+        const long long at = u - (k ? a.end[k - 1] : 0);
+        unsigned* to       = a.ptr[k] + 4 * at;
+        const int words    = u == a.end[k] - 1 ? a.words[k] : 4;
+        if (words == 4 && ((uintptr_t)to & 15) == 0)
+            *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+        else
+            for (int i = 0; i < words; ++i) to[i] = 0u;
+    }
 }
 
 // ApplyTangent (PointRenderer.cu:1325-1341): pose <- exp_se3(t) * pose in double; tangent = (translation, rotation).
@@ -2962,6 +3012,36 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
     return VETR_OK;
 }
 
+// Launches zero_buffers_kernel on the context's stream; `bytes` are multiples of 4, as are the addresses.
+static int zero_buffers(vetr_ctx* ctx, void* const* buffers, const int64_t* bytes, int n)
+{
+    ZeroArgs a;
+    a.n = 0;
+    long long total = 0;
+    for (int i = 0; i < n; ++i)
+    {
+        if (bytes[i] == 0) continue;
+        const long long words = bytes[i] / 4, units = (words + 3) / 4;
+        total += units;
+        a.ptr[a.n] = (unsigned*)buffers[i], a.end[a.n] = total, a.words[a.n] = (int)(words - 4 * (units - 1));
+        ++a.n;
+    }
+    if (a.n == 0) return VETR_OK;
+    ctx->launches += 1;
+    zero_buffers_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, ctx->sm_count * 32ll), 256, 0, ctx->stream>>>(a);
+    VETR_CUDA(ctx, cudaGetLastError());
+    return VETR_OK;
+}
+
+extern "C" int vetr_zero_buffers(vetr_ctx* ctx, void* const* buffers, const int64_t* bytes, int n)
+{
+    if (!ctx || n < 0 || n > VETR_MAX_ZERO || (n > 0 && (!buffers || !bytes))) return VETR_E_INVALID_ARG;
+    for (int i = 0; i < n; ++i)
+        if (bytes[i] < 0 || bytes[i] % 4 != 0 || (bytes[i] > 0 && (!buffers[i] || ((uintptr_t)buffers[i] & 3) != 0))) return VETR_E_INVALID_ARG;
+    VETR_CUDA(ctx, cudaSetDevice(ctx->device));
+    return zero_buffers(ctx, buffers, bytes, n);
+}
+
 extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr_cloud* cloud, const vetr_texture* texture,
                             const vetr_cameras* cameras, const vetr_view* views, int n_views, const float* dropout,
                             const vetr_lists* lists, float* const* out_color, float* const* out_weight,
@@ -3007,8 +3087,12 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         VETR_CUDA(ctx, cudaGetLastError());
         return VETR_OK;
     }
-    VETR_CUDA(ctx, cudaMemsetAsync(f.counts, 0, f.PT * sizeof(int), st));
-    VETR_CUDA(ctx, cudaMemsetAsync(f.status, 0, 4 * sizeof(int), st));
+    {
+        void* const buffers[2] = {f.counts, f.status};
+        const int64_t bytes[2] = {(int64_t)(f.PT * sizeof(int)), 4 * sizeof(int)};
+        rc = zero_buffers(ctx, buffers, bytes, 2);
+        if (rc != VETR_OK) return rc;
+    }
     const int point_ctas = (f.n + kProjThreads * kPointsPerThread - 1) / (kProjThreads * kPointsPerThread);
     if (point_ctas > 0)
     {
@@ -3161,19 +3245,18 @@ extern "C" int vetr_finalize_gradients(vetr_ctx* ctx, int channels, int n_tex, c
     if (!ctx) return VETR_E_INVALID_ARG;
     VETR_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
-    const int n_kernels = (g_desc && g_texture && n_tex > 0) + (g_points && n > 0) + (g_pose && g_pose_count && n_img > 0) +
-                          (g_intr && g_intr_count && n_cam > 0);
-    PassScope t(ctx, VETR_T_FINALIZE, n_kernels);
-    if (g_desc && g_texture && n_tex > 0)
-    {
-        if (channels != 3 && channels != 4) return VETR_E_INVALID_ARG;
-        transpose_desc_kernel<<<(n_tex + 255) / 256, 256, 0, st>>>((const float4*)g_desc, g_texture, n_tex, channels);
-    }
-    if (g_points && n > 0) normalize_points_kernel<<<(n + 255) / 256, 256, 0, st>>>((float4*)g_points, g_points_count, n);
-    if (g_pose && g_pose_count && n_img > 0)
-        normalize_rows_kernel<double, 6><<<(n_img + 127) / 128, 128, 0, st>>>(g_pose, g_pose_count, n_img);
-    if (g_intr && g_intr_count && n_cam > 0)
-        normalize_rows_kernel<float, 13><<<(n_cam + 127) / 128, 128, 0, st>>>(g_intr, g_intr_count, n_cam);
+    if (g_desc && g_texture && n_tex > 0 && channels != 3 && channels != 4) return VETR_E_INVALID_ARG;
+    const auto blocks = [](bool wanted, int rows) { return wanted && rows > 0 ? (unsigned)((rows + 255ll) / 256) : 0u; };
+    FinalizeArgs a;
+    a.g_desc = (const float4*)g_desc, a.g_texture = g_texture, a.g_points = (float4*)g_points, a.g_points_count = g_points_count;
+    a.g_pose = g_pose, a.g_pose_count = g_pose_count, a.g_intr = g_intr, a.g_intr_count = g_intr_count;
+    a.C = channels, a.n_tex = n_tex, a.n = n, a.n_img = n_img, a.n_cam = n_cam;
+    a.desc_end   = blocks(g_desc && g_texture, n_tex);
+    a.points_end = a.desc_end + blocks(g_points != nullptr, n);
+    a.pose_end   = a.points_end + blocks(g_pose && g_pose_count, n_img);
+    const unsigned grid = a.pose_end + blocks(g_intr && g_intr_count, n_cam);
+    PassScope t(ctx, VETR_T_FINALIZE, grid > 0);
+    if (grid > 0) finalize_kernel<<<grid, 256, 0, st>>>(a);
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }

@@ -230,16 +230,20 @@ class Rasterizer:
         f32 = dict(dtype=torch.float32, device=self.device)
         g = accum
         if g is None:
-            g = dict(desc=torch.zeros(n_tex, 4, **f32), conf=torch.zeros(n_tex, **f32),
-                     background=torch.zeros(Cn, **f32))
+            # one launch zeroes them all: a fill of its own each costs more than the buffers of a small scene
+            g = dict(desc=torch.empty(n_tex, 4, **f32), conf=torch.empty(n_tex, **f32),
+                     background=torch.empty(Cn, **f32))
             if want_points:
-                g["points"] = torch.zeros(n, 4, **f32)
+                g["points"] = torch.empty(n, 4, **f32)
             if want_pose:
-                g["pose"] = torch.zeros(poses.shape[0], 6, dtype=torch.float64, device=self.device)
-                g["pose_count"] = torch.zeros(poses.shape[0], **f32)
+                g["pose"] = torch.empty(poses.shape[0], 6, dtype=torch.float64, device=self.device)
+                g["pose_count"] = torch.empty(poses.shape[0], **f32)
             if want_intrinsics:
-                g["intrinsics"] = torch.zeros(intrinsics.shape[0], 13, **f32)
-                g["intrinsics_count"] = torch.zeros(intrinsics.shape[0], **f32)
+                g["intrinsics"] = torch.empty(intrinsics.shape[0], 13, **f32)
+                g["intrinsics_count"] = torch.empty(intrinsics.shape[0], **f32)
+            bufs = list(g.values())
+            sizes = (C.c_int64 * len(bufs))(*[t.nbytes for t in bufs])
+            self._check(lib.vetr_zero_buffers(self._ctx, _ptr_array(bufs), sizes, len(bufs)), "vetr_zero_buffers")
         grad_color = [x.contiguous() for x in grad_color]
         for (b0, b1, lists, varr) in s["groups"]:
             oc = [t[b0:b1] for t in s["color"]]
