@@ -329,8 +329,7 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 //
 // kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of
 // up to four spheres does not pay for eight, and has room for the coordinates (asin, atan2, two square roots) of the first
-// sweep.  Four spheres of 1024 x 1024, one 1920x1080 view: 1040 -> 965 us.  What is left does not follow the instruction
-// count any more: 30 M reductions of single floats.
+// sweep.  Four spheres of 1024 x 1024, one 1920x1080 view: 1040 -> 965 us.
 #ifndef VETR_ENV_BACK_CTAS
 #    define VETR_ENV_BACK_CTAS 3
 #endif
