@@ -138,9 +138,10 @@ typedef struct vetr_lists
                               need_point_gradient is set; level_mask must be the one the forward call wrote.  Neither
                               needs initialising.  Mode 3 keeps a fragment's corner in the two top bits of the record's
                               descriptor index, so n_tex must stay below 2^30 there. */
-    float*    pixel_scratch; /* [n_views*P*8] 16-byte aligned scratch of vetr_backward in modes 1-3: channel-interleaved
-                                copies of out_color and grad_color over the pixel space (eight 16-byte loads fetch all
-                                neighbour values of a fragment).  Needs no initialising. */
+    float*    pixel_scratch; /* [n_views*P*8] 16-byte aligned scratch of vetr_backward, required in modes 1-3, used in mode 0
+                                where it is given (else slower loads): channel-interleaved copies of out_color and
+                                grad_color over the pixel space (eight 16-byte loads fetch all neighbour values of a
+                                fragment).  Needs no initialising. */
 } vetr_lists;
 
 typedef struct vetr_ctx vetr_ctx;

@@ -125,3 +125,27 @@ def test_zero_buffers(rasterizer):
             assert torch.equal(t, want)
     assert L.lib().vetr_zero_buffers(rasterizer._ctx, ptrs, (C.c_int64 * 1)(6), 1) == L.E_INVALID_ARG
     assert L.lib().vetr_zero_buffers(rasterizer._ctx, None, None, 17) == L.E_INVALID_ARG
+
+
+# ---- mode 0: backward with the interleaved image copies, and without pixel scratch
+
+
+@pytest.mark.parametrize("channels, ghost", [(4, 0), (3, 0), (4, 1)])
+def test_mode0_backward_scratch(monkeypatch, channels, ghost):
+    from vet_b200 import render
+
+    sc = scenes.tiny_scene(n=9000, w=93, h=61, n_views=2, seed=13, channels=channels, crop=True)  # 7475 pixels a view
+    dropout = (np.random.default_rng(2).random((2, sc.n)) < 0.2).astype(np.float32)
+    params = default_params(render_mode=0, num_channels=channels, ghost_gradients=ghost)
+    ora = util.run_oracle(sc, params, dropout=dropout)
+    grads = util.random_grads(ora["fwd"]["color"], seed=3)
+    ora = util.run_oracle(sc, params, grads=grads, dropout=dropout)
+    for scratch in (True, False):
+        if not scratch:
+            monkeypatch.setattr(render.FragmentLists, "ensure_pixel_scratch", lambda self: None)
+        rast = render.Rasterizer(0)
+        gpu = util.run_gpu(rast, sc, params, grads=grads, dropout=dropout)
+        # the forward image differs from the oracle's in the last bits (descriptors are summed in no fixed order), and an
+        # addend (T - I) * G inherits that relative to |I * G|: the bound of the mode-0 parity tests
+        util.compare_backward(gpu["bwd_raw"], ora, channels, rtol=2e-5, floor_rel=1e-6)
+        rast.close()
