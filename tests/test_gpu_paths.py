@@ -51,6 +51,33 @@ def test_grid_loss_paths(rasterizer, case):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0, equal_nan=True)
 
 
+@pytest.mark.parametrize("offset", [2e5, 1e6])
+def test_grid_loss_far_from_the_origin(rasterizer, offset):
+    """A scene far from the origin: the corners of a box are rounded to the grid of the world coordinates (1/64 of a unit at 2e5,
+    where a cell is 0.4 units wide), so its faces bend and their diagonals stick out of the edges' outline; at 1e6 the projected box
+    is no longer in one piece row by row.  Coverage stays exact."""
+    import torch
+
+    w, h, cells = 640, 360, 48
+    sc = scenes.config_planar(64, w, h, 800.0, n_views=2, seed=5)
+    bb_min, bb_len = _grid(cells, 10.0)
+    shift = np.array([1.0, 0.7, -0.4]) * offset
+    bb_min = (bb_min + shift).astype(np.float32)
+    for pose in sc.poses:  # x -> R x + t seen from the shifted scene: t - R shift
+        q, v = pose[:3], shift
+        uv = 2 * np.cross(q, v)
+        pose[4:7] -= v + pose[3] * uv + np.cross(q, uv)
+    loss = np.random.default_rng(1).random((1, h, w)).astype(np.float32)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    for view in sc.views:
+        ref_v, ref_c = O.grid_loss(sc, view, bb_min, bb_len, loss)
+        value, count = torch.zeros(len(bb_min), device=rasterizer.device), torch.zeros(len(bb_min), dtype=torch.int32, device=rasterizer.device)
+        rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), view, t(bb_min), t(bb_len), t(loss), value, count)
+        assert (ref_c > 0).sum() > 1000
+        np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+        np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
 # ---- lists of more than 256 fragments: their sort (runs of 32, merges, up to 2048 in shared memory), their fold (blocks of
 # 1024), their sweeps (blocks of 768; mode 2: up to 1024, up to 4096)
 

@@ -5,15 +5,20 @@
 // The reference tests every pixel of a cell's screen rectangle against the twelve triangles of the box (two per face) and
 // issues two global atomics per covered pixel.  Those tests are what bounds a per-pixel form (twelve triangles of three
 // edge functions in strict fp32 for each of some 600 M pixels at 128^3 cells and 1920 x 1080: 7.3 ms).  Here a lane owns one
-// pixel ROW of a cell: the twelve triangles are the two layers of the box's convex outline, so what they cover of a row is
-// the run of pixels between its leftmost and rightmost crossing with the box's edges, and the run's loss is a difference
+// pixel ROW of a cell: the twelve triangles are a closed surface, so what they cover of a row is the run of pixels between its
+// leftmost and rightmost crossing with the 18 segments (12 edges, 6 face diagonals), and the run's loss is a difference
 // of two running sums of that image row (fp64, formed once per call).  0.95 ms at the same sizes.
 //
+// Why one run: a row cuts the surface in a connected set if the part of the surface above it and the part below are both
+// connected (the surface is a sphere), and they are for every row if only one corner has no higher neighbour along the 18
+// segments and only one has no lower neighbour.  grid_prepare counts them.  Nothing else is asked of the corners: faces may be
+// bent, as they are far from the origin, where the corners are rounded to the grid of the world coordinates.
+//
 // The numbers stay those of the per-pixel tests, rounding included: a row in which any pixel comes so close to one of the
-// 18 segments (12 edges, 6 face diagonals) that the strict fp32 edge functions could disagree with the outline goes
-// through the per-pixel test (grid_exact_row), and cells for which the outline argument does not hold - a face seen
-// nearly edge-on, corners far outside the image, a lens distortion (straight edges do not stay straight), rectangles
-// whose fp32 pixel coordinates may skip a number, a loss image with Inf or NaN - are walked pixel by pixel as a whole.
+// 18 segments that the strict fp32 edge functions could disagree with it goes through the per-pixel test
+// (grid_exact_row), and cells for which the argument does not hold - several highest or lowest corners, a face seen
+// nearly edge-on, corners far outside the image, a lens distortion, rectangles whose fp32 pixel coordinates may skip a
+// number, a loss image with Inf or NaN - are walked pixel by pixel as a whole.
 #pragma once
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -70,6 +75,7 @@ constexpr int kGridChunk    = 512;              // pixels of a rectangle one war
 constexpr int kGridRowChunk = 32;               // rows of a queued chunk; cells of up to that many rows are not queued
 constexpr int kGridQueueCap = 4 * 1024 * 1024;  // (cell, chunk) pairs handed to the second kernel
 constexpr int kGridSegments = 18;               // 12 edges, then 6 face diagonals
+constexpr unsigned long long kGridNeighbours = 0x72bdcbc76151b17eull;  // byte c: the corners that share a segment with corner c
 constexpr int kGridCtas     = 6;                // resident CTAs per SM the kernels are compiled for (5: the same, 8: 10 % slower)
 
 // Running sums of |loss| along every image row, one CTA per row, four pixels per thread and step.  fp64: a run's sum is
@@ -185,7 +191,7 @@ __device__ __noinline__ void grid_cell_pixels(const GridArgs& a, int c, int lane
     }
 }
 
-// Base run of a row: the pixels between the leftmost and rightmost crossing of the outline.
+// Base run of a row: the pixels between its leftmost and rightmost crossing.
 __device__ __forceinline__ void grid_run(const GridArgs& a, const int4 rect, int j, float L, float R, double& sum, int& hits)
 {
     const int xl = (int)fmaxf(ceilf(L), 0.f), xr = (int)fminf(floorf(R), (float)(rect.z - 1));
@@ -195,7 +201,7 @@ __device__ __forceinline__ void grid_run(const GridArgs& a, const int4 rect, int
     hits += xr - xl + 1;
 }
 
-// One row of one cell in which pixels lie in the band of a segment (a whole warp): the outline's run of pixels, corrected
+// One row of one cell in which pixels lie in the band of a segment (a whole warp): the run of pixels, corrected
 // where the per-pixel test disagrees.  Lane k owns segment k.  The pixels of a short band are taken one by one, a triangle per
 // lane; those of a long one (a nearly horizontal segment) 32 at a time, a pixel per lane.
 __device__ __noinline__ void grid_exact_row(const GridArgs& a, const GridWarpSmem& s, int slot, int j, double& sum, int& hits)
@@ -211,7 +217,7 @@ __device__ __noinline__ void grid_exact_row(const GridArgs& a, const GridWarpSme
         const float yc = fminf(fmaxf(y, q.y), q.z);
         const float xs = fmaf(yc - q.y, q.w, q.x), h = s.half[lane][slot];
         if (fabsf(y - yc) <= s.rho[slot]) x0 = (int)fmaxf(ceilf(xs - h), 0.f), x1 = (int)fminf(floorf(xs + h), (float)(rect.z - 1));
-        if (lane < 12 && y == yc) L = R = xs;
+        if (y == yc) L = R = xs;
     }
     for (int o = 16; o > 0; o >>= 1)
     {
@@ -274,14 +280,15 @@ struct GridCell
 //
 // Bands.  With all differences of coordinates below E (the box's extent on the screen, plus one pixel) the strict fp32 edge
 // function of an edge of length l is off by less than 8.4 E l 2^-24, i.e. its sign is certain farther than 5e-7 E pixels from
-// the edge's line, and a crossing computed here is off by less than 4e-7 E (1 + |dx/dy|) along the row.  A pixel inside the
-// outline and farther than 5e-7 E from all segments lies inside some triangle of the front layer with all three signs certain.
-// A pixel outside the outline fails every triangle for certain if it is farther than 5e-7 E / sin(half the smallest angle)
-// <= 1e-6 E kappa from it, kappa = the largest (product of the two longer sides) / (2 area) of the twelve triangles.  So the
-// band of a diagonal is rho = 1e-6 E wide, that of an edge (kappa + 0.5) rho, and along a row of slope dx/dy = k a band of
-// height rho reaches rho (1 + |k|) to either side.
-// Cells whose band would be wider than a quarter pixel, or with a triangle so thin that the rounding of its corners (a few
-// units in the last place of a pixel coordinate) could bend the outline, take the per-pixel form.
+// the edge's line, and a crossing computed here is off by less than 4e-7 E (1 + |dx/dy|) along the row.  A pixel of the run
+// that is farther than 5e-7 E from all segments lies inside some triangle with all three signs certain.  A pixel outside
+// the run lies in no triangle.  It fails one whose side is nearest for certain if it is farther than 5e-7 E from that side,
+// and one whose corner is nearest if it is farther than 5e-7 E / sin(half the smallest angle) <= 1e-6 E kappa from that
+// corner, kappa = the largest (product of the two longer sides) / (2 area) of the twelve triangles.  So the
+// band of a diagonal is rho = 1e-6 E wide, that of an edge (kappa + 0.5) rho, which also covers all corners, and along a row
+// of slope dx/dy = k a band of height rho reaches rho (1 + |k|) to either side.
+// All this takes the projected corners as they are, whatever rounding went into them.  Cells whose band would be wider than a
+// quarter pixel, or with a triangle as thin as a few units in the last place of a pixel coordinate, take the per-pixel form.
 __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs& a, const Camera& cam, GridWarpSmem& s, int c, bool no_rows)
 {
     const int lane = threadIdx.x & 31, slot = lane >> 3, corner = lane & 7;
@@ -327,11 +334,22 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
         kappa = fmaxf(kappa, __shfl_xor_sync(0xffffffffu, kappa, o));
         thin  = fminf(thin, __shfl_xor_sync(0xffffffffu, thin, o));
     }
+    // corners without a higher (lower) neighbour; equal rows are told apart by the corner's number
+    unsigned higher = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+    {
+        const float y = s.pp[slot][k].y;
+        if (y > ip.y || (y == ip.y && k > corner)) higher |= 1u << k;
+    }
+    const unsigned near = (unsigned)(kGridNeighbours >> (8 * corner)) & 0xffu;
+    const unsigned tops = __ballot_sync(0xffffffffu, (higher & near) == 0), bottoms = __ballot_sync(0xffffffffu, (~higher & near) == 0);
+    const bool one_run  = __popc(tops >> (8 * slot) & 0xffu) == 1 && __popc(bottoms >> (8 * slot) & 0xffu) == 1;
     const float size = (float)max(a.w, a.h);
     const float rho = 1e-6f * E, rho_edge = rho * (kappa + 0.5f);
     const float skip = 1.f - size * 2.4e-7f;  // fp32 column / row numbers count up without a gap below this fraction
     // (written so that a NaN anywhere selects the per-pixel form)
-    cell.by_rows = cell.total > 0 && cell.x_size > 0 && cell.y_size > 0 && E < 2e4f && rho_edge < 0.25f &&
+    cell.by_rows = cell.total > 0 && cell.x_size > 0 && cell.y_size > 0 && one_run && E < 2e4f && rho_edge < 0.25f &&
                    thin > 4e-3f * (1.f + (size + E) * (1.f / 2048.f)) && mn.x - floorf(mn.x) < skip && mn.y - floorf(mn.y) < skip;
     if (cell.by_rows)
     {
@@ -378,21 +396,13 @@ __device__ __forceinline__ void grid_rows(const GridArgs& a, const GridWarpSmem&
             const float rho = s.rho[slot];
             float L = CUDART_INF_F, R = -CUDART_INF_F;
 #pragma unroll 6
-            for (int q = 0; q < 12; ++q)
+            for (int q = 0; q < kGridSegments; ++q)
             {
                 const float4 g = s.seg[q][slot];
                 const float yc = fminf(fmaxf(y, g.y), g.z), dy = fabsf(y - yc);
                 const float xs = fmaf(yc - g.y, g.w, g.x);
                 close |= dy <= rho && fabsf(xs - rintf(xs)) <= s.half[q][slot];
                 if (dy == 0.f) L = fminf(L, xs), R = fmaxf(R, xs);
-            }
-#pragma unroll
-            for (int q = 12; q < kGridSegments; ++q)
-            {
-                const float4 g = s.seg[q][slot];
-                const float yc = fminf(fmaxf(y, g.y), g.z), dy = fabsf(y - yc);
-                const float xs = fmaf(yc - g.y, g.w, g.x);
-                close |= dy <= rho && fabsf(xs - rintf(xs)) <= s.half[q][slot];
             }
             if (!close) grid_run(a, s.rect[slot], j, L, R, sum, hits);
         }
