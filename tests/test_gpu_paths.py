@@ -78,6 +78,28 @@ def test_grid_loss_far_from_the_origin(rasterizer, offset):
         np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+def test_grid_loss_wide_range(rasterizer):
+    """Rows with one pixel of 1e12 among losses of 1e-3, and a block of zeros: what a cell covers beside that pixel keeps its
+    relative accuracy (sums of non-negative fp32 terms, 1e-5), and a cell over zeros only stays exactly zero."""
+    import torch
+
+    w, h = 640, 360
+    sc = scenes.config_planar(64, w, h, 800.0, n_views=1, seed=5)
+    bb_min, bb_len = _grid(40, 10.0)
+    rng = np.random.default_rng(2)
+    loss = (1e-3 * rng.standard_normal((2, h, w))).astype(np.float32)
+    loss[:, 100:200, 300:420] = 0
+    loss[0, ::3, 40] = 1e12
+    loss[1, 1::3, 290] = 1e12
+    ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    assert ((ref_c > 0) & (ref_v == 0)).sum() > 50 and (ref_v > 1e11).sum() > 50
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(len(bb_min), device=rasterizer.device), torch.zeros(len(bb_min), dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+    np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
 # ---- lists of more than 256 fragments: their sort (runs of 32, merges, up to 2048 in shared memory), their fold (blocks of
 # 1024), their sweeps (blocks of 768; mode 2: up to 1024, up to 4096)
 

@@ -7,7 +7,7 @@
 // edge functions in strict fp32 for each of some 600 M pixels at 128^3 cells and 1920 x 1080: 7.3 ms).  Here a lane owns one
 // pixel ROW of a cell: the twelve triangles are a closed surface, so what they cover of a row is the run of pixels between its
 // leftmost and rightmost crossing with the 18 segments (12 edges, 6 face diagonals), and the run's loss is a difference
-// of two running sums of that image row (fp64, formed once per call).  0.95 ms at the same sizes.
+// of two running sums of that image row (fp64, formed once per call).  0.92 ms at the same sizes.
 //
 // Why one run: a row cuts the surface in a connected set if the part of the surface above it and the part below are both
 // connected (the surface is a sphere), and they are for every row if only one corner has no higher neighbour along the 18
@@ -78,8 +78,9 @@ constexpr int kGridSegments = 18;               // 12 edges, then 6 face diagona
 constexpr unsigned long long kGridNeighbours = 0x72bdcbc76151b17eull;  // byte c: the corners that share a segment with corner c
 constexpr int kGridCtas     = 6;                // resident CTAs per SM the kernels are compiled for (5: the same, 8: 10 % slower)
 
-// Running sums of |loss| along every image row, one CTA per row, four pixels per thread and step.  fp64: a run's sum is
-// off by less than 2^-52 of its row's sum.
+// Running sums of |loss| along every image row, one CTA per row, four pixels per thread and step.  A sum is formed in fp64 from
+// what lies to its left and nothing else, in at most 8 w / 1024 + 17 additions one after the other: it is off by less than
+// that many times 2^-53 of itself (1920 pixels: 33, 16384 pixels: 145).
 __global__ void __launch_bounds__(256) grid_row_sums_kernel(const __grid_constant__ GridArgs a)
 {
     __shared__ double s_warp[8];
@@ -107,7 +108,8 @@ __global__ void __launch_bounds__(256) grid_row_sums_kernel(const __grid_constan
         }
         if (lane == 31) s_warp[warp] = inc;
         __syncthreads();
-        double off = before + inc - sum;
+        double off = __shfl_up_sync(0xffffffffu, inc, 1);  // (not inc - sum: what lies to the right must leave no rounding here)
+        off        = before + (lane == 0 ? 0.0 : off);
         for (int w = 0; w < 8; ++w)
         {
             if (w < warp) off += s_warp[w];
@@ -191,14 +193,42 @@ __device__ __noinline__ void grid_cell_pixels(const GridArgs& a, int c, int lane
     }
 }
 
-// Base run of a row: the pixels between its leftmost and rightmost crossing.
-__device__ __forceinline__ void grid_run(const GridArgs& a, const int4 rect, int j, float L, float R, double& sum, int& hits)
+// Base run of a row: the pixels between its leftmost and rightmost crossing.  Its loss is a difference of two running sums, whose
+// rounding goes with the larger one.  A difference 2^20 times smaller than that - a run behind a pixel a million times
+// brighter, or over pixels without loss - is formed pixel by pixel instead (grid_run_pixels; for a row with pixels in a band the
+// whole cell is, see grid_rows).  Any other is off by less than 145 x 2^-52 x 2^20 = 3.4e-8 of itself up to 16384 pixels a row, half a
+// unit in the last place of the fp32 result.  (Letting grid_exact_row repeat such a row by itself cost registers: 995 instead
+// of 915 us at the sizes above.)
+constexpr int kGridCancelBits = 20;
+
+__device__ __forceinline__ bool grid_cancels(double sum, double scale)  // (high words: the exponent and 20 bits behind it)
 {
-    const int xl = (int)fmaxf(ceilf(L), 0.f), xr = (int)fminf(floorf(R), (float)(rect.z - 1));
-    if (xl > xr) return;
-    const double* p = a.prefix + (long long)(rect.y + j) * (a.w + 1) + rect.x;
-    sum += p[xr + 1] - p[xl];
-    hits += xr - xl + 1;
+    return __double2hiint(sum) < __double2hiint(scale) - (kGridCancelBits << 20);
+}
+__device__ __forceinline__ bool grid_run_ends(const int4 rect, float L, float R, int& xl, int& xr)
+{
+    xl = (int)fmaxf(ceilf(L), 0.f), xr = (int)fminf(floorf(R), (float)(rect.z - 1));
+    return xl <= xr;
+}
+__device__ __forceinline__ const double* grid_prefix(const GridArgs& a, int y) { return a.prefix + (long long)y * (a.w + 1); }
+__device__ __forceinline__ int grid_run(const GridArgs& a, const int4 rect, int j, float L, float R, double& sum, bool* cancels = nullptr)
+{
+    int xl, xr;
+    if (!grid_run_ends(rect, L, R, xl, xr)) return 0;
+    const double* p  = grid_prefix(a, rect.y + j) + rect.x;
+    const double end = p[xr + 1], run = end - p[xl];
+    if (cancels) *cancels = grid_cancels(run, end);
+    sum += run;
+    return xr - xl + 1;
+}
+__device__ __noinline__ double grid_run_pixels(const GridArgs& a, const GridWarpSmem& s, int slot, int j, float L, float R)
+{
+    int xl, xr;
+    double sum = 0.0;
+    const int4 rect = s.rect[slot];
+    if (!grid_run_ends(rect, L, R, xl, xr)) return sum;
+    for (int x = xl; x <= xr; ++x) sum += (double)grid_pixel_loss(a, rect.x + x, rect.y + j);
+    return sum;
 }
 
 // One row of one cell in which pixels lie in the band of a segment (a whole warp): the run of pixels, corrected
@@ -224,7 +254,7 @@ __device__ __noinline__ void grid_exact_row(const GridArgs& a, const GridWarpSme
         L = fminf(L, __shfl_xor_sync(0xffffffffu, L, o));
         R = fmaxf(R, __shfl_xor_sync(0xffffffffu, R, o));
     }
-    if (lane == 0) grid_run(a, rect, j, L, R, sum, hits);
+    if (lane == 0) hits += grid_run(a, rect, j, L, R, sum);
     const unsigned all = __ballot_sync(0xffffffffu, x0 <= x1);
     const int t = min(lane, 11);
     const float2 v0 = s.pp[slot][kGridTriangles[t][0]], v1 = s.pp[slot][kGridTriangles[t][1]], v2 = s.pp[slot][kGridTriangles[t][2]];
@@ -379,32 +409,50 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
     return cell;
 }
 
-// Rows [row0, row0 + rows) of the cell of every slot, eight at a time; adds each cell's totals.
-__device__ __forceinline__ void grid_rows(const GridArgs& a, const GridWarpSmem& s, int row0, int rows, int c)
+// Leftmost and rightmost crossing of row j with the segments of a cell; true if a pixel lies in the band of one.
+__device__ __forceinline__ bool grid_crossings(const GridWarpSmem& s, int slot, int j, float& L, float& R)
+{
+    const float y = (float)j, rho = s.rho[slot];
+    bool close = false;
+    L = CUDART_INF_F, R = -CUDART_INF_F;
+#pragma unroll 6
+    for (int q = 0; q < kGridSegments; ++q)
+    {
+        const float4 g = s.seg[q][slot];
+        const float yc = fminf(fmaxf(y, g.y), g.z), dy = fabsf(y - yc);
+        const float xs = fmaf(yc - g.y, g.w, g.x);
+        close |= dy <= rho && fabsf(xs - rintf(xs)) <= s.half[q][slot];
+        if (dy == 0.f) L = fminf(L, xs), R = fmaxf(R, xs);
+    }
+    return close;
+}
+
+// Rows [row0, row0 + rows) of the cell of every slot, eight at a time; adds each cell's totals.  Returns true (in all eight lanes) if
+// they are not to be had like this - a row with pixels in a band comes out small against the running sums, or against pixels
+// taken out of its run - and adds nothing then.
+__device__ __forceinline__ bool grid_rows(const GridArgs& a, const GridWarpSmem& s, int row0, int rows, int c)
 {
     const int lane = threadIdx.x & 31, slot = lane >> 3, corner = lane & 7;
     const int most = __reduce_max_sync(0xffffffffu, rows);
-    double sum = 0.0;
-    int hits   = 0;
+    double sum  = 0.0;
+    int hits    = 0;
+    bool refuse = false;
     for (int base = 0; base < most; base += 8)
     {
         const int i = base + corner, j = row0 + i;
         bool close  = false;
         if (i < rows)
         {
-            const float y   = (float)j;
-            const float rho = s.rho[slot];
-            float L = CUDART_INF_F, R = -CUDART_INF_F;
-#pragma unroll 6
-            for (int q = 0; q < kGridSegments; ++q)
+            float L, R;
+            close = grid_crossings(s, slot, j, L, R);
+            if (!close)
             {
-                const float4 g = s.seg[q][slot];
-                const float yc = fminf(fmaxf(y, g.y), g.z), dy = fabsf(y - yc);
-                const float xs = fmaf(yc - g.y, g.w, g.x);
-                close |= dy <= rho && fabsf(xs - rintf(xs)) <= s.half[q][slot];
-                if (dy == 0.f) L = fminf(L, xs), R = fmaxf(R, xs);
+                double run   = 0.0;
+                bool cancels = false;
+                hits += grid_run(a, s.rect[slot], j, L, R, run, &cancels);
+                if (cancels) run = grid_run_pixels(a, s, slot, j, L, R);
+                sum += run;
             }
-            if (!close) grid_run(a, s.rect[slot], j, L, R, sum, hits);
         }
         unsigned todo = __ballot_sync(0xffffffffu, close);
         while (todo)
@@ -418,20 +466,26 @@ __device__ __forceinline__ void grid_rows(const GridArgs& a, const GridWarpSmem&
             __syncwarp();
             for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
             rh = __reduce_add_sync(0xffffffffu, rh);
-            if (lane == from) sum += rs, hits += rh;
+            if (lane == from && rh > 0)
+            {
+                refuse |= grid_cancels(rs, grid_prefix(a, s.rect[slot].y + je)[a.w]);
+                sum += rs, hits += rh;
+            }
         }
     }
+    refuse = (__ballot_sync(0xffffffffu, refuse) >> (8 * slot) & 0xffu) != 0;
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1)
     {
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
         hits += __shfl_xor_sync(0xffffffffu, hits, o);
     }
-    if (corner == 0 && hits > 0)
+    if (corner == 0 && hits > 0 && !refuse)
     {
         atomicAdd(a.value + c, (float)sum);
         atomicAdd(a.count + c, hits);
     }
+    return refuse;
 }
 
 // Per-pixel form of the cells of the slots in `which` (bits 0, 8, 16, 24).
@@ -489,8 +543,8 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
             for (int k = lane; k < chunks && at + k < kGridQueueCap; k += 32) queue[at + k] = fits ? make_int2(ci, k) : make_int2(-1, 0);
             if (fits && (lane >> 3) == (from >> 3)) here = false;
         }
-        grid_rows(a, s, 0, here && cell.by_rows ? cell.y_size : 0, c);
-        const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && here && !cell.by_rows);
+        const bool refused  = grid_rows(a, s, 0, here && cell.by_rows ? cell.y_size : 0, c);
+        const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && here && (!cell.by_rows || refused));
         grid_pixels(a, s, cell, c, slow, 0, cell.total);
     }
 }
@@ -513,11 +567,12 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_chunk_ke
         const int mine = e * kGridGroup + (lane >> 3);
         const int2 q   = mine < n ? queue[mine] : make_int2(-1, 0);
         const GridCell cell = grid_prepare(f, a, s_cam, s, q.x, no_rows);
-        const int row0 = q.y * kGridRowChunk;
-        grid_rows(a, s, row0, cell.by_rows ? min(kGridRowChunk, cell.y_size - row0) : 0, q.x);
-        const long long first = (long long)q.y * kGridChunk;
-        const unsigned slow   = __ballot_sync(0xffffffffu, (lane & 7) == 0 && cell.total > 0 && !cell.by_rows);
-        grid_pixels(a, s, cell, q.x, slow, first, min(first + kGridChunk, cell.total));
+        const int row0      = q.y * kGridRowChunk;
+        const bool refused  = grid_rows(a, s, row0, cell.by_rows ? min(kGridRowChunk, cell.y_size - row0) : 0, q.x);
+        const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && cell.total > 0 && (!cell.by_rows || refused));
+        const int unit      = cell.by_rows ? kGridRowChunk * cell.x_size : kGridChunk;  // pixels of a chunk
+        const long long first = (long long)q.y * unit;
+        grid_pixels(a, s, cell, q.x, slow, first, min(first + unit, cell.total));
     }
 }
 
