@@ -347,7 +347,7 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
     if (no_rows) return cell;
     const float2 mn = cell.mn;
     const float E   = fmaxf(hi.x - lo.x, hi.y - lo.y) + 1.f;
-    float kappa = 0.f, thin = CUDART_INF_F;  // thin: smallest altitude of a triangle
+    float kappa = 0.f, thin = CUDART_INF_F;  // thin: smallest altitude of a triangle, 0 if one has no area or a corner is NaN
     for (int t = corner; t < 12; t += 8)
     {
         const float2 p0 = s.pp[slot][kGridTriangles[t][0]], p1 = s.pp[slot][kGridTriangles[t][1]], p2 = s.pp[slot][kGridTriangles[t][2]];
@@ -355,7 +355,7 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
         const float area2 = fabsf(ux * vy - uy * vx);
         const float a2 = ux * ux + uy * uy, b2 = vx * vx + vy * vy, c2 = wx * wx + wy * wy;
         const float l2 = fmaxf(a2, fmaxf(b2, c2)), m2 = fmaxf(fminf(a2, b2), fminf(fmaxf(a2, b2), c2));  // longest, second longest
-        kappa = fmaxf(kappa, sqrtf(l2 * m2) / area2), thin = fminf(thin, area2 * rsqrtf(l2));
+        kappa = fmaxf(kappa, sqrtf(l2 * m2) / area2), thin = fminf(thin, area2 > 0.f ? area2 * rsqrtf(l2) : 0.f);
     }
     __syncwarp();
 #pragma unroll
@@ -378,7 +378,7 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
     const float size = (float)max(a.w, a.h);
     const float rho = 1e-6f * E, rho_edge = rho * (kappa + 0.5f);
     const float skip = 1.f - size * 2.4e-7f;  // fp32 column / row numbers count up without a gap below this fraction
-    // (written so that a NaN anywhere selects the per-pixel form)
+    // (a NaN or infinite corner selects the per-pixel form through thin, or through E)
     cell.by_rows = cell.total > 0 && cell.x_size > 0 && cell.y_size > 0 && one_run && E < 2e4f && rho_edge < 0.25f &&
                    thin > 4e-3f * (1.f + (size + E) * (1.f / 2048.f)) && mn.x - floorf(mn.x) < skip && mn.y - floorf(mn.y) < skip;
     if (cell.by_rows)
