@@ -100,6 +100,49 @@ def test_grid_loss_wide_range(rasterizer):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+def test_grid_loss_recorded(rasterizer):
+    """Recorded calls: a graph stays good when a larger image has come since, and an image larger than any before can be
+    recorded (without room for its running sums the cells are walked pixel by pixel)."""
+    import torch
+
+    from vet_b200.render import Rasterizer
+
+    rast = Rasterizer(0)
+    bb_min, bb_len = _grid(21, 10.0)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rast.device)  # noqa: E731
+
+    def call(w, h, seed):
+        sc = scenes.config_planar(64, w, h, 0.6 * w, n_views=1, seed=3)
+        loss = np.random.default_rng(seed).random((3, h, w)).astype(np.float32)
+        value, count = torch.zeros(len(bb_min), device=rast.device), torch.zeros(len(bb_min), dtype=torch.int32, device=rast.device)
+        args = (t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+
+        def check():
+            torch.cuda.synchronize()
+            ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+            np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+            np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+            value.zero_(), count.zero_()
+
+        return lambda: rast.grid_loss(*args), check
+
+    run, check = call(160, 120, 1)
+    run(), check()
+    graphs = []
+    for size, seed in (((160, 120), 2), ((400, 300), 3)):
+        run, check = call(*size, seed)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run()
+        graphs.append((graph, check, run))  # (run holds the graph's tensors)
+    run, check = call(640, 480, 4)
+    run(), check()
+    for graph, check, _ in graphs:
+        graph.replay(), check()
+    rast.close()
+
+
 # ---- lists of more than 256 fragments: their sort (runs of 32, merges, up to 2048 in shared memory), their fold (blocks of
 # 1024), their sweeps (blocks of 768; mode 2: up to 1024, up to 4096)
 

@@ -18,7 +18,7 @@
 // 18 segments that the strict fp32 edge functions could disagree with it goes through the per-pixel test
 // (grid_exact_row), and cells for which the argument does not hold - several highest or lowest corners, a face seen
 // nearly edge-on, corners far outside the image, a lens distortion, rectangles whose fp32 pixel coordinates may skip a
-// number, a loss image with Inf or NaN - are walked pixel by pixel as a whole.
+// number, a loss image with Inf or NaN, no room for the running sums - are walked pixel by pixel as a whole.
 #pragma once
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -34,7 +34,8 @@ struct GridArgs
     float* value;
     int* count;
     double* prefix;   // [h][w + 1]: sum over the channels of |loss| of the pixels left of x in the row
-    int* non_finite;  // set when a pixel's loss is Inf or NaN (a running sum would carry it to the right)
+    int* no_rows;     // not 0: no running sums, either for want of room or because a pixel's loss is Inf or NaN (they would
+                      // carry it to the right)
     int n_cells, channels, h, w, view;
 };
 
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(256) grid_row_sums_kernel(const __grid_constan
         __syncthreads();
     }
     if (threadIdx.x == 0 && (a.w & 1023) == 0) row[a.w] = before;
-    if (__any_sync(0xffffffffu, bad) && lane == 0) *a.non_finite = 1;
+    if (__any_sync(0xffffffffu, bad) && lane == 0) *a.no_rows = 1;
 }
 
 __constant__ signed char kGridSegEnds[kGridSegments][2] = {{0, 1}, {2, 4}, {3, 5}, {6, 7}, {0, 2}, {1, 4}, {3, 6}, {5, 7}, {0, 3},
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     GridWarpSmem& s    = s_warp[warp];
-    const bool no_rows = s_cam.has_dist || *a.non_finite != 0;
+    const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
     const int n_groups = (a.n_cells + kGridGroup - 1) / kGridGroup;
     for (int group = blockIdx.x * kGridWarps + warp; group < n_groups; group += gridDim.x * kGridWarps)
     {
@@ -559,7 +560,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_chunk_ke
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     GridWarpSmem& s    = s_warp[warp];
-    const bool no_rows = s_cam.has_dist || *a.non_finite != 0;
+    const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
     // reservations past the capacity were never written: those cells were done by the first kernel
     const int n = min(*queue_count, kGridQueueCap);
     for (int e = blockIdx.x * kGridWarps + warp; e * kGridGroup < n; e += gridDim.x * kGridWarps)

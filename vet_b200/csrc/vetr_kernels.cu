@@ -2725,8 +2725,11 @@ struct vetr_ctx
     long long* tile_sums = nullptr;  // scan scratch
     long long tile_cap   = 0;
     int2* grid_queue     = nullptr;  // (cell, chunk) queue of vetr_grid_loss, allocated by its first call
-    int* grid_queue_count = nullptr;  // {queue length, non-finite loss seen}
-    double* grid_prefix  = nullptr;  // running sums of the loss image's rows, grown on demand
+    int* grid_queue_count = nullptr;  // {queue length, no cell by rows}
+    // running sums of the loss image's rows: the last one is in use, the ones before it were outgrown and stay until the context
+    // goes, because a recorded graph may still write to them (each at least twice the one before: together no more than the last)
+    double* grid_prefix[32] = {};
+    int grid_prefix_n         = 0;
     long long grid_prefix_cap = 0;
     // scratch of vetr_knn_radius, grown on demand: per point (sorted copy, cell, queue) and per cell (starts, ends)
     float4* knn_sorted   = nullptr;
@@ -2911,7 +2914,7 @@ extern "C" void vetr_destroy(vetr_ctx* ctx)
     cudaSetDevice(ctx->device);
     if (ctx->tile_sums) cudaFree(ctx->tile_sums);
     if (ctx->grid_queue) cudaFree(ctx->grid_queue);
-    cudaFree(ctx->grid_prefix);
+    for (int i = 0; i < ctx->grid_prefix_n; ++i) cudaFree(ctx->grid_prefix[i]);
     cudaFree(ctx->knn_sorted), cudaFree(ctx->knn_point_cell), cudaFree(ctx->knn_queue);
     cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends), cudaFree(ctx->knn_tile_sums), cudaFree(ctx->points_flags);
     for (int i = 0; i < VETR_T_N; ++i)
@@ -3319,6 +3322,31 @@ extern "C" int vetr_exchange_finalize_part(vetr_ctx* ctx, const vetr_exchange* e
     return VETR_OK;
 }
 
+// Room for n running sums, or nullptr where none is to be had: while the stream is being recorded, which forbids allocation,
+// or when the device is full.
+static double* grid_prefix(vetr_ctx* ctx, long long n)
+{
+    if (n > ctx->grid_prefix_cap)
+    {
+        cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(ctx->stream, &recording) != cudaSuccess || recording != cudaStreamCaptureStatusNone)
+        {
+            cudaGetLastError();
+            return nullptr;
+        }
+        const long long twice = 2 * ctx->grid_prefix_cap, cap = std::max(n, twice);
+        double* p = nullptr;
+        if (ctx->grid_prefix_n == 32 || cudaMalloc(&p, (size_t)cap * sizeof(double)) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return nullptr;
+        }
+        ctx->grid_prefix[ctx->grid_prefix_n++] = p;
+        ctx->grid_prefix_cap = cap;
+    }
+    return ctx->grid_prefix[ctx->grid_prefix_n - 1];
+}
+
 extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vetr_view* view, float dist_cutoff, int n_cells,
                               const float* cell_bb_min, const float* cell_bb_len, const float* loss_img, int channels,
                               float* cell_value, int32_t* cell_access_count)
@@ -3348,18 +3376,11 @@ extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vet
             VETR_CUDA(ctx, cudaMalloc(&ctx->grid_queue, (size_t)kGridQueueCap * sizeof(int2) + 256));
             ctx->grid_queue_count = reinterpret_cast<int*>(ctx->grid_queue + kGridQueueCap);
         }
-        const long long sums = (long long)view->h * (view->w + 1);
-        if (sums > ctx->grid_prefix_cap)
-        {
-            cudaFree(ctx->grid_prefix);
-            ctx->grid_prefix = nullptr, ctx->grid_prefix_cap = 0;
-            VETR_CUDA(ctx, cudaMalloc(&ctx->grid_prefix, (size_t)sums * sizeof(double)));
-            ctx->grid_prefix_cap = sums;
-        }
-        a.prefix = ctx->grid_prefix, a.non_finite = ctx->grid_queue_count + 1;
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, 2 * sizeof(int), ctx->stream));
-        ctx->launches += 3;
-        grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
+        a.prefix = grid_prefix(ctx, (long long)view->h * (view->w + 1)), a.no_rows = ctx->grid_queue_count + 1;
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, sizeof(int), ctx->stream));
+        VETR_CUDA(ctx, cudaMemsetAsync(a.no_rows, a.prefix ? 0 : 1, sizeof(int), ctx->stream));
+        ctx->launches += 2 + (a.prefix != nullptr);
+        if (a.prefix) grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
         const int groups = (n_cells + kGridGroup - 1) / kGridGroup;
         const int ctas   = std::min((groups + kGridWarps - 1) / kGridWarps, ctx->sm_count * 12);
         grid_loss_kernel<<<ctas, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
