@@ -320,16 +320,18 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 //   d env / d colour_s = T_s alpha_s G,    d env / d alpha_s = T_s (D_s - rest_s),
 //   rest_s = sum over the spheres behind s of their contribution per unit of transmittance behind s
 //          = alpha_{s+1} D_{s+1} + (1 - alpha_{s+1}) rest_{s+1}
-// (no division by 1 - alpha, which a saturated sigmoid makes zero).  First sweep, front to back: sample, keep alpha, D, T,
-// the texel coordinates and the colours' signs.  Second sweep, back to front: the gradients of the sphere's samples,
+// (no division by 1 - alpha, which a saturated sigmoid makes zero).  First sweep, front to back: sample, keep alpha, D, T
+// and the colours' signs.  Second sweep, back to front: the gradients of the sphere's samples,
 // scattered to the eight corners of its tap.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920
 // pixels crosses a few hundred texels), so before the atomics the lanes of a warp that share a base texel, in runs of
-// consecutive lanes, are summed with a segmented shuffle reduction, as many steps as the warp's longest run takes, and the
-// run's first lane issues one atomic per corner and value.
+// consecutive lanes, are summed with a segmented shuffle reduction and the run's first lane issues one atomic per corner and
+// value.  (Ending the reduction at the warp's longest run, five values side by side, was measured slower: 843 -> 955 us with
+// four spheres, 1890 -> 2390 us with eight.)
 //
-// kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of
-// up to four spheres does not pay for eight, and has room for the coordinates (asin, atan2, two square roots) of the first
-// sweep.  Four spheres of 1024 x 1024, one 1920x1080 view: 1040 -> 965 us.
+// kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of up to four spheres does not
+// pay for eight, and has room for the texel coordinates (asin, atan2, two square roots) of the first sweep; with eight they
+// are formed anew (kept: 2420 us).  1920x1080, four levels, one view: four spheres of 1024 x 1024 843 us, five of
+// 512 x 512 1110, eight 1890 us (one kernel for up to eight, without kept coordinates: 967, 1157, 1971 us).
 #ifndef VETR_ENV_BACK_CTAS
 #    define VETR_ENV_BACK_CTAS 3
 #endif
@@ -364,7 +366,8 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 if (ch < a.C) G[ch] = g[ch * per_view];
             ray = env_ray(s_cam[p.b], a.lw[p.l], a.lh[p.l], a.scale[p.l], p.x, p.y);
         }
-        float alpha[kMaxSpheres], dot[kMaxSpheres], Tin[kMaxSpheres], ix[kMaxSpheres], iy[kMaxSpheres];
+        constexpr bool kKeep = kMaxSpheres <= 4;
+        float alpha[kMaxSpheres], dot[kMaxSpheres], Tin[kMaxSpheres], ix[kKeep ? kMaxSpheres : 1], iy[kKeep ? kMaxSpheres : 1];
         unsigned hits     = 0;  // bit s: the ray hits sphere s
         unsigned negative = 0;  // bit 4 s + ch: the raw colour sample is negative (S <= 8, C <= 4)
         unsigned zero     = 0;  // the raw colour sample is exactly zero (abs has no gradient there)
@@ -372,14 +375,15 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
 #pragma unroll
         for (int s = 0; s < kMaxSpheres; ++s)
         {
-            alpha[s] = 0.f, dot[s] = 0.f, Tin[s] = T, ix[s] = 0.f, iy[s] = 0.f;
+            alpha[s] = 0.f, dot[s] = 0.f, Tin[s] = T;
+            float x = 0.f, y = 0.f;
             if (s < a.S && active)
             {
-                if (env_coordinates(a, ray, s, ix[s], iy[s]))
+                if (env_coordinates(a, ray, s, x, y))
                 {
                     hits |= 1u << s;
                     EnvCorners c;
-                    env_corners(a, env_tap_at(a, ix[s], iy[s], s), c);
+                    env_corners(a, env_tap_at(a, x, y, s), c);
                     alpha[s] = 1.f;
                     if (s != a.S - 1) alpha[s] = 1.f / (1.f + expf(-env_fetch(a.density, c)));
                     float d = 0.f;
@@ -398,6 +402,7 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                         }
                     dot[s] = d;
                 }
+                if (kKeep) ix[kKeep ? s : 0] = x, iy[kKeep ? s : 0] = y;
                 T = (1.f - alpha[s]) * T;
             }
         }
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
             int key = -1 - lane;                      // never equal between lanes
             if (live)
             {
-                const EnvTap t = env_tap_at(a, ix[s], iy[s], s);
+                const EnvTap t = kKeep ? env_tap_at(a, ix[kKeep ? s : 0], iy[kKeep ? s : 0], s) : env_tap(a, ray, s);
                 env_corners(a, t, c);
                 key   = (t.z0 * a.R + t.y0) * a.R + t.x0;
                 gv[0] = s == a.S - 1 ? 0.f : g_alpha * (alpha[s] * (1.f - alpha[s]));  // alpha is the sigmoid
@@ -445,35 +450,25 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 const int other = __shfl_down_sync(0xffffffffu, seg, 1 << k);
                 if (lane + (1 << k) < 32 && other == seg) same |= 1u << k;
             }
-            const unsigned steps = __reduce_or_sync(0xffffffffu, same);  // bits 0 .. k: a run of more than 2^k lanes
 #pragma unroll
             for (int q = 0; q < 8; ++q)
             {
                 // a corner no lane of the warp uses (outside the texture, or the empty z slice of a tap that sits on a slice)
                 if (!__any_sync(0xffffffffu, c.off[q] >= 0 && c.w[q] != 0.f)) continue;
-                float x[5];
 #pragma unroll
-                for (int v = 0; v < 5; ++v) x[v] = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
-                // (one atomic per lane without this pre-sum was measured 3 % slower)
-#pragma unroll
-                for (int k = 0; k < 5; ++k)
+                for (int v = 0; v < 5; ++v)
                 {
-                    if (!(steps >> k & 1)) break;
+                    if (v > a.C) continue;
+                    if (v == 0 && s == a.S - 1) continue;  // the last sphere's alpha is a constant
+                    float x = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
 #pragma unroll
-                    for (int v = 0; v < 5; ++v)
+                    for (int k = 0; k < 5; ++k)
                     {
-                        if (v > a.C) continue;
-                        const float y = __shfl_down_sync(0xffffffffu, x[v], 1 << k);
-                        if (same >> k & 1) x[v] += y;
+                        const float y = __shfl_down_sync(0xffffffffu, x, 1 << k);
+                        if (same >> k & 1) x += y;
                     }
-                }
-                if (head && c.off[q] >= 0)
-                {
-#pragma unroll
-                    for (int v = 0; v < 5; ++v)
-                        // (value 0: the last sphere's alpha is a constant)
-                        if (v <= a.C && !(v == 0 && s == a.S - 1) && x[v] != 0.f)
-                            atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + c.off[q], x[v]);
+                    if (head && c.off[q] >= 0 && x != 0.f)
+                        atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + c.off[q], x);
                 }
             }
         }
