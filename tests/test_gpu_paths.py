@@ -219,6 +219,32 @@ def test_zero_buffers(rasterizer):
     assert L.lib().vetr_zero_buffers(rasterizer._ctx, None, None, 17) == L.E_INVALID_ARG
 
 
+# ---- camera gradients: the image-space gradients of a point's fragments are summed in fp64
+
+
+def test_pose_gradient_of_cancelling_fragments(rasterizer):
+    """One point of mode 3 between four pixels, every product a power of two: the corners' gradients along x are 2^24, 1,
+    -2^24 and 0.  Their sum is 1; a sum in fp32 gives 0."""
+    import torch
+
+    dev = rasterizer.device
+    w = h = 16
+    f32 = dict(dtype=torch.float32, device=dev)
+    position = torch.tensor([[(6.5 - 8) / 64 * 2, (7.5 - 8) / 64 * 2, 2.0, 0.01]], **f32)
+    index = torch.zeros(1, dtype=torch.int32, device=dev)
+    texture, confidence, background = torch.tensor([[1.0], [0], [0], [0]], **f32), torch.ones(1, 1, **f32), torch.zeros(4, **f32)
+    poses = torch.tensor([[0, 0, 0, 1, 0, 0, 0, 0]], dtype=torch.float64, device=dev)
+    intrinsics = torch.tensor([[64.0, 64, 8, 8] + [0] * 9], **f32)
+    params = default_params(render_mode=3, num_layers=1, drop_out_points_by_radius=0)
+    rasterizer.forward(position, index, texture, confidence, background, poses, intrinsics, [scenes.View(w, h)], params)
+    grad = torch.zeros(1, 4, h, w, **f32)
+    grad[0, 0, 7, 6], grad[0, 0, 7, 7], grad[0, 0, 8, 6] = -2.0 ** 25, 2.0, 2.0 ** 25
+    raw = rasterizer.backward_raw([grad])
+    assert raw["points"][0, 3].item() == 4
+    assert raw["pose"][0, 0].item() == 32.0  # f / z
+    assert raw["intrinsics"][0, 2].item() == 0.5  # K_gradient_factor
+
+
 # ---- mode 0: backward with the interleaved image copies, and without pixel scratch
 
 

@@ -1293,16 +1293,18 @@ __device__ void reduce_cam(const Frame& f, const BackPtrs& bp, CamAcc<kIntr>& ac
 
 // Image-space gradient of all fragments of a point in one view, brought to level 0.  The chain of Jacobians behind it is
 // linear and differs between the levels only by the factor 0.5^level of the crop matrix (a power of two: exact), so the
-// camera gradients, sums over many points, take it once per point and view instead of once per fragment.
+// camera gradients, sums over many points, take it once per point and view instead of once per fragment.  Summed in fp64: the
+// terms of a point cancel (the Jacobians of a bilinear point's four corners add up to zero), and what they leave goes through
+// the chain with one rounding to fp32, not with one per fragment.
 struct PointGrad
 {
-    float x, y;
+    double x, y;
     int hits;
-    __device__ __forceinline__ void clear() { x = y = 0.f, hits = 0; }
+    __device__ __forceinline__ void clear() { x = y = 0.0, hits = 0; }
     __device__ __forceinline__ void add(float2 g, int level)
     {
         const float scale = level_scale(level);
-        x += g.x * scale, y += g.y * scale, ++hits;
+        x += (double)(g.x * scale), y += (double)(g.y * scale), ++hits;
     }
     static __device__ __forceinline__ float level_scale(int level) { return __int_as_float((127 - level) << 23); }
 };
@@ -1322,7 +1324,7 @@ template <bool kIntr>
 __device__ __forceinline__ void camera_terms(const Frame& f, const Camera& cam, const PointJac& jac, const PointGrad& g,
                                              CamAcc<kIntr>& acc)
 {
-    const ViewGrad v = project_backward_view(jac, make_float2(g.x, g.y), cam, cam.crop);
+    const ViewGrad v = project_backward_view(jac, make_float2((float)g.x, (float)g.y), cam, cam.crop);
     float g_pose[6];
     project_backward_pose(jac, v, g_pose);
 #pragma unroll
