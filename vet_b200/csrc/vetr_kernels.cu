@@ -1294,8 +1294,8 @@ __device__ void reduce_cam(const Frame& f, const BackPtrs& bp, CamAcc<kIntr>& ac
 // Image-space gradient of all fragments of a point in one view, brought to level 0.  The chain of Jacobians behind it is
 // linear and differs between the levels only by the factor 0.5^level of the crop matrix (a power of two: exact), so the
 // camera gradients, sums over many points, take it once per point and view instead of once per fragment.  Summed in fp64: the
-// terms of a point cancel (the Jacobians of a bilinear point's four corners add up to zero), and what they leave goes through
-// the chain with one rounding to fp32, not with one per fragment.
+// terms of a point cancel (the Jacobians of a bilinear point's four corners add up to zero).  They stay fp64 through the
+// camera's matrices, so that the sum is rounded to fp32 no more often than a single fragment's gradient is.
 struct PointGrad
 {
     double x, y;
@@ -1315,7 +1315,7 @@ __device__ __forceinline__ void point_terms(const Camera& cam, const PointJac& j
     const float scale = PointGrad::level_scale(level);
     const float crop2[5] = {cam.crop[0] * scale, cam.crop[1] * scale, 0.f, 0.f, cam.crop[4] * scale};  // IntrinsicsPinhole::scale
     float g[3];
-    project_backward_point(cam, project_backward_view(jac, dR, cam, crop2), g);
+    project_backward_point(cam, project_backward_view(jac, dR.x, dR.y, cam, crop2), g);
     gp.x += g[0], gp.y += g[1], gp.z += g[2], gp.w += 1.f;
 }
 
@@ -1324,7 +1324,7 @@ template <bool kIntr>
 __device__ __forceinline__ void camera_terms(const Frame& f, const Camera& cam, const PointJac& jac, const PointGrad& g,
                                              CamAcc<kIntr>& acc)
 {
-    const ViewGrad v = project_backward_view(jac, make_float2((float)g.x, (float)g.y), cam, cam.crop);
+    const ViewGrad v = project_backward_view(jac, g.x, g.y, cam, cam.crop);
     float g_pose[6];
     project_backward_pose(jac, v, g_pose);
 #pragma unroll

@@ -247,13 +247,16 @@ struct ViewGrad
     float gv[3];
 };
 
-__device__ __forceinline__ ViewGrad project_backward_view(const PointJac& j, float2 grad, const Camera& cam, const float cropK[5])
+// (Real = double, for a gradient that is a sum: the matrices in fp64, rounded to fp32 once behind them)
+template <typename Real>
+__device__ __forceinline__ ViewGrad project_backward_view(const PointJac& j, Real grad_x, Real grad_y, const Camera& cam, const float cropK[5])
 {
     ViewGrad o;
     // grad_p_rot = rot^T grad ; grad_p_k2 = J_p_K2^T grad_p_rot ; then J_p_K1^T, J_p_dis^T, J_div^T
-    const float2 g_rot = make_float2(cam.rot[0] * grad.x + cam.rot[2] * grad.y, cam.rot[1] * grad.x + cam.rot[3] * grad.y);
-    o.g_k2 = make_float2(cropK[0] * g_rot.x, cropK[4] * g_rot.x + cropK[1] * g_rot.y);
-    o.g_k1 = make_float2(cam.K[0] * o.g_k2.x, cam.K[4] * o.g_k2.x + cam.K[1] * o.g_k2.y);
+    const Real rx = cam.rot[0] * grad_x + cam.rot[2] * grad_y, ry = cam.rot[1] * grad_x + cam.rot[3] * grad_y;
+    const Real k2x = cropK[0] * rx, k2y = cropK[4] * rx + cropK[1] * ry;
+    o.g_k2 = make_float2((float)k2x, (float)k2y);
+    o.g_k1 = make_float2((float)(cam.K[0] * k2x), (float)(cam.K[4] * k2x + cam.K[1] * k2y));
     float2 g_dis = o.g_k1;
     if (cam.has_dist)
         g_dis = make_float2(j.Jpd[0] * o.g_k1.x + j.Jpd[2] * o.g_k1.y, j.Jpd[1] * o.g_k1.x + j.Jpd[3] * o.g_k1.y);
