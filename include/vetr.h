@@ -138,10 +138,10 @@ typedef struct vetr_lists
                               need_point_gradient is set; level_mask must be the one the forward call wrote.  Neither
                               needs initialising.  Mode 3 keeps a fragment's corner in the two top bits of the record's
                               descriptor index, so n_tex must stay below 2^30 there. */
-    float*    pixel_scratch; /* [n_views*P*8] 16-byte aligned scratch of vetr_backward, required in modes 1-3, used in mode 0
-                                where it is given (else slower loads): channel-interleaved copies of out_color and
-                                grad_color over the pixel space (eight 16-byte loads fetch all neighbour values of a
-                                fragment).  Needs no initialising. */
+    float*    pixel_scratch; /* [n_views*P*8] 16-byte aligned scratch of vetr_backward in modes 1-3: channel-interleaved
+                                copies of out_color and grad_color over the pixel space (eight 16-byte loads fetch all
+                                neighbour values of a fragment).  Needs no initialising.  Mode 0 does not touch it, unless
+                                vetr_backward_phase is given VETR_BACKWARD_PIXEL_SCRATCH. */
 } vetr_lists;
 
 typedef struct vetr_ctx vetr_ctx;
@@ -218,6 +218,9 @@ int vetr_backward(vetr_ctx* ctx, const vetr_params* params, const vetr_cloud* cl
  * g_intr; in mode 3 also g_conf).  vetr_backward is both.  Mode 0 does everything in the first phase. */
 #define VETR_BACKWARD_FRAGMENTS 1
 #define VETR_BACKWARD_POINTS 2
+/* Beside VETR_BACKWARD_FRAGMENTS: lists->pixel_scratch (as large as in modes 1-3) may be used in mode 0 too, which is faster
+ * where points are no fewer than pixels.  Without effect in the other modes, or where pixel_scratch is NULL. */
+#define VETR_BACKWARD_PIXEL_SCRATCH 4
 int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, const vetr_cloud* cloud, const vetr_texture* texture,
                         const vetr_cameras* cameras, const vetr_view* views, int n_views, const float* dropout,
                         const vetr_lists* lists, const float* const* out_color, const float* const* grad_color,

@@ -267,3 +267,41 @@ def test_mode0_backward_scratch(monkeypatch, channels, ghost):
         # addend (T - I) * G inherits that relative to |I * G|: the bound of the mode-0 parity tests
         util.compare_backward(gpu["bwd_raw"], ora, channels, rtol=2e-5, floor_rel=1e-6)
         rast.close()
+
+
+def test_mode0_leaves_the_scratch_of_other_modes_alone(rasterizer):
+    """vetr_backward in mode 0 does not touch lists->pixel_scratch, which it has no use for: a caller may keep a buffer of any
+    size there."""
+    import ctypes as C
+
+    import torch
+
+    from vet_b200 import _lib as L
+
+    sc = scenes.tiny_scene(n=9000, w=93, h=61, n_views=2, seed=13)
+    params = default_params(render_mode=0)
+    grads = [torch.from_numpy(g).to(rasterizer.device) for g in
+             util.random_grads(util.run_gpu(rasterizer, sc, params)["fwd"]["color"], seed=3)]
+    want = rasterizer.backward_raw(grads)
+    s = rasterizer._saved
+    b0, b1, lists, views = s["groups"][0]
+    lists.ensure_pixel_scratch()
+    lists.pixel_scratch.fill_(7.0)
+    got = {k: torch.zeros_like(v) for k, v in want.items()}
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    arr = lambda ts: (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])  # noqa: E731
+    rc = L.lib().vetr_backward(rasterizer._ctx, C.byref(s["prm"]), C.byref(s["cloud"]), C.byref(s["tex"]), C.byref(s["cams"]),
+                               views, b1 - b0, None, C.byref(lists.c), arr(s["color"]), arr(grads), p(got["desc"]),
+                               p(got["conf"]), p(got["points"]), p(got["background"]), p(got["pose"]), p(got["pose_count"]),
+                               p(got["intrinsics"]), p(got["intrinsics_count"]))
+    assert rc == L.OK
+    assert bool((lists.pixel_scratch == 7.0).all())
+    assert torch.equal(got["points"][:, 3], want["points"][:, 3])
+    for k in want:  # the same addends (sums in no fixed order)
+        assert torch.allclose(got[k], want[k], rtol=1e-4, atol=1e-5 * float(want[k].abs().max())), k
+    # the word for it goes with the per-fragment phase; other bits are refused as before
+    for phases in (0, 4, 6, 8, 11):
+        assert L.lib().vetr_backward_phase(rasterizer._ctx, C.byref(s["prm"]), C.byref(s["cloud"]), C.byref(s["tex"]),
+                                           C.byref(s["cams"]), views, b1 - b0, None, C.byref(lists.c), arr(s["color"]),
+                                           arr(grads), p(got["desc"]), p(got["conf"]), None, p(got["background"]), None, None,
+                                           None, None, phases) == L.E_INVALID_ARG

@@ -82,7 +82,7 @@ EXPORTS = [
     "vetr_zero_buffers",
 ]
 ENV_ADD, ENV_NOT_AT_POINTS, ENV_DEPTH_TEST_WEIGHT, ENV_NO_DISTORTION_CHECK = 1, 2, 4, 8
-BACKWARD_FRAGMENTS, BACKWARD_POINTS = 1, 2
+BACKWARD_FRAGMENTS, BACKWARD_POINTS, BACKWARD_PIXEL_SCRATCH = 1, 2, 4
 SEG_DESC, SEG_POINTS, SEG_CONF = 1, 2, 4
 TIMING_NAMES = ["count", "scan", "collect", "sort_blend", "backward", "finalize", "point_backward", "exchange", "envmap", "knn"]
 

@@ -3148,6 +3148,9 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
                                    float* g_conf, float* g_points, float* g_background, double* g_pose,
                                    float* g_pose_count, float* g_intr, float* g_intr_count, int phases)
 {
+    const bool use_scratch = phases & VETR_BACKWARD_PIXEL_SCRATCH;
+    if (use_scratch && !(phases & VETR_BACKWARD_FRAGMENTS)) return VETR_E_INVALID_ARG;
+    phases &= ~VETR_BACKWARD_PIXEL_SCRATCH;
     if ((phases & ~(VETR_BACKWARD_FRAGMENTS | VETR_BACKWARD_POINTS)) != 0 || phases == 0) return VETR_E_INVALID_ARG;
     Frame f;
     int rc = fill_frame(ctx, f, params, cloud, texture, cameras, views, n_views, lists);
@@ -3172,8 +3175,8 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         if (!(phases & VETR_BACKWARD_FRAGMENTS)) return VETR_OK;  // mode 0 has one phase
         // Channel-interleaved copies: 9 gathers of 16 bytes per fragment instead of 36 of 4.  They cost 11 ps per pixel and save
         // 13 ps per point and view (2 M points, 2 views 1280x720: 234 -> 181 + 27 us), hence only where points are no fewer
-        // than pixels.
-        if (((uintptr_t)f.img4 & 15) != 0 || f.n < f.Prm) f.img4 = f.grad4 = nullptr;
+        // than pixels; and only with the caller's word that the scratch is there, because mode 0 can do without.
+        if (!use_scratch || ((uintptr_t)f.img4 & 15) != 0 || f.n < f.Prm) f.img4 = f.grad4 = nullptr;
         PassScope t(ctx, VETR_T_BACKWARD, 2 + (f.img4 != nullptr));
         cudaStream_t st = ctx->stream;
         if (f.img4) pack_images_kernel<<<(unsigned)((f.Prm * n_views + 255) / 256), 256, 0, st>>>(f, bp);

@@ -258,7 +258,8 @@ class Rasterizer:
                                          C.byref(lists.c), _ptr_array(oc), _ptr_array(gc),
                                          _ptr(g["desc"]), _ptr(g["conf"]), _ptr(g.get("points")), _ptr(g["background"]),
                                          _ptr(g.get("pose")), _ptr(g.get("pose_count")), _ptr(g.get("intrinsics")),
-                                         _ptr(g.get("intrinsics_count")), phases)
+                                         _ptr(g.get("intrinsics_count")),
+                                         phases | L.BACKWARD_PIXEL_SCRATCH if phases & L.BACKWARD_FRAGMENTS else phases)
             self._check(rc, "vetr_backward_phase")
         return g
 

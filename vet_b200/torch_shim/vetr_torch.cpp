@@ -386,16 +386,17 @@ variable_list PointRender::backward(AutogradContext* ctx, variable_list grad_out
         auto pc = level_ptrs(color, b0), pg = level_ptrs(gcolor, b0);
         std::vector<const float*> cpc(pc.begin(), pc.end()), cpg(pg.begin(), pg.end());
         const bool has_dropout = dropout.numel() > 0;
-        check(vetr_backward(vc, &prm, &in.cloud, &in.tex, &in.cams, views.data(), nb,
-                            has_dropout ? dropout.data_ptr<float>() + (int64_t)b0 * dropout.stride(0) : nullptr,
-                            &lists, cpc.data(), cpg.data(),
-                            g_desc.data_ptr<float>(), g_conf.data_ptr<float>(),
-                            g_points.defined() ? g_points.data_ptr<float>() : nullptr, g_background.data_ptr<float>(),
-                            g_pose.defined() ? g_pose.data_ptr<double>() : nullptr,
-                            g_pose.defined() ? g_pose_count.data_ptr<float>() : nullptr,
-                            g_intr.defined() ? g_intr.data_ptr<float>() : nullptr,
-                            g_intr.defined() ? g_intr_count.data_ptr<float>() : nullptr),
-              "vetr_backward");
+        check(vetr_backward_phase(vc, &prm, &in.cloud, &in.tex, &in.cams, views.data(), nb,
+                                  has_dropout ? dropout.data_ptr<float>() + (int64_t)b0 * dropout.stride(0) : nullptr,
+                                  &lists, cpc.data(), cpg.data(),
+                                  g_desc.data_ptr<float>(), g_conf.data_ptr<float>(),
+                                  g_points.defined() ? g_points.data_ptr<float>() : nullptr, g_background.data_ptr<float>(),
+                                  g_pose.defined() ? g_pose.data_ptr<double>() : nullptr,
+                                  g_pose.defined() ? g_pose_count.data_ptr<float>() : nullptr,
+                                  g_intr.defined() ? g_intr.data_ptr<float>() : nullptr,
+                                  g_intr.defined() ? g_intr_count.data_ptr<float>() : nullptr,
+                                  VETR_BACKWARD_FRAGMENTS | VETR_BACKWARD_POINTS | VETR_BACKWARD_PIXEL_SCRATCH),
+              "vetr_backward_phase");
         // mode 2 flags lists it had to skip in the status words: looked at when the next call starts
         if (prm.render_mode == VETR_MODE_FUZZY_BLEND) cache.NoteStatus(t[3], t[2].size(0), nb, true);
     }
