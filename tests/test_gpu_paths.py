@@ -305,3 +305,33 @@ def test_mode0_leaves_the_scratch_of_other_modes_alone(rasterizer):
                                            C.byref(s["cams"]), views, b1 - b0, None, C.byref(lists.c), arr(s["color"]),
                                            arr(grads), p(got["desc"]), p(got["conf"]), None, p(got["background"]), None, None,
                                            None, None, phases) == L.E_INVALID_ARG
+
+
+# ---- per-point pass: several runs of 256 points per block (2 and the most, 8), several views, a partial last run
+
+
+@pytest.mark.parametrize("mode", [1, 3])
+@pytest.mark.parametrize("tiles, w, h, views", [(2, 320, 240, 3), (8, 640, 480, 2)])
+def test_point_backward_tiles(rasterizer, mode, tiles, w, h, views):
+    import torch
+
+    per_tile = 256 * 4 * torch.cuda.get_device_properties(rasterizer.device).multi_processor_count
+    n = tiles * per_tile + 257  # the rule: as many runs per block as leave four blocks per SM
+    sc = scenes.config_planar(n, w, h, 0.9 * w, n_views=views, seed=17)
+    rng = np.random.default_rng(6)  # gradients without cancellation inside a term: thin fragments of one sign, no background
+    sc.texture[:], sc.background[:] = 0, 0
+    sc.texture[0] = rng.uniform(1, 2, n)
+    sc.confidence *= np.float32(0.002)
+    params = default_params(render_mode=mode, num_layers=2)
+    ora = util.run_oracle(sc, params)
+    grads = util.l1_grads(ora["fwd"]["color"], seed=3)
+    ora = util.run_oracle(sc, params, grads=grads)
+    gpu = util.run_gpu(rasterizer, sc, params, grads=grads)
+    util.compare_forward(gpu, ora, exact_images=True)
+    util.compare_backward(gpu["bwd_raw"], ora, sc.channels)
+    on = [torch.from_numpy(g).to(rasterizer.device) for g in grads]
+    for want_pose in (True, False):  # the kernel without intrinsics, with and without a pose
+        part = rasterizer.backward_raw(on, want_pose=want_pose, want_intrinsics=False)
+        np.testing.assert_array_equal(part["points"].cpu().numpy(), gpu["bwd_raw"]["points"])  # one owner per point, fixed order
+    pose = rasterizer.backward_raw(on, want_intrinsics=False)["pose"].cpu().numpy()
+    np.testing.assert_allclose(pose, gpu["bwd_raw"]["pose"], rtol=1e-6, atol=1e-9 * np.abs(pose).max())

@@ -4,7 +4,7 @@
 //
 // The reference tests every pixel of a cell's screen rectangle against the twelve triangles of the box (two per face) and
 // issues two global atomics per covered pixel.  Those tests are what bounds a per-pixel form (twelve triangles of three
-// edge functions in strict fp32 for each of some 600 M pixels at 128^3 cells and 1920 x 1080: 7.3 ms).  Here a lane owns one
+// edge functions in strict fp32 for each of some 600 M pixels at 128^3 cells and 1920 x 1080: 7.9 ms).  Here a lane owns one
 // pixel ROW of a cell: the twelve triangles are a closed surface, so what they cover of a row is the run of pixels between its
 // leftmost and rightmost crossing with the 18 segments (12 edges, 6 face diagonals), and the run's loss is a difference
 // of two running sums of that image row (fp64, formed once per call).  0.92 ms at the same sizes.

@@ -24,13 +24,13 @@
 //   pack_images_kernel       channel-interleaved copies of the forward image and its gradient
 //   backward_kernel          per work item: stream sorted records, image-space gradient of each fragment (parked for
 //                            the per-point pass), O(n) transmittance / suffix sweeps per pixel, vector reductions of
-//                            descriptor / confidence gradients (+ _long variants; mode 3 forms its spatial gradient here)
-//   point_backward_kernel    modes 1, 2: one thread per point over all views: projection Jacobians per fragment,
-//                            position gradient written once, camera gradients reduced per CTA and view
+//                            descriptor / confidence gradients (+ _long variants; mode 3 parks the alpha gradient)
+//   point_backward_kernel    one thread per point over all views: projection Jacobians per fragment, position gradient
+//                            written once, camera gradients reduced per CTA and view (mode 3: confidence gradient too)
 //   fuzzy_dt_*               mode 0 (no lists): depth pre-pass, splat, combine, per-point backward
 //   exchange_finalize_kernel multi-GPU: sum over ranks + epilogue over NVLink peer memory (plain or multicast)
-//   grid_loss_kernel         error-grid rasterisation (one warp per grid cell)
-//   transpose / normalize / apply_tangent   small epilogues
+//   grid_row_sums / grid_loss (+ _chunk)   error-grid rasterisation (four cells per warp, a lane per pixel row)
+//   zero_buffers / finalize / apply_tangent   zero fill, epilogue, pose update
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -3612,7 +3612,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         cell *= 0.5f, cells = finer;
         d[0] = d2[0], d[1] = d2[1], d[2] = d2[2];
     }
-    if (cells > ctx->knn_cap_cells)  // no iteration counted, as when all points coincide
+    if (cells > ctx->knn_cap_cells)  // all points coincide: no iteration ran
     {
         cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends);
         ctx->knn_starts = nullptr, ctx->knn_ends = nullptr, ctx->knn_cap_cells = 0;
