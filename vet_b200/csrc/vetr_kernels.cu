@@ -1992,8 +1992,10 @@ __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __g
 // fragment, 600 us like this; mode 3, 3 M points x 2 views: 1587 -> 326 us.
 constexpr int kPointTilesMax = 8;
 
-template <bool kIntr, bool kBilinear>
-__global__ void __launch_bounds__(kProjThreads, kIntr || kBilinear ? 3 : 4)
+// kCam: 0 = no camera gradients (their sums are not kept: a step of 20 M points and 8 views 1.5 % slower with them than before they were
+// fp64, 1.4 % faster without), 1 = pose, 2 = intrinsics (and the pose where it is wanted).
+template <int kCam, bool kBilinear>
+__global__ void __launch_bounds__(kProjThreads, kCam == 2 || kBilinear ? 3 : 4)
     point_backward_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp, int tiles)
 {
     extern __shared__ __align__(16) float4 s_gp[];  // [tiles][kProjThreads], every thread its own column
@@ -2002,9 +2004,9 @@ __global__ void __launch_bounds__(kProjThreads, kIntr || kBilinear ? 3 : 4)
     if (f.status[1] != 0) return;  // overflow / skipped list: some fragments never parked a value
     if (threadIdx.x < f.n_views) s_cam[threadIdx.x] = load_camera(f, threadIdx.x);
     __syncthreads();
-    const int first     = blockIdx.x * (kProjThreads * tiles) + threadIdx.x;
-    const bool want_cam = bp.g_pose != nullptr || kIntr;
-    const bool spatial  = f.need_point_grad != 0;
+    const int first      = blockIdx.x * (kProjThreads * tiles) + threadIdx.x;
+    constexpr bool kIntr = kCam == 2;
+    const bool spatial   = f.need_point_grad != 0;
     for (int it = 0; it < tiles; ++it) s_gp[it * kProjThreads + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int b = 0; b < f.n_views; ++b)
     {
@@ -2035,7 +2037,7 @@ __global__ void __launch_bounds__(kProjThreads, kIntr || kBilinear ? 3 : 4)
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l)
                     if ((mask >> l & 1u) && __float_as_int(dR[l].x) != kNoGradientBits)
                     {
-                        g.add(dR[l], l);
+                        if (kCam) g.add(dR[l], l);
                         point_terms(s_cam[b], jac, dR[l], l, gp);
                     }
             }
@@ -2071,20 +2073,20 @@ __global__ void __launch_bounds__(kProjThreads, kIntr || kBilinear ? 3 : 4)
                         if (!jac_ok) continue;
                         const float single = conf * gl[c];
                         const float2 dR    = make_float2(jx * single, jy * single);
-                        g.add(dR, l);
+                        if (kCam) g.add(dR, l);
                         point_terms(s_cam[b], jac, dR, l, gp);
                     }
                 }
                 if (gconf != 0.f) red_add(bp.g_conf + tex, gconf);
             }
             s_gp[it * kProjThreads + threadIdx.x] = gp;
-            if (want_cam && g.hits)
+            if (kCam && g.hits)
             {
                 camera_terms<kIntr>(f, s_cam[b], jac, g, acc);
                 any = true;
             }
         }
-        if (want_cam && __syncthreads_or(any)) reduce_cam<kIntr>(f, bp, acc, b, s_red);
+        if (kCam && __syncthreads_or(any)) reduce_cam<kIntr>(f, bp, acc, b, s_red);
     }
     if (bp.g_points)
         for (int it = 0; it < tiles; ++it)
@@ -2265,10 +2267,11 @@ __global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_c
 
 // RenderBackward (RenderBackward.cu:131-474): one thread per point and view.  Pixel positions come from the backward's own
 // copy of the projection, which leaves out the crop rotation (RenderBackward.cu:78-116).
-template <bool kIntr>
+template <int kCam>  // as in point_backward_kernel
 __global__ void __launch_bounds__(kProjThreads, 4) fuzzy_dt_backward_kernel(const __grid_constant__ Frame f,
                                                                          const __grid_constant__ BackPtrs bp)
 {
+    constexpr bool kIntr = kCam == 2;
     __shared__ Camera s_cam;
     __shared__ double s_red[kProjThreads / 32][kCamValues];
     const int b = blockIdx.y;
@@ -2316,17 +2319,17 @@ __global__ void __launch_bounds__(kProjThreads, 4) fuzzy_dt_backward_kernel(cons
                 if (!(point_grad && px.interior)) continue;
                 const float4 d  = load_descriptor(f, tex);
                 const float2 dR = f.img4 ? neighbour_gradient(f, row_major_index(f, px), lw, d) : neighbour_gradient_planar(f, bp, px, d);
-                grad.add(dR, l);
+                if (kCam) grad.add(dR, l);
                 point_terms(cam, jac, dR, l, gp);
             }
-            if (grad.hits)
+            if (gp.w != 0.f)
             {
-                camera_terms<kIntr>(f, cam, jac, grad, acc);
+                if (kCam) camera_terms<kIntr>(f, cam, jac, grad, acc);
                 if (bp.g_points) red_add_v4(bp.g_points + pid, gp);
             }
         }
     }
-    if (bp.g_pose != nullptr || kIntr) reduce_cam<kIntr>(f, bp, acc, b, s_red);
+    if (kCam) reduce_cam<kIntr>(f, bp, acc, b, s_red);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -3184,10 +3187,8 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         if (ctas > 0)
         {
-            if (g_intr)
-                fuzzy_dt_backward_kernel<true><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f, bp);
-            else
-                fuzzy_dt_backward_kernel<false><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f, bp);
+            const auto kernel = g_intr ? fuzzy_dt_backward_kernel<2> : g_pose ? fuzzy_dt_backward_kernel<1> : fuzzy_dt_backward_kernel<0>;
+            kernel<<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f, bp);
         }
         VETR_CUDA(ctx, cudaGetLastError());
         return VETR_OK;
@@ -3233,21 +3234,9 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         const int tiles   = std::max(1, std::min(kPointTilesMax, f.n / (kProjThreads * ctx->sm_count * 4)));
         const int ctas    = (f.n + kProjThreads * tiles - 1) / (kProjThreads * tiles);
         const size_t smem = (size_t)tiles * kProjThreads * sizeof(float4);
-        cudaStream_t st = ctx->stream;
-        if (bilinear)
-        {
-            if (g_intr)
-                point_backward_kernel<true, true><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
-            else
-                point_backward_kernel<false, true><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
-        }
-        else
-        {
-            if (g_intr)
-                point_backward_kernel<true, false><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
-            else
-                point_backward_kernel<false, false><<<ctas, kProjThreads, smem, st>>>(f, bp, tiles);
-        }
+        const auto kernel = bilinear ? (g_intr ? point_backward_kernel<2, true> : g_pose ? point_backward_kernel<1, true> : point_backward_kernel<0, true>)
+                                     : (g_intr ? point_backward_kernel<2, false> : g_pose ? point_backward_kernel<1, false> : point_backward_kernel<0, false>);
+        kernel<<<ctas, kProjThreads, smem, ctx->stream>>>(f, bp, tiles);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
