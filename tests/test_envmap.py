@@ -207,6 +207,14 @@ def test_fixture_restatement_and_libtorch_values():
     assert np.all(np.abs(gc - g["env_torch_g_color"]) <= 1e-5 * mc + 1e-7)
 
 
+def test_slices_of_up_to_five_spheres_are_exact():
+    """The kernels take four corners per sample where grid_sample's third coordinate, formed in fp32, is the sphere's number."""
+    f = np.float32
+    for S in range(2, 9):
+        exact = all((((f(s) / f(S - 1) * f(2) - f(1)) + f(1)) / f(2)) * f(S - 1) == s for s in range(S))
+        assert exact == (S <= 5), S
+
+
 # ---------------------------------------------------------------------------------------------------------
 # CUDA kernels against the restatement
 
@@ -296,3 +304,10 @@ def test_gpu_envmap_against_fixture():
     for mine, ref, mag in ((gd, g["env_torch_g_density"], g["env_mag_density"]), (gc, g["env_torch_g_color"], g["env_mag_color"]),
                            (gd, g["env_g_density"], g["env_mag_density"]), (gc, g["env_g_color"], g["env_mag_color"])):
         assert np.all(np.abs(mine - ref) <= util.env_grad_tolerance(mag, env))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S", [2, 5, 6, 7])
+def test_gpu_envmap_on_either_side_of_flat_slices(S):
+    """Two and five spheres: samples on their slices; six and seven: some samples reach into the neighbouring slice."""
+    test_gpu_envmap_matches_oracle(0, False, S, 0)

@@ -32,7 +32,8 @@ struct EnvArgs  // kernel parameter block
 {
     int n_views, L, S, R, C, up_axis, non_subzero, flags;
     int lw[VETR_MAX_LAYERS], lh[VETR_MAX_LAYERS];
-    long long lend[VETR_MAX_LAYERS];  // pixels of levels 0..l over all views (running total)
+    float inv_lw[VETR_MAX_LAYERS];
+    int lend[VETR_MAX_LAYERS];        // pixels of levels 0..l over all views (running total; below 2^30)
     float scale[VETR_MAX_LAYERS];     // 0.5^l
     float radii[kEnvMaxSpheres];
     EnvView views[VETR_MAX_VIEWS];
@@ -125,13 +126,6 @@ __device__ __forceinline__ EnvRay env_ray(const EnvCam& c, int lw, int lh, float
     return ray;
 }
 
-struct EnvTap  // one sphere's sample: base texel and trilinear weights
-{
-    bool hit;
-    int x0, y0, z0;
-    float wx[2], wy[2], wz[2];
-};
-
 __device__ __forceinline__ float env_unnormalize(float c, int size) { return ((c + 1.f) / 2.f) * (float)(size - 1); }
 
 // CreateSampleUVMapAllSpheres for one sphere (EnvironmentMap.cu:620-682): texel coordinates of the ray's sample, false if
@@ -162,65 +156,64 @@ __device__ __forceinline__ bool env_coordinates(const EnvArgs& a, const EnvRay& 
     return true;
 }
 
-// grid_sample's coordinate arithmetic for sphere s.
-__device__ __forceinline__ EnvTap env_tap_at(const EnvArgs& a, float ix, float iy, int s)
-{
-    EnvTap t;
-    t.hit = true;
-    const float z  = a.S == 1 ? 0.f : (float)s / (float)(a.S - 1) * 2.f - 1.f;
-    const float iz = env_unnormalize(z, a.S);
-    const float fx = floorf(ix), fy = floorf(iy), fz = floorf(iz);
-    // the base texel, kept inside [-2, size] so that the int conversion and the + 1 of the far corners are defined for
-    // every float (anything out there is outside the texture and reads zero either way)
-    t.x0 = (int)fminf(fmaxf(fx, -2.f), (float)a.R), t.y0 = (int)fminf(fmaxf(fy, -2.f), (float)a.R);
-    t.z0 = (int)fminf(fmaxf(fz, -2.f), (float)a.S);
-    t.wx[1] = ix - fx, t.wx[0] = (fx + 1.f) - ix;
-    t.wy[1] = iy - fy, t.wy[0] = (fy + 1.f) - iy;
-    t.wz[1] = iz - fz, t.wz[0] = (fz + 1.f) - iz;
-    return t;
-}
+// Up to kEnvFlatSpheres spheres, grid_sample's third coordinate of sphere s, formed in fp32 as unnormalize(2 s / (S - 1) - 1),
+// is s exactly: a sample lies on its slice, has four corners instead of eight, and offsets are taken inside the slice.  With
+// six and more some come out beside the slice (0.99999994 for s = 1 of 6), and the neighbouring slice gets its share.
+constexpr int kEnvFlatSpheres = 5;
 
-__device__ __forceinline__ EnvTap env_tap(const EnvArgs& a, const EnvRay& ray, int s)
-{
-    float ix, iy;
-    if (env_coordinates(a, ray, s, ix, iy)) return env_tap_at(a, ix, iy, s);
-    EnvTap t;
-    t.hit = false;
-    t.x0 = t.y0 = t.z0 = 0;
-    t.wx[0] = t.wx[1] = t.wy[0] = t.wy[1] = t.wz[0] = t.wz[1] = 0.f;
-    return t;
-}
-
-// The eight corners of a tap: texel offset inside one [S,R,R] plane (-1 = outside, reads zero) and weight.
+// The corners of sphere s's sample: texel offset inside the slice (flat) or inside one [S,R,R] plane, and weight; outside the
+// texture -1 and 0.  Corners of weight 0 read nothing, whatever the texel holds.
+template <bool kFlat>
 struct EnvCorners
 {
-    int off[8];
-    float w[8];
+    static constexpr int N = kFlat ? 4 : 8;
+    int off[N];
+    float w[N];
 };
 
-__device__ __forceinline__ void env_corners(const EnvArgs& a, const EnvTap& t, EnvCorners& c)
+// Fills the corners and returns the base texel's index, which samples with the same corners share (`alone`, an index of the
+// caller's, where the base texel lies outside the texture).
+template <bool kFlat>
+__device__ __forceinline__ int env_corners(const EnvArgs& a, float ix, float iy, int s, EnvCorners<kFlat>& c, int alone = -1)
 {
+    const float fx = floorf(ix), fy = floorf(iy);
+    // the base texel, kept inside [-2, size] so that the int conversion and the + 1 of the far corners are defined for
+    // every float (anything out there is outside the texture and reads zero either way)
+    const int x0 = (int)fminf(fmaxf(fx, -2.f), (float)a.R), y0 = (int)fminf(fmaxf(fy, -2.f), (float)a.R);
+    const float wx[2] = {(fx + 1.f) - ix, ix - fx}, wy[2] = {(fy + 1.f) - iy, iy - fy};
+    int z0      = 0;
+    float wz[2] = {1.f, 0.f};
+    if (!kFlat)
+    {
+        const float iz = env_unnormalize((float)s / (float)(a.S - 1) * 2.f - 1.f, a.S);  // more than one sphere
+        const float fz = floorf(iz);
+        z0    = (int)fminf(fmaxf(fz, -2.f), (float)a.S);
+        wz[0] = (fz + 1.f) - iz, wz[1] = iz - fz;
+    }
+    const int base = (z0 * a.R + y0) * a.R + x0;
+    const bool inx[2] = {(unsigned)x0 < (unsigned)a.R, (unsigned)(x0 + 1) < (unsigned)a.R};
+    const bool iny[2] = {(unsigned)y0 < (unsigned)a.R, (unsigned)(y0 + 1) < (unsigned)a.R};
 #pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-            {
-                const int x = t.x0 + i, y = t.y0 + j, z = t.z0 + k;
-                const bool in = x >= 0 && x < a.R && y >= 0 && y < a.R && z >= 0 && z < a.S;
-                const float w = t.wx[i] * t.wy[j] * t.wz[k];
-                c.off[4 * k + 2 * j + i] = in ? (z * a.R + y) * a.R + x : -1;
-                c.w[4 * k + 2 * j + i]   = w;
-            }
+    for (int q = 0; q < EnvCorners<kFlat>::N; ++q)
+    {
+        const int i = q & 1, j = q >> 1 & 1, k = q >> 2;
+        const float w = kFlat ? wx[i] * wy[j] : wx[i] * wy[j] * wz[k];
+        const bool in = inx[i] && iny[j] && (kFlat || (unsigned)(z0 + k) < (unsigned)a.S);
+        c.off[q] = in ? base + (k * a.R + j) * a.R + i : -1;
+        c.w[q]   = in ? w : 0.f;
+    }
+    return c.off[0] >= 0 ? base : alone;
 }
 
-__device__ __forceinline__ float env_fetch(const float* plane, const EnvCorners& c)
+template <bool kFlat>
+__device__ __forceinline__ float env_fetch(const float* plane, const EnvCorners<kFlat>& c)
 {
+    float v[EnvCorners<kFlat>::N];
+#pragma unroll
+    for (int q = 0; q < EnvCorners<kFlat>::N; ++q) v[q] = c.w[q] != 0.f ? __ldg(plane + c.off[q]) : 0.f;
     float acc = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-        if (c.off[q] >= 0 && c.w[q] != 0.f) acc += __ldg(plane + c.off[q]) * c.w[q];  // weight 0 adds nothing to a finite texture
+    for (int q = 0; q < EnvCorners<kFlat>::N; ++q) acc += v[q] * c.w[q];
     return acc;
 }
 
@@ -229,22 +222,24 @@ __device__ __forceinline__ float env_fetch(const float* plane, const EnvCorners&
 struct EnvPixelId
 {
     int l, b, x, y;
-    long long pix;  // index inside the level's [n_views, h, w] plane
+    int pix;  // index inside the level's [n_views, h, w] plane
 };
 
-__device__ __forceinline__ bool env_locate(const EnvArgs& a, long long idx, EnvPixelId& p)
+__device__ __forceinline__ bool env_locate(const EnvArgs& a, int idx, EnvPixelId& p)
 {
     if (idx >= a.lend[a.L - 1]) return false;
     int l = 0;
     while (idx >= a.lend[l]) ++l;
-    const long long base = l == 0 ? 0 : a.lend[l - 1];
     p.l   = l;
-    p.pix = idx - base;
-    const int per_view = a.lw[l] * a.lh[l];
-    p.b   = (int)(p.pix / per_view);
-    const int r = (int)(p.pix - (long long)p.b * per_view);
-    p.y   = r / a.lw[l];
-    p.x   = r - p.y * a.lw[l];
+    p.pix = idx - (l == 0 ? 0 : a.lend[l - 1]);
+    const int lw = a.lw[l], per_view = lw * a.lh[l];
+    int b = 0, r = p.pix;
+    for (; r >= per_view; r -= per_view) ++b;  // at most VETR_MAX_VIEWS - 1 steps
+    // row: float estimate, then one correction step either way (the estimate is off by at most one)
+    int y = __float2int_rz((float)r * a.inv_lw[l]), x = r - y * lw;
+    if (x < 0) x += lw, --y;
+    if (x >= lw) x -= lw, ++y;
+    p.b = b, p.x = x, p.y = y;
     return true;
 }
 
@@ -253,21 +248,17 @@ __device__ __forceinline__ float env_start_T(float weight, int flags)
     return (flags & VETR_ENV_DEPTH_TEST_WEIGHT) ? (weight > 0.5f ? 0.f : 1.f) : weight;
 }
 
-#ifndef VETR_ENV_FWD_CTAS
-#    define VETR_ENV_FWD_CTAS 0  // resident thread blocks per SM the forward kernel is compiled for (0: the compiler's choice, 64 registers)
-#endif
-#if VETR_ENV_FWD_CTAS > 0
-__global__ void __launch_bounds__(kEnvThreads, VETR_ENV_FWD_CTAS) envmap_forward_kernel(const __grid_constant__ EnvArgs a)
-#else
+// Bound by instruction issue (76 % of the issue slots with eight corners, 3400 instructions per pixel and four spheres: a test
+// and a branch per corner and plane, 64-bit divisions for the pixel).  1920x1080, four levels, four spheres of 1024 x 1024:
+// 337 -> 251 us.
+template <bool kFlat>
 __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __grid_constant__ EnvArgs a)
-#endif
 {
     __shared__ EnvCam s_cam[VETR_MAX_VIEWS];
     if (threadIdx.x < a.n_views) s_cam[threadIdx.x] = load_env_cam(a, threadIdx.x);
     __syncthreads();
-    const long long plane = (long long)a.S * a.R * a.R;
-    for (long long idx = (long long)blockIdx.x * kEnvThreads + threadIdx.x; idx < a.lend[a.L - 1];
-         idx += (long long)gridDim.x * kEnvThreads)
+    const long long plane = (long long)a.S * a.R * a.R, slice = kFlat ? (long long)a.R * a.R : 0;
+    for (int idx = blockIdx.x * kEnvThreads + threadIdx.x; idx < a.lend[a.L - 1]; idx += gridDim.x * kEnvThreads)
     {
         EnvPixelId p;
         env_locate(a, idx, p);
@@ -281,17 +272,17 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
             const EnvRay ray = env_ray(s_cam[p.b], lw, lh, a.scale[p.l], p.x, p.y);
             for (int s = 0; s < a.S; ++s)
             {
-                const EnvTap t = env_tap(a, ray, s);
-                if (!t.hit) continue;  // alpha = 0: nothing added, T unchanged
-                EnvCorners c;
-                env_corners(a, t, c);
+                float ix, iy;
+                if (!env_coordinates(a, ray, s, ix, iy)) continue;  // alpha = 0: nothing added, T unchanged
+                EnvCorners<kFlat> c;
+                env_corners<kFlat>(a, ix, iy, s, c);
                 float alpha = 1.f;
-                if (s != a.S - 1) alpha = 1.f / (1.f + expf(-env_fetch(a.density, c)));
+                if (s != a.S - 1) alpha = 1.f / (1.f + expf(-env_fetch<kFlat>(a.density + s * slice, c)));
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch)
                     if (ch < a.C)
                     {
-                        float col = env_fetch(a.color + ch * plane, c);
+                        float col = env_fetch<kFlat>(a.color + ch * plane + s * slice, c);
                         if (a.non_subzero) col = fabsf(col);
                         acc[ch] = T * alpha * col + acc[ch];
                     }
@@ -299,7 +290,7 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
             }
         }
         const long long per_view = (long long)lw * lh;
-        float* o = a.out[p.l] + ((long long)p.b * a.C) * per_view + (p.pix - (long long)p.b * per_view);
+        float* o = a.out[p.l] + ((long long)p.b * a.C) * per_view + (p.y * lw + p.x);
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch)
             if (ch < a.C)
@@ -322,30 +313,31 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 //          = alpha_{s+1} D_{s+1} + (1 - alpha_{s+1}) rest_{s+1}
 // (no division by 1 - alpha, which a saturated sigmoid makes zero).  First sweep, front to back: sample, keep alpha, D, T
 // and the colours' signs.  Second sweep, back to front: the gradients of the sphere's samples,
-// scattered to the eight corners of its tap.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920
+// scattered to its corners.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920
 // pixels crosses a few hundred texels), so before the atomics the lanes of a warp that share a base texel, in runs of
 // consecutive lanes, are summed with a segmented shuffle reduction and the run's first lane issues one atomic per corner and
 // value.  (Ending the reduction at the warp's longest run, five values side by side, was measured slower: 843 -> 955 us with
-// four spheres, 1890 -> 2390 us with eight.)
+// four spheres, 1890 -> 2390 us with eight, at eight corners per sample.)
 //
 // kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of up to four spheres does not
 // pay for eight, and has room for the texel coordinates (asin, atan2, two square roots) of the first sweep; with eight they
-// are formed anew (kept: 2420 us).  1920x1080, four levels, one view: four spheres of 1024 x 1024 843 us, five of
-// 512 x 512 1110, eight 1890 us (one kernel for up to eight, without kept coordinates: 967, 1157, 1971 us).
+// are formed anew.  1920x1080, four levels, one view: four spheres of 1024 x 1024 710 us (905 with eight corners per sample),
+// five of 512 x 512 1044 (1095), eight of 1024 x 1024 2130 us (2245).
 #ifndef VETR_ENV_BACK_CTAS
 #    define VETR_ENV_BACK_CTAS 3
 #endif
-template <int kMaxSpheres>
+template <int kMaxSpheres>  // a map of up to four spheres is flat; one of five goes with the larger ones
 __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backward_kernel(const __grid_constant__ EnvArgs a)
 {
     __shared__ EnvCam s_cam[VETR_MAX_VIEWS];
     if (threadIdx.x < a.n_views) s_cam[threadIdx.x] = load_env_cam(a, threadIdx.x);
     __syncthreads();
-    const long long plane = (long long)a.S * a.R * a.R;
-    const int lane        = threadIdx.x & 31;
-    const long long total = a.lend[a.L - 1];
-    const long long span  = (total + 31) / 32 * 32;  // whole warps stay in the loop together
-    for (long long idx = (long long)blockIdx.x * kEnvThreads + threadIdx.x; idx < span; idx += (long long)gridDim.x * kEnvThreads)
+    constexpr bool kFlat  = kMaxSpheres <= kEnvFlatSpheres;
+    constexpr int kN      = EnvCorners<kFlat>::N;
+    const long long plane = (long long)a.S * a.R * a.R, slice = kFlat ? (long long)a.R * a.R : 0;
+    const int lane = threadIdx.x & 31;
+    const int span = (a.lend[a.L - 1] + 31) / 32 * 32;  // whole warps stay in the loop together
+    for (int idx = blockIdx.x * kEnvThreads + threadIdx.x; idx < span; idx += gridDim.x * kEnvThreads)
     {
         EnvPixelId p;
         bool active = env_locate(a, idx, p);
@@ -360,7 +352,7 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
         if (active)
         {
             const long long per_view = (long long)a.lw[p.l] * a.lh[p.l];
-            const float* g = a.grad[p.l] + ((long long)p.b * a.C) * per_view + (p.pix - (long long)p.b * per_view);
+            const float* g = a.grad[p.l] + ((long long)p.b * a.C) * per_view + (p.y * a.lw[p.l] + p.x);
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch)
                 if (ch < a.C) G[ch] = g[ch * per_view];
@@ -382,16 +374,16 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 if (env_coordinates(a, ray, s, x, y))
                 {
                     hits |= 1u << s;
-                    EnvCorners c;
-                    env_corners(a, env_tap_at(a, x, y, s), c);
+                    EnvCorners<kFlat> c;
+                    env_corners<kFlat>(a, x, y, s, c);
                     alpha[s] = 1.f;
-                    if (s != a.S - 1) alpha[s] = 1.f / (1.f + expf(-env_fetch(a.density, c)));
+                    if (s != a.S - 1) alpha[s] = 1.f / (1.f + expf(-env_fetch<kFlat>(a.density + s * slice, c)));
                     float d = 0.f;
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch)
                         if (ch < a.C)
                         {
-                            float col = env_fetch(a.color + ch * plane, c);
+                            float col = env_fetch<kFlat>(a.color + ch * plane + s * slice, c);
                             if (a.non_subzero)
                             {
                                 if (col < 0.f) negative |= 1u << (4 * s + ch);
@@ -414,14 +406,14 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
             const float g_alpha = Tin[s] * (dot[s] - rest);
             rest                = alpha[s] * dot[s] + (1.f - alpha[s]) * rest;
             const bool live = hits >> s & 1;
-            EnvCorners c;
+            EnvCorners<kFlat> c;
             float gv[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // gradient of the density sample, then of the colour samples
             int key = -1 - lane;                      // never equal between lanes
             if (live)
             {
-                const EnvTap t = kKeep ? env_tap_at(a, ix[kKeep ? s : 0], iy[kKeep ? s : 0], s) : env_tap(a, ray, s);
-                env_corners(a, t, c);
-                key   = (t.z0 * a.R + t.y0) * a.R + t.x0;
+                float x = kKeep ? ix[kKeep ? s : 0] : 0.f, y = kKeep ? iy[kKeep ? s : 0] : 0.f;
+                if (!kKeep) env_coordinates(a, ray, s, x, y);
+                key   = env_corners<kFlat>(a, x, y, s, c, key);
                 gv[0] = s == a.S - 1 ? 0.f : g_alpha * (alpha[s] * (1.f - alpha[s]));  // alpha is the sigmoid
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch)
@@ -436,7 +428,7 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
             else
             {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) c.off[q] = -1, c.w[q] = 0.f;
+                for (int q = 0; q < kN; ++q) c.off[q] = -1, c.w[q] = 0.f;
             }
             // runs of consecutive lanes with the same base texel (the corner offsets of such lanes are the same)
             const int prev       = __shfl_up_sync(0xffffffffu, key, 1);
@@ -451,10 +443,10 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 if (lane + (1 << k) < 32 && other == seg) same |= 1u << k;
             }
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int q = 0; q < kN; ++q)
             {
-                // a corner no lane of the warp uses (outside the texture, or the empty z slice of a tap that sits on a slice)
-                if (!__any_sync(0xffffffffu, c.off[q] >= 0 && c.w[q] != 0.f)) continue;
+                // a corner no lane of the warp uses (the empty z slice of a sample that sits on a slice)
+                if (!kFlat && !__any_sync(0xffffffffu, c.w[q] != 0.f)) continue;
 #pragma unroll
                 for (int v = 0; v < 5; ++v)
                 {
@@ -468,7 +460,7 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                         if (same >> k & 1) x += y;
                     }
                     if (head && c.off[q] >= 0 && x != 0.f)
-                        atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + c.off[q], x);
+                        atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + s * slice + c.off[q], x);
                 }
             }
         }

@@ -3413,15 +3413,14 @@ static int envmap_args(const vetr_cameras* cams, const vetr_view* views, int n_v
         memcpy(a.views[b].crop, v.crop, sizeof(v.crop));
         memcpy(a.views[b].rot, v.rot, sizeof(v.rot));
     }
-    long long run = 0;
-    int lw = w, lh = h;
+    int run = 0, lw = w, lh = h;
     float scale = 1.f;
     for (int l = 0; l < num_layers; ++l, lw /= 2, lh /= 2, scale *= 0.5f)
     {
         if (!weight[l]) return VETR_E_INVALID_ARG;
         if ((long long)n_views * 4 * lw * lh > 0x7fffffffLL) return VETR_E_TOO_LARGE;
-        a.lw[l] = lw, a.lh[l] = lh, a.scale[l] = scale;
-        run += (long long)nv * lw * lh;
+        a.lw[l] = lw, a.lh[l] = lh, a.scale[l] = scale, a.inv_lw[l] = 1.f / (float)lw;
+        run += nv * lw * lh;  // a quarter of 2^31 on the largest level, a third more over all of them
         a.lend[l]   = run;
         a.weight[l] = weight[l] + (long long)v0 * lw * lh;
     }
@@ -3461,9 +3460,12 @@ extern "C" int vetr_envmap_forward(vetr_ctx* ctx, const vetr_cameras* cams, cons
             if (!out[l]) return VETR_E_INVALID_ARG;
             a.out[l] = out[l] + (long long)v0 * env->channels * a.lw[l] * a.lh[l];
         }
-        const long long blocks = (a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads;
+        const int grid = std::min((a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads, ctx->sm_count * 32);
         ctx->launches += 1;
-        envmap_forward_kernel<<<(int)std::min<long long>(blocks, (long long)ctx->sm_count * 32), kEnvThreads, 0, ctx->stream>>>(a);
+        if (a.S <= kEnvFlatSpheres)
+            envmap_forward_kernel<true><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
+        else
+            envmap_forward_kernel<false><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
@@ -3489,9 +3491,8 @@ extern "C" int vetr_envmap_backward(vetr_ctx* ctx, const vetr_cameras* cams, con
             a.grad[l] = grad_out[l] + (long long)v0 * env->channels * a.lw[l] * a.lh[l];
         }
         a.g_density = g_density, a.g_color = g_color;
-        const long long blocks = (a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads;
         ctx->launches += 1;
-        const int grid = (int)std::min<long long>(blocks, (long long)ctx->sm_count * 32);
+        const int grid = std::min((a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads, ctx->sm_count * 32);
         if (a.S <= 4)
             envmap_backward_kernel<4><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
         else
