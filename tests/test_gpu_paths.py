@@ -335,3 +335,19 @@ def test_point_backward_tiles(rasterizer, mode, tiles, w, h, views):
         np.testing.assert_array_equal(part["points"].cpu().numpy(), gpu["bwd_raw"]["points"])  # one owner per point, fixed order
     pose = rasterizer.backward_raw(on, want_intrinsics=False)["pose"].cpu().numpy()
     np.testing.assert_allclose(pose, gpu["bwd_raw"]["pose"], rtol=1e-6, atol=1e-9 * np.abs(pose).max())
+
+
+# ---- mode 2: groups of one, of a few, of the whole list, with the background (beyond a window of 1e5 every depth is in)
+
+
+@pytest.mark.parametrize("accept", [0.0, 0.003, 0.5, 9e4, 3e5])
+@pytest.mark.parametrize("n, w, h", [(6000, 96, 64), (30000, 16, 12)])
+def test_mode2_group_sizes(rasterizer, accept, n, w, h):
+    sc = scenes.tiny_scene(n=n, w=w, h=h, n_views=1, seed=17)
+    for env in (0, 1):
+        params = default_params(render_mode=2, drop_out_points_by_radius=0, num_layers=3, depth_accept_blend=accept, use_environment_map=env)
+        g = util.l1_grads(util.run_oracle(sc, params)["fwd"]["color"], seed=3)
+        ora = util.run_oracle(sc, params, grads=g)
+        gpu = util.run_gpu(rasterizer, sc, params, grads=g)
+        util.compare_forward(gpu, ora, exact_images=True)
+        util.compare_backward(gpu["bwd_raw"], ora, sc.channels)

@@ -808,6 +808,9 @@ struct FuzzyFold
     {
         if (n_acc > 0) flush();
     }
+    // Once the first group is closed, every later fragment is a group of its own (depths are positive, so none lies within
+    // `accept` of -100000 unless `accept` is larger than that): what follows is the plain fold, without the averages.
+    __device__ __forceinline__ bool plain_from_here(float accept) const { return last_min_d == -100000.f && accept <= 100000.f; }
 };
 
 // ---------------------------------------------------------------------------------------------------------
@@ -889,27 +892,25 @@ __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const 
             int cnt = se - ss;
             if (f.dbg_max_len > 0) cnt = min(cnt, f.dbg_max_len);
             Fold fold;
+            fold.init();
+            int r = ss;
             if (f.mode == VETR_MODE_FUZZY_BLEND)
             {
                 FuzzyFold ff;
                 ff.init();
-                for (int r = ss; r < ss + cnt; ++r)
+                while (r < ss + cnt && !ff.plain_from_here(f.accept_blend))
                 {
-                    const int u = s.perm[r];
+                    const int u = s.perm[r++];
                     ff.add(__uint_as_float((unsigned)(s.key[u] >> 32)), s.alpha[u], s.desc[u], f.accept_blend);
                 }
                 ff.finish();
                 fold = ff.fold;
             }
-            else
+            for (; r < ss + cnt; ++r)
             {
-                fold.init();
-                for (int r = ss; r < ss + cnt; ++r)
-                {
-                    const int u = s.perm[r];
-                    fold.add(s.alpha[u], s.desc[u]);
-                    if (bilinear && fold.T < 0.001f) break;
-                }
+                const int u = s.perm[r];
+                fold.add(s.alpha[u], s.desc[u]);
+                if (bilinear && fold.T < 0.001f) break;
             }
             fold.background(f, bg);
             float depth = se > ss ? __uint_as_float((unsigned)(s.key[s.perm[ss]] >> 32)) : kMaxDepth;
@@ -1028,9 +1029,9 @@ __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __g
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LongBlendSmem& s = *reinterpret_cast<LongBlendSmem*>(smem_raw);
-    __shared__ FuzzyFold s_fuzzy;  // carried between blocks (mode 2)
+    __shared__ FuzzyFold s_fuzzy;  // carried between blocks (mode 2, until its first group is closed)
     __shared__ float s_T, s_color[4];
-    __shared__ int s_used, s_stop;
+    __shared__ int s_used, s_stop, s_grouped;
     const int tid       = threadIdx.x;
     const int n_items   = f.status[3];
     const bool bilinear = f.mode == VETR_MODE_BILINEAR_BLEND, fuzzy = f.mode == VETR_MODE_FUZZY_BLEND;
@@ -1051,8 +1052,9 @@ __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __g
         if (tid == 0)
         {
             s_fuzzy.init();
-            s_T    = 1.f;
-            s_stop = 0;
+            s_T       = 1.f;
+            s_stop    = 0;
+            s_grouped = fuzzy;
         }
         if (tid < 4) s_color[tid] = 0.f;
         __syncthreads();
@@ -1069,18 +1071,39 @@ __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __g
             }
             if (m + tid < ((m + 3) & ~3)) s.fold.alpha[m + tid] = 0.f;
             __syncthreads();
-            if (fuzzy)
+            bool chain = true;
+            if (s_grouped)
             {
+                // mode 2: one thread forms the first group; what it took is left behind as fragments that change nothing
+                __syncthreads();  // all threads have read s_grouped
                 if (tid == 0)
                 {
                     FuzzyFold ff = s_fuzzy;
-                    for (int i = 0; i < m; ++i)
+                    int i        = 0;
+                    while (i < m && !ff.plain_from_here(f.accept_blend))
+                    {
                         ff.add(s.fold.depth[i], s.fold.alpha[i],
                                make_float4(s.fold.desc[0][i], s.fold.desc[1][i], s.fold.desc[2][i], s.fold.desc[3][i]), f.accept_blend);
+                        ++i;
+                    }
+                    if (ff.plain_from_here(f.accept_blend))
+                    {
+                        ff.finish();
+                        s_T = ff.fold.T;
+                        for (int k = 0; k < 4; ++k) s_color[k] = ff.fold.c[k];
+                        s_grouped = 0;
+                    }
                     s_fuzzy = ff;
+                    s_used  = i;
                 }
+                __syncthreads();
+                const int taken = s_used;
+                chain           = !s_grouped;
+                for (int i = tid; chain && i < taken; i += kLongThreads)
+                    s.fold.alpha[i] = s.fold.desc[0][i] = s.fold.desc[1][i] = s.fold.desc[2][i] = s.fold.desc[3][i] = 0.f;
+                __syncthreads();
             }
-            else
+            if (chain)
             {
                 if (tid == 0)
                 {
@@ -1113,7 +1136,7 @@ __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __g
         if (tid == 0)
         {
             Fold fold;
-            if (fuzzy)
+            if (s_grouped)
             {
                 FuzzyFold ff = s_fuzzy;
                 ff.finish();
@@ -1153,7 +1176,7 @@ struct BackSmem
     int pid[kCap];
     int tex[kCap];
     float alpha[kCap];
-    float dot[kCap];     // d_i . G (mode 2: replaced by the confidence gradient)
+    float dot[kCap];     // d_i . G (mode 2: replaced by the gradient of the group's confidence)
     float trans[kCap];   // T_i ; NaN = fragment not blended (early termination / list truncation)
     float4 grad[kMaxPixels];  // incoming gradient of the pixel
     int seg_end[kMaxPixels + 1];
@@ -1176,13 +1199,10 @@ __device__ __forceinline__ float* suffix_of(BackSmem& s)
         return reinterpret_cast<float*>(s.pid);
 }
 
-// Mode 2 additionally needs every fragment's descriptor and depth (groups average them) and two group markers.
+// Mode 2 additionally needs every fragment's depth; the suffix sums take the memory of the point indices as in mode 1.
 struct BackSmemFuzzy : BackSmem
 {
-    float4 desc[kCap];
     float depth[kCap];
-    float gv[kCap];               // at the first fragment of a group: sum_c G_c * colour_c * T * conf of that group
-    unsigned char gfirst[kCap];   // 1 = first fragment of its group
 };
 
 // Gradient accumulation with fire-and-forget reductions.  The gradient buffers are never read by these kernels, so
@@ -1441,12 +1461,11 @@ constexpr int kNoGradientBits = 0x7fffffff;
 // coalesced position loads and without atomics, instead of a position gather per fragment here.
 template <bool kBilinear>
 __device__ __forceinline__ void fragment_stage_a(const Frame& f, BackSmem& s, int g, const PixInfo& px, float4 G, int slot,
-                                                 uint4 h, uint4 payload, bool blended, float4* desc_out = nullptr,
-                                                 float* depth_out = nullptr)
+                                                 uint4 h, uint4 payload, bool blended, float* depth_out = nullptr)
 {
     const float4 d = as_float4(payload);
     const int pid  = (int)h.x;
-    if (desc_out) desc_out[slot] = d, depth_out[slot] = __uint_as_float(h.y);
+    if (depth_out) depth_out[slot] = __uint_as_float(h.y);
     s.pid[slot]    = pid;
     s.tex[slot]    = (int)h.w;
     s.alpha[slot]  = __uint_as_float(h.z);
@@ -1563,85 +1582,131 @@ __device__ __forceinline__ float alpha_gradient(float T, float a, float dot, flo
 // first depth of every group, the background is an entry of depth 100000 (confidence 1, colour = background), a
 // group's descriptor / confidence gradients are shared equally by its fragments, and the term a later group passes to
 // the confidence of an earlier fragment uses that fragment's GROUP confidence and is not divided by the group size.
-// Leaves the factor of G of the descriptor gradient in trans[] (NaN = not blended) and the confidence gradient in dot[].
-__device__ __forceinline__ void sweep_list_fuzzy(const Frame& f, float* alpha, float* dot, float* trans, const float4* desc,
-                                                 const float* depth, float* gv, unsigned char* gfirst, int ss, int se,
-                                                 float4 G, float4 bgc, float bg_acc[4])
+//
+// Three steps, with a barrier between them: fuzzy_groups (one thread per list) cuts the list into groups and runs the chain of
+// transmittances, fuzzy_group_terms (a thread per fragment) forms what hangs on a group's mean colour, fuzzy_suffix (one
+// thread per list) sums from the back; fuzzy_alpha_gradient puts a fragment's confidence gradient together.  Bound by the latency
+// of the two chains, which are down to a comparison and a multiplication, and an addition, per fragment; four groups of one
+// fragment each go through a step together.  1 M points, 801x603, one view: backward_kernel 295 -> 169 us, lists of more than 256
+// fragments 105 -> 61 us (before: everything in the list's own thread, descriptors in shared memory, half as many CTAs per SM).
+//
+// fuzzy_groups: n fragments of one list.  Leaves the transmittance in front of its group in trans[] (NaN = not blended), the
+// group's confidence in alpha[], and in group[], which takes the memory of depth[], its number of members at the first of
+// them (negative if the background belongs to the group too; it is not counted) and 0 at the others.  Returns the suffix sum
+// behind the last fragment.
+__device__ __forceinline__ float fuzzy_groups(const Frame& f, float* alpha, float* trans, float* depth, int n, float4 G, float4 bgc,
+                                              float bg_acc[4])
 {
-    int cnt = se - ss;
+    int* group = reinterpret_cast<int*>(depth);
+    int cnt    = n;
     if (f.dbg_max_len > 0) cnt = min(cnt, f.dbg_max_len);
-    for (int i = ss + cnt; i < se; ++i) trans[i] = __int_as_float(0x7fffffff);
-    const int list_size = f.use_env ? cnt : cnt + 1;
-    float last_min_d = 0.f, acc_conf = 0.f, T = 1.f, S_tail = 0.f;
-    float4 acc_desc = make_float4(0.f, 0.f, 0.f, 0.f);
-    int n_acc = 0, start = 0;
-    auto close_group = [&]()
+    const float accept = f.accept_blend;
+    bool background    = !f.use_env;  // still to come
+    float T            = 1.f;
+    int i              = 0;
+    while (i < cnt)
     {
-        const float inv_w = n_acc == 1 ? 1.f : 1.f / (float)n_acc;  // every group but a few is a single fragment
-        const float conf  = acc_conf * inv_w;
-        const float4 col  = make_float4(acc_desc.x * inv_w, acc_desc.y * inv_w, acc_desc.z * inv_w, acc_desc.w * inv_w);
-        const float g_alpha = dot4(col, G, f.C) * T;
-        float v = 0.f;
-        v += G.x * col.x * T * conf;
-        v += G.y * col.y * T * conf;
-        v += G.z * col.z * T * conf;
-        if (f.C > 3) v += G.w * col.w * T * conf;
-        for (int t = start; t < start + n_acc; ++t)
+        const float d0 = depth[i];
+        if (i > 0 && i + 4 < cnt)
         {
-            if (t < cnt)
+            const float d1 = depth[i + 1], d2 = depth[i + 2], d3 = depth[i + 3], d4 = depth[i + 4];
+            if (!(d1 - d0 < accept) && !(d2 - d1 < accept) && !(d3 - d2 < accept) && !(d4 - d3 < accept))
             {
-                trans[ss + t]  = T * conf * inv_w;
-                dot[ss + t]    = g_alpha * inv_w;
-                alpha[ss + t]  = conf;  // the group's confidence, used below for earlier fragments
-                gfirst[ss + t] = t == start;
-                gv[ss + t]     = v;
-            }
-            else
-            {
-                bg_acc[0] += T * conf * G.x * inv_w, bg_acc[1] += T * conf * G.y * inv_w, bg_acc[2] += T * conf * G.z * inv_w;
-                if (f.C > 3) bg_acc[3] += T * conf * G.w * inv_w;
+                const float t1 = vetr_new_T(T, alpha[i]), t2 = vetr_new_T(t1, alpha[i + 1]), t3 = vetr_new_T(t2, alpha[i + 2]);
+                trans[i] = T, trans[i + 1] = t1, trans[i + 2] = t2, trans[i + 3] = t3;
+                T        = vetr_new_T(t3, alpha[i + 3]);
+                group[i] = group[i + 1] = group[i + 2] = group[i + 3] = 1;
+                i += 4;
+                continue;
             }
         }
-        if (start >= cnt) S_tail = v;  // the group consists of the background entry alone
+        // one group: fragments within `accept` of its first depth (the first group of a list may also be measured from 0)
+        const float ref = i == 0 && d0 < accept ? 0.f : d0;
+        float conf      = alpha[i];
+        int j           = i + 1;
+        for (; j < cnt && depth[j] - ref < accept; ++j) conf += alpha[j];
+        const bool joined = background && j == cnt && kMaxDepth - ref < accept;
+        const int members = j - i;
+        float inv_w       = 1.f;
+        if (joined) conf += 1.f;
+        if (members + joined > 1) inv_w = 1.f / (float)(members + joined), conf *= inv_w;
+        for (int t = i; t < j; ++t) trans[t] = T, alpha[t] = conf, group[t] = 0;
+        group[i] = joined ? -members : members;
+        if (joined)
+        {
+            bg_acc[0] += T * conf * G.x * inv_w, bg_acc[1] += T * conf * G.y * inv_w, bg_acc[2] += T * conf * G.z * inv_w;
+            if (f.C > 3) bg_acc[3] += T * conf * G.w * inv_w;
+            background = false;
+        }
         T = vetr_new_T(T, conf);
-    };
-    for (int i = 0; i < list_size; ++i)
+        i = j;
+    }
+    for (i = cnt; i < n; ++i) trans[i] = __int_as_float(0x7fffffff), group[i] = 0;
+    if (!background) return 0.f;
+    bg_acc[0] += T * G.x, bg_acc[1] += T * G.y, bg_acc[2] += T * G.z;
+    if (f.C > 3) bg_acc[3] += T * G.w;
+    float v = G.x * bgc.x * T + G.y * bgc.y * T + G.z * bgc.z * T;
+    if (f.C > 3) v += G.w * bgc.w * T;
+    return v;
+}
+
+// The thread of a group's first fragment i, for all members: the factor of G of the descriptor gradient in trans[], the group's
+// own part of the confidence gradient in dot[] (d . G on entry), and in suffix[] what the group passes to the ones before it
+// (the other members hold a zero).  The mean colour of several members is summed in list order.  recs: the list's records.
+__device__ __forceinline__ void fuzzy_group_terms(const Frame& f, const float* alpha, float* dot, float* trans, float* suffix,
+                                                  int group, const uint4* recs, int i, float4 G, float4 bgc)
+{
+    const int members = abs(group);
+    const float T = trans[i], conf = alpha[i];
+    float4 col    = as_float4(recs[2 * i + 1]);
+    float inv_w = 1.f, q = dot[i];
+    if (group != 1)
     {
-        const bool fg = i != cnt;
-        const float d = fg ? depth[ss + i] : kMaxDepth;
-        if (!(d - last_min_d < f.accept_blend))
+        for (int t = 1; t < members; ++t)
         {
-            if (i != 0) close_group();
-            acc_conf = 0.f, n_acc = 0, acc_desc = make_float4(0.f, 0.f, 0.f, 0.f);
-            last_min_d = d;
-            start      = i;
+            const float4 d = as_float4(recs[2 * (i + t) + 1]);
+            col.x += d.x, col.y += d.y, col.z += d.z, col.w += d.w;
         }
-        const float4 c = fg ? desc[ss + i] : bgc;
-        acc_conf += fg ? alpha[ss + i] : 1.f;
-        acc_desc.x += c.x, acc_desc.y += c.y, acc_desc.z += c.z, acc_desc.w += c.w;
-        ++n_acc;
+        if (group < 0) col.x += bgc.x, col.y += bgc.y, col.z += bgc.z, col.w += bgc.w;
+        inv_w = 1.f / (float)(members + (group < 0));
+        col.x *= inv_w, col.y *= inv_w, col.z *= inv_w, col.w *= inv_w;
+        q = dot4(col, G, f.C);
     }
-    if (n_acc > 0) close_group();
-    float S = S_tail;  // sum of v over the groups after the current one
-    int t = cnt;
-    for (; t >= 4; t -= 4)  // operands of four steps requested together
+    const float g_alpha = q * T;
+    float v = 0.f;
+    v += G.x * col.x * T * conf;
+    v += G.y * col.y * T * conf;
+    v += G.z * col.z * T * conf;
+    if (f.C > 3) v += G.w * col.w * T * conf;
+    for (int t = i; t < i + members; ++t)
     {
-        const int q = ss + t - 4;
-        const float a0 = alpha[q], a1 = alpha[q + 1], a2 = alpha[q + 2], a3 = alpha[q + 3];
-        const float d0 = dot[q], d1 = dot[q + 1], d2 = dot[q + 2], d3 = dot[q + 3];
-        const float S2 = gfirst[q + 3] ? S + gv[q + 3] : S, S1 = gfirst[q + 2] ? S2 + gv[q + 2] : S2;
-        const float S0 = gfirst[q + 1] ? S1 + gv[q + 1] : S1;
-        dot[q + 3] = d3 - S / (1 - a3 + 1e-9f), dot[q + 2] = d2 - S2 / (1 - a2 + 1e-9f);
-        dot[q + 1] = d1 - S1 / (1 - a1 + 1e-9f), dot[q] = d0 - S0 / (1 - a0 + 1e-9f);
-        S = gfirst[q] ? S0 + gv[q] : S0;
-    }
-    for (; t > 0; --t)
-    {
-        const int q = ss + t - 1;
-        dot[q] -= S / (1 - alpha[q] + 1e-9f);
-        if (gfirst[q]) S += gv[q];
+        trans[t]  = T * conf * inv_w;
+        dot[t]    = g_alpha * inv_w;
+        suffix[t] = t == i ? v : 0.f;
     }
 }
+
+// Sums what the groups behind a fragment's group pass to it; S: what comes from behind the list.
+__device__ __forceinline__ void fuzzy_suffix(const Frame& f, float* suffix, int n, float S)
+{
+    int i = n;
+    if (f.dbg_max_len > 0) i = min(i, f.dbg_max_len);
+    for (; i >= 4; i -= 4)
+    {
+        const float v3 = suffix[i - 1], v2 = suffix[i - 2], v1 = suffix[i - 3], v0 = suffix[i - 4];
+        const float S2 = S + v3, S1 = S2 + v2, S0 = S1 + v1;
+        suffix[i - 1] = S, suffix[i - 2] = S2, suffix[i - 3] = S1, suffix[i - 4] = S0;
+        S = S0 + v0;
+    }
+    for (; i > 0; --i)
+    {
+        const float v = suffix[i - 1];
+        suffix[i - 1] = S;
+        S += v;
+    }
+}
+
+__device__ __forceinline__ float fuzzy_alpha_gradient(float conf, float dot, float suffix) { return dot - suffix / (1 - conf + 1e-9f); }
 
 // Background gradient and the confidence term the reference routes to descriptor 0: CTA reduction, one atomic each.
 __device__ __forceinline__ void reduce_background(const Frame& f, const BackPtrs& bp, BackSmem& s, const float bg_acc[4],
@@ -1692,8 +1757,8 @@ struct BackSmemOf<false, true>
 
 // Position / camera gradients are left to point_backward_kernel in every mode.
 template <bool kFuzzy, bool kBilinear>
-__global__ void __launch_bounds__(kThreads, kFuzzy ? 1 : kBackCtas) backward_kernel(const __grid_constant__ Frame f,
-                                                                                   const __grid_constant__ BackPtrs bp)
+__global__ void __launch_bounds__(kThreads, kBackCtas) backward_kernel(const __grid_constant__ Frame f,
+                                                                       const __grid_constant__ BackPtrs bp)
 {
     static_assert(!(kFuzzy && kBilinear), "mode 2 and mode 3 exclude each other");
     using Smem = typename BackSmemOf<kFuzzy, kBilinear>::type;
@@ -1735,33 +1800,42 @@ __global__ void __launch_bounds__(kThreads, kFuzzy ? 1 : kBackCtas) backward_ker
                 const int a = seg_lookup(s.seg, parity, s.seg_end, i);
                 const bool blended = f.dbg_max_len <= 0 || i - s.seg_end[a] < f.dbg_max_len;  // list truncation
                 if constexpr (kFuzzy)
-                    fragment_stage_a<false>(f, s, lo + a, s.pix[a], s.grad[a], i, h, d, blended, s.desc, s.depth);
+                    fragment_stage_a<false>(f, s, lo + a, s.pix[a], s.grad[a], i, h, d, blended, s.depth);
                 else
                     fragment_stage_a<kBilinear>(f, s, lo + a, s.pix[a], s.grad[a], i, h, d, blended);
             }
             __syncthreads();
+            [[maybe_unused]] float S_behind = 0.f;
             if (tid < np && s.pix[tid].valid)
             {
                 if constexpr (kFuzzy)
-                    sweep_list_fuzzy(f, s.alpha, s.dot, s.trans, s.desc, s.depth, s.gv, s.gfirst, s.seg_end[tid], s.seg_end[tid + 1],
-                                     s.grad[tid], bgc, bg_acc);
+                {
+                    const int ss = s.seg_end[tid];
+                    S_behind     = fuzzy_groups(f, s.alpha + ss, s.trans + ss, s.depth + ss, s.seg_end[tid + 1] - ss, s.grad[tid], bgc, bg_acc);
+                }
                 else
                     sweep_list<kBilinear>(f, s, s.seg_end[tid], s.seg_end[tid + 1], s.grad[tid], bgc, bg_acc, p0_acc);
             }
             __syncthreads();
+            if constexpr (kFuzzy)
+            {
+                for (int i = tid; i < nf; i += kThreads)
+                    if (const int group = __float_as_int(s.depth[i]))
+                        fuzzy_group_terms(f, s.alpha, s.dot, s.trans, suffix_of<false>(s), group, f.recs + 2 * (size_t)f0, i,
+                                          s.grad[seg_lookup(s.seg, parity, s.seg_end, i)], bgc);
+                __syncthreads();
+                if (tid < np) fuzzy_suffix(f, suffix_of<false>(s) + s.seg_end[tid], s.seg_end[tid + 1] - s.seg_end[tid], S_behind);
+                __syncthreads();
+            }
             for (int i = tid; i < nf; i += kThreads)
             {
                 const float Ti     = s.trans[i];
                 const bool blended = Ti == Ti;  // NaN: the list ended before this fragment
                 if (!kBilinear && !blended) continue;
                 const int a = seg_lookup(s.seg, parity, s.seg_end, i);
-                float Ta = Ti, galpha = s.dot[i];  // mode 2 left both behind
-                if constexpr (!kFuzzy)
-                {
-                    const float al = s.alpha[i];
-                    galpha = alpha_gradient(Ti, al, galpha, suffix_of<kBilinear>(s)[i]);
-                    Ta     = Ti * al;
-                }
+                const float al = s.alpha[i], suffix = suffix_of<kBilinear>(s)[i];
+                const float galpha = kFuzzy ? fuzzy_alpha_gradient(al, s.dot[i], suffix) : alpha_gradient(Ti, al, s.dot[i], suffix);
+                const float Ta     = kFuzzy ? Ti : Ti * al;
                 fragment_stage_b<kBilinear>(f, bp, s.pix[a], s.grad[a], kBilinear ? s.pid[i] : 0, s.tex[i], Ta, galpha, blended);
             }
         }
@@ -1908,14 +1982,12 @@ constexpr int kFuzzyMidMax  = 1024;
 template <int kMax>
 struct FuzzyLongSmem
 {
-    float4 desc[kMax];
     int tex[kMax];
     float alpha[kMax];
     float dot[kMax];
     float trans[kMax];
     float depth[kMax];
-    float gv[kMax];
-    unsigned char gfirst[kMax];
+    float suffix[kMax];
 };
 
 // Lists of more than kMin and up to kMax fragments.
@@ -1951,7 +2023,7 @@ __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __g
             const uint4 h  = f.recs[2 * (size_t)(e0 + i)];
             const float4 d = as_float4(f.recs[2 * (size_t)(e0 + i) + 1]);
             s.tex[i] = (int)h.w, s.alpha[i] = __uint_as_float(h.z), s.depth[i] = __uint_as_float(h.y);
-            s.desc[i] = d;
+            s.dot[i] = dot4(d, G, f.C);
             const bool blended = f.dbg_max_len <= 0 || i < f.dbg_max_len;
             if (f.need_point_grad)
                 f.point_grad[((size_t)px.view * f.L + px.level) * f.n + (int)h.x] =
@@ -1959,14 +2031,21 @@ __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __g
                                        : make_float2(__int_as_float(kNoGradientBits), 0.f);
         }
         __syncthreads();
-        if (tid == 0) sweep_list_fuzzy(f, s.alpha, s.dot, s.trans, s.desc, s.depth, s.gv, s.gfirst, 0, n, G, bgc, bg_acc);
+        float S_behind = 0.f;
+        if (tid == 0) S_behind = fuzzy_groups(f, s.alpha, s.trans, s.depth, n, G, bgc, bg_acc);
+        __syncthreads();
+        for (int i = tid; i < n; i += kThreads)
+            if (const int group = __float_as_int(s.depth[i]))
+                fuzzy_group_terms(f, s.alpha, s.dot, s.trans, s.suffix, group, f.recs + 2 * (size_t)e0, i, G, bgc);
+        __syncthreads();
+        if (tid == 0) fuzzy_suffix(f, s.suffix, n, S_behind);
         __syncthreads();
         for (int i = tid; i < n; i += kThreads)
         {
             const float coef = s.trans[i];
             if (coef != coef) continue;
             red_add_v4(bp.g_desc + s.tex[i], make_float4(coef * G.x, coef * G.y, coef * G.z, f.C > 3 ? coef * G.w : 0.f));
-            red_add(bp.g_conf + s.tex[i], s.dot[i]);
+            red_add(bp.g_conf + s.tex[i], fuzzy_alpha_gradient(s.alpha[i], s.dot[i], s.suffix[i]));
         }
     }
     if (tid == 0)
