@@ -63,3 +63,24 @@ def test_gpu_rejects_indices_outside_the_cloud():
             rast.remove_points(100, torch.tensor(bad, dtype=torch.int64, device="cuda"))
         assert ei.value.status == _lib.E_INVALID_ARG
     rast.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 255, 1023, 1025, 70_001])
+def test_gpu_many_arrays_of_all_widths(n):
+    """More arrays than one launch moves, widths of one to six words, blocks that the points do not fill."""
+    from vet_b200.render import Rasterizer
+
+    rng = np.random.default_rng(n)
+    remove = rng.integers(0, n, size=n // 3).astype(np.int64)
+    keep = np.setdiff1d(np.arange(n), remove)
+    last = [rng.standard_normal((rows, n)).astype(np.float32) for rows in (1, 2, 5) * 4]
+    first = [rng.standard_normal((n, width)).astype(np.float32) for width in (1, 2, 3, 4, 5, 6) * 2]
+    rast = Rasterizer(0)
+    t = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    _, got_last, got_first = rast.remove_points(n, t(remove), [t(a) for a in last], [t(a) for a in first])
+    for g, a in zip(got_last, last):
+        assert np.array_equal(g.cpu().numpy(), a[:, keep])
+    for g, a in zip(got_first, first):
+        assert np.array_equal(g.cpu().numpy(), a[keep])
+    rast.close()

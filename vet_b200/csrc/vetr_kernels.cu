@@ -3771,13 +3771,24 @@ extern "C" int vetr_gather_points(vetr_ctx* ctx, int n, int n_kept, const int32_
     }
     if (n == 0 || n_kept == 0) return VETR_OK;
     VETR_CUDA(ctx, cudaSetDevice(ctx->device));
+    GatherArgs g;
+    memset(&g, 0, sizeof(g));
+    g.new_index = new_index, g.n = n, g.n_kept = n_kept;
+    long long rows = 0;
     for (int k = 0; k < n_arrays; ++k)
     {
         const vetr_point_array& a = arrays[k];
-        const long long total = (long long)a.rows * n;
-        const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)ctx->sm_count * 16);
-        points_gather_kernel<<<blocks, 256, 0, ctx->stream>>>((const uint32_t*)a.src, (uint32_t*)a.dst, new_index, n, n_kept, a.rows, a.width);
+        rows += a.rows;
+        g.src[g.arrays] = (const uint32_t*)a.src, g.dst[g.arrays] = (uint32_t*)a.dst;
+        g.row_end[g.arrays] = (int)rows, g.width[g.arrays] = a.width;
+        ++g.arrays;
+        // a launch when the table is full, at the end, and where one more array would leave the row counter's range
+        if (g.arrays < kGatherArrays && k + 1 < n_arrays && rows + arrays[k + 1].rows <= 0x7fffffff) continue;
+        const int blocks = (int)((n + 256ll * kGatherPoints - 1) / (256 * kGatherPoints));
+        const int share  = std::max(1, ctx->sm_count * 16 / blocks);  // sixteen blocks per SM
+        points_gather_kernel<<<dim3(blocks, (unsigned)std::min<long long>(std::min(share, 65535), rows)), 256, 0, ctx->stream>>>(g);
         ctx->launches += 1;
+        g.arrays = 0, rows = 0;
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
