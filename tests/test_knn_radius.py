@@ -141,3 +141,17 @@ def test_gpu_full_size_properties():
     d2 = ((xyz[sub, None, :] - xyz[None, :, :]) ** 2)
     d2 = (d2[..., 0] + d2[..., 1]) + d2[..., 2]
     assert np.array_equal(a[sub], np.sqrt(np.partition(d2, 4, axis=1)[:, 4]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_gpu_dense_sheet_and_outliers(axis):
+    """Rows of the grid with hundreds of candidates (a sheet along or across them) in the cubes of isolated points, cells of many points
+    whose neighbours are passed over, points on the faces of cells."""
+    rng = np.random.default_rng(axis)
+    sheet = rng.uniform(-1, 1, size=(12000, 3)).astype(np.float32)
+    sheet[:, axis] = rng.normal(0, 1e-3, size=12000)
+    sheet[:2000] = np.round(sheet[:2000] * 32) / 32
+    xyz = np.concatenate([sheet, rng.uniform(-1, 1, size=(300, 3)).astype(np.float32) * np.float32(1.5)])
+    for k in (1, 4, 8, 16):
+        assert np.array_equal(_gpu(xyz, k), O.knn_radius(xyz, k)), k

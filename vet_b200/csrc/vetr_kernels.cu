@@ -2815,13 +2815,12 @@ struct vetr_ctx
     double* grid_prefix[32] = {};
     int grid_prefix_n         = 0;
     long long grid_prefix_cap = 0;
-    // scratch of vetr_knn_radius, grown on demand: per point (sorted copy, cell, queue) and per cell (starts, ends)
+    // scratch of vetr_knn_radius, grown on demand: per point (sorted copy, cell, queue) and per cell (first slot)
     float4* knn_sorted   = nullptr;
     int* knn_point_cell  = nullptr;
     int* knn_queue       = nullptr;
     long long knn_cap_points = 0;
-    int* knn_starts      = nullptr;
-    int* knn_ends        = nullptr;
+    int* knn_cells       = nullptr;
     long long knn_cap_cells = 0;
     int* knn_tile_sums   = nullptr;  // 16384 tile sums, then 16 words: bounds[6], occupied (64 bit), queue count, 2 of the point removal
     int* points_flags    = nullptr;  // keep flags of vetr_remove_points_plan
@@ -3000,7 +2999,7 @@ extern "C" void vetr_destroy(vetr_ctx* ctx)
     if (ctx->grid_queue) cudaFree(ctx->grid_queue);
     for (int i = 0; i < ctx->grid_prefix_n; ++i) cudaFree(ctx->grid_prefix[i]);
     cudaFree(ctx->knn_sorted), cudaFree(ctx->knn_point_cell), cudaFree(ctx->knn_queue);
-    cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends), cudaFree(ctx->knn_tile_sums), cudaFree(ctx->points_flags);
+    cudaFree(ctx->knn_cells), cudaFree(ctx->knn_tile_sums), cudaFree(ctx->points_flags);
     for (int i = 0; i < VETR_T_N; ++i)
         for (int k = 0; k < 2; ++k)
             if (ctx->ev[i][k]) cudaEventDestroy(ctx->ev[i][k]);
@@ -3644,7 +3643,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     float cell = ext > 0.f ? ext / 32.f : 1.f;
     int d[3];
     long long cells = dims_for(cell, d);
-    bool counted = false;  // knn_starts and knn_point_cell hold the counts and cells of the current cell size
+    bool counted = false;  // knn_cells and knn_point_cell hold the counts and cells of the current cell size
     for (int iter = 0; iter < 24 && ext > 0.f; ++iter)
     {
         int d2[3];
@@ -3658,18 +3657,17 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         }
         if (cells > ctx->knn_cap_cells)
         {
-            cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends);
-            ctx->knn_starts = nullptr, ctx->knn_ends = nullptr, ctx->knn_cap_cells = 0;
+            cudaFree(ctx->knn_cells);
+            ctx->knn_cells = nullptr, ctx->knn_cap_cells = 0;
             const long long cap = std::min(kKnnMaxCells, std::max(cells * 8, 1ll << 20));
-            VETR_CUDA(ctx, cudaMalloc(&ctx->knn_starts, (size_t)cap * sizeof(int)));
-            VETR_CUDA(ctx, cudaMalloc(&ctx->knn_ends, (size_t)cap * sizeof(int)));
+            VETR_CUDA(ctx, cudaMalloc(&ctx->knn_cells, (size_t)(cap + kKnnCellsPad) * sizeof(int)));
             ctx->knn_cap_cells = cap;
         }
         g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_starts, 0, (size_t)cells * sizeof(int), st));
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
         VETR_CUDA(ctx, cudaMemsetAsync(d_occ, 0, sizeof(unsigned long long), st));
-        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, ctx->knn_point_cell);
-        knn_occupied_kernel<<<(int)std::min<long long>((cells + 255) / 256, ctx->sm_count * 16), 256, 0, st>>>(ctx->knn_starts, cells, d_occ);
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
+        knn_occupied_kernel<<<(int)std::min<long long>((cells + 255) / 256, ctx->sm_count * 16), 256, 0, st>>>(ctx->knn_cells + kKnnCellsPad, cells, d_occ);
         unsigned long long occupied = 0;
         VETR_CUDA(ctx, cudaMemcpyAsync(&occupied, d_occ, sizeof(occupied), cudaMemcpyDeviceToHost, st));
         VETR_CUDA(ctx, cudaStreamSynchronize(st));
@@ -3683,33 +3681,33 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     }
     if (cells > ctx->knn_cap_cells)  // all points coincide: no iteration ran
     {
-        cudaFree(ctx->knn_starts), cudaFree(ctx->knn_ends);
-        ctx->knn_starts = nullptr, ctx->knn_ends = nullptr, ctx->knn_cap_cells = 0;
+        cudaFree(ctx->knn_cells);
+        ctx->knn_cells = nullptr, ctx->knn_cap_cells = 0;
         const long long cap = std::max(cells, 1ll << 20);
-        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_starts, (size_t)cap * sizeof(int)));
-        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_ends, (size_t)cap * sizeof(int)));
+        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_cells, (size_t)(cap + kKnnCellsPad) * sizeof(int)));
         ctx->knn_cap_cells = cap;
     }
     g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
 
     // counting sort into the chosen grid
     const int n_tiles = (int)((cells + kKnnScanTile - 1) / kKnnScanTile);
+    // the scatter advances every cell's first slot to the next cell's: one entry further down they are first slots again
+    int* const cursor = ctx->knn_cells + kKnnCellsPad;
     VETR_CUDA(ctx, cudaMemsetAsync(d_queue_count, 0, sizeof(int), st));
     if (!counted)
     {
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_starts, 0, (size_t)cells * sizeof(int), st));
-        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_starts, ctx->knn_point_cell);
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
         ctx->launches += 1;
     }
-    knn_tile_sums_kernel<<<n_tiles, 256, 0, st>>>(ctx->knn_starts, cells, ctx->knn_tile_sums);
+    knn_tile_sums_kernel<<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums);
     knn_spine_kernel<<<1, 1024, 0, st>>>(ctx->knn_tile_sums, n_tiles);
-    knn_apply_kernel<<<n_tiles, 256, 0, st>>>(ctx->knn_starts, cells, ctx->knn_tile_sums, ctx->knn_starts);
-    VETR_CUDA(ctx, cudaMemcpyAsync(ctx->knn_ends, ctx->knn_starts, (size_t)cells * sizeof(int), cudaMemcpyDeviceToDevice, st));
-    knn_scatter_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, ctx->knn_ends, ctx->knn_sorted);
+    knn_apply_kernel<<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums, cursor);
+    knn_scatter_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, cursor, ctx->knn_sorted);
 
     // search
     KnnSearch a;
-    a.g = g, a.sorted = ctx->knn_sorted, a.starts = ctx->knn_starts, a.ends = ctx->knn_ends, a.n = n;
+    a.g = g, a.sorted = ctx->knn_sorted, a.first = cursor - 1, a.n = n;
     const int k1 = std::min(k, n - 1) + 1;  // list entries that count: the point itself and its k nearest
     a.slack = 1e-3f * cell + 4e-6f * (maxabs + ext);
     a.radius = radius, a.radius_stride = radius_stride, a.queue = ctx->knn_queue, a.queue_count = d_queue_count;

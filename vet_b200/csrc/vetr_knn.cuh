@@ -4,7 +4,7 @@
 // the cells around its own in growing cubes until the k-th nearest distance found so far is smaller than the distance to
 // the cube's faces, beyond which nothing has been looked at.  Most points end after the first cube of 3 x 3 x 3 cells,
 // with one thread per point; the rest (isolated points, whose cubes grow to tens of cells a side) go to a queue and are
-// finished by one warp per point, whose lanes split the rows of a cube that grows by half from stage to stage.
+// finished by one warp per point, whose lanes split the candidates of a cube that grows from stage to stage.
 //
 // The result is the (k+1)-th smallest of a multiset of fp32 squared distances, each formed as (dx dx + dy dy) + dz dz
 // without contraction, so it does not depend on the order in which candidates are met and is bit-equal to an all-pairs
@@ -18,6 +18,7 @@ namespace vetr
 {
 constexpr int kKnnMaxK       = 16;
 constexpr int kKnnScanTile   = 4096;       // cells per thread block of the scan (256 threads x 16)
+constexpr int kKnnCellsPad   = 4;          // zeros in front of the per-cell array (the first cell begins at slot 0), a whole 16 bytes
 constexpr long long kKnnMaxCells = 1ll << 26;  // 64 Mi cells: 16384 scan tiles, one spine block
 
 struct KnnGrid
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(256) knn_apply_kernel(const int* counts, long 
 }
 
 // Counting sort, last step: sorted[slot] = (x, y, z, index bits); cursor[cell] starts at the cell's first slot and ends
-// at its last + 1.
+// at its last + 1, the first slot of the next cell.
 __global__ void __launch_bounds__(256) knn_scatter_kernel(const float* __restrict__ pos, int stride, int n, const int* __restrict__ point_cell,
                                                           int* cursor, float4* sorted)
 {
@@ -223,8 +224,7 @@ struct KnnSearch
 {
     KnnGrid g;
     const float4* sorted;
-    const int* starts;  // first slot of a cell
-    const int* ends;    // last slot + 1
+    const int* first;  // [cells + 1]: first slot of a cell, which ends where the cell behind it begins
     int n;
     int dummies;   // list entries pre-filled with -inf so that the (k+1)-th smallest distance sits in the last entry
     float slack;   // rounding allowance of the cube-face distances
@@ -288,92 +288,164 @@ __device__ __forceinline__ float knn_margin(const KnnSearch& a, float x, float y
 
 __device__ __forceinline__ bool knn_done(float kth_d2, float margin) { return margin > 0.f && kth_d2 <= margin * margin; }
 
-// First pass: one thread per point (in cell order, so that a warp's points share their cells), the cube of 3^3 cells.
+// Square of a distance to a cell's face, rounding allowance taken off.
+__device__ __forceinline__ float knn_gap2(const KnnSearch& a, float d)
+{
+    d = fmaxf(d - a.slack, 0.f);
+    return d * d;
+}
+
+// First pass: one thread per point (in cell order, so that a warp's points share their cells), the cube of 3^3 cells.  The
+// point's own cell comes first: in a dense cell it holds neighbours closer than the cell's faces, and the other cells, nearest
+// first, are passed over where they lie beyond the k-th distance found so far (a later candidate would have to be smaller, so
+// the result is the same).  Bound by instruction issue, 75 % of the slots at half the lanes.  4 M points of a planar scene with
+// 5 % outliers, k = 4: 969 -> 769 us (before: all 27 cells, row by row from one corner).
 template <int KMAX>
 __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ KnnSearch a)
 {
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= a.n) return;
-    const float4 p = a.sorted[i];
+    const float4 p   = a.sorted[i];
+    const KnnGrid& g = a.g;
     int cx, cy, cz;
-    knn_cell_of(a.g, p.x, p.y, p.z, cx, cy, cz);
+    const int own = knn_cell_of(g, p.x, p.y, p.z, cx, cy, cz);
     float best[KMAX];
 #pragma unroll
     for (int j = 0; j < KMAX; ++j) best[j] = j < a.dummies ? -CUDART_INF_F : CUDART_INF_F;
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, a.g.nx - 1);
-    for (int z = max(cz - 1, 0); z <= min(cz + 1, a.g.nz - 1); ++z)
-        for (int y = max(cy - 1, 0); y <= min(cy + 1, a.g.ny - 1); ++y)
+    const float xlo = knn_gap2(a, p.x - (g.ox + (float)cx * g.cell)), xhi = knn_gap2(a, (g.ox + (float)(cx + 1) * g.cell) - p.x);
+    const float ylo = knn_gap2(a, p.y - (g.oy + (float)cy * g.cell)), yhi = knn_gap2(a, (g.oy + (float)(cy + 1) * g.cell) - p.y);
+    const float zlo = knn_gap2(a, p.z - (g.oz + (float)cz * g.cell)), zhi = knn_gap2(a, (g.oz + (float)(cz + 1) * g.cell) - p.z);
+    knn_scan_slots<KMAX>(a, a.first[own], a.first[own + 1], p.x, p.y, p.z, best);
+    // steps 0, 1: the neighbours along x; 2..9: the other rows of three cells, those that share a face with the own row first
+#pragma unroll 1
+    for (int t = 0; t < 10; ++t)
+    {
+        const int dy = (int)(0x88585u >> (2 * t) & 3) - 1, dz = (int)(0xa0855u >> (2 * t) & 3) - 1;  // two bits a step
+        const int y = cy + dy, z = cz + dz;
+        if ((unsigned)y >= (unsigned)g.ny || (unsigned)z >= (unsigned)g.nz) continue;
+        const float gap = (dy < 0 ? ylo : dy > 0 ? yhi : 0.f) + (dz < 0 ? zlo : dz > 0 ? zhi : 0.f);
+        const float kth = best[KMAX - 1];
+        if (!(gap < kth)) continue;
+        const bool left = cx > 0 && gap + xlo < kth, right = cx < g.nx - 1 && gap + xhi < kth;
+        int c0 = cx - left, c1 = cx + right;  // the row's cells are consecutive slots
+        if (t == 0)
         {
-            const int row = (z * a.g.ny + y) * a.g.nx;
-            knn_scan_slots<KMAX>(a, a.starts[row + x0], a.ends[row + x1], p.x, p.y, p.z, best);  // x-neighbours are contiguous
+            if (!left) continue;
+            c1 = c0;
         }
+        else if (t == 1)
+        {
+            if (!right) continue;
+            c0 = c1;
+        }
+        const int row = (z * g.ny + y) * g.nx;
+        knn_scan_slots<KMAX>(a, a.first[row + c0], a.first[row + c1 + 1], p.x, p.y, p.z, best);
+    }
     if (knn_done(best[KMAX - 1], knn_margin(a, p.x, p.y, p.z, cx, cy, cz, 1)))
         a.radius[(size_t)__float_as_int(p.w) * a.radius_stride] = sqrtf(best[KMAX - 1]);
     else
         a.queue[atomicAdd(a.queue_count, 1)] = i;
 }
 
-// Second pass: one warp per queued point.  The cube [c - R, c + R]^3 grows its half-width R by half from stage to stage.  The
-// rows (y, z) of the cube that lie inside the grid are dealt to the lanes; the cells of a row are consecutive in the sorted
-// array, so a row costs one or two range look-ups whatever its length: the whole row if it lies outside the previous
-// cube, else the two pieces left and right of it.  After each stage the stopping rule is applied to the cube's faces.
+// Second pass: one warp per queued point.  The cube [c - R, c + R]^3 grows from stage to stage.  The rows (y, z) of the cube that
+// lie inside the grid are dealt to the lanes; the cells of a row are consecutive in the sorted array, so a row is one range of
+// slots, or two (left and right of the cube already visited), and rows or their ends that lie beyond the k-th distance known so
+// far are left out.  The ranges of 32 rows are then laid end to end and every lane takes every 32nd candidate of them.
+// After each stage the stopping rule is applied to the cube's faces.
+//
+// Where the cube of an isolated point meets a dense surface, a few rows hold hundreds of candidates: with a lane scanning
+// the whole of its row the others waited for it.  4 M points of a planar scene with 5 % outliers, k = 4: 1054 -> 557 us.
 template <int KMAX>
 __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ KnnSearch a)
 {
-    const int lane = threadIdx.x & 31;
-    const int n_q  = *a.queue_count;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane   = threadIdx.x & 31;
+    const int n_q    = *a.queue_count;
+    const KnnGrid& g = a.g;
     for (int w = blockIdx.x * 4 + (threadIdx.x >> 5); w < n_q; w += gridDim.x * 4)
     {
         const float4 p = a.sorted[a.queue[w]];
         int cx, cy, cz;
-        knn_cell_of(a.g, p.x, p.y, p.z, cx, cy, cz);
+        knn_cell_of(g, p.x, p.y, p.z, cx, cy, cz);
         float best[KMAX];
 #pragma unroll
         for (int j = 0; j < KMAX; ++j) best[j] = (lane == 0 && j < a.dummies) ? -CUDART_INF_F : CUDART_INF_F;
-        const int r_max = max(max(max(cx, a.g.nx - 1 - cx), max(cy, a.g.ny - 1 - cy)), max(cz, a.g.nz - 1 - cz));
+        float kth       = CUDART_INF_F;  // k-th smallest of all lanes' candidates so far
+        const int r_max = max(max(max(cx, g.nx - 1 - cx), max(cy, g.ny - 1 - cy)), max(cz, g.nz - 1 - cz));
         int r_prev = -1;  // half-width of the cube already visited (-1: nothing yet)
-        for (int r = 1;; r = min(r + max(r / 2, 1), max(r_max, 1)))  // 1, 2, 3, 4, 6, 9, 13, ...
+        for (int r = min(2, max(r_max, 1));; r = min(r + max(r / 2, 2), max(r_max, 1)))  // 2, 4, 6, 9, 13, ...
         {
-            const int ylo = max(cy - r, 0), yhi = min(cy + r, a.g.ny - 1), zlo = max(cz - r, 0), zhi = min(cz + r, a.g.nz - 1);
+            const int ylo = max(cy - r, 0), yhi = min(cy + r, g.ny - 1), zlo = max(cz - r, 0), zhi = min(cz + r, g.nz - 1);
             const int wz = zhi - zlo + 1, rows = (yhi - ylo + 1) * wz;  // <= ny nz <= 2^26
-            const int x0 = max(cx - r, 0), x1 = min(cx + r, a.g.nx - 1);
-            for (int t = lane; t < rows; t += 32)
+            for (int base = 0; base < rows; base += 32)
             {
-                const int y = ylo + t / wz, z = zlo + t % wz;
-                const int row = (z * a.g.ny + y) * a.g.nx;
-                if (abs(y - cy) > r_prev || abs(z - cz) > r_prev)
-                    knn_scan_slots<KMAX>(a, a.starts[row + x0], a.ends[row + x1], p.x, p.y, p.z, best);
-                else
+                int b0 = 0, n0 = 0, b1 = 0, n1 = 0;  // the lane's row: its one or two ranges of slots
+                const int t = base + lane;
+                if (t < rows)
                 {
-                    const int left = cx - r_prev - 1, right = cx + r_prev + 1;  // the cells next to the visited piece
-                    if (left >= x0) knn_scan_slots<KMAX>(a, a.starts[row + x0], a.ends[row + left], p.x, p.y, p.z, best);
-                    if (right <= x1) knn_scan_slots<KMAX>(a, a.starts[row + right], a.ends[row + x1], p.x, p.y, p.z, best);
+                    const int y = ylo + t / wz, z = zlo + t % wz;
+                    float gap = 0.f;
+                    if (y != cy) gap += knn_gap2(a, y < cy ? p.y - (g.oy + (float)(y + 1) * g.cell) : (g.oy + (float)y * g.cell) - p.y);
+                    if (z != cz) gap += knn_gap2(a, z < cz ? p.z - (g.oz + (float)(z + 1) * g.cell) : (g.oz + (float)z * g.cell) - p.z);
+                    if (gap < kth)
+                    {
+                        const float reach = sqrtf(kth - gap) + a.slack;  // cells follow the coordinate: none beyond it can count
+                        const int x0 = max(cx - r, knn_cell_coord(p.x - reach, g.ox, g.inv_cell, g.nx));
+                        const int x1 = min(cx + r, knn_cell_coord(p.x + reach, g.ox, g.inv_cell, g.nx));
+                        const int* row   = a.first + (z * g.ny + y) * g.nx;
+                        const bool inner = abs(y - cy) <= r_prev && abs(z - cz) <= r_prev;
+                        // the cells next to the visited piece
+                        const int end = inner ? min(cx - r_prev - 1, x1) : x1, begin = max(cx + r_prev + 1, x0);
+                        if (x0 <= end) b0 = row[x0], n0 = row[end + 1] - b0;
+                        if (inner && begin <= x1) b1 = row[begin], n1 = row[x1 + 1] - b1;
+                    }
                 }
-            }
-            // The stopping rule wants the KMAX-th smallest distance of all lanes to lie inside the cube, i.e. KMAX of the
-            // lanes' entries: a count says so, and the lists are merged only once, at the end.  (4 M points of a planar scene with
-            // 5 % outliers, k = 4: 1432 us with a merge per stage, 1070 us like this.)
-            const float margin = knn_margin(a, p.x, p.y, p.z, cx, cy, cz, r);
-            unsigned inside    = 0;
+                int upto = n0 + n1;  // candidates of this lane's row and the rows before it
+                for (int o = 1; o < 32; o <<= 1)
+                {
+                    const int v = __shfl_up_sync(kAll, upto, o);
+                    if (lane >= o) upto += v;
+                }
+                const int total = __shfl_sync(kAll, upto, 31);
+                if (total == 0) continue;
+                const int before = upto - n0 - n1;
+                for (int first = 0; first < total; first += 32)
+                {
+                    const int c = first + lane;
+                    int owner   = 0;  // first lane whose rows reach beyond candidate c (31 behind the last)
 #pragma unroll
-            for (int j = 0; j < KMAX; ++j) inside += knn_done(best[j], margin);
-            if (r >= r_max || __reduce_add_sync(0xffffffffu, inside) >= KMAX)
-            {
-                // KMAX times, take the smallest head of all lanes
-                float kth = 0.f;
+                    for (int o = 16; o > 0; o >>= 1)
+                        if (__shfl_sync(kAll, upto, owner + o - 1) <= c) owner += o;
+                    const int at = c - __shfl_sync(kAll, before, owner), n_left = __shfl_sync(kAll, n0, owner);
+                    const int left = __shfl_sync(kAll, b0, owner), right = __shfl_sync(kAll, b1, owner);
+                    if (c < total)
+                    {
+                        const float4 q = __ldg(a.sorted + (at < n_left ? left + at : right + at - n_left));
+                        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+                        const float d  = dx * dx + dy * dy + dz * dz;
+                        if (d < best[KMAX - 1]) knn_insert<KMAX>(best, d);
+                    }
+                }
+                // the k-th smallest of all lanes: k times, take the smallest head off its list (of a copy)
+                float rest[KMAX];
+#pragma unroll
+                for (int j = 0; j < KMAX; ++j) rest[j] = best[j];
 #pragma unroll 1
                 for (int j = 0; j < KMAX; ++j)
                 {
-                    kth = best[0];
-                    for (int o = 16; o > 0; o >>= 1) kth = fminf(kth, __shfl_xor_sync(0xffffffffu, kth, o));
-                    const unsigned holders = __ballot_sync(0xffffffffu, best[0] == kth);
+                    kth = rest[0];
+                    for (int o = 16; o > 0; o >>= 1) kth = fminf(kth, __shfl_xor_sync(kAll, kth, o));
+                    const unsigned holders = __ballot_sync(kAll, rest[0] == kth);
                     if (lane == __ffs(holders) - 1)
                     {
 #pragma unroll
-                        for (int q = 0; q + 1 < KMAX; ++q) best[q] = best[q + 1];
-                        best[KMAX - 1] = CUDART_INF_F;
+                        for (int q = 0; q + 1 < KMAX; ++q) rest[q] = rest[q + 1];
+                        rest[KMAX - 1] = CUDART_INF_F;
                     }
                 }
+            }
+            if (r >= r_max || knn_done(kth, knn_margin(a, p.x, p.y, p.z, cx, cy, cz, r)))
+            {
                 if (lane == 0) a.radius[(size_t)__float_as_int(p.w) * a.radius_stride] = sqrtf(kth);
                 break;
             }
