@@ -77,3 +77,35 @@ def test_static_scan_rejects_sizes_beyond_its_scratch(rasterizer):
     assert L.lib().vetr_scan_counts_static(0, None, p, too_many, 0, p, p, p, 1 << 40) == L.E_TOO_LARGE
     assert L.lib().vetr_scan_counts_static(0, None, p, 16, 0, p, p, p, 0) == L.E_INVALID_ARG  # item table too small
     assert L.lib().vetr_scan_counts_static(0, None, None, 16, 0, p, p, p, 64) == L.E_INVALID_ARG
+
+
+@pytest.mark.parametrize("n", [1, 3, 1023, 4095, 4096, 4097, 3 * 4096 + 5])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_static_scan_of_ragged_and_unaligned_arrays(rasterizer, n, shift):
+    """Ends of tiles and of 16-byte accesses; shift = 1: arrays that start 4 bytes behind a 16-byte boundary; lists long enough
+    to span several work items."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    c = rng.integers(0, 9, size=n) * (rng.random(n) < 0.7)
+    c[rng.integers(0, n, size=3)] = 1700
+    dev = rasterizer.device
+    counts = torch.zeros(n + 8, dtype=torch.int32, device=dev)
+    counts[shift:shift + n] = torch.from_numpy(c.astype(np.int32)).to(dev)
+    counts[shift + n:] = 99  # not part of the array
+    ends = torch.full((n + 8,), -7, dtype=torch.int32, device=dev)
+    status = torch.empty(4, dtype=torch.int32, device=dev)
+    n_items = int(L.lib().vetr_item_table_entries(int(c.sum()), n))
+    items = torch.full((n_items,), -7, dtype=torch.int32, device=dev)
+    p = lambda t, k=0: C.c_void_p(t.data_ptr() + 4 * k)  # noqa: E731
+    assert L.lib().vetr_scan_counts_static(0, None, p(counts, shift), n, int(c.sum()), p(ends, shift), p(status), p(items), n_items) == L.OK
+    torch.cuda.synchronize()
+    start = np.cumsum(c) - c
+    e = ends.cpu().numpy()
+    np.testing.assert_array_equal(e[shift:shift + n], start)
+    assert (e[:shift] == -7).all() and (e[shift + n:] == -7).all()
+    work = np.cumsum(c) + 4 * (np.arange(n) + 1)  # work up to and with a pixel; item k opens at the first that exceeds 512 k
+    total = -(-int(work[-1]) // ITEM_UNITS)
+    assert status.cpu().tolist() == [int(c.sum()), 0, int(c.max()), total]
+    want = np.searchsorted(work, ITEM_UNITS * np.arange(total), side="right").tolist() + [n]
+    assert items[:total + 1].cpu().tolist() == want

@@ -114,12 +114,17 @@ __global__ void __launch_bounds__(256) knn_occupied_kernel(const int* __restrict
 }
 
 // Exclusive scan of the cell counts in three kernels: sums of tiles, scan of the tile sums by one block, scan inside the tiles.
+template <bool kVec>
 __global__ void __launch_bounds__(256) knn_tile_sums_kernel(const int* __restrict__ counts, long long n_cells, int* tile_sums)
 {
     const long long base = (long long)blockIdx.x * kKnnScanTile;
     int s = 0;
-    for (int k = threadIdx.x; k < kKnnScanTile; k += 256)
-        if (base + k < n_cells) s += counts[base + k];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+    {
+        const int4 c = scan_load<kVec>(counts, base + r * 1024 + threadIdx.x * 4, n_cells);
+        s += c.x + c.y + c.z + c.w;
+    }
     __shared__ int part[8];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
@@ -174,37 +179,23 @@ __global__ void __launch_bounds__(1024) knn_spine_kernel(int* tile_sums, int n_t
         }
 }
 
-// starts[cell] = exclusive scan of counts (in place is allowed: starts may alias counts).
+// starts[cell] = exclusive scan of counts (in place is allowed: starts may alias counts).  17 M cells: 80 -> 16 us (before: 16 consecutive
+// cells per thread).
+template <bool kVec>
 __global__ void __launch_bounds__(256) knn_apply_kernel(const int* counts, long long n_cells, const int* __restrict__ tile_sums, int* starts)
 {
-    __shared__ int warp_tot[8];
-    const long long base = (long long)blockIdx.x * kKnnScanTile + threadIdx.x * 16;
-    int local[16], s = 0;
+    __shared__ int s_warp[32];
+    const long long base = (long long)blockIdx.x * kKnnScanTile;
+    int4 c[4];
+    int before[4];
+    scan_tile<kVec>(counts, base, n_cells, s_warp, c, before);
+    const int offset = tile_sums[blockIdx.x];
 #pragma unroll
-    for (int k = 0; k < 16; ++k)
+    for (int r = 0; r < 4; ++r)
     {
-        local[k] = base + k < n_cells ? counts[base + k] : 0;
-        s += local[k];
+        const int s0 = offset + before[r], s1 = s0 + c[r].x, s2 = s1 + c[r].y;
+        scan_store<kVec>(starts, base + r * 1024 + threadIdx.x * 4, n_cells, make_int4(s0, s1, s2, s2 + c[r].z));
     }
-    int incl = s;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1)
-    {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    int before = 0;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    int run = tile_sums[blockIdx.x] + before + incl - s;
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-        if (base + k < n_cells)
-        {
-            starts[base + k] = run;
-            run += local[k];
-        }
 }
 
 // Counting sort, last step: sorted[slot] = (x, y, z, index bits); cursor[cell] starts at the cell's first slot and ends
