@@ -340,7 +340,7 @@ def test_point_backward_tiles(rasterizer, mode, tiles, w, h, views):
 # ---- mode 2: groups of one, of a few, of the whole list, with the background (beyond a window of 1e5 every depth is in)
 
 
-@pytest.mark.parametrize("accept", [0.0, 0.003, 0.5, 9e4, 3e5])
+@pytest.mark.parametrize("accept", [1e-6, 0.003, 0.5, 9e4, 3e5])  # (0: an empty first group, 0 / 0 as in the reference)
 @pytest.mark.parametrize("n, w, h", [(6000, 96, 64), (30000, 16, 12)])
 def test_mode2_group_sizes(rasterizer, accept, n, w, h):
     sc = scenes.tiny_scene(n=n, w=w, h=h, n_views=1, seed=17)
