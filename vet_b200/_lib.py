@@ -5,6 +5,7 @@ import ctypes as C
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
+HOST_PATH = os.path.join(_HERE, "_host.so")
 LIB_PATH = os.environ.get("VETR_LIB", os.path.join(_HERE, "libvetr.so"))  # VETR_LIB: a tuning variant of the library
 
 MAX_LAYERS = 5
@@ -87,6 +88,7 @@ SEG_DESC, SEG_POINTS, SEG_CONF = 1, 2, 4
 TIMING_NAMES = ["count", "scan", "collect", "sort_blend", "backward", "finalize", "point_backward", "exchange", "envmap", "knn"]
 
 _lib = None
+_bound = None
 
 
 class VetrError(RuntimeError):
@@ -152,3 +154,19 @@ def lib():
         L.vetr_gather_points.argtypes = [vp, C.c_int, C.c_int, vp, C.POINTER(PointArray), C.c_int]
         _lib = L
     return _lib
+
+
+def host():
+    """The native host side of render.py (csrc/vetr_host.cpp), bound to the loaded library."""
+    global _bound
+    if _bound is None:
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m vet_b200.build`.")
+        import torch  # noqa: F401  (its libraries come first)
+
+        from . import _host
+
+        names = ("vetr_forward", "vetr_backward_phase", "vetr_finalize_gradients", "vetr_l1_loss_grad", "vetr_zero_buffers")
+        _host.bind(*[C.cast(getattr(lib(), n), C.c_void_p).value for n in names])
+        _bound = _host
+    return _bound

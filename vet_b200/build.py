@@ -20,6 +20,10 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
          "-Xcompiler", "-fPIC", "-shared", "-ccbin", "/usr/bin/g++"]
 
 
+HOST_PATH = os.path.join(_HERE, "_host.so")
+HOST_SOURCES = [os.path.join(_HERE, "csrc", "vetr_host.cpp")]
+
+
 def needs_build() -> bool:
     if not os.path.exists(LIB_PATH):
         return True
@@ -32,7 +36,31 @@ def build(force: bool = False, verbose: bool = False, defines=(), out: str = LIB
     if force or out != LIB_PATH or needs_build():
         cmd = [NVCC] + FLAGS + [f"-D{d}" for d in defines] + (["-Xptxas", "-v"] if verbose else []) + ["-o", out] + SOURCES
         subprocess.check_call(cmd)
+    if out == LIB_PATH:
+        build_host(force)
     return out
+
+
+def build_host(force: bool = False) -> str:
+    """Builds _host.so, the native host side of render.py: a CPython extension over libtorch (host code only, g++).  It
+    reaches libvetr.so through addresses, so it does not link it."""
+    if not force and os.path.exists(HOST_PATH):
+        t = os.path.getmtime(HOST_PATH)
+        if all(os.path.getmtime(p) <= t for p in HOST_SOURCES + [os.path.join(_HERE, "..", "include", "vetr.h")]):
+            return HOST_PATH
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ce
+
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=" + str(int(torch._C._GLIBCXX_USE_CXX11_ABI))]
+    for inc in ce.include_paths("cuda") + [sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", inc]
+    cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+                           "-Wl,-rpath," + torch_lib]
+    subprocess.check_call(cmd)
+    return HOST_PATH
 
 
 SHIM_PATH = os.path.join(_HERE, "libvetr_torch.so")

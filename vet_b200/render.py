@@ -119,7 +119,7 @@ class Rasterizer:
         """Without an explicit stream the context follows torch's current stream (also the capture stream of
         torch.cuda.graph, so a whole step of forward + backward can be recorded into a CUDA graph and replayed)."""
         if self._stream is None:
-            cur = torch.cuda.current_stream(self.device).cuda_stream
+            cur = torch._C._cuda_getCurrentRawStream(self.device.index)
             if cur != self._cur_stream:
                 self._check(L.lib().vetr_set_stream(self._ctx, C.c_void_p(cur)), "vetr_set_stream")
                 self._cur_stream = cur
@@ -131,9 +131,7 @@ class Rasterizer:
     # ---- helpers -----------------------------------------------------------------------------------------
     def _views(self, views):
         arr = (L.View * len(views))()
-        for i, v in enumerate(views):
-            arr[i] = L.View(v.w, v.h, v.image_index, v.camera_index, v.camera_model, (C.c_float * 5)(*v.crop),
-                            (C.c_float * 4)(*v.rot))
+        L.host().views(C.addressof(arr), views)
         return arr
 
     def _lists(self, slot: int, n_pixels_total: int, capacity: int, exact: bool = False) -> FragmentLists:
@@ -148,21 +146,17 @@ class Rasterizer:
     def forward(self, position, index, texture, confidence, background, poses, intrinsics, views, params: dict,
                 dropout=None, capacity: Optional[int] = None, want_weight=True, want_mask=False, want_depth=False):
         """Returns dict(color=[L x [B,C,h,w]], weight=..., mask=..., depth=...).  Keeps what backward() needs."""
-        lib = L.lib()
+        lib, host = L.lib(), L.host()
         self._sync_stream()
-        prm = L.Params(**{k: params[k] for k, _ in L.Params._fields_})
+        prm = L.Params()
+        host.params(C.addressof(prm), params, texture.shape[0])
         B, Cn, Ln = len(views), texture.shape[0], prm.num_layers
-        prm.num_channels = Cn
         w, h = views[0].w, views[0].h
         sizes = level_sizes(w, h, Ln)
         P = int(lib.vetr_pyramid_pixels(w, h, Ln))
         if P <= 0:
             raise L.VetrError(L.E_INVALID_ARG, "vetr_pyramid_pixels")
-        f32 = dict(dtype=torch.float32, device=self.device)
-        color = [torch.empty(B, Cn, hh, ww, **f32) for (ww, hh) in sizes]
-        weight = [torch.empty(B, 1, hh, ww, **f32) for (ww, hh) in sizes] if want_weight else None
-        mask = [torch.empty(B, 1, hh, ww, **f32) for (ww, hh) in sizes] if want_mask else None
-        depth = [torch.empty(B, 1, hh, ww, **f32) for (ww, hh) in sizes] if want_depth else None
+        color, weight, mask, depth = host.images(self.device, B, Cn, w, h, Ln, want_weight, want_mask, want_depth)
         cloud = L.Cloud(position.data_ptr(), index.data_ptr(), position.shape[0])
         tex = L.Texture(texture.data_ptr(), confidence.data_ptr(), background.data_ptr(), texture.shape[1])
         cams = L.Cameras(poses.data_ptr(), intrinsics.data_ptr(), poses.shape[0], intrinsics.shape[0])
@@ -175,11 +169,8 @@ class Rasterizer:
             if prm.render_mode == 3 or (prm.render_mode in (1, 2) and prm.need_point_gradient):
                 lists.ensure_level_mask(nb * position.shape[0])
             varr = self._views(views[b0:b1])
-            sl = lambda ts: None if ts is None else [t[b0:b1] for t in ts]
-            dro = None if dropout is None else dropout[b0:b1]
-            rc = lib.vetr_forward(self._ctx, C.byref(prm), C.byref(cloud), C.byref(tex), C.byref(cams), varr, nb,
-                                  _ptr(dro), C.byref(lists.c), _ptr_array(sl(color)), _ptr_array(sl(weight)),
-                                  _ptr_array(sl(mask)), _ptr_array(sl(depth)))
+            rc = host.forward(self._ctx.value, C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
+                              C.addressof(varr), nb, b0, dropout, C.addressof(lists.c), Ln, color, weight, mask, depth)
             self._check(rc, "vetr_forward")
             groups.append((b0, b1, lists, varr))
         self._saved = dict(prm=prm, cloud=cloud, tex=tex, cams=cams, groups=groups, color=color, P=P, sizes=sizes,
@@ -222,44 +213,32 @@ class Rasterizer:
         `phases`: 1 = the per-fragment kernels only, 2 = the per-point pass only (with the `accum` of the first call and the
         same `grad_color`), 3 = both (vetr_backward_phase)."""
         s = self._saved
-        lib = L.lib()
+        host = L.host()
         self._sync_stream()
+        ctx = self._ctx.value
         position, index, texture = s["tensors"][0], s["tensors"][1], s["tensors"][2]
-        poses, intrinsics = s["tensors"][5], s["tensors"][6]
+        poses, intrinsics, dropout = s["tensors"][5], s["tensors"][6], s["tensors"][7]
         n, n_tex, Cn = position.shape[0], texture.shape[1], texture.shape[0]
-        f32 = dict(dtype=torch.float32, device=self.device)
         g = accum
         if g is None:
-            # one launch zeroes them all: a fill of its own each costs more than the buffers of a small scene
-            g = dict(desc=torch.empty(n_tex, 4, **f32), conf=torch.empty(n_tex, **f32),
-                     background=torch.empty(Cn, **f32))
-            if want_points:
-                g["points"] = torch.empty(n, 4, **f32)
-            if want_pose:
-                g["pose"] = torch.empty(poses.shape[0], 6, dtype=torch.float64, device=self.device)
-                g["pose_count"] = torch.empty(poses.shape[0], **f32)
-            if want_intrinsics:
-                g["intrinsics"] = torch.empty(intrinsics.shape[0], 13, **f32)
-                g["intrinsics_count"] = torch.empty(intrinsics.shape[0], **f32)
-            bufs = list(g.values())
-            sizes = (C.c_int64 * len(bufs))(*[t.nbytes for t in bufs])
-            self._check(lib.vetr_zero_buffers(self._ctx, _ptr_array(bufs), sizes, len(bufs)), "vetr_zero_buffers")
+            names = ["desc", "conf", "background"] + ["points"] * bool(want_points)
+            names += ["pose", "pose_count"] * bool(want_pose) + ["intrinsics", "intrinsics_count"] * bool(want_intrinsics)
+            bufs = host.gradients(ctx, self.device, n if want_points else None, n_tex, Cn, poses.shape[0] if want_pose else None,
+                                  intrinsics.shape[0] if want_intrinsics else None)
+            if isinstance(bufs, int):
+                self._check(bufs, "vetr_zero_buffers")
+            g = dict(zip(names, bufs))
         grad_color = [x.contiguous() for x in grad_color]
         for (b0, b1, lists, varr) in s["groups"]:
-            oc = [t[b0:b1] for t in s["color"]]
-            gc = [t[b0:b1] for t in grad_color]
-            dro = s["tensors"][7]
             lists.ensure_pixel_scratch()
             if lists.level_mask is not None:  # 2 floats per (view, level, point), 4 (one per bilinear corner) in mode 3
                 per = 4 if s["prm"].render_mode == 3 else 2
                 lists.ensure_point_grad((b1 - b0) * s["prm"].num_layers * n * per)
-            rc = lib.vetr_backward_phase(self._ctx, C.byref(s["prm"]), C.byref(s["cloud"]), C.byref(s["tex"]),
-                                         C.byref(s["cams"]), varr, b1 - b0, _ptr(None if dro is None else dro[b0:b1]),
-                                         C.byref(lists.c), _ptr_array(oc), _ptr_array(gc),
-                                         _ptr(g["desc"]), _ptr(g["conf"]), _ptr(g.get("points")), _ptr(g["background"]),
-                                         _ptr(g.get("pose")), _ptr(g.get("pose_count")), _ptr(g.get("intrinsics")),
-                                         _ptr(g.get("intrinsics_count")),
-                                         phases | L.BACKWARD_PIXEL_SCRATCH if phases & L.BACKWARD_FRAGMENTS else phases)
+            rc = host.backward(ctx, C.addressof(s["prm"]), C.addressof(s["cloud"]), C.addressof(s["tex"]), C.addressof(s["cams"]),
+                               C.addressof(varr), b1 - b0, b0, dropout, C.addressof(lists.c), s["prm"].num_layers, s["color"], grad_color,
+                               g["desc"], g["conf"], g.get("points"), g["background"], g.get("pose"), g.get("pose_count"),
+                               g.get("intrinsics"), g.get("intrinsics_count"),
+                               phases | L.BACKWARD_PIXEL_SCRATCH if phases & L.BACKWARD_FRAGMENTS else phases)
             self._check(rc, "vetr_backward_phase")
         return g
 
@@ -267,15 +246,11 @@ class Rasterizer:
         """Raw sums -> the reference's return tensors (PointRenderer.cu:1251-1322): texture [C,n_tex], confidence
         [1,n_tex], background [C], points [n,4] averaged by hit count, pose tangent and intrinsics averaged."""
         self._sync_stream()
-        n_tex = g["desc"].shape[0]
-        Cn = g["background"].shape[0]
-        g_texture = torch.empty(Cn, n_tex, dtype=torch.float32, device=self.device)
         pts, pose, intr = g.get("points"), g.get("pose"), g.get("intrinsics")
-        rc = L.lib().vetr_finalize_gradients(
-            self._ctx, Cn, n_tex, _ptr(g["desc"]), _ptr(g_texture), 0 if pts is None else pts.shape[0], _ptr(pts), None,
-            0 if pose is None else pose.shape[0], _ptr(pose), _ptr(g.get("pose_count")),
-            0 if intr is None else intr.shape[0], _ptr(intr), _ptr(g.get("intrinsics_count")))
-        self._check(rc, "vetr_finalize_gradients")
+        g_texture = L.host().finalize(self._ctx.value, self.device, g["background"].shape[0], g["desc"], pts, pose,
+                                      g.get("pose_count"), intr, g.get("intrinsics_count"))
+        if isinstance(g_texture, int):
+            self._check(g_texture, "vetr_finalize_gradients")
         return dict(texture=g_texture, confidence=g["conf"].view(1, -1), background=g["background"], points=pts,
                     pose=pose, intrinsics=intr)
 
@@ -389,10 +364,7 @@ class Rasterizer:
     def l1_loss_grad(self, images, targets, grads, loss):
         """loss (device scalar) = sum over levels of mean |image - target|; grads[l] = sign(image - target) / numel, one launch."""
         self._sync_stream()
-        n = len(images)
-        numel = (C.c_int64 * n)(*[t.numel() for t in images])
-        rc = L.lib().vetr_l1_loss_grad(self._ctx, n, _ptr_array(images), _ptr_array(targets), _ptr_array(grads), numel, _ptr(loss))
-        self._check(rc, "vetr_l1_loss_grad")
+        self._check(L.host().l1_loss_grad(self._ctx.value, images, targets, grads, loss), "vetr_l1_loss_grad")
 
     def set_timing(self, enable: bool):
         self._sync_stream()
