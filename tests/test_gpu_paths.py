@@ -351,3 +351,33 @@ def test_mode2_group_sizes(rasterizer, accept, n, w, h):
         gpu = util.run_gpu(rasterizer, sc, params, grads=g)
         util.compare_forward(gpu, ora, exact_images=True)
         util.compare_backward(gpu["bwd_raw"], ora, sc.channels)
+
+
+# ---- error grid: groups of cells that are left out before their corners are projected
+
+
+@pytest.mark.parametrize("crop", [False, True])
+def test_grid_loss_cells_around_the_edges_of_the_view(rasterizer, crop):
+    """Boxes of all sizes around the camera and the border of the image, in groups of four that lie across it or just beside it:
+    none that covers a pixel may be left out (coverage is exact).  A number of cells that fills no group."""
+    import torch
+
+    w, h = 321, 243
+    sc = scenes.config_planar(64, w, h, 200.0, n_views=1, seed=3)
+    if crop:
+        sc.views[0].crop = (1.3, 0.8, 12.0, -9.0, 0.05)
+        sc.views[0].rot = (0.8, -0.6, 0.6, 0.8)
+    rng = np.random.default_rng(2)
+    n = 20_003
+    centre = np.repeat(rng.uniform(-12, 12, size=(n // 4 + 1, 3)), 4, axis=0)[:n]  # neighbours close to each other, as in a grid
+    size = np.repeat(10.0 ** rng.uniform(-2.5, 0.5, size=(n // 4 + 1, 1)), 4, axis=0)[:n]
+    bb_min = (centre + size * rng.uniform(-1, 1, size=(n, 3))).astype(np.float32)
+    bb_len = np.broadcast_to(size, (n, 3)).astype(np.float32).copy()
+    loss = rng.standard_normal((3, h, w)).astype(np.float32)
+    ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    assert (ref_c > 0).sum() > 1000 and (ref_c == 0).sum() > 1000
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+    np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)

@@ -506,7 +506,74 @@ __device__ __forceinline__ void grid_pixels(const GridArgs& a, const GridWarpSme
     }
 }
 
-// First kernel: one warp per group of four cells.  Cells with many rows (next to the camera a cell covers 10^5 pixels) and
+// Half-spaces that hold no cell to be drawn: behind the camera, and left, right, above and below what grid_rectangle keeps of the
+// image.  The image position of a point with z > 0 is A (x / z, y / z) + b (no distortion), so "left of u" is n . v < 0 with
+// n = (A11, A12, b1 - u) for the point v in camera space, and w . p + d < 0 for the point p in the world.  A box lies in it if
+// its support w . c + d + |w| . h does (c centre, h half extents).  A cell with a corner behind the camera is not drawn, so the
+// other corners' z need not be looked at.  Bounds are moved outwards by two pixels and by what fp32 may be off.
+struct GridPlane
+{
+    float w[3], d, size;  // size: |n| . |t|, what the rounding of d is measured by
+};
+constexpr int kGridPlanes = 5;
+__device__ __forceinline__ GridPlane grid_plane(const GridArgs& a, const Camera& cam, int k)
+{
+    // K, crop and rotation about the image centre, one after the other
+    const float a11 = cam.crop[0] * cam.K[0], a12 = cam.crop[0] * cam.K[4] + cam.crop[4] * cam.K[1];
+    const float b1  = cam.crop[0] * cam.K[2] + cam.crop[4] * cam.K[3] + cam.crop[2] - cam.cx;
+    const float a22 = cam.crop[1] * cam.K[1], b2 = cam.crop[1] * cam.K[3] + cam.crop[3] - cam.cy;
+    const float A[2][2] = {{cam.rot[0] * a11, cam.rot[0] * a12 + cam.rot[1] * a22}, {cam.rot[2] * a11, cam.rot[2] * a12 + cam.rot[3] * a22}};
+    const float b[2]    = {cam.rot[0] * b1 + cam.rot[1] * b2 + cam.cx, cam.rot[2] * b1 + cam.rot[3] * b2 + cam.cy};
+    float n[3] = {0.f, 0.f, 1.f};
+    if (k > 0)
+    {
+        const int axis     = (k - 1) >> 1;
+        const float size   = (float)(axis ? a.h : a.w), border = 32.f, out = 2.f + 1e-5f * (fabsf(b[axis]) + size);
+        const bool far     = !(k & 1);
+        const float sign   = far ? -1.f : 1.f;
+        n[0] = sign * A[axis][0], n[1] = sign * A[axis][1];
+        n[2] = far ? size - border + out - b[axis] : b[axis] - border + out;
+    }
+    GridPlane p;
+    for (int j = 0; j < 3; ++j) p.w[j] = n[0] * cam.R[j] + n[1] * cam.R[3 + j] + n[2] * cam.R[6 + j];
+    p.d    = n[0] * cam.V.tx + n[1] * cam.V.ty + n[2] * cam.V.tz;
+    p.size = fabsf(n[0] * cam.V.tx) + fabsf(n[1] * cam.V.ty) + fabsf(n[2] * cam.V.tz);
+    return p;
+}
+
+// True if no cell of the group is drawn (false for anything that is not a number).
+__device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridPlane* planes, int group)
+{
+    float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+    bool number = true;
+    for (int c = group * kGridGroup; c < min((group + 1) * kGridGroup, a.n_cells); ++c)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+        {
+            const float b = a.bb_min[3 * c + j], e = b + a.bb_len[3 * c + j];
+            lo[j] = fminf(lo[j], fminf(b, e)), hi[j] = fmaxf(hi[j], fmaxf(b, e));
+            number &= fabsf(e) < 1e30f;
+        }
+    bool out = false;
+#pragma unroll
+    for (int k = 0; k < kGridPlanes; ++k)
+    {
+        const GridPlane p = planes[k];
+        float v = p.d, size = p.size;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+        {
+            const float centre = 0.5f * lo[j] + 0.5f * hi[j], half = 0.5f * hi[j] - 0.5f * lo[j], reach = fabsf(p.w[j]) * half;
+            v += p.w[j] * centre + reach, size += fabsf(p.w[j] * centre) + reach;
+        }
+        out |= v < -1e-5f * size;
+    }
+    return number && out;
+}
+
+// First kernel: one warp per group of four cells.  A warp's next 32 groups are looked at first, a lane each: groups that lie
+// altogether out of sight are left out before their corners are projected, which costs about 200 instructions per group.
+// 128^3 cells, 1920x1080: grid_loss_kernel 682 -> 592 us.  Cells with many rows (next to the camera a cell covers 10^5 pixels) and
 // large rectangles in the per-pixel form are cut into chunks that go to a queue, so that the second kernel can spread them
 // over all SMs.  If the queue is full the warp does the whole cell itself.
 __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
@@ -519,9 +586,24 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     GridWarpSmem& s    = s_warp[warp];
     const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
-    const int n_groups = (a.n_cells + kGridGroup - 1) / kGridGroup;
-    for (int group = blockIdx.x * kGridWarps + warp; group < n_groups; group += gridDim.x * kGridWarps)
+    const int n_groups = (a.n_cells + kGridGroup - 1) / kGridGroup, stride = gridDim.x * kGridWarps;
+    __shared__ GridPlane s_planes[kGridPlanes];
+    if (threadIdx.x < kGridPlanes) s_planes[threadIdx.x] = grid_plane(a, s_cam, threadIdx.x);
+    __syncthreads();
+    unsigned todo = 0;  // groups first + k stride still to do (bit k)
+    int first = blockIdx.x * kGridWarps + warp - 32 * stride;
+    for (;;)
     {
+        if (todo == 0)
+        {
+            first += 32 * stride;
+            if (first >= n_groups) break;
+            const int mine = first + lane * stride;
+            todo = __ballot_sync(0xffffffffu, mine < n_groups && (s_cam.has_dist || !grid_out_of_sight(a, s_planes, mine)));
+            continue;
+        }
+        const int group = first + (__ffs(todo) - 1) * stride;
+        todo &= todo - 1;
         const int c         = group * kGridGroup + (lane >> 3);
         const GridCell cell = grid_prepare(f, a, s_cam, s, c < a.n_cells ? c : -1, no_rows);
         if (!__any_sync(0xffffffffu, cell.total > 0)) continue;
