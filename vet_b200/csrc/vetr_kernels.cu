@@ -1471,27 +1471,32 @@ __device__ __forceinline__ float4 load_grad(const Frame& f, int g) { return __ld
 
 // Channel-interleaved copies of the forward image and of its gradient over the global pixel space (the caller's
 // tensors are planar [view, channel, y, x] per level).
-__global__ void __launch_bounds__(256) pack_images_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp)
+__device__ __forceinline__ float4 pack_pixel(const Frame& f, const BackPtrs& bp, long long r, int& view, int& l, int& o)
 {
-    // one thread per pixel in plain row-major order (view, level, y, x): coalesced reads of the planar tensors
-    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= f.Prm * f.n_views) return;
-    const int Prm  = (int)f.Prm;
-    int view = 0;
+    // pixels in plain row-major order (view, level, y, x): coalesced reads of the planar tensors
+    const int Prm = (int)f.Prm;
+    view = 0, l = 0;
 #pragma unroll
     for (int i = 1; i < VETR_MAX_VIEWS; ++i)
         if (i < f.n_views && r >= (long long)i * Prm) view = i;
     const int q = (int)(r - (long long)view * Prm);
-    int l = 0;
 #pragma unroll
     for (int i = 1; i < VETR_MAX_LAYERS; ++i)
         if (i < f.L && q >= (int)f.rbase[i]) l = i;
-    const int o  = q - (int)f.rbase[l];  // y * w + x
-    const int hw = f.lw[l] * f.lh[l];
+    o = q - (int)f.rbase[l];  // y * w + x
+    const int hw   = f.lw[l] * f.lh[l];
     const float* I = bp.out_color[l] + (size_t)(view * f.C) * hw + o;
     const float* G = bp.grad_color[l] + (size_t)(view * f.C) * hw + o;
+    const float4 g = make_float4(__ldg(G), __ldg(G + hw), __ldg(G + 2 * hw), f.C > 3 ? __ldg(G + 3 * hw) : 0.f);
     f.img4[r]  = make_float4(__ldg(I), __ldg(I + hw), __ldg(I + 2 * hw), f.C > 3 ? __ldg(I + 3 * hw) : 0.f);
-    f.grad4[r] = make_float4(__ldg(G), __ldg(G + hw), __ldg(G + 2 * hw), f.C > 3 ? __ldg(G + 3 * hw) : 0.f);
+    f.grad4[r] = g;
+    return g;
+}
+__global__ void __launch_bounds__(256) pack_images_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp)
+{
+    const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int view, l, o;
+    if (r < f.Prm * f.n_views) pack_pixel(f, bp, r, view, l, o);
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b, int C)
@@ -2281,10 +2286,17 @@ __device__ __forceinline__ float4 load_grad_planar(const Frame& f, const BackPtr
     return g;
 }
 
-__global__ void fill_int_kernel(int* p, int v, long long n)
+// Start of a call: no depth, empty accumulators, status.
+__global__ void __launch_bounds__(256) fuzzy_dt_clear_kernel(const __grid_constant__ Frame f)
 {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
+    const long long g = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (g < f.PT)
+    {
+        f.ends[g]      = __float_as_int(kMaxDepth);
+        const uint4 no = make_uint4(0u, 0u, 0u, 0u);
+        store_sector(f.recs + 2 * (size_t)g, no, no);
+    }
+    if (g < 4) f.status[g] = 0;
 }
 
 // kPass 0: DepthPrepassMulti (RenderForward.cu:180-308; no drop-out test).  kPass 1: RenderForwardMulti (:312-406).
@@ -2368,20 +2380,12 @@ __global__ void __launch_bounds__(256) fuzzy_dt_combine_kernel(const __grid_cons
     }
 }
 
-// CombineAndFillBackward (RenderBackward.cu:27-76): the background colour receives the gradient of every empty pixel.
-__global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_constant__ Frame f,
-                                                                   const __grid_constant__ BackPtrs bp)
+// CombineAndFillBackward (RenderBackward.cu:27-76): the background colour receives the gradient of every empty pixel.  With
+// interleaved copies the kernel that makes them has every pixel's gradient at hand and sums these as well (2 views 1280x720:
+// 39 us for both, before 27 + 27 us in two launches); without them the empty pixels are visited by themselves.
+__device__ __forceinline__ void fuzzy_dt_background_sum(const Frame& f, const BackPtrs& bp, const float (&v)[4])
 {
     __shared__ float s_red[8][4];
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < f.PT; g += (long long)gridDim.x * blockDim.x)
-        if (f.counts[g] == 0)
-        {
-            const PixInfo px = decode_pixel(f, (unsigned)g);
-            if (!px.valid) continue;
-            const float4 G = load_grad_planar(f, bp, px);
-            v[0] += G.x, v[1] += G.y, v[2] += G.z, v[3] += G.w;
-        }
     for (int k = 0; k < 4; ++k)
     {
         float x = v[k];
@@ -2395,6 +2399,37 @@ __global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_c
         for (int w = 0; w < 8; ++w) x += s_red[w][threadIdx.x];
         if (x != 0.f) atomicAdd(bp.g_background + threadIdx.x, x);
     }
+}
+__global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_constant__ Frame f,
+                                                                   const __grid_constant__ BackPtrs bp)
+{
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < f.PT; g += (long long)gridDim.x * blockDim.x)
+        if (f.counts[g] == 0)
+        {
+            const PixInfo px = decode_pixel(f, (unsigned)g);
+            if (!px.valid) continue;
+            const float4 G = load_grad_planar(f, bp, px);
+            v[0] += G.x, v[1] += G.y, v[2] += G.z, v[3] += G.w;
+        }
+    fuzzy_dt_background_sum(f, bp, v);
+}
+__global__ void __launch_bounds__(256) fuzzy_dt_pack_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp)
+{
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    const long long total = f.Prm * f.n_views;
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < total; r += (long long)gridDim.x * blockDim.x)
+    {
+        int view, l, o;
+        const float4 G = pack_pixel(f, bp, r, view, l, o);
+        const int w    = f.lw[l];
+        // row: float estimate, then one correction step either way (the estimate is off by at most one)
+        int y = __float2int_rz((float)o * f.inv_lw[l]), x = o - y * w;
+        if (x < 0) x += w, --y;
+        if (x >= w) x -= w, ++y;
+        if (f.counts[view * (int)f.P + (int)f.lbase[l] + pixel_offset(w, x, y)] == 0) v[0] += G.x, v[1] += G.y, v[2] += G.z, v[3] += G.w;
+    }
+    fuzzy_dt_background_sum(f, bp, v);
 }
 
 // RenderBackward (RenderBackward.cu:131-474): one thread per point and view.  Pixel positions come from the backward's own
@@ -2918,13 +2953,6 @@ struct PassScope
         }                                         \
     } while (0)
 
-static int __float_as_int_host(float v)
-{
-    int i;
-    memcpy(&i, &v, 4);
-    return i;
-}
-
 // Pixel space of one view: every level's height is padded to a multiple of kBand rows (the banded order of pixel_offset).
 // rbase / *row_major: the same levels in plain row-major order without padding.
 static int64_t pyramid(int w, int h, int L, int* lw, int* lh, long long* lbase, long long* rbase = nullptr,
@@ -3217,12 +3245,10 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     if (f.mode == VETR_MODE_FUZZY_DT)
     {
         if (f.capacity < f.PT) return VETR_E_INVALID_ARG;  // the fragment buffer holds one accumulator record per pixel
-        VETR_CUDA(ctx, cudaMemsetAsync(f.status, 0, 4 * sizeof(int), st));
-        VETR_CUDA(ctx, cudaMemsetAsync(f.recs, 0, (size_t)f.PT * 32, st));
         const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         {
             PassScope t(ctx, VETR_T_COUNT, 2 + (ctas > 0));
-            fill_int_kernel<<<(unsigned)((f.PT + 255) / 256), 256, 0, st>>>(f.ends, __float_as_int_host(kMaxDepth), f.PT);
+            fuzzy_dt_clear_kernel<<<(unsigned)((f.PT + 255) / 256), 256, 0, st>>>(f);
             if (ctas > 0) fuzzy_dt_point_kernel<0><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f);
         }
         if (ctas > 0)
@@ -3318,10 +3344,12 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         // 13 ps per point and view (2 M points, 2 views 1280x720: 234 -> 181 + 27 us), hence only where points are no fewer
         // than pixels; and only with the caller's word that the scratch is there, because mode 0 can do without.
         if (!use_scratch || ((uintptr_t)f.img4 & 15) != 0 || f.n < f.Prm) f.img4 = f.grad4 = nullptr;
-        PassScope t(ctx, VETR_T_BACKWARD, 2 + (f.img4 != nullptr));
+        PassScope t(ctx, VETR_T_BACKWARD, 2);
         cudaStream_t st = ctx->stream;
-        if (f.img4) pack_images_kernel<<<(unsigned)((f.Prm * n_views + 255) / 256), 256, 0, st>>>(f, bp);
-        fuzzy_dt_background_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(f, bp);
+        if (f.img4)
+            fuzzy_dt_pack_kernel<<<ctx->sm_count * 16, 256, 0, st>>>(f, bp);
+        else
+            fuzzy_dt_background_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(f, bp);
         const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         if (ctas > 0)
         {
