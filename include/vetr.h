@@ -413,7 +413,7 @@ int vetr_scan_counts_static(int device, void* cuda_stream, const int32_t* counts
 enum
 {
     VETR_T_COUNT = 0,    /* project + count */
-    VETR_T_SCAN,         /* the three scan kernels */
+    VETR_T_SCAN,         /* the two scan kernels */
     VETR_T_COLLECT,      /* project + collect */
     VETR_T_SORT_BLEND,   /* sort + blend */
     VETR_T_BACKWARD,     /* backward */

@@ -438,9 +438,75 @@ __device__ __forceinline__ void scan_tile(const int* in, long long base, long lo
     for (int r = 0; r < 4; ++r) before[r] += s_warp[r * 8 + warp];
 }
 
+// True in the last block of a grid to come here (in all its threads): what the blocks before it wrote is then visible to it.
+// *ticket is 0 before.
+__device__ __forceinline__ bool last_block(unsigned* ticket)
+{
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last;
+}
+
+// One block: exclusive scan of the tile sums in place; writes F, the overflow flag and the number of work items.
+__device__ void scan_spine(long long* tile_sums, int n_tiles, long long n_pixels, long long capacity, int* status, int* item_start)
+{
+    constexpr int kEach = 8;  // consecutive tiles per thread
+    __shared__ long long s_warp[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long carry = 0;
+    for (int base = 0; base < n_tiles; base += 256 * kEach)
+    {
+        const int first = base + threadIdx.x * kEach;
+        long long v[kEach], own = 0;
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+        {
+            v[k] = first + k < n_tiles ? __ldcg(tile_sums + first + k) : 0;
+            own += v[k];
+        }
+        long long inc = own;
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        __syncthreads();  // the previous round's sums have been read
+        if (lane == 31) s_warp[warp] = inc;
+        __syncthreads();
+        long long run = carry + inc - own;
+        for (int w = 0; w < 8; ++w)
+        {
+            if (w < warp) run += s_warp[w];
+            carry += s_warp[w];
+        }
+#pragma unroll
+        for (int k = 0; k < kEach; ++k)
+        {
+            if (first + k < n_tiles) tile_sums[first + k] = run;
+            run += v[k];
+        }
+    }
+    if (threadIdx.x == 0)
+    {
+        const long long F   = carry;
+        const bool overflow = F > capacity || F > 0x7fffffffLL;
+        status[0]           = (int)(F > 0x7fffffffLL ? 0x7fffffffLL : F);
+        status[1]           = overflow ? 1 : 0;
+        const long long work = F + (long long)kPixelWork * n_pixels;
+        const int items      = overflow ? 0 : (int)((work + kQuantum - 1) / kQuantum);
+        status[3]            = items;
+        item_start[items]    = (int)n_pixels;  // sentinel
+    }
+}
+
+// Sums of the tiles; the last block to finish scans them (a launch of its own for that cost a small scene as much as the tiles).
 template <bool kVec>
-__global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restrict__ counts, long long n,
-                                                             long long* __restrict__ tile_sums, int* status)
+__global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restrict__ counts, long long n, long long* tile_sums, int* status,
+                                                             long long capacity, int* item_start, unsigned* ticket)
 {
     __shared__ long long s_sum[8];
     __shared__ int s_max[8];
@@ -467,57 +533,7 @@ __global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restri
         tile_sums[blockIdx.x] = sum;
         if (mx > 0) atomicMax(status + 2, mx);
     }
-}
-
-// One CTA: exclusive scan of the tile sums in place; writes F, the overflow flag and the number of work items.
-__global__ void __launch_bounds__(1024) scan_spine_kernel(long long* tile_sums, int n_tiles, long long n_pixels,
-                                                          long long capacity, int* status, int* item_start)
-{
-    __shared__ long long s_warp[32];
-    __shared__ long long s_carry;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (int base = 0; base < n_tiles; base += 1024)
-    {
-        int i         = base + threadIdx.x;
-        long long v   = i < n_tiles ? tile_sums[i] : 0;
-        long long inc = v;
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            long long t = __shfl_up_sync(0xffffffffu, inc, o);
-            if ((threadIdx.x & 31) >= o) inc += t;
-        }
-        if ((threadIdx.x & 31) == 31) s_warp[threadIdx.x >> 5] = inc;
-        __syncthreads();
-        if (threadIdx.x < 32)
-        {
-            long long w = s_warp[threadIdx.x];
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                long long t = __shfl_up_sync(0xffffffffu, w, o);
-                if (threadIdx.x >= o) w += t;
-            }
-            s_warp[threadIdx.x] = w;
-        }
-        __syncthreads();
-        long long carry  = s_carry;
-        long long before = carry + (threadIdx.x >= 32 ? s_warp[(threadIdx.x >> 5) - 1] : 0) + inc - v;
-        if (i < n_tiles) tile_sums[i] = before;
-        __syncthreads();
-        if (threadIdx.x == 1023) s_carry = carry + s_warp[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-    {
-        long long F   = s_carry;
-        bool overflow = F > capacity || F > 0x7fffffffLL;
-        status[0]     = (int)(F > 0x7fffffffLL ? 0x7fffffffLL : F);
-        status[1]     = overflow ? 1 : 0;
-        long long work = F + (long long)kPixelWork * n_pixels;
-        int items      = overflow ? 0 : (int)((work + kQuantum - 1) / kQuantum);
-        status[3]      = items;
-        item_start[items] = (int)n_pixels;  // sentinel
-    }
+    if (last_block(ticket)) scan_spine(tile_sums, (int)gridDim.x, n, capacity, status, item_start);
 }
 
 // Writes the exclusive offsets and cuts the pixel space into work items: with work(p) = end(p) + kPixelWork*(p+1)
@@ -3030,7 +3046,7 @@ static int ensure_scratch(vetr_ctx* ctx, long long n_tiles)
         if (ctx->tile_sums) cudaFree(ctx->tile_sums);
         ctx->tile_sums = nullptr;
         long long cap  = n_tiles + n_tiles / 4 + 16;
-        VETR_CUDA(ctx, cudaMalloc(&ctx->tile_sums, cap * sizeof(long long)));
+        VETR_CUDA(ctx, cudaMalloc(&ctx->tile_sums, (cap + 1) * sizeof(long long)));  // and the ticket
         ctx->tile_cap = cap;
     }
     return VETR_OK;
@@ -3182,12 +3198,11 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
 }
 
 // Launches zero_buffers_kernel on the context's stream; `bytes` are multiples of 4, as are the addresses.
-static void launch_scan(const int* counts, long long n, long long capacity, long long* tile_sums, int n_tiles, int* ends, int* status,
-                        int* items, cudaStream_t st)
+static void launch_scan(const int* counts, long long n, long long capacity, long long* tile_sums, unsigned* ticket, int n_tiles, int* ends,
+                        int* status, int* items, cudaStream_t st)
 {
     const bool vec = (((uintptr_t)counts | (uintptr_t)ends) & 15) == 0;
-    (vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, status);
-    scan_spine_kernel<<<1, 1024, 0, st>>>(tile_sums, n_tiles, n, capacity, status, items);
+    (vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, status, capacity, items, ticket);
     (vec ? scan_apply_kernel<true> : scan_apply_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, ends, status, items);
 }
 
@@ -3264,9 +3279,9 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         return VETR_OK;
     }
     {
-        void* const buffers[2] = {f.counts, f.status};
-        const int64_t bytes[2] = {(int64_t)(f.PT * sizeof(int)), 4 * sizeof(int)};
-        rc = zero_buffers(ctx, buffers, bytes, 2);
+        void* const buffers[3] = {f.counts, f.status, ctx->tile_sums + ctx->tile_cap};
+        const int64_t bytes[3] = {(int64_t)(f.PT * sizeof(int)), 4 * sizeof(int), sizeof(long long)};
+        rc = zero_buffers(ctx, buffers, bytes, 3);
         if (rc != VETR_OK) return rc;
     }
     const int point_ctas = (f.n + kProjThreads * kPointsPerThread - 1) / (kProjThreads * kPointsPerThread);
@@ -3277,8 +3292,8 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     }
     const int n_tiles = (int)((f.PT + kScanTile - 1) / kScanTile);
     {
-        PassScope t(ctx, VETR_T_SCAN, 3);
-        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, n_tiles, f.ends, f.status, f.item_start, st);
+        PassScope t(ctx, VETR_T_SCAN, 2);
+        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, st);
     }
     if (point_ctas > 0)
     {
@@ -3943,7 +3958,7 @@ extern "C" int vetr_read_status(vetr_ctx* ctx, const vetr_lists* lists, int64_t*
 namespace vetr
 {
 constexpr int kStaticScanTiles = 16384;  // 16384 tiles x 4096 pixels = 67 108 864 pixels per call
-static __device__ __align__(256) long long g_static_tile_sums[kStaticScanTiles];
+static __device__ __align__(256) long long g_static_tile_sums[kStaticScanTiles + 1];  // and the ticket
 }  // namespace vetr
 static long long* g_static_tile_ptr[64] = {};  // device address of the array above, per device ordinal
 
@@ -3980,7 +3995,8 @@ extern "C" int vetr_scan_counts_static(int device, void* cuda_stream, const int3
     cudaStream_t st      = (cudaStream_t)cuda_stream;
     // the status words are accumulated into (longest list is an atomic maximum): start them at zero
     if (cudaMemsetAsync(status, 0, 4 * sizeof(int), st) != cudaSuccess) return VETR_E_CUDA;
-    launch_scan(counts, n_pixels, capacity, tile_sums, (int)n_tiles, ends, status, items, st);
+    if (cudaMemsetAsync(tile_sums + kStaticScanTiles, 0, sizeof(long long), st) != cudaSuccess) return VETR_E_CUDA;
+    launch_scan(counts, n_pixels, capacity, tile_sums, reinterpret_cast<unsigned*>(tile_sums + kStaticScanTiles), (int)n_tiles, ends, status, items, st);
     return cudaGetLastError() == cudaSuccess ? VETR_OK : VETR_E_CUDA;
 }
 
