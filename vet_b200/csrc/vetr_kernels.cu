@@ -210,25 +210,31 @@ __device__ __forceinline__ bool point_is_live(const Frame& f, int b, int pid)
     return true;
 }
 
+// The collection waits for its atomics (54 % of the issue slots), so it wants warps: blocks of 128 threads, twelve per SM (42
+// registers).  8 M points x 4 views: 648 us (656 with the positions requested behind the camera); six, seven or eight blocks of
+// 256: 671, 664, 664, fourteen of 128: 659, twenty-four of 64: 653, five of 256: 725.  The count pass is bound by instruction
+// issue (82 %) and stays at 256 threads: 321 us, six blocks 319, twelve of 128 341.
+constexpr int kCollectThreads = 128, kCollectCtas = 12;
 template <bool kCollect, int kPts>
-__global__ void __launch_bounds__(kProjThreads) project_kernel(const __grid_constant__ Frame f)
+__global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCollect ? kCollectCtas : 5) project_kernel(const __grid_constant__ Frame f)
 {
+    constexpr int kThreadsHere = kCollect ? kCollectThreads : kProjThreads;
     __shared__ Camera s_cam;
-    const int b = blockIdx.y;
+    const int b     = blockIdx.y;
+    const int first = blockIdx.x * (kThreadsHere * kPts) + threadIdx.x;
+
+    float4 pos[kPts];  // requested before the camera, which the block waits for
+#pragma unroll
+    for (int it = 0; it < kPts; ++it)
+    {
+        const int pid = first + it * kThreadsHere;
+        pos[it]       = pid < f.n ? __ldg(f.position + pid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     if (threadIdx.x == 0) s_cam = load_camera(f, b);
     __syncthreads();
     const Camera& cam   = s_cam;
     const int vbase     = b * (int)f.P;
     const bool bilinear = f.mode == VETR_MODE_BILINEAR_BLEND;
-    const int first     = blockIdx.x * (kProjThreads * kPts) + threadIdx.x;
-
-    float4 pos[kPts];
-#pragma unroll
-    for (int it = 0; it < kPts; ++it)
-    {
-        const int pid = first + it * kProjThreads;
-        pos[it]       = pid < f.n ? __ldg(f.position + pid) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
 
     if (!bilinear)
     {
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(kProjThreads) project_kernel(const __grid_cons
 #pragma unroll
         for (int it = 0; it < kPts; ++it)
         {
-            const int pid = first + it * kProjThreads;
+            const int pid = first + it * kThreadsHere;
 #pragma unroll
             for (int l = 0; l < VETR_MAX_LAYERS; ++l) g[it][l] = -1;
             zbits[it] = 0;
@@ -282,7 +288,7 @@ __global__ void __launch_bounds__(kProjThreads) project_kernel(const __grid_cons
 #pragma unroll
         for (int it = 0; it < kPts; ++it)
         {
-            const int pid = first + it * kProjThreads;
+            const int pid = first + it * kThreadsHere;
             if (pid >= f.n) break;
             unsigned bits = 0;
 #pragma unroll
@@ -310,7 +316,7 @@ __global__ void __launch_bounds__(kProjThreads) project_kernel(const __grid_cons
 #pragma unroll
     for (int it = 0; it < kPts; ++it)
     {
-        const int pid = first + it * kProjThreads;
+        const int pid = first + it * kThreadsHere;
         if (pid >= f.n) break;
         unsigned level_bits = 0;
         Projected pr;
@@ -3298,8 +3304,8 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     if (point_ctas > 0)
     {
         PassScope t(ctx, VETR_T_COLLECT, 1);
-        const int ctas = (f.n + kProjThreads * kCollectPoints - 1) / (kProjThreads * kCollectPoints);
-        project_kernel<true, kCollectPoints><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f);
+        const int ctas = (f.n + kCollectThreads * kCollectPoints - 1) / (kCollectThreads * kCollectPoints);
+        project_kernel<true, kCollectPoints><<<dim3(ctas, n_views), kCollectThreads, 0, st>>>(f);
     }
     {
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
