@@ -381,3 +381,26 @@ def test_grid_loss_cells_around_the_edges_of_the_view(rasterizer, crop):
     assert (ref_c > 0).sum() > 1000 and (ref_c == 0).sum() > 1000
     np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
+# ---- mode 0 without camera gradients: the pixels of all levels are looked up together
+
+
+@pytest.mark.parametrize("layers, ghost, by_radius", [(1, 0, 1), (4, 1, 1), (5, 0, 0), (5, 0, 1)])
+def test_mode0_backward_without_cameras(rasterizer, layers, ghost, by_radius):
+    """Against the oracle; counts of hits per point and which descriptors are reached are exact."""
+    sc = scenes.tiny_scene(n=9000, w=93, h=61, n_views=2, seed=13, crop=True)
+    dropout = (np.random.default_rng(2).random((2, sc.n)) < 0.2).astype(np.float32)
+    params = default_params(render_mode=0, num_layers=layers, ghost_gradients=ghost, drop_out_points_by_radius=by_radius)
+    ora = util.run_oracle(sc, params, dropout=dropout)
+    grads = util.random_grads(ora["fwd"]["color"], seed=3)
+    ora = util.run_oracle(sc, params, grads=grads, dropout=dropout)
+    gpu = util.run_gpu(rasterizer, sc, params, grads=grads, dropout=dropout)
+    import torch
+
+    on = [torch.from_numpy(g).to(rasterizer.device) for g in grads]
+    plain = rasterizer.backward_raw(on, want_pose=False, want_intrinsics=False)
+    raw = dict(gpu["bwd_raw"], **{k: v.cpu().numpy() for k, v in plain.items()})
+    # the bound of the other mode-0 tests (see test_mode0_backward_scratch)
+    util.compare_backward(raw, ora, 4, rtol=2e-5, floor_rel=1e-6)
+    assert np.array_equal(raw["points"][:, 3], gpu["bwd_raw"]["points"][:, 3]) and raw["points"][:, 3].sum() > 0
