@@ -84,3 +84,29 @@ def test_gpu_many_arrays_of_all_widths(n):
     for g, a in zip(got_first, first):
         assert np.array_equal(g.cpu().numpy(), a[keep])
     rast.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 2500])
+@pytest.mark.parametrize("width", [2, 3, 5, 7, 8, 16, 33, 64, 255, 256, 257, 4095, 4097])
+def test_gpu_wide_rows(n, width):
+    """Rows of any width, cut into pieces: widths beside the 256 threads of a block and the 4096 words of a piece, several rows of
+    rows, a last block that the points do not fill."""
+    from vet_b200 import _lib as L
+    from vet_b200.render import Rasterizer
+
+    rows = 2 if n * width < 1_000_000 else 1
+    rng = np.random.default_rng(n * 10007 + width)
+    src = torch.from_numpy(rng.integers(-2**31, 2**31, size=(rows, n, width)).astype(np.int32)).cuda()
+    gone = rng.random(n) < 0.3
+    new_index = np.where(gone, -1, np.cumsum(~gone) - 1).astype(np.int32)
+    kept = int((~gone).sum())
+    dst = torch.full((rows, kept + 1, width), 7, dtype=torch.int32, device="cuda")  # one element more: not to be written
+    rast = Rasterizer(0)
+    index = torch.from_numpy(new_index).cuda()
+    array = L.PointArray(src.data_ptr(), dst.data_ptr(), rows, width)
+    assert L.lib().vetr_gather_points(rast._ctx, n, kept, index.data_ptr(), array, 1) == L.OK
+    got = dst.cpu().numpy().reshape(-1)
+    want = src.cpu().numpy()[:, ~gone].reshape(-1)
+    assert np.array_equal(got[:want.size], want) and (got[want.size:] == 7).all()
+    rast.close()

@@ -37,6 +37,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <limits>
 #include <new>
 #include <vector>
 
@@ -3893,6 +3894,39 @@ extern "C" int vetr_remove_points_plan(vetr_ctx* ctx, int n, const int64_t* remo
     return VETR_OK;
 }
 
+// Launches `kernel` for the arrays of which a row is units_of(width) > 0 units of work, up to kGatherArrays of them at a time.
+template <typename Total, typename Kernel, typename Units>
+static void gather_arrays(vetr_ctx* ctx, Kernel kernel, int n, int n_kept, const int32_t* new_index, const vetr_point_array* arrays, int n_arrays,
+                          Units units_of)
+{
+    GatherArgs<Total> g;
+    memset(&g, 0, sizeof(g));
+    g.new_index = new_index, g.n = n, g.n_kept = n_kept;
+    long long total   = 0;
+    const auto launch = [&]()
+    {
+        if (g.arrays == 0) return;
+        const int blocks = (int)(((long long)n + kGatherBlock - 1) / kGatherBlock);
+        const int share  = std::max(1, ctx->sm_count * 16 / blocks);  // sixteen blocks per SM
+        kernel<<<dim3(blocks, (unsigned)std::min<long long>(std::min(share, 65535), total)), 256, 0, ctx->stream>>>(g);
+        ctx->launches += 1;
+        g.arrays = 0, total = 0;
+    };
+    for (int k = 0; k < n_arrays; ++k)
+    {
+        const vetr_point_array& a = arrays[k];
+        const long long units     = (long long)a.rows * units_of(a.width);
+        if (units == 0) continue;
+        // a launch when the table is full, and where one more array would leave the counter's range
+        if (g.arrays == kGatherArrays || total + units > (long long)std::numeric_limits<Total>::max()) launch();
+        total += units;
+        g.src[g.arrays] = (const uint32_t*)a.src, g.dst[g.arrays] = (uint32_t*)a.dst;
+        g.end[g.arrays] = (Total)total, g.width[g.arrays] = a.width;
+        ++g.arrays;
+    }
+    launch();
+}
+
 extern "C" int vetr_gather_points(vetr_ctx* ctx, int n, int n_kept, const int32_t* new_index, const vetr_point_array* arrays, int n_arrays)
 {
     if (!ctx || n < 0 || n_kept < 0 || n_kept > n || n_arrays < 0 || (n_arrays > 0 && !arrays) || (n > 0 && !new_index))
@@ -3905,25 +3939,9 @@ extern "C" int vetr_gather_points(vetr_ctx* ctx, int n, int n_kept, const int32_
     }
     if (n == 0 || n_kept == 0) return VETR_OK;
     VETR_CUDA(ctx, cudaSetDevice(ctx->device));
-    GatherArgs g;
-    memset(&g, 0, sizeof(g));
-    g.new_index = new_index, g.n = n, g.n_kept = n_kept;
-    long long rows = 0;
-    for (int k = 0; k < n_arrays; ++k)
-    {
-        const vetr_point_array& a = arrays[k];
-        rows += a.rows;
-        g.src[g.arrays] = (const uint32_t*)a.src, g.dst[g.arrays] = (uint32_t*)a.dst;
-        g.row_end[g.arrays] = (int)rows, g.width[g.arrays] = a.width;
-        ++g.arrays;
-        // a launch when the table is full, at the end, and where one more array would leave the row counter's range
-        if (g.arrays < kGatherArrays && k + 1 < n_arrays && rows + arrays[k + 1].rows <= 0x7fffffff) continue;
-        const int blocks = (int)((n + 256ll * kGatherPoints - 1) / (256 * kGatherPoints));
-        const int share  = std::max(1, ctx->sm_count * 16 / blocks);  // sixteen blocks per SM
-        points_gather_kernel<<<dim3(blocks, (unsigned)std::min<long long>(std::min(share, 65535), rows)), 256, 0, ctx->stream>>>(g);
-        ctx->launches += 1;
-        g.arrays = 0, rows = 0;
-    }
+    gather_arrays<int>(ctx, points_gather_kernel, n, n_kept, new_index, arrays, n_arrays, [](int width) { return width <= kGatherNarrow ? 1 : 0; });
+    gather_arrays<long long>(ctx, points_gather_pieces_kernel, n, n_kept, new_index, arrays, n_arrays,
+                             [](int width) { return width <= kGatherNarrow ? 0 : gather_pieces(width); });
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }
