@@ -383,6 +383,29 @@ def test_grid_loss_cells_around_the_edges_of_the_view(rasterizer, crop):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("n", [28 * 28416 - 4, 28 * 28416 + 4, 1_000_001])
+def test_grid_loss_many_cells(rasterizer, n):
+    """Cell numbers around and above the one from which on groups are looked at first on 148 SMs (28 groups of four for each of 7104
+    warps): small and large boxes around the camera and the border of the image; coverage is exact."""
+    import torch
+
+    w, h = 321, 243
+    sc = scenes.config_planar(64, w, h, 200.0, n_views=1, seed=3)
+    rng = np.random.default_rng(n)
+    centre = np.repeat(rng.uniform(-12, 12, size=(n // 4 + 1, 3)), 4, axis=0)[:n]
+    size = np.repeat(10.0 ** rng.uniform(-2.5, 0.2, size=(n // 4 + 1, 1)), 4, axis=0)[:n]
+    bb_min = (centre + size * rng.uniform(-1, 1, size=(n, 3))).astype(np.float32)
+    bb_len = np.broadcast_to(size, (n, 3)).astype(np.float32).copy()
+    loss = rng.standard_normal((3, h, w)).astype(np.float32)
+    ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    assert (ref_c > 0).sum() > 10_000 and (ref_c == 0).sum() > 10_000
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+    np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
 # ---- mode 0 without camera gradients: the pixels of all levels are looked up together
 
 

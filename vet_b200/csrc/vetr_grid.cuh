@@ -571,11 +571,17 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
     return number && out;
 }
 
-// First kernel: one warp per group of four cells.  A warp's next 32 groups are looked at first, a lane each: groups that lie
+// First kernel: one warp per group of four cells.  kCull: a warp's next 32 groups are looked at first, a lane each; groups that lie
 // altogether out of sight are left out before their corners are projected, which costs about 200 instructions per group.
-// 128^3 cells, 1920x1080: grid_loss_kernel 682 -> 592 us.  Cells with many rows (next to the camera a cell covers 10^5 pixels) and
-// large rectangles in the per-pixel form are cut into chunks that go to a queue, so that the second kernel can spread them
-// over all SMs.  If the queue is full the warp does the whole cell itself.
+// Cells with many rows (next to the camera a cell covers 10^5 pixels) and large rectangles in the per-pixel form are cut into
+// chunks that go to a queue, so that the second kernel can spread them over all SMs.  If the queue is full the warp does the
+// whole cell itself.
+//
+// Looking ahead wants groups to look at: with few per warp it saves less than the second reading of the boxes and the half-spaces cost.
+// The whole call, 1920x1080, without and with it: camera on an orbit inside the grid 80^3 cells (18 groups a warp) 615 and 642 us,
+// 96^3 (31) 739 and 725, 128^3 (74) 1036 and 984; all cells in sight 64^3 (9) 197 and 203, 80^3 309 and 321, 128^3 907 and 937.
+constexpr int kGridCullGroups = 28;  // groups per warp from which on the launch takes kCull
+template <bool kCull>
 __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
                                                                      int2* queue, int* queue_count)
 {
@@ -587,9 +593,12 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
     GridWarpSmem& s    = s_warp[warp];
     const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
     const int n_groups = (a.n_cells + kGridGroup - 1) / kGridGroup, stride = gridDim.x * kGridWarps;
-    __shared__ GridPlane s_planes[kGridPlanes];
-    if (threadIdx.x < kGridPlanes) s_planes[threadIdx.x] = grid_plane(a, s_cam, threadIdx.x);
-    __syncthreads();
+    __shared__ GridPlane s_planes[kCull ? kGridPlanes : 1];
+    if (kCull)
+    {
+        if (threadIdx.x < kGridPlanes) s_planes[threadIdx.x] = grid_plane(a, s_cam, threadIdx.x);
+        __syncthreads();
+    }
     unsigned todo = 0;  // groups first + k stride still to do (bit k)
     int first = blockIdx.x * kGridWarps + warp - 32 * stride;
     for (;;)
@@ -599,7 +608,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
             first += 32 * stride;
             if (first >= n_groups) break;
             const int mine = first + lane * stride;
-            todo = __ballot_sync(0xffffffffu, mine < n_groups && (s_cam.has_dist || !grid_out_of_sight(a, s_planes, mine)));
+            todo = __ballot_sync(0xffffffffu, mine < n_groups && (!kCull || s_cam.has_dist || !grid_out_of_sight(a, s_planes, mine)));
             continue;
         }
         const int group = first + (__ffs(todo) - 1) * stride;
