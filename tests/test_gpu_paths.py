@@ -427,3 +427,26 @@ def test_mode0_backward_without_cameras(rasterizer, layers, ghost, by_radius):
     # the bound of the other mode-0 tests (see test_mode0_backward_scratch)
     util.compare_backward(raw, ora, 4, rtol=2e-5, floor_rel=1e-6)
     assert np.array_equal(raw["points"][:, 3], gpu["bwd_raw"]["points"][:, 3]) and raw["points"][:, 3].sum() > 0
+
+
+def test_calls_after_close_are_refused():
+    """Every call of a closed rasterizer raises VetrError with the library's status for a missing context."""
+    import torch
+    from vet_b200 import _lib as L
+    from vet_b200.render import Rasterizer, scene_to_device
+
+    rast = Rasterizer(0)
+    sc = scenes.tiny_scene(n=500, w=40, h=32, n_views=1, seed=3)
+    tensors = scene_to_device(sc, rast.device)
+    fwd = rast.forward(*tensors, sc.views, default_params())
+    grads, loss = [torch.ones_like(c) for c in fwd["color"]], torch.zeros((), device=rast.device)
+    raw = rast.backward_raw(grads)
+    torch.cuda.synchronize()
+    rast.close()
+    calls = [lambda: rast.forward(*tensors, sc.views, default_params()), lambda: rast.backward_raw(grads),
+             lambda: rast.backward_raw(grads, accum=raw), lambda: rast.finalize(raw),
+             lambda: rast.l1_loss_grad(fwd["color"], grads, grads, loss)]
+    for call in calls:
+        with pytest.raises(L.VetrError) as e:
+            call()
+        assert e.value.status == L.E_INVALID_ARG

@@ -129,6 +129,10 @@ class Rasterizer:
             raise L.VetrError(rc, where, L.lib().vetr_last_cuda_error(self._ctx))
 
     # ---- helpers -----------------------------------------------------------------------------------------
+    def _context(self) -> int:
+        """The context's address for the native host side; 0 after close(), which the library refuses."""
+        return self._ctx.value or 0
+
     def _views(self, views):
         arr = (L.View * len(views))()
         L.host().views(C.addressof(arr), views)
@@ -169,7 +173,7 @@ class Rasterizer:
             if prm.render_mode == 3 or (prm.render_mode in (1, 2) and prm.need_point_gradient):
                 lists.ensure_level_mask(nb * position.shape[0])
             varr = self._views(views[b0:b1])
-            rc = host.forward(self._ctx.value, C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
+            rc = host.forward(self._context(), C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
                               C.addressof(varr), nb, b0, dropout, C.addressof(lists.c), Ln, color, weight, mask, depth)
             self._check(rc, "vetr_forward")
             groups.append((b0, b1, lists, varr))
@@ -215,7 +219,7 @@ class Rasterizer:
         s = self._saved
         host = L.host()
         self._sync_stream()
-        ctx = self._ctx.value
+        ctx = self._context()
         position, index, texture = s["tensors"][0], s["tensors"][1], s["tensors"][2]
         poses, intrinsics, dropout = s["tensors"][5], s["tensors"][6], s["tensors"][7]
         n, n_tex, Cn = position.shape[0], texture.shape[1], texture.shape[0]
@@ -247,7 +251,7 @@ class Rasterizer:
         [1,n_tex], background [C], points [n,4] averaged by hit count, pose tangent and intrinsics averaged."""
         self._sync_stream()
         pts, pose, intr = g.get("points"), g.get("pose"), g.get("intrinsics")
-        g_texture = L.host().finalize(self._ctx.value, self.device, g["background"].shape[0], g["desc"], pts, pose,
+        g_texture = L.host().finalize(self._context(), self.device, g["background"].shape[0], g["desc"], pts, pose,
                                       g.get("pose_count"), intr, g.get("intrinsics_count"))
         if isinstance(g_texture, int):
             self._check(g_texture, "vetr_finalize_gradients")
@@ -364,7 +368,7 @@ class Rasterizer:
     def l1_loss_grad(self, images, targets, grads, loss):
         """loss (device scalar) = sum over levels of mean |image - target|; grads[l] = sign(image - target) / numel, one launch."""
         self._sync_stream()
-        self._check(L.host().l1_loss_grad(self._ctx.value, images, targets, grads, loss), "vetr_l1_loss_grad")
+        self._check(L.host().l1_loss_grad(self._context(), images, targets, grads, loss), "vetr_l1_loss_grad")
 
     def set_timing(self, enable: bool):
         self._sync_stream()
