@@ -59,3 +59,14 @@ def test_wrong_arguments_raise():
     with pytest.raises(ValueError):
         L.host().l1_loss_grad(8, [t, t], [t], [t, t], t)  # a target too few
     assert L.host().l1_loss_grad(8, [t] * 6, [t] * 6, [t] * 6, t) == L.E_INVALID_ARG
+
+
+def test_crop_and_rotation_with_too_many_entries():
+    """The rasterizer answers as an array does that is given too many initialisers; fewer leave the rest at zero."""
+    from vet_b200.render import Rasterizer
+
+    for bad in (View(8, 8, crop=(1.0,) * 6), View(8, 8, rot=(1.0,) * 5)):
+        with pytest.raises(IndexError):
+            Rasterizer._views(None, [bad])
+    arr = Rasterizer._views(None, [View(8, 8, crop=(1, 2, 3), rot=())])
+    assert list(arr[0].crop) == [1, 2, 3, 0, 0] and list(arr[0].rot) == [0, 0, 0, 0]

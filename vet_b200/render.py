@@ -135,7 +135,10 @@ class Rasterizer:
 
     def _views(self, views):
         arr = (L.View * len(views))()
-        L.host().views(C.addressof(arr), views)
+        try:
+            L.host().views(C.addressof(arr), views)
+        except ValueError as e:  # more entries of crop or rot than there are
+            raise IndexError(str(e)) from None
         return arr
 
     def _lists(self, slot: int, n_pixels_total: int, capacity: int, exact: bool = False) -> FragmentLists:
