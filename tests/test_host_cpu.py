@@ -70,3 +70,108 @@ def test_crop_and_rotation_with_too_many_entries():
             Rasterizer._views(None, [bad])
     arr = Rasterizer._views(None, [View(8, 8, crop=(1, 2, 3), rot=())])
     assert list(arr[0].crop) == [1, 2, 3, 0, 0] and list(arr[0].rot) == [0, 0, 0, 0]
+
+
+class _Array:
+    """Device memory of another library: a tensor's methods, but not a torch.Tensor."""
+
+    def __init__(self, t):
+        self.t, self.shape = t, tuple(t.shape)
+
+    def data_ptr(self):
+        return self.t.data_ptr()
+
+    def numel(self):
+        return self.t.numel()
+
+    def __getitem__(self, k):
+        return _Array(self.t[k])
+
+
+class _SubTensor(torch.Tensor):
+    pass
+
+
+@pytest.fixture
+def recorded():
+    """The native host side bound to functions that record what they are given; bound to the library again afterwards."""
+    import vet_b200._lib as lib
+
+    calls = []
+
+    def fake(name, n):
+        @C.CFUNCTYPE(C.c_int, *[C.c_void_p] * n)
+        def f(*a):
+            calls.append((name, a))
+            return 0
+        return f
+
+    fakes = [fake("forward", 13), fake("backward", 20), fake("finalize", 14), fake("l1", 7), fake("zero", 4)]
+    L.host().bind(*[C.cast(f, C.c_void_p).value for f in fakes])
+    yield calls
+    lib._bound = None
+    lib.host()
+
+
+def _levels(address, n):
+    return [C.c_void_p.from_address(address + 8 * k).value for k in range(n)]
+
+
+@pytest.mark.parametrize("kind", [lambda t: t, _Array, lambda t: t.as_subclass(_SubTensor), torch.nn.Parameter])
+@pytest.mark.parametrize("b0", [0, 8])
+def test_addresses_of_a_group_of_views(recorded, kind, b0):
+    """Views from b0 on: images, drop-out flags and gradients start at view b0, whatever kind of tensor they come in."""
+    host, views = L.host(), 11
+    img = [torch.zeros(views, 4, 6 >> l, 8 >> l) for l in range(2)]
+    plane = [torch.zeros(views, 1, 6 >> l, 8 >> l) for l in range(2)]
+    drop = torch.zeros(views, 33)
+    want = lambda ts: [t[b0:].data_ptr() for t in ts]  # noqa: E731
+    frame = (1, 2, 3, 4, 5, 6, 3, b0, kind(drop), 7, 2)
+    tables = {}  # the level tables live on the native stack, so they are read during the call
+
+    @C.CFUNCTYPE(C.c_int, *[C.c_void_p] * 13)
+    def forward(*a):
+        tables["dropout"] = a[7]
+        tables["forward"] = [_levels(p, 2) for p in a[9:13]]
+        return 0
+
+    @C.CFUNCTYPE(C.c_int, *[C.c_void_p] * 20)
+    def backward(*a):
+        tables["backward"] = [_levels(p, 2) for p in a[9:11]]
+        tables["gradients"] = a[11:19]
+        tables["dropout_backward"] = a[7]
+        return 0
+
+    names = ("vetr_finalize_gradients", "vetr_l1_loss_grad", "vetr_zero_buffers")
+    host.bind(C.cast(forward, C.c_void_p).value, C.cast(backward, C.c_void_p).value,
+              *[C.cast(getattr(L.lib(), n), C.c_void_p).value for n in names])
+    ts = lambda x: [kind(t) for t in x]  # noqa: E731
+    assert host.forward(*frame, ts(img), ts(plane), ts(plane), ts(plane)) == 0
+    assert tables["dropout"] == drop[b0:].data_ptr()
+    assert tables["forward"] == [want(img)] + [want(plane)] * 3
+    grads = [torch.zeros(5, 4), torch.zeros(5), torch.zeros(9, 4), torch.zeros(4)]
+    assert host.backward(*frame, ts(img), ts(img), *ts(grads), None, None, None, None, 3) == 0
+    assert tables["backward"] == [want(img)] * 2 and tables["dropout_backward"] == drop[b0:].data_ptr()
+    assert list(tables["gradients"]) == [t.data_ptr() for t in grads] + [None] * 4
+
+
+@pytest.mark.parametrize("kind", [lambda t: t, _Array, lambda t: t.as_subclass(_SubTensor)])
+def test_sizes_of_any_tensor(recorded, kind):
+    host = L.host()
+    out = host.finalize(1, torch.device("cpu"), 3, kind(torch.zeros(7, 4)), kind(torch.zeros(9, 4)), kind(torch.zeros(2, 6)),
+                        kind(torch.zeros(2)), kind(torch.zeros(3, 13)), kind(torch.zeros(3)))
+    assert tuple(out.shape) == (3, 7)
+    name, a = recorded[-1]
+    assert name == "finalize" and (a[2], a[5], a[8], a[11]) == (7, 9, 2, 3)
+    image = [torch.zeros(2, 4, 3, 5)]
+    assert host.l1_loss_grad(1, [kind(t) for t in image], [kind(t) for t in image], [kind(t) for t in image], kind(torch.zeros(()))) == 0
+    assert recorded[-1][0] == "l1" and recorded[-1][1][1] == 1
+    with pytest.raises(TypeError):
+        host.l1_loss_grad(1, [np.zeros(4)], image, image, image[0])
+
+
+def test_whole_numbers_are_cut_to_32_bits():
+    params = default_params(debug_max_list_length=2**70 + 5, viewer_only=True)
+    want, got = L.Params(**{k: params[k] for k, _ in L.Params._fields_}), L.Params()
+    L.host().params(C.addressof(got), params, 4)
+    assert got.debug_max_list_length == want.debug_max_list_length and got.viewer_only == want.viewer_only == 1

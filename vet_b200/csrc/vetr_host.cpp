@@ -41,6 +41,13 @@ long long integer(PyObject* o)
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
+int32_t whole(PyObject* o)  // anything with __index__, cut to 32 bits as ctypes does
+{
+    THPObjectPtr i            = held(PyNumber_Index(o));
+    const unsigned long long v = PyLong_AsUnsignedLongLongMask(i.get());
+    if (v == ~0ull && PyErr_Occurred()) throw python_error();
+    return (int32_t)v;
+}
 float real(PyObject* o)
 {
     const double v = PyFloat_AsDouble(o);
@@ -52,15 +59,47 @@ T* address(PyObject* o)
 {
     return reinterpret_cast<T*>(integer(o));
 }
-const at::Tensor& tensor(PyObject* o)
+// Tensors may be torch's own, or any object that answers to data_ptr() and the few others of a tensor's methods used here.
+const at::Tensor* plain_tensor(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+THPObjectPtr attribute(PyObject* o, const char* name)
 {
-    if (!THPVariable_Check(o)) throw torch::TypeError("expected a tensor");
-    return THPVariable_Unpack(o);
+    THPObjectPtr a(PyObject_GetAttrString(o, name));
+    if (!a && PyErr_ExceptionMatches(PyExc_AttributeError))
+    {
+        PyErr_Clear();
+        throw torch::TypeError("expected a tensor");
+    }
+    return held(a.release());
+}
+void* storage(PyObject* o)
+{
+    if (const at::Tensor* t = plain_tensor(o)) return t->data_ptr();
+    return address<void>(held(PyObject_CallNoArgs(attribute(o, "data_ptr").get())).get());
+}
+// The same from the first dimension's index b0 on.
+void* storage_from(PyObject* o, long long b0)
+{
+    if (b0 == 0) return storage(o);
+    if (const at::Tensor* t = plain_tensor(o)) return static_cast<char*>(t->data_ptr()) + b0 * t->stride(0) * (long long)t->element_size();
+    THPObjectPtr start = held(PyLong_FromLongLong(b0)), slice = held(PySlice_New(start.get(), nullptr, nullptr));
+    return storage(held(PyObject_GetItem(o, slice.get())).get());
+}
+long long numel(PyObject* o)
+{
+    if (const at::Tensor* t = plain_tensor(o)) return t->numel();
+    return integer(held(PyObject_CallNoArgs(attribute(o, "numel").get())).get());
+}
+int rows(PyObject* o)  // of a tensor, or 0 for None
+{
+    if (o == Py_None) return 0;
+    if (const at::Tensor* t = plain_tensor(o)) return (int)t->size(0);
+    THPObjectPtr shape = attribute(o, "shape");
+    return (int)integer(held(PySequence_GetItem(shape.get(), 0)).get());
 }
 template <typename T>
 T* data(PyObject* o)  // a tensor, or None
 {
-    return o == Py_None ? nullptr : static_cast<T*>(tensor(o).data_ptr());
+    return o == Py_None ? nullptr : static_cast<T*>(storage(o));
 }
 at::TensorOptions on(PyObject* device, at::ScalarType type = at::kFloat)
 {
@@ -79,11 +118,7 @@ struct Levels
         if (list == Py_None) return;
         THPObjectPtr items = sequence(list);
         require(levels <= VETR_MAX_LAYERS && PySequence_Fast_GET_SIZE(items.get()) >= levels, "one tensor per level");
-        for (int l = 0; l < levels; ++l)
-        {
-            const at::Tensor& t = tensor(PySequence_Fast_GET_ITEM(items.get(), l));
-            p[l] = static_cast<char*>(t.data_ptr()) + (b0 ? b0 * t.stride(0) * (long long)t.element_size() : 0);
-        }
+        for (int l = 0; l < levels; ++l) p[l] = storage_from(PySequence_Fast_GET_ITEM(items.get(), l), b0);
         given = true;
     }
     template <typename T>
@@ -155,7 +190,7 @@ PyObject* params(const Call& c)
         THPObjectPtr key = held(PyUnicode_InternFromString(name));
         return held(PyObject_GetItem(c[1], key.get()));
     };
-    const auto i = [&](const char* name) { return (int32_t)integer(held(PyNumber_Index(get(name).get())).get()); };
+    const auto i = [&](const char* name) { return whole(get(name).get()); };
     const auto f = [&](const char* name) { return real(get(name).get()); };
     p.render_mode = i("render_mode"), p.num_layers = i("num_layers"), i("num_channels"), p.num_channels = (int32_t)integer(c[2]);
     p.drop_out_points_by_radius = i("drop_out_points_by_radius"), p.drop_out_radius_threshold = f("drop_out_radius_threshold");
@@ -177,7 +212,7 @@ PyObject* views(const Call& c)
     for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(items.get()); ++k)
     {
         PyObject* v    = PySequence_Fast_GET_ITEM(items.get(), k);
-        const auto i   = [&](const char* name) { return (int32_t)integer(held(PyNumber_Index(held(PyObject_GetAttrString(v, name)).get())).get()); };
+        const auto i   = [&](const char* name) { return whole(held(PyObject_GetAttrString(v, name)).get()); };
         const auto f   = [&](const char* name, float* to, Py_ssize_t n)
         {
             THPObjectPtr a = held(PyObject_GetAttrString(v, name)), s = sequence(a.get());
@@ -210,10 +245,10 @@ struct Frame
     explicit Frame(const Call& c)
         : ctx(address<vetr_ctx>(c[0])), params(address<const vetr_params>(c[1])), cloud(address<const vetr_cloud>(c[2])),
           texture(address<const vetr_texture>(c[3])), cameras(address<const vetr_cameras>(c[4])), views(address<const vetr_view>(c[5])),
-          n_views((int)integer(c[6])), b0(integer(c[7])), dropout(data<const float>(c[8])), lists(address<const vetr_lists>(c[9])),
+          n_views((int)integer(c[6])), b0(integer(c[7])),
+          dropout(c[8] == Py_None ? nullptr : static_cast<const float*>(storage_from(c[8], b0))), lists(address<const vetr_lists>(c[9])),
           levels((int)integer(c[10]))
     {
-        if (dropout && b0) dropout += b0 * tensor(c[8]).stride(0);
     }
 };
 
@@ -284,10 +319,9 @@ PyObject* finalize(const Call& c)
 {
     c.expect(9);
     vetr_ctx* ctx   = address<vetr_ctx>(c[0]);
-    const int C     = (int)integer(c[2]), n_tex = (int)tensor(c[3]).size(0);
-    const auto rows = [&](int i) { return c[i] == Py_None ? 0 : (int)tensor(c[i]).size(0); };
+    const int C     = (int)integer(c[2]), n_tex = rows(c[3]);
     at::Tensor out  = at::empty({C, n_tex}, on(c[1]));
-    const int n = rows(4), n_img = rows(5), n_cam = rows(7);
+    const int n = rows(c[4]), n_img = rows(c[5]), n_cam = rows(c[7]);
     const float* desc       = data<const float>(c[3]);
     float *texture          = static_cast<float*>(out.data_ptr()), *points = data<float>(c[4]), *intr = data<float>(c[7]);
     double* pose            = data<double>(c[5]);
@@ -310,7 +344,7 @@ PyObject* l1_loss_grad(const Call& c)
     const int n = (int)PySequence_Fast_GET_SIZE(images.get());
     const Levels image(images.get(), 0, n), target(c[2], 0, n), grad(c[3], 0, n);
     int64_t numel[VETR_MAX_LAYERS] = {};
-    for (int l = 0; l < n; ++l) numel[l] = tensor(PySequence_Fast_GET_ITEM(images.get(), l)).numel();
+    for (int l = 0; l < n; ++l) numel[l] = ::numel(PySequence_Fast_GET_ITEM(images.get(), l));
     float* loss = data<float>(c[4]);
     int rc;
     Py_BEGIN_ALLOW_THREADS
