@@ -182,6 +182,24 @@ def test_many_views_grouped(rasterizer):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_many_views_grouped_step(rasterizer, mode):
+    """A batch of more views than one launch takes, with point drop-out: every image of the later group and what the backward pass
+    adds for it, against the oracle."""
+    views = 11
+    sc = scenes.tiny_scene(n=2500, w=44, h=36, n_views=views, seed=72, crop=True)
+    params = default_params(render_mode=mode, num_layers=3)
+    dropout = (np.random.default_rng(5).random((views, sc.n)) < 0.3).astype(np.float32)
+    if mode == 0:
+        _mode0_roundtrip(rasterizer, sc, params, dropout=dropout)
+        return
+    grads = util.random_grads(util.run_oracle(sc, params, dropout=dropout)["fwd"]["color"], seed=6)
+    ora = util.run_oracle(sc, params, grads=grads, dropout=dropout)
+    gpu = util.run_gpu(rasterizer, sc, params, grads=grads, dropout=dropout)
+    util.compare_forward(gpu, ora, exact_images=True)
+    util.compare_backward(gpu["bwd_raw"], ora, sc.channels)
+
+
 def test_plumbing_config_l1(rasterizer):
     """Configuration 1 of the benchmark set: 100k points, one 512x512 view, L1 loss against a seeded target."""
     sc = scenes.config_plumbing()
