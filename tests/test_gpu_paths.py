@@ -450,3 +450,24 @@ def test_calls_after_close_are_refused():
         with pytest.raises(L.VetrError) as e:
             call()
         assert e.value.status == L.E_INVALID_ARG
+
+
+def test_follows_the_current_stream(monkeypatch):
+    """Kernels go to torch's current stream, which is asked for through public interfaces only."""
+    import torch
+    from vet_b200.render import Rasterizer, scene_to_device
+
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    rast = Rasterizer(0)
+    sc = scenes.tiny_scene(n=500, w=40, h=32, n_views=1, seed=3)
+    tensors = scene_to_device(sc, rast.device)
+    want = rast.forward(*tensors, sc.views, default_params())["color"][0].clone()
+    assert rast._cur_stream == torch.cuda.current_stream(rast.device).cuda_stream
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream(rast.device)
+    with torch.cuda.stream(side):
+        got = rast.forward(*tensors, sc.views, default_params())["color"][0]
+        assert rast._cur_stream == side.cuda_stream != 0
+        side.synchronize()  # nothing else is waited for
+        assert torch.equal(got, want)
+    rast.close()

@@ -57,7 +57,7 @@ def build_host(force: bool = False) -> str:
     cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=" + str(int(torch._C._GLIBCXX_USE_CXX11_ABI))]
     for inc in ce.include_paths("cuda") + [sysconfig.get_paths()["include"]]:
         cmd += ["-isystem", inc]
-    cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+    cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
                            "-Wl,-rpath," + torch_lib]
     subprocess.check_call(cmd)
     return HOST_PATH

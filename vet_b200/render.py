@@ -119,7 +119,7 @@ class Rasterizer:
         """Without an explicit stream the context follows torch's current stream (also the capture stream of
         torch.cuda.graph, so a whole step of forward + backward can be recorded into a CUDA graph and replayed)."""
         if self._stream is None:
-            cur = torch._C._cuda_getCurrentRawStream(self.device.index)
+            cur = L.host().current_stream(self.device.index)
             if cur != self._cur_stream:
                 self._check(L.lib().vetr_set_stream(self._ctx, C.c_void_p(cur)), "vetr_set_stream")
                 self._cur_stream = cur
