@@ -175,3 +175,59 @@ def test_whole_numbers_are_cut_to_32_bits():
     want, got = L.Params(**{k: params[k] for k, _ in L.Params._fields_}), L.Params()
     L.host().params(C.addressof(got), params, 4)
     assert got.debug_max_list_length == want.debug_max_list_length and got.viewer_only == want.viewer_only == 1
+
+
+def test_native_host_side_is_built_anew_when_its_makers_change(monkeypatch, tmp_path):
+    """Another torch, another interpreter, other flags, a changed source or a file of unknown origin: built again; else not.  With
+    every variant of the library, and not at all where there is no torch."""
+    import importlib.util
+    import sys
+    import sysconfig
+
+    from vet_b200 import build as B
+
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert L.HOST_PATH == B.HOST_PATH and B.HOST_PATH.endswith("_host" + suffix)
+    target, source = tmp_path / ("_host" + suffix), tmp_path / "host.cpp"
+    source.write_text("")
+    commands = []
+
+    def compiler(cmd):
+        commands.append(cmd)
+        if "-o" in cmd and cmd[cmd.index("-o") + 1] == str(target):
+            target.write_text("built")
+
+    monkeypatch.setattr(B.subprocess, "check_call", compiler)
+    monkeypatch.setattr(B, "HOST_PATH", str(target))
+    monkeypatch.setattr(B, "HOST_SOURCES", [str(source)])
+
+    def built():
+        n = len(commands)
+        B.build_host()
+        return len(commands) - n
+
+    target.write_text("of unknown origin")
+    assert (built(), built()) == (1, 0)
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0")
+        assert (built(), built()) == (1, 0)
+    assert built() == 1
+    with monkeypatch.context() as m:
+        m.setattr(sys, "version", "0.0")
+        assert built() == 1
+    with monkeypatch.context() as m:
+        m.setattr(torch._C, "_GLIBCXX_USE_CXX11_ABI", not torch._C._GLIBCXX_USE_CXX11_ABI)
+        assert built() == 1
+    assert (built(), built()) == (1, 0)
+    os.utime(source, (os.path.getmtime(target) + 10,) * 2)
+    assert built() == 1
+    # a variant of the library comes with it
+    target.unlink()
+    commands.clear()
+    B.build(out=str(tmp_path / "variant.so"))
+    assert len(commands) == 2 and target.exists()
+    find = importlib.util.find_spec
+    target.unlink()
+    monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
+    B.build(out=str(tmp_path / "variant.so"))
+    assert not target.exists()

@@ -3,9 +3,10 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
-HOST_PATH = os.path.join(_HERE, "_host.so")
+HOST_PATH = os.path.join(_HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 LIB_PATH = os.environ.get("VETR_LIB", os.path.join(_HERE, "libvetr.so"))  # VETR_LIB: a tuning variant of the library
 
 MAX_LAYERS = 5

@@ -7,9 +7,11 @@ which fp32 atomics sum.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libvetr.so")
@@ -20,7 +22,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
          "-Xcompiler", "-fPIC", "-shared", "-ccbin", "/usr/bin/g++"]
 
 
-HOST_PATH = os.path.join(_HERE, "_host.so")
+HOST_PATH = os.path.join(_HERE, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))  # the suffix names the interpreter it is for
 HOST_SOURCES = [os.path.join(_HERE, "csrc", "vetr_host.cpp")]
 
 
@@ -36,20 +38,14 @@ def build(force: bool = False, verbose: bool = False, defines=(), out: str = LIB
     if force or out != LIB_PATH or needs_build():
         cmd = [NVCC] + FLAGS + [f"-D{d}" for d in defines] + (["-Xptxas", "-v"] if verbose else []) + ["-o", out] + SOURCES
         subprocess.check_call(cmd)
-    if out == LIB_PATH:
-        build_host(force)
+    if importlib.util.find_spec("torch") is not None:  # the C ABI needs none of it
+        build_host(force)  # the same for every variant: it reaches the library through addresses
     return out
 
 
 def build_host(force: bool = False) -> str:
-    """Builds _host.so, the native host side of render.py: a CPython extension over libtorch (host code only, g++).  It
+    """Builds the native host side of render.py: a CPython extension over libtorch (host code only, g++).  It
     reaches libvetr.so through addresses, so it does not link it."""
-    if not force and os.path.exists(HOST_PATH):
-        t = os.path.getmtime(HOST_PATH)
-        if all(os.path.getmtime(p) <= t for p in HOST_SOURCES + [os.path.join(_HERE, "..", "include", "vetr.h")]):
-            return HOST_PATH
-    import sysconfig
-
     import torch
     from torch.utils import cpp_extension as ce
 
@@ -59,7 +55,16 @@ def build_host(force: bool = False) -> str:
         cmd += ["-isystem", inc]
     cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
                            "-Wl,-rpath," + torch_lib]
+    # up to date: newer than its sources, made by this command with this torch and this interpreter
+    made_by, made_by_path = "\n".join([torch.__version__, sys.version] + [c.replace(_HERE, ".") for c in cmd]), HOST_PATH + ".made_by"
+    if not force and os.path.exists(HOST_PATH) and os.path.exists(made_by_path):
+        t = os.path.getmtime(HOST_PATH)
+        with open(made_by_path) as f:
+            if f.read() == made_by and all(os.path.getmtime(p) <= t for p in HOST_SOURCES + [os.path.join(_HERE, "..", "include", "vetr.h")]):
+                return HOST_PATH
     subprocess.check_call(cmd)
+    with open(made_by_path, "w") as f:
+        f.write(made_by)
     return HOST_PATH
 
 
