@@ -471,3 +471,47 @@ def test_follows_the_current_stream(monkeypatch):
         side.synchronize()  # nothing else is waited for
         assert torch.equal(got, want)
     rast.close()
+
+
+@pytest.mark.parametrize("n", [500, 1])
+@pytest.mark.parametrize("mode, forward, backward", [
+    (0, 4, 1 + 2 + 1),  # clear, nearest depth, splat, combine; gradients cleared, pack or background, points, epilogue
+    (1, 7, 1 + 4 + 1),  # clear, count, two of the scan, collect, two of sort + blend; pack, lists, long lists, points
+    (2, 7, 1 + 5 + 1),  # long lists in two kernels
+    (3, 7, 1 + 4 + 1)])
+def test_launch_count(mode, forward, backward, n):
+    """vetr_launch_count counts every kernel once."""
+    from vet_b200.render import Rasterizer, scene_to_device
+    import torch
+
+    rast = Rasterizer(0)
+    sc = scenes.tiny_scene(n=n, w=40, h=32, n_views=1, seed=3)
+    tensors, params = scene_to_device(sc, rast.device), default_params(render_mode=mode)
+    before = rast.launch_count()
+    grads = [torch.ones_like(c) for c in rast.forward(*tensors, sc.views, params)["color"]]
+    between = rast.launch_count()
+    rast.finalize(rast.backward_raw(grads))
+    assert (between - before, rast.launch_count() - between) == (forward, backward)
+    rast.close()
+
+
+def test_launch_count_of_an_empty_cloud():
+    """Mode 0 without points: the clearing and combining kernels, then the background sum."""
+    import torch
+    from vet_b200.render import Rasterizer, scene_to_device
+
+    class NoPoints:  # an empty tensor has no address, which the library wants
+        shape = (0, 4)
+
+        def __init__(self, t):
+            self.data_ptr = t.data_ptr
+
+    rast = Rasterizer(0)
+    sc = scenes.tiny_scene(n=8, w=40, h=32, n_views=1, seed=3)
+    position, index, *rest = scene_to_device(sc, rast.device)
+    before = rast.launch_count()
+    out = rast.forward(NoPoints(position), NoPoints(index), *rest, sc.views, default_params(render_mode=0))
+    assert rast.launch_count() - before == 2
+    rast.backward_raw([torch.ones_like(c) for c in out["color"]], want_points=False)
+    assert rast.launch_count() - before == 2 + 1 + 1  # gradients cleared, background summed
+    rast.close()

@@ -3296,7 +3296,7 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         if (f.capacity < f.PT) return VETR_E_INVALID_ARG;  // the fragment buffer holds one accumulator record per pixel
         const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         {
-            PassScope t(ctx, VETR_T_COUNT, 2 + (ctas > 0));
+            PassScope t(ctx, VETR_T_COUNT, 1 + (ctas > 0));
             fuzzy_dt_clear_kernel<<<(unsigned)((f.PT + 255) / 256), 256, 0, st>>>(f);
             if (ctas > 0) fuzzy_dt_point_kernel<0><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f);
         }
@@ -3393,13 +3393,13 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         // 13 ps per point and view (2 M points, 2 views 1280x720: 234 -> 181 + 27 us), hence only where points are no fewer
         // than pixels; and only with the caller's word that the scratch is there, because mode 0 can do without.
         if (!use_scratch || ((uintptr_t)f.img4 & 15) != 0 || f.n < f.Prm) f.img4 = f.grad4 = nullptr;
-        PassScope t(ctx, VETR_T_BACKWARD, 2);
+        const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
+        PassScope t(ctx, VETR_T_BACKWARD, 1 + (ctas > 0));
         cudaStream_t st = ctx->stream;
         if (f.img4)
             fuzzy_dt_pack_kernel<<<ctx->sm_count * 16, 256, 0, st>>>(f, bp);
         else
             fuzzy_dt_background_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(f, bp);
-        const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         if (ctas > 0)
         {
             const auto kernel = g_intr ? fuzzy_dt_backward_kernel<2> : g_pose ? fuzzy_dt_backward_kernel<1> : fuzzy_dt_backward_kernel<0>;
