@@ -311,3 +311,20 @@ def test_gpu_envmap_against_fixture():
 def test_gpu_envmap_on_either_side_of_flat_slices(S):
     """Two and five spheres: samples on their slices; six and seven: some samples reach into the neighbouring slice."""
     test_gpu_envmap_matches_oracle(0, False, S, 0)
+
+
+@pytest.mark.gpu
+def test_gpu_envmap_of_a_very_tall_image():
+    """2^24 rows, the most whose numbers are exact in fp32: a pixel's row is formed from an estimate that is off by two there.  A small
+    focal length and a centre near the last rows make neighbouring rows differ."""
+    w, h = 3, 2**24
+    sc = util.env_scene(n_views=1)
+    sc.views = [scenes.View(w, h, image_index=sc.views[0].image_index)]
+    sc.intrinsics[:, :4] = (2.0, 3.0, 1.0, h - 20)
+    env = util.env_map(np.random.default_rng(0), S=1, R=32, C=1)
+    weight = [np.ones((1, 1, h, w), np.float32)]
+    want = O.envmap_forward(sc, sc.views, 1, env, weight)[0][0, 0, -60:]
+    got = util.env_gpu_run(sc, env, 1, weight, 0)[0][0, 0, -60:]
+    tol = util.env_sample_tolerance(env)
+    assert (np.abs(np.diff(want, axis=0)) > 10 * tol).all(axis=1).sum() > 30
+    assert np.abs(got - want).max() <= tol

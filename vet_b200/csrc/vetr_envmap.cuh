@@ -235,10 +235,10 @@ __device__ __forceinline__ bool env_locate(const EnvArgs& a, int idx, EnvPixelId
     const int lw = a.lw[l], per_view = lw * a.lh[l];
     int b = 0, r = p.pix;
     for (; r >= per_view; r -= per_view) ++b;  // at most VETR_MAX_VIEWS - 1 steps
-    // row: float estimate, then one correction step either way (the estimate is off by at most one)
+    // row: float estimate, then correction steps either way (the estimate is off by at most one up to 2^23 rows)
     int y = __float2int_rz((float)r * a.inv_lw[l]), x = r - y * lw;
-    if (x < 0) x += lw, --y;
-    if (x >= lw) x -= lw, ++y;
+    while (x < 0) x += lw, --y;
+    while (x >= lw) x -= lw, ++y;
     p.b = b, p.x = x, p.y = y;
     return true;
 }
