@@ -392,7 +392,8 @@ int vetr_get_lists(vetr_ctx* ctx, const vetr_lists* lists, int w, int h, int num
  * as a call of its own that allocates nothing.  It has no counterpart in the reference; it exists for hosts that cannot
  * allocate device memory while they render (a frame loop that cannot take the device-wide stall of cudaMalloc, a process
  * whose device memory was handed out once by an arena, a region where allocation is forbidden).  The scan's scratch, one
- * partial sum per 4096 pixels, is a fixed 128 KB array inside the library image on every GPU that loads it.
+ * partial sum per 4096 pixels and a counter (128 KB and eight bytes), is a fixed array inside the library image on every GPU that
+ * loads it.
  *   limit       n_pixels <= 67 108 864 (16384 tiles); more returns VETR_E_TOO_LARGE
  *   inputs      counts [n_pixels] int32 device array; capacity as in vetr_lists
  *   outputs     ends [n_pixels] = exclusive scan of counts (the start of every list; vetr_forward's collection pass later
@@ -401,8 +402,9 @@ int vetr_get_lists(vetr_ctx* ctx, const vetr_lists* lists, int w, int h, int num
  * The first call on a device looks up the array's device address (cudaGetSymbolAddress) and should therefore come before
  * any stream capture on that device; it is not safe to make that first call from two threads at once.  The kernels are
  * launched on `device`; the caller's current device is the same after the call as before it.  All calls share
- * the one array: it is fully rewritten by every call (nothing needs clearing), the status words are zeroed by the call,
- * and two calls whose kernels overlap on the GPU (different streams, same device) race.  Calls no cudaMalloc / cudaFree. */
+ * the one array: every call rewrites the partial sums it uses and clears the counter and the status words itself, so the caller
+ * has nothing to clear; two calls whose kernels overlap on the GPU (different streams, same device) race.  Calls no
+ * cudaMalloc / cudaFree. */
 int vetr_scan_counts_static(int device, void* cuda_stream, const int32_t* counts, int64_t n_pixels, int64_t capacity,
                             int32_t* ends, int32_t* status, int32_t* items, int64_t items_capacity);
 
@@ -417,8 +419,8 @@ enum
     VETR_T_COLLECT,      /* project + collect */
     VETR_T_SORT_BLEND,   /* sort + blend */
     VETR_T_BACKWARD,     /* backward */
-    VETR_T_FINALIZE,     /* transpose + normalisation kernels */
-    VETR_T_POINT_BACKWARD, /* per-point pass of the backward step (modes 1 and 2) */
+    VETR_T_FINALIZE,     /* epilogue */
+    VETR_T_POINT_BACKWARD, /* per-point pass of the backward step (modes 1 to 3) */
     VETR_T_EXCHANGE,     /* vetr_exchange_finalize */
     VETR_T_ENVMAP,       /* vetr_envmap_forward / vetr_envmap_backward */
     VETR_T_KNN,          /* vetr_knn_radius */

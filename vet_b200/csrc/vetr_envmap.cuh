@@ -248,9 +248,9 @@ __device__ __forceinline__ float env_start_T(float weight, int flags)
     return (flags & VETR_ENV_DEPTH_TEST_WEIGHT) ? (weight > 0.5f ? 0.f : 1.f) : weight;
 }
 
-// Bound by instruction issue (76 % of the issue slots with eight corners, 3400 instructions per pixel and four spheres: a test
-// and a branch per corner and plane, 64-bit divisions for the pixel).  1920x1080, four levels, four spheres of 1024 x 1024:
-// 337 -> 251 us.
+// Bound by instruction issue (74 % of the slots, 2300 instructions per pixel and four spheres; 3400 with eight corners per sample, a
+// test and a branch per corner and plane, and 64-bit divisions for the pixel).  1920x1080, four levels, four spheres of 1024 x 1024:
+// 335 -> 231 us; five of 512 x 512 397 -> 266, eight of 1024 x 1024 661 -> 584.
 template <bool kFlat>
 __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __grid_constant__ EnvArgs a)
 {
@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 //
 // kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of up to four spheres does not
 // pay for eight, and has room for the texel coordinates (asin, atan2, two square roots) of the first sweep; with eight they
-// are formed anew.  1920x1080, four levels, one view: four spheres of 1024 x 1024 710 us (905 with eight corners per sample),
-// five of 512 x 512 1044 (1095), eight of 1024 x 1024 2130 us (2245).
+// are formed anew.  1920x1080, four levels, one view: four spheres of 1024 x 1024 708 us (902 with eight corners per sample),
+// five of 512 x 512 1064 (1112), eight of 1024 x 1024 2140 us (2295).
 #ifndef VETR_ENV_BACK_CTAS
 #    define VETR_ENV_BACK_CTAS 3
 #endif

@@ -4,7 +4,8 @@
 // that is called.  No state but those addresses.
 //
 // Why: a training batch of a small scene is bound by the host.  5 k points, two views 96x64, camera gradients: a pass takes
-// 173 us with these steps in Python (65 us of it on the device), 87 us like this; 100 k points at 512x512 158 -> 112 us.
+// 173 to 181 us with these steps in Python (64 us of it on the device), 84 to 89 us like this; 100 k points at 512x512 158 to
+// 164 and 105 to 112 us (several GPUs; both times include a scan that became 3 us faster meanwhile).
 #include <Python.h>
 
 #include <c10/cuda/CUDAStream.h>

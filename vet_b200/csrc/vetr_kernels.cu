@@ -17,7 +17,8 @@
 //
 // Kernels (nothing here is a contraction, so no tensor cores)
 //   project_kernel<count>    stream positions, strict-fp32 projection, per-level pixel, one reduction per fragment
-//   scan_*                   three-phase exclusive scan of counts -> ends, total F, longest list, work-item table
+//   scan_*                   exclusive scan of counts -> ends, total F, longest list, work-item table, in two kernels (the last block
+//                            of the first scans the sums of the tiles)
 //   project_kernel<collect>  re-project, reserve all slots of a thread's points, then store the 32-byte records
 //   sort_blend_kernel        per work item: stage records in shared memory, rank-sort each list by (depth, index),
 //                            write the sorted records back, blend front to back, write all outputs (+ _long variant)
@@ -211,10 +212,10 @@ __device__ __forceinline__ bool point_is_live(const Frame& f, int b, int pid)
     return true;
 }
 
-// The collection waits for its atomics (54 % of the issue slots), so it wants warps: blocks of 128 threads, twelve per SM (42
+// The collection waits for its atomics (55 % of the issue slots), so it wants warps: blocks of 128 threads, twelve per SM (40
 // registers).  8 M points x 4 views: 648 us (656 with the positions requested behind the camera); six, seven or eight blocks of
 // 256: 671, 664, 664, fourteen of 128: 659, twenty-four of 64: 653, five of 256: 725.  The count pass is bound by instruction
-// issue (82 %) and stays at 256 threads: 321 us, six blocks 319, twelve of 128 341.
+// issue (89 %) and stays at 256 threads: 320 us, six blocks 319, twelve of 128 341.
 constexpr int kCollectThreads = 128, kCollectCtas = 12;
 template <bool kCollect, int kPts>
 __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCollect ? kCollectCtas : 5) project_kernel(const __grid_constant__ Frame f)
@@ -2055,9 +2056,13 @@ __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_co
 // into blocks).  Lists beyond kFuzzyLongMax are skipped and flagged in the status word (the reference itself sorts only
 // the first 4096 fragments of a list, AlphaListSort.cu:289-290, so its result for longer lists is not defined either).
 //
-// Launched twice: lists of up to kFuzzyMidMax fragments, several of which fit an SM, and the longer ones, one per SM.  The
-// sweep of a list is one thread's chain, so a launch with few such lists takes as long as the longest of them (1 M points,
-// 801x603: 115 us in either form), one with many as long as they take one SM's turn.
+// Launched twice: lists of up to kFuzzyMidMax fragments, eight of which fit an SM, and the longer ones, one per SM.  Two steps of a
+// list are one thread's chain each (fuzzy_groups, fuzzy_suffix), so a launch with few lists takes as long as the longest of them: 1 M
+// points, 801x603, 61 us with the line anywhere from 512 to 4096 (one launch for all).  With lists on both sides of the line the
+// two launches follow each other, so that no line is the best one everywhere.  Both launches, without a drop-out radius, line at
+// 512 / 1024 / 2048 / 4096: 60 k points, 8 views 200x150 (174 lists up to 851) 284 / 166 / 176 / 175 us; 200 k, one view (188 up to
+// 1024, 11 up to 2252) 459 / 547 / 633 / 361; 400 k, 4 views 400x300 (1256 and 16 up to 1496) 956 / 616 / 527 / 686; 1 M, 8 views
+// 801x603 (3731 and 50 up to 2041) 2101 / 1524 / 837 / 1353.
 constexpr int kFuzzyLongMax = 4096;  // what the reference sorts of a list (AlphaListSort.cu:289-290)
 constexpr int kFuzzyMidMax  = 1024;
 template <int kMax>
@@ -2487,7 +2492,7 @@ __global__ void __launch_bounds__(kProjThreads, 4) fuzzy_dt_backward_kernel(cons
             float2 ip     = pr.ip;
             float radius  = pr.radius_px;
             // Without camera gradients there are registers to request count and depth of the point's pixel on all levels together;
-            // with them that costs spills.  Bound by the latency of the gathers (43 % of the issue slots): 2 M points, 2 views
+            // with them that costs spills.  Bound by the latency of the gathers (62 % of the issue slots, 23 of 32 lanes): 2 M points, 2 views
             // 1280x720, the whole pass: 214 -> 196 us; in this form with pose and intrinsics gradients 269 -> 275.
             constexpr bool kTogether = kCam == 0;
             int hits[VETR_MAX_LAYERS], nearest[VETR_MAX_LAYERS];
@@ -3231,7 +3236,8 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
     return VETR_OK;
 }
 
-// Launches zero_buffers_kernel on the context's stream; `bytes` are multiples of 4, as are the addresses.
+// The two kernels of the scan.  *ticket and status[0..3] are zero on the stream before it (a ticket that is not would have the sums of
+// the tiles scanned too early).
 static void launch_scan(const int* counts, long long n, long long capacity, long long* tile_sums, unsigned* ticket, int n_tiles, int* ends,
                         int* status, int* items, cudaStream_t st)
 {
@@ -3240,6 +3246,7 @@ static void launch_scan(const int* counts, long long n, long long capacity, long
     (vec ? scan_apply_kernel<true> : scan_apply_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, ends, status, items);
 }
 
+// Launches zero_buffers_kernel on the context's stream; `bytes` are multiples of 4, as are the addresses.
 static int zero_buffers(vetr_ctx* ctx, void* const* buffers, const int64_t* bytes, int n)
 {
     ZeroArgs a;
