@@ -545,15 +545,28 @@ __device__ __forceinline__ GridPlane grid_plane(const GridArgs& a, const Camera&
 __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridPlane* planes, int group)
 {
     float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    bool number = true;
-    for (int c = group * kGridGroup; c < min((group + 1) * kGridGroup, a.n_cells); ++c)
+    bool number     = true;
+    const auto take = [&](int j, float b, float e)
+    {
+        lo[j] = fminf(lo[j], fminf(b, e)), hi[j] = fmaxf(hi[j], fmaxf(b, e));
+        number &= fabsf(e) < 1e30f;
+    };
+    const int c0 = group * kGridGroup;
+    if (c0 + kGridGroup <= a.n_cells && (((uintptr_t)a.bb_min | (uintptr_t)a.bb_len) & 15) == 0)
+    {
+        // the group's four boxes are three 16-byte words of either array (the lanes' groups lie far apart: a load per number would
+        // be 32 accesses each)
+        const float4* m = reinterpret_cast<const float4*>(a.bb_min) + 3 * (size_t)group;
+        const float4* s = reinterpret_cast<const float4*>(a.bb_len) + 3 * (size_t)group;
+        const float4 m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2), s0 = __ldg(s), s1 = __ldg(s + 1), s2 = __ldg(s + 2);
+        take(0, m0.x, m0.x + s0.x), take(1, m0.y, m0.y + s0.y), take(2, m0.z, m0.z + s0.z), take(0, m0.w, m0.w + s0.w);
+        take(1, m1.x, m1.x + s1.x), take(2, m1.y, m1.y + s1.y), take(0, m1.z, m1.z + s1.z), take(1, m1.w, m1.w + s1.w);
+        take(2, m2.x, m2.x + s2.x), take(0, m2.y, m2.y + s2.y), take(1, m2.z, m2.z + s2.z), take(2, m2.w, m2.w + s2.w);
+    }
+    else
+        for (int c = c0; c < min(c0 + kGridGroup, a.n_cells); ++c)
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
-        {
-            const float b = a.bb_min[3 * c + j], e = b + a.bb_len[3 * c + j];
-            lo[j] = fminf(lo[j], fminf(b, e)), hi[j] = fmaxf(hi[j], fmaxf(b, e));
-            number &= fabsf(e) < 1e30f;
-        }
+            for (int j = 0; j < 3; ++j) take(j, a.bb_min[3 * c + j], a.bb_min[3 * c + j] + a.bb_len[3 * c + j]);
     bool out = false;
 #pragma unroll
     for (int k = 0; k < kGridPlanes; ++k)
@@ -577,10 +590,14 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
 // chunks that go to a queue, so that the second kernel can spread them over all SMs.  If the queue is full the warp does the
 // whole cell itself.
 //
-// Looking ahead wants groups to look at: with few per warp it saves less than the second reading of the boxes and the half-spaces cost.
-// The whole call, 1920x1080, without and with it: camera on an orbit inside the grid 80^3 cells (18 groups a warp) 615 and 642 us,
-// 96^3 (31) 739 and 725, 128^3 (74) 1036 and 984; all cells in sight 64^3 (9) 197 and 203, 80^3 309 and 321, 128^3 907 and 937.
-constexpr int kGridCullGroups = 28;  // groups per warp from which on the launch takes kCull
+// Looking ahead wants groups to look at: with few per warp it saves less than the half-spaces and the second reading of the boxes cost,
+// unless the image is so small that there is little but the projection.  The whole call without and with it, camera on an orbit inside
+// the grid: 1920x1080 64^3 cells (9 groups a warp) 406 to 535 and 397 to 544 us (three cameras), 96^3 556 to 737 and 510 to 705, 128^3 941
+// to 1096 and 825 to 1006; 640x480 48^3 (4) 213 to 268 and 211 to 270, 56^3 (6) 167 to 208 and 154 to 205, 96^3 311 to 445 and 278 to
+// 412; 160x120 48^3 60 to 84 and 57 to 79, 40^3 (2) no difference.  All cells in sight: 64^3 186 and 189, 128^3 903 and 901, 48^3 at
+// 640x480 71 and 73.  (With a load per number instead of 16 bytes at a time all of that was 5 % slower than without looking.)
+constexpr int kGridCullGroups = 6, kGridCullGroupsSmall = 3, kGridCullCells = 4;  // groups per warp; in images of no more than a
+                                                                                  // pixel per kGridCullCells cells
 template <bool kCull>
 __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
                                                                      int2* queue, int* queue_count)

@@ -3599,7 +3599,8 @@ extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vet
         if (a.prefix) grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
         const int groups = (n_cells + kGridGroup - 1) / kGridGroup;
         const int ctas   = std::min((groups + kGridWarps - 1) / kGridWarps, ctx->sm_count * 12);
-        const bool cull  = groups / kGridCullGroups >= ctas * kGridWarps;
+        const bool small = n_cells / kGridCullCells >= (long long)view->w * view->h;
+        const bool cull  = groups / (small ? kGridCullGroupsSmall : kGridCullGroups) >= ctas * kGridWarps;
         (cull ? grid_loss_kernel<true> : grid_loss_kernel<false>)<<<ctas, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
         grid_loss_chunk_kernel<<<ctx->sm_count * 16, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
     }
