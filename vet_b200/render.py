@@ -94,11 +94,13 @@ class Rasterizer:
             raise RuntimeError("vet_b200.Rasterizer needs a CUDA device; there is no CPU path")
         self.device = torch.device("cuda", device)
         self._ctx = C.c_void_p()
+        self._current_stream = L.host().current_stream
         st = C.c_void_p(stream.cuda_stream) if stream is not None else None
         self._stream = stream
         rc = L.lib().vetr_create(C.byref(self._ctx), device, st)
         if rc != L.OK:
             raise L.VetrError(rc, "vetr_create")
+        self._address = self._ctx.value  # for the native host side; 0 after close(), which the library refuses
         self._lists_cache = {}
         self._saved = None
         self._cur_stream = 0 if stream is None else stream.cuda_stream
@@ -108,6 +110,7 @@ class Rasterizer:
         if self._ctx:
             L.lib().vetr_destroy(self._ctx)
             self._ctx = C.c_void_p()
+            self._address = 0
 
     def __del__(self):
         try:
@@ -119,7 +122,7 @@ class Rasterizer:
         """Without an explicit stream the context follows torch's current stream (also the capture stream of
         torch.cuda.graph, so a whole step of forward + backward can be recorded into a CUDA graph and replayed)."""
         if self._stream is None:
-            cur = L.host().current_stream(self.device.index)
+            cur = self._current_stream(self.device.index)
             if cur != self._cur_stream:
                 self._check(L.lib().vetr_set_stream(self._ctx, C.c_void_p(cur)), "vetr_set_stream")
                 self._cur_stream = cur
@@ -129,10 +132,6 @@ class Rasterizer:
             raise L.VetrError(rc, where, L.lib().vetr_last_cuda_error(self._ctx))
 
     # ---- helpers -----------------------------------------------------------------------------------------
-    def _context(self) -> int:
-        """The context's address for the native host side; 0 after close(), which the library refuses."""
-        return self._ctx.value or 0
-
     def _views(self, views):
         arr = (L.View * len(views))()
         try:
@@ -176,7 +175,7 @@ class Rasterizer:
             if prm.render_mode == 3 or (prm.render_mode in (1, 2) and prm.need_point_gradient):
                 lists.ensure_level_mask(nb * position.shape[0])
             varr = self._views(views[b0:b1])
-            rc = host.forward(self._context(), C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
+            rc = host.forward(self._address, C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
                               C.addressof(varr), nb, b0, dropout, C.addressof(lists.c), Ln, color, weight, mask, depth)
             self._check(rc, "vetr_forward")
             groups.append((b0, b1, lists, varr))
@@ -222,7 +221,7 @@ class Rasterizer:
         s = self._saved
         host = L.host()
         self._sync_stream()
-        ctx = self._context()
+        ctx = self._address
         position, index, texture = s["tensors"][0], s["tensors"][1], s["tensors"][2]
         poses, intrinsics, dropout = s["tensors"][5], s["tensors"][6], s["tensors"][7]
         n, n_tex, Cn = position.shape[0], texture.shape[1], texture.shape[0]
@@ -254,7 +253,7 @@ class Rasterizer:
         [1,n_tex], background [C], points [n,4] averaged by hit count, pose tangent and intrinsics averaged."""
         self._sync_stream()
         pts, pose, intr = g.get("points"), g.get("pose"), g.get("intrinsics")
-        g_texture = L.host().finalize(self._context(), self.device, g["background"].shape[0], g["desc"], pts, pose,
+        g_texture = L.host().finalize(self._address, self.device, g["background"].shape[0], g["desc"], pts, pose,
                                       g.get("pose_count"), intr, g.get("intrinsics_count"))
         if isinstance(g_texture, int):
             self._check(g_texture, "vetr_finalize_gradients")
@@ -371,7 +370,7 @@ class Rasterizer:
     def l1_loss_grad(self, images, targets, grads, loss):
         """loss (device scalar) = sum over levels of mean |image - target|; grads[l] = sign(image - target) / numel, one launch."""
         self._sync_stream()
-        self._check(L.host().l1_loss_grad(self._context(), images, targets, grads, loss), "vetr_l1_loss_grad")
+        self._check(L.host().l1_loss_grad(self._address, images, targets, grads, loss), "vetr_l1_loss_grad")
 
     def set_timing(self, enable: bool):
         self._sync_stream()
