@@ -4013,7 +4013,7 @@ extern "C" int vetr_read_status(vetr_ctx* ctx, const vetr_lists* lists, int64_t*
 // Some hosts must not allocate device memory while they render: an interactive viewer whose frame loop cannot afford
 // the device-wide stall of cudaMalloc / cudaFree, a process whose device memory is handed out once at start-up by an
 // arena it does not own, or code running inside a region where the driver forbids allocation.  For them the scan's
-// only scratch (one partial sum per tile of 4096 pixels) lives in a fixed array inside the library image instead of a
+// only scratch (one partial sum per tile of 4096 pixels, and the ticket) lives in a fixed array inside the library image instead of a
 // buffer grown on demand.  Every GPU that loads the library carries these 128 KB until the process exits.
 namespace vetr
 {
