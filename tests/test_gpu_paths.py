@@ -410,6 +410,32 @@ def test_grid_loss_many_cells(rasterizer, n, w, h, shift):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("n", [1, 3, 5, 31, 33, 130])
+def test_grid_loss_rows_and_corners(rasterizer, n):
+    """Boxes whose front face covers 1 to 200 rows, among them the numbers around a chunk of 64 rows, with corners on whole and half
+    pixels (the front face stands at depth 1 of a focal length of 256, the back face at depth 2): exact coverage."""
+    import torch
+
+    w, h = 400, 300
+    sc = scenes.config_planar(64, w, h, 256.0, n_views=1, seed=3)
+    sc.poses = np.array([[0, 0, 0, 1, 0, 0, 0, 0]], np.float64)
+    sc.intrinsics[0, :4] = 256.0, 256.0, 200.0, 150.0
+    rng = np.random.default_rng(n)
+    rows = np.resize(np.array([64, 65, 63, 128, 127, 129, 1, 2, 32, 33, 200, 192, 193]), n)
+    u, v = rng.integers(32, 200, n), rng.integers(32, 60, n)
+    columns = rng.integers(1, 150, n)
+    bb_min = np.stack([(u - 200) / 256, (v - 150) / 256, np.ones(n)], 1).astype(np.float32)
+    bb_len = np.stack([columns / 256, rows / 256, np.ones(n)], 1).astype(np.float32)
+    loss = rng.standard_normal((3, h, w)).astype(np.float32)
+    ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    assert (ref_c > 0).any()
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+    np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
 # ---- mode 0 without camera gradients: the pixels of all levels are looked up together
 
 

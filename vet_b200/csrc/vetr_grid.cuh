@@ -7,7 +7,7 @@
 // edge functions in strict fp32 for each of some 600 M pixels at 128^3 cells and 1920 x 1080: 7.9 ms).  Here a lane owns one
 // pixel ROW of a cell: the twelve triangles are a closed surface, so what they cover of a row is the run of pixels between its
 // leftmost and rightmost crossing with the 18 segments (12 edges, 6 face diagonals), and the run's loss is a difference
-// of two running sums of that image row (fp64, formed once per call).  0.92 ms at the same sizes.
+// of two running sums of that image row (fp64, formed once per call).  0.63 ms at the same sizes.
 //
 // Why one run: a row cuts the surface in a connected set if the part of the surface above it and the part below are both
 // connected (the surface is a sphere), and they are for every row if only one corner has no higher neighbour along the 18
@@ -71,12 +71,14 @@ __device__ __forceinline__ float grid_pixel_loss(const GridArgs& a, int x, int y
 
 constexpr int kGridWarps    = 4;
 constexpr int kGridGroup    = 4;                // cells a warp takes together: eight lanes each
-constexpr int kGridChunk    = 512;              // pixels of a rectangle one warp walks in the per-pixel form (4096: a warp with
-                                                // four such chunks ends 0.3 ms after the others)
-constexpr int kGridRowChunk = 32;               // rows of a queued chunk; cells of up to that many rows are not queued
+constexpr int kGridChunk      = 64;             // pixels of a rectangle one warp walks in the per-pixel form (256: a warp with four such chunks
+                                                // ends late, 128^3 cells at 1920x1080 681 instead of 631 us; 512: 50 us more)
+constexpr int kGridRowChunk   = 64;             // rows of a queued chunk; cells of up to that many rows are not queued (32: 702 instead of 655 us,
+                                                // 35^3 cells at 160x120 45 instead of 37; 128: 835 instead of 805)
+constexpr int kGridExactLanes = 6;              // rows of a warp with pixels to be tested from which on their own lanes test them (2 to 6 the same;
+                                                // never: 1089 instead of 958 us with the bands as wide as they were then)
 constexpr int kGridQueueCap = 4 * 1024 * 1024;  // (cell, chunk) pairs handed to the second kernel
 constexpr int kGridSegments = 18;               // 12 edges, then 6 face diagonals
-constexpr unsigned long long kGridNeighbours = 0x72bdcbc76151b17eull;  // byte c: the corners that share a segment with corner c
 constexpr int kGridCtas     = 6;                // resident CTAs per SM the kernels are compiled for (5: the same, 8: 10 % slower)
 
 // Running sums of |loss| along every image row, one CTA per row, four pixels per thread and step.  A sum is formed in fp64 from
@@ -125,30 +127,49 @@ __global__ void __launch_bounds__(256) grid_row_sums_kernel(const __grid_constan
     if (__any_sync(0xffffffffu, bad) && lane == 0) *a.no_rows = 1;
 }
 
-__constant__ signed char kGridSegEnds[kGridSegments][2] = {{0, 1}, {2, 4}, {3, 5}, {6, 7}, {0, 2}, {1, 4}, {3, 6}, {5, 7}, {0, 3},
-                                                           {1, 5}, {2, 6}, {4, 7}, {0, 4}, {1, 7}, {5, 6}, {0, 6}, {0, 5}, {4, 6}};
-__constant__ signed char kGridTriangles[12][3] = {{0, 1, 4}, {0, 4, 2}, {1, 5, 7}, {1, 7, 4}, {5, 3, 6}, {5, 6, 7},
-                                                  {3, 0, 6}, {0, 6, 2}, {3, 0, 5}, {0, 5, 1}, {2, 4, 6}, {4, 6, 7}};
+#define VETR_GRID_SEGMENTS                                                                                                                  \
+    {{0, 1}, {2, 4}, {3, 5}, {6, 7}, {0, 2}, {1, 4}, {3, 6}, {5, 7}, {0, 3}, {1, 5}, {2, 6}, {4, 7}, {0, 4}, {1, 7}, {5, 6}, {0, 6}, {0, 5}, {4, 6}}
+#define VETR_GRID_TRIANGLES                                                                                                                 \
+    {{0, 1, 4}, {0, 4, 2}, {1, 5, 7}, {1, 7, 4}, {5, 3, 6}, {5, 6, 7}, {3, 0, 6}, {0, 6, 2}, {3, 0, 5}, {0, 5, 1}, {2, 4, 6}, {4, 6, 7}}
+__constant__ signed char kGridSegEnds[kGridSegments][2] = VETR_GRID_SEGMENTS;
+__constant__ signed char kGridTriangles[12][3]          = VETR_GRID_TRIANGLES;
+// The same for loops that are unrolled.
+struct GridTables
+{
+    int ends[kGridSegments][2] = VETR_GRID_SEGMENTS, triangles[12][3] = VETR_GRID_TRIANGLES;
+    int sides[12][3] = {};  // segments between corners 0 1, 0 2 and 1 2 of a triangle
+    constexpr GridTables()
+    {
+        for (int t = 0; t < 12; ++t)
+            for (int k = 0; k < 3; ++k)
+                for (int g = 0; g < kGridSegments; ++g)
+                {
+                    const int p = triangles[t][k == 2], q = triangles[t][k == 0 ? 1 : 2];
+                    if ((ends[g][0] == p && ends[g][1] == q) || (ends[g][0] == q && ends[g][1] == p)) sides[t][k] = g;
+                }
+    }
+};
 
 struct GridWarpSmem
 {
-    float2 pp[kGridGroup][8];               // projected corners
-    float4 seg[kGridSegments][kGridGroup];  // {x at y0, y0, y1, dx/dy}, relative to the rectangle's first pixel
-    float half[kGridSegments][kGridGroup];  // half-width of the band around the segment, along the row
-    int4 rect[kGridGroup];                  // first column, first row, columns, rows
-    float rho[kGridGroup];                  // height of the band beyond the segment's ends
+    float2 corner[8][33];                   // projected corners of up to 32 cells, a lane's cell per column
+    float2 pp[kGridGroup][8];               // those of the group in work
+    float4 seg[kGridSegments][kGridGroup];   // {x at row 0, dx/dy, middle row, half the rows}, relative to the rectangle's first pixel
+    float2 band[kGridSegments][kGridGroup];  // {half-width of the band along the row, half the rows with what the band adds to them}
+    int4 rect[kGridGroup];                   // first column, first row, columns, rows
+    int2 spot[kGridGroup][8];                // {row, column} of the pixel next to a corner, row -1 if it is far enough away
+    int spots[kGridGroup];                   // not 0: there are some
+    int2 todo[64];                          // {cell, chunk} to be prepared
 };
 
 // Corner order of the reference: (0,0,0) (1,0,0) (0,1,0) (0,0,1) (1,1,0) (1,0,1) (0,1,1) (1,1,1).
-__device__ __forceinline__ float2 grid_project_corner(const Frame& f, const GridArgs& a, const Camera& cam, int c, int corner, bool& behind)
+__device__ __forceinline__ float2 grid_project_corner(const Frame& f, const Camera& cam, const float (&box)[3], const float (&len)[3], int corner,
+                                                       bool& behind)
 {
-    const float fx = (corner == 1 || corner == 4 || corner == 5 || corner == 7) ? 1.f : 0.f;
-    const float fy = (corner == 2 || corner == 4 || corner == 6 || corner == 7) ? 1.f : 0.f;
-    const float fz = (corner == 3 || corner == 5 || corner == 6 || corner == 7) ? 1.f : 0.f;
-    const float4 pos = make_float4(VA(a.bb_min[3 * c], VM(a.bb_len[3 * c], fx)), VA(a.bb_min[3 * c + 1], VM(a.bb_len[3 * c + 1], fy)),
-                                   VA(a.bb_min[3 * c + 2], VM(a.bb_len[3 * c + 2], fz)), 0.f);
+    const float fx = 0xb2 >> corner & 1 ? 1.f : 0.f, fy = 0xd4 >> corner & 1 ? 1.f : 0.f, fz = 0xe8 >> corner & 1 ? 1.f : 0.f;
+    const float4 pos   = make_float4(VA(box[0], VM(len[0], fx)), VA(box[1], VM(len[1], fy)), VA(box[2], VM(len[2], fz)), 0.f);
     const Projected pr = project_point(pos, cam, f.dist_cutoff);
-    behind = pr.z <= 0.f;  // one corner behind the camera: the whole cell is ignored
+    behind |= pr.z <= 0.f;
     return pr.ip;
 }
 
@@ -174,10 +195,14 @@ __device__ __noinline__ void grid_cell_pixels(const GridArgs& a, int c, int lane
     for (int i = 0; i < 8; ++i) pp[i] = s_pp[i];
     float sum = 0.f;
     int hits  = 0;
-    for (long long xy = first + lane; xy < last; xy += 32)
+    // (a rectangle has no more pixels than the image, hence 32 bits; in images below 64 pixels across x_size can be negative)
+    const int width = abs(x_size), turn = x_size < 0 ? -1 : 1, dx = 32 % width, dy = 32 / width * turn;
+    int x = ((int)first + lane) % width, y = ((int)first + lane) / width * turn;
+    for (unsigned xy = (unsigned)first + lane; xy < (unsigned)last; xy += 32, x += dx, y += dy)
     {
-        const int x_c = (int)VA((float)(int)(xy % x_size), mn.x);
-        const int y_c = (int)VA((float)(int)(xy / x_size), mn.y);
+        if (x >= width) x -= width, y += turn;
+        const int x_c = (int)VA((float)x, mn.x);
+        const int y_c = (int)VA((float)y, mn.y);
         if (!point_in_box(make_float2((float)x_c, (float)y_c), pp)) continue;
         sum += grid_pixel_loss(a, x_c, y_c);
         ++hits;
@@ -232,6 +257,87 @@ __device__ __noinline__ double grid_run_pixels(const GridArgs& a, const GridWarp
     return sum;
 }
 
+// Crossing of row y with segment k of a slot's cell, extended beyond its ends; true if it lies on the segment.
+__device__ __forceinline__ bool grid_crossing(const GridWarpSmem& s, int k, int slot, float y, float& xs)
+{
+    const float4 g = s.seg[k][slot];
+    xs             = __fmaf_rn(g.y, y, g.x);
+    return fabsf(y - g.z) <= g.w;
+}
+// Pixels [x0, x1] of the row that lie in the segment's band.
+__device__ __forceinline__ void grid_band(const GridWarpSmem& s, const int4 rect, int k, int slot, float y, float xs, int& x0, int& x1)
+{
+    const float2 b = s.band[k][slot];
+    x0 = 1, x1 = 0;
+    if (fabsf(y - s.seg[k][slot].z) <= b.y) x0 = (int)fmaxf(ceilf(xs - b.x), 0.f), x1 = (int)fminf(floorf(xs + b.x), (float)(rect.z - 1));
+}
+
+// Leftmost and rightmost crossing of row j with the segments of a cell; true if a pixel lies in the band of one.  Bound by instruction
+// issue, 13 per segment.
+__device__ __forceinline__ bool grid_crossings(const GridWarpSmem& s, int slot, int j, float& L, float& R)
+{
+    const float y = (float)j;
+    bool close = false;
+    L = CUDART_INF_F, R = -CUDART_INF_F;
+#pragma unroll 6
+    for (int q = 0; q < kGridSegments; ++q)
+    {
+        const float4 g = s.seg[q][slot];
+        const float2 b = s.band[q][slot];
+        const float t = fabsf(y - g.z), xs = __fmaf_rn(g.y, y, g.x);
+        const float column = (xs + 12582912.f) - 12582912.f;  // the nearest whole number up to 2^22; beyond that the row is not near the segment
+        close |= t <= b.y && fabsf(xs - column) <= b.x;
+        if (t <= g.w) L = fminf(L, xs), R = fmaxf(R, xs);
+    }
+    if (s.spots[slot])
+        for (int k = 0; k < 8; ++k) close |= s.spot[slot][k].x == j;
+    return close;
+}
+
+// One row whose bands hold no more than four pixels, by the lane it belongs to, where several rows of a warp's have some: the run L to R of
+// pixels, corrected where the per-pixel test disagrees.  False, and nothing done, if there are more pixels.
+__device__ __noinline__ bool grid_exact_lane(const GridArgs& a, const GridWarpSmem& s, int slot, int j, float L, float R, double& sum, int& hits)
+{
+    const int4 rect = s.rect[slot];
+    const float y   = (float)j;
+    int at[4] = {-1, -1, -1, -1};
+#pragma unroll 1
+    for (int k = 0; k < kGridSegments + 8; ++k)
+    {
+        float xs;
+        int x0 = 1, x1 = 0;
+        if (k < kGridSegments)
+        {
+            grid_crossing(s, k, slot, y, xs);
+            grid_band(s, rect, k, slot, y, xs, x0, x1);
+        }
+        else
+        {
+            const int2 spot = s.spot[slot][k - kGridSegments];
+            if (spot.x == j && spot.y >= 0 && spot.y < rect.z) x0 = x1 = spot.y;
+        }
+        if (x1 - x0 > 3) return false;
+        for (int x = x0; x <= x1; ++x)
+        {
+            if (x == at[0] || x == at[1] || x == at[2] || x == at[3]) continue;
+            if (at[3] >= 0) return false;
+            at[3] = at[2], at[2] = at[1], at[1] = at[0], at[0] = x;
+        }
+    }
+    sum  = 0.0;
+    hits = grid_run(a, rect, j, L, R, sum);
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n)
+    {
+        const int x = at[0];
+        if (x < 0) break;
+        at[0] = at[1], at[1] = at[2], at[2] = at[3], at[3] = -1;
+        const int change = (int)point_in_box(make_float2((float)(rect.x + x), (float)(rect.y + j)), s.pp[slot]) - (int)((float)x >= L && (float)x <= R);
+        if (change != 0) sum += (double)change * (double)grid_pixel_loss(a, rect.x + x, rect.y + j), hits += change;
+    }
+    return true;
+}
+
 // One row of one cell in which pixels lie in the band of a segment (a whole warp): the run of pixels, corrected
 // where the per-pixel test disagrees.  Lane k owns segment k.  The pixels of a short band are taken one by one, a triangle per
 // lane; those of a long one (a nearly horizontal segment) 32 at a time, a pixel per lane.
@@ -244,11 +350,15 @@ __device__ __noinline__ void grid_exact_row(const GridArgs& a, const GridWarpSme
     int x0 = 1, x1 = 0;  // pixels in the band of the lane's segment
     if (lane < kGridSegments)
     {
-        const float4 q = s.seg[lane][slot];
-        const float yc = fminf(fmaxf(y, q.y), q.z);
-        const float xs = fmaf(yc - q.y, q.w, q.x), h = s.half[lane][slot];
-        if (fabsf(y - yc) <= s.rho[slot]) x0 = (int)fmaxf(ceilf(xs - h), 0.f), x1 = (int)fminf(floorf(xs + h), (float)(rect.z - 1));
-        if (y == yc) L = R = xs;
+        float xs;
+        const bool crossed = grid_crossing(s, lane, slot, y, xs);
+        grid_band(s, rect, lane, slot, y, xs, x0, x1);
+        if (crossed) L = R = xs;
+    }
+    else if (lane < kGridSegments + 8)
+    {
+        const int2 spot = s.spot[slot][lane - kGridSegments];
+        if (spot.x == j && spot.y >= 0 && spot.y < rect.z) x0 = x1 = spot.y;
     }
     for (int o = 16; o > 0; o >>= 1)
     {
@@ -298,16 +408,17 @@ __device__ __noinline__ void grid_exact_row(const GridArgs& a, const GridWarpSme
     }
 }
 
-// What eight lanes know of their cell.
+// What is known of a cell.
 struct GridCell
 {
-    float2 mn;  // first pixel of the rectangle (fp32, not truncated)
-    int x_size, y_size;
-    long long total;  // pixels of the rectangle; 0: nothing to do
-    bool by_rows;     // row form; otherwise per-pixel form
+    float2 mn;            // first pixel of the rectangle (fp32, not truncated)
+    int x_size, y_size;   // of the rectangle
+    bool by_rows;         // row form; otherwise per-pixel form
+    float rho, zone;      // reach of a segment's band and of a corner's
+    __device__ __forceinline__ long long total() const { return (long long)x_size * y_size; }  // pixels; 0: nothing to do
 };
 
-// Projects the corners of the cells of a warp (cell c of the lane's slot, or -1), forms rectangles and segments.
+// Projects the corners of the lane's cell c (-1: none) and forms its rectangle and bands.
 //
 // Bands.  With all differences of coordinates below E (the box's extent on the screen, plus one pixel) the strict fp32 edge
 // function of an edge of length l is off by less than 8.4 E l 2^-24, i.e. its sign is certain farther than 5e-7 E pixels from
@@ -315,76 +426,98 @@ struct GridCell
 // that is farther than 5e-7 E from all segments lies inside some triangle with all three signs certain.  A pixel outside
 // the run lies in no triangle.  It fails one whose side is nearest for certain if it is farther than 5e-7 E from that side,
 // and one whose corner is nearest if it is farther than 5e-7 E / sin(half the smallest angle) <= 1e-6 E kappa from that
-// corner, kappa = the largest (product of the two longer sides) / (2 area) of the twelve triangles.  So the
-// band of a diagonal is rho = 1e-6 E wide, that of an edge (kappa + 0.5) rho, which also covers all corners, and along a row
-// of slope dx/dy = k a band of height rho reaches rho (1 + |k|) to either side.
-// All this takes the projected corners as they are, whatever rounding went into them.  Cells whose band would be wider than a
+// corner, kappa = the largest (product of the two longer sides) / (2 area) of the twelve triangles, 1 / the sine of the smallest
+// angle.  So the band of a segment is rho = 1e-6 E wide, which along a row of slope dx/dy = k reaches rho (1 + |k|) to either side,
+// and that of a corner (kappa + 0.5) rho (the half more than covers the rounding of kappa, some 1e-6 kappa: corners' bands above
+// a quarter pixel are refused) and at least 7 rho: a pixel above or below a segment of |k| <= 4 that is nearest to a point inside it is at
+// most sqrt(17) rho away from its end, so that only flatter segments have to be followed beyond their ends.  (All of the edges' bands
+// as wide as the corners' want 3 % of the rows tested pixel by pixel, a sixth of the whole call.)
+// All this takes the projected corners as they are, whatever rounding went into them.  Cells whose corners' bands would be wider than a
 // quarter pixel, or with a triangle as thin as a few units in the last place of a pixel coordinate, take the per-pixel form.
 __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs& a, const Camera& cam, GridWarpSmem& s, int c, bool no_rows)
 {
-    const int lane = threadIdx.x & 31, slot = lane >> 3, corner = lane & 7;
+    constexpr GridTables kTab;
+    const int lane = threadIdx.x & 31;
     GridCell cell;
-    cell.x_size = cell.y_size = 0, cell.total = 0, cell.by_rows = false, cell.mn = make_float2(0.f, 0.f);
-    bool behind = true;
-    float2 ip   = make_float2(0.f, 0.f);
-    if (c >= 0) ip = grid_project_corner(f, a, cam, c, corner, behind);
-    const unsigned behind_lanes = __ballot_sync(0xffffffffu, behind);
-    const bool visible          = (behind_lanes >> (8 * slot) & 0xffu) == 0;
-    if (!__any_sync(0xffffffffu, visible)) return cell;
-    float2 lo = make_float2(fminf(ip.x, 10000000.f), fminf(ip.y, 10000000.f));
-    float2 hi = make_float2(fmaxf(ip.x, -10000000.f), fmaxf(ip.y, -10000000.f));
+    cell.x_size = cell.y_size = 0, cell.by_rows = false, cell.mn = make_float2(0.f, 0.f), cell.rho = cell.zone = 0.f;
+    if (c < 0) return cell;
+    float box[3], len[3];
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1)
-    {
-        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o)), lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o)), hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-    }
-    cell.mn = lo;
-    if (visible) cell.total = grid_rectangle(a, cell.mn, hi, cell.x_size, cell.y_size);
-    if (!__any_sync(0xffffffffu, cell.total > 0)) return cell;
-    __syncwarp();  // the previous cells' segments have been read
-    s.pp[slot][corner] = ip;
-    __syncwarp();
-    if (no_rows) return cell;
-    const float2 mn = cell.mn;
-    const float E   = fmaxf(hi.x - lo.x, hi.y - lo.y) + 1.f;
-    float kappa = 0.f, thin = CUDART_INF_F;  // thin: smallest altitude of a triangle, 0 if one has no area or a corner is NaN
-    for (int t = corner; t < 12; t += 8)
-    {
-        const float2 p0 = s.pp[slot][kGridTriangles[t][0]], p1 = s.pp[slot][kGridTriangles[t][1]], p2 = s.pp[slot][kGridTriangles[t][2]];
-        const float ux = p1.x - p0.x, uy = p1.y - p0.y, vx = p2.x - p0.x, vy = p2.y - p0.y, wx = vx - ux, wy = vy - uy;
-        const float area2 = fabsf(ux * vy - uy * vx);
-        const float a2 = ux * ux + uy * uy, b2 = vx * vx + vy * vy, c2 = wx * wx + wy * wy;
-        const float l2 = fmaxf(a2, fmaxf(b2, c2)), m2 = fmaxf(fminf(a2, b2), fminf(fmaxf(a2, b2), c2));  // longest, second longest
-        kappa = fmaxf(kappa, sqrtf(l2 * m2) / area2), thin = fminf(thin, area2 > 0.f ? area2 * rsqrtf(l2) : 0.f);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1)
-    {
-        kappa = fmaxf(kappa, __shfl_xor_sync(0xffffffffu, kappa, o));
-        thin  = fminf(thin, __shfl_xor_sync(0xffffffffu, thin, o));
-    }
-    // corners without a higher (lower) neighbour; equal rows are told apart by the corner's number
-    unsigned higher = 0;
-#pragma unroll
+    for (int k = 0; k < 3; ++k) box[k] = a.bb_min[3 * (size_t)c + k], len[k] = a.bb_len[3 * (size_t)c + k];
+    bool behind = false;  // one corner behind the camera: the whole cell is ignored
+    float2 lo = make_float2(10000000.f, 10000000.f), hi = make_float2(-10000000.f, -10000000.f);
+#pragma unroll 1
     for (int k = 0; k < 8; ++k)
     {
-        const float y = s.pp[slot][k].y;
-        if (y > ip.y || (y == ip.y && k > corner)) higher |= 1u << k;
+        const float2 ip   = grid_project_corner(f, cam, box, len, k, behind);
+        s.corner[k][lane] = ip;
+        lo.x = fminf(lo.x, ip.x), lo.y = fminf(lo.y, ip.y), hi.x = fmaxf(hi.x, ip.x), hi.y = fmaxf(hi.y, ip.y);
     }
-    const unsigned near = (unsigned)(kGridNeighbours >> (8 * corner)) & 0xffu;
-    const unsigned tops = __ballot_sync(0xffffffffu, (higher & near) == 0), bottoms = __ballot_sync(0xffffffffu, (~higher & near) == 0);
-    const bool one_run  = __popc(tops >> (8 * slot) & 0xffu) == 1 && __popc(bottoms >> (8 * slot) & 0xffu) == 1;
+    cell.mn = lo;
+    if (behind || grid_rectangle(a, cell.mn, hi, cell.x_size, cell.y_size) <= 0)
+    {
+        cell.x_size = cell.y_size = 0;
+        return cell;
+    }
+    if (no_rows) return cell;
+    float2 p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = s.corner[k][lane];
+    const float E = fmaxf(hi.x - lo.x, hi.y - lo.y) + 1.f;
+    // squared lengths, and which corners have a higher or a lower neighbour; equal rows are told apart by the corner's number
+    float len2[kGridSegments];
+    unsigned higher = 0, lower = 0;
+#pragma unroll
+    for (int k = 0; k < kGridSegments; ++k)
+    {
+        const int i = kTab.ends[k][0], j = kTab.ends[k][1];  // i < j
+        const float dx = p[j].x - p[i].x, dy = p[j].y - p[i].y;
+        len2[k]       = __fmaf_rn(dx, dx, dy * dy);
+        const bool up = p[j].y >= p[i].y;
+        higher |= up ? 1u << i : 1u << j, lower |= up ? 1u << j : 1u << i;
+    }
+    const bool one_run = __popc(higher) == 7 && __popc(lower) == 7;
+    float sine = 1.f, thin = CUDART_INF_F;  // of the smallest angle; smallest altitude of a triangle (0: without area, or a NaN corner)
+#pragma unroll
+    for (int t = 0; t < 12; ++t)
+    {
+        const float2 p0 = p[kTab.triangles[t][0]], p1 = p[kTab.triangles[t][1]], p2 = p[kTab.triangles[t][2]];
+        const float area2 = fabsf((p1.x - p0.x) * (p2.y - p0.y) - (p1.y - p0.y) * (p2.x - p0.x));
+        const float a2 = len2[kTab.sides[t][0]], b2 = len2[kTab.sides[t][1]], c2 = len2[kTab.sides[t][2]];
+        const float l2 = fmaxf(a2, fmaxf(b2, c2)), m2 = fmaxf(fminf(a2, b2), fminf(fmaxf(a2, b2), c2));  // longest, second longest
+        const float altitude = area2 > 0.f ? area2 * rsqrtf(l2) : 0.f;
+        thin = fminf(thin, altitude), sine = fminf(sine, area2 > 0.f ? altitude * rsqrtf(m2) : 0.f);
+    }
     const float size = (float)max(a.w, a.h);
-    const float rho = 1e-6f * E, rho_edge = rho * (kappa + 0.5f);
+    cell.rho = 1e-6f * E, cell.zone = cell.rho * fmaxf(1.f / sine + 0.5f, 7.f);
     const float skip = 1.f - size * 2.4e-7f;  // fp32 column / row numbers count up without a gap below this fraction
     // (a NaN or infinite corner selects the per-pixel form through thin, or through E)
-    cell.by_rows = cell.total > 0 && cell.x_size > 0 && cell.y_size > 0 && one_run && E < 2e4f && rho_edge < 0.25f &&
-                   thin > 4e-3f * (1.f + (size + E) * (1.f / 2048.f)) && mn.x - floorf(mn.x) < skip && mn.y - floorf(mn.y) < skip;
+    cell.by_rows = cell.x_size > 0 && cell.y_size > 0 && one_run && E < 2e4f && cell.zone < 0.25f &&
+                   thin > 4e-3f * (1.f + (size + E) * (1.f / 2048.f)) && cell.mn.x - floorf(cell.mn.x) < skip && cell.mn.y - floorf(cell.mn.y) < skip;
+    return cell;
+}
+
+// What lane `from` knows of its cell.
+__device__ __forceinline__ GridCell grid_cell_of(const GridCell& cell, int from)
+{
+    GridCell g;
+    g.mn      = make_float2(__shfl_sync(0xffffffffu, cell.mn.x, from), __shfl_sync(0xffffffffu, cell.mn.y, from));
+    g.x_size  = __shfl_sync(0xffffffffu, cell.x_size, from), g.y_size = __shfl_sync(0xffffffffu, cell.y_size, from);
+    g.by_rows = __shfl_sync(0xffffffffu, (int)cell.by_rows, from) != 0;
+    g.rho     = __shfl_sync(0xffffffffu, cell.rho, from), g.zone = __shfl_sync(0xffffffffu, cell.zone, from);
+    return g;
+}
+
+// Corners, segments and rectangles of a group of four cells, eight lanes each; from: the lane that the slot's cell was prepared by.
+__device__ __forceinline__ void grid_segments(GridWarpSmem& s, const GridCell& cell, int from)
+{
+    const int lane = threadIdx.x & 31, slot = lane >> 3, corner = lane & 7;
+    __syncwarp();  // the previous group's have been read, this one's corners written
+    s.pp[slot][corner] = s.corner[corner][from];
+    __syncwarp();
     if (cell.by_rows)
     {
-        const float bx = floorf(mn.x), by = floorf(mn.y);
+        const float bx = floorf(cell.mn.x), by = floorf(cell.mn.y);
         for (int k = corner; k < kGridSegments; k += 8)
         {
             float2 p = s.pp[slot][kGridSegEnds[k][0]], q = s.pp[slot][kGridSegEnds[k][1]];
@@ -394,38 +527,27 @@ __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs&
                 p = q, q = t;
             }
             p.x -= bx, p.y -= by, q.x -= bx, q.y -= by;
-            const float dx = q.x - p.x, dy = q.y - p.y, r = k < 12 ? rho_edge : rho;
+            const float dx = q.x - p.x, dy = q.y - p.y, rho = cell.rho;
             const bool flat = dy < 1e-3f;  // as good as horizontal: the band covers the whole segment
-            const float k_  = flat ? 0.f : dx / dy;
-            s.seg[k][slot]  = make_float4(flat ? p.x + 0.5f * dx : p.x, p.y, q.y, k_);
-            s.half[k][slot] = flat ? 0.5f * fabsf(dx) + 4.f * r : fminf(r * (1.f + fabsf(k_)), fabsf(dx) + 2.f * r);
+            const float k_  = flat ? 0.f : dx / dy, rows = 0.5f * dy, steep = fabsf(k_);
+            s.seg[k][slot]  = make_float4(flat ? p.x + 0.5f * dx : __fmaf_rn(-k_, p.y, p.x), k_, p.y + rows, rows);
+            const bool beyond = flat || steep > 4.f;  // followed beyond its ends: by rho in height, the last term of its reach along the row
+            // (which is also for the rounding of the crossing where the reach is cut: 1.2e-7 E |dx/dy|)
+            float half = flat ? 0.5f * fabsf(dx) + 4.f * rho : fminf(rho * (1.f + steep), fabsf(dx) + 2.f * rho);
+            if (beyond) half += 1.25f * rho * steep;
+            s.band[k][slot] = make_float2(half, beyond ? rows + rho : rows);
         }
-    }
-    if (corner == 0)
-    {
-        s.rect[slot] = make_int4((int)floorf(mn.x), (int)floorf(mn.y), cell.x_size, cell.y_size);
-        s.rho[slot]  = rho_edge;
+        const float2 c = s.pp[slot][corner];
+        const float x = rintf(c.x), y = rintf(c.y);
+        const bool next = fabsf(c.x - x) <= cell.zone && fabsf(c.y - y) <= cell.zone;
+        s.spot[slot][corner] = next ? make_int2((int)y - (int)by, (int)x - (int)bx) : make_int2(-1, 0);
+        if (corner == 0) s.spots[slot] = 0;
+        __syncwarp(0xffu << (8 * slot));
+        if (next) s.spots[slot] = 1;
+        if (corner == 0)
+            s.rect[slot] = make_int4((int)bx, (int)by, cell.x_size, cell.y_size);
     }
     __syncwarp();
-    return cell;
-}
-
-// Leftmost and rightmost crossing of row j with the segments of a cell; true if a pixel lies in the band of one.
-__device__ __forceinline__ bool grid_crossings(const GridWarpSmem& s, int slot, int j, float& L, float& R)
-{
-    const float y = (float)j, rho = s.rho[slot];
-    bool close = false;
-    L = CUDART_INF_F, R = -CUDART_INF_F;
-#pragma unroll 6
-    for (int q = 0; q < kGridSegments; ++q)
-    {
-        const float4 g = s.seg[q][slot];
-        const float yc = fminf(fmaxf(y, g.y), g.z), dy = fabsf(y - yc);
-        const float xs = fmaf(yc - g.y, g.w, g.x);
-        close |= dy <= rho && fabsf(xs - rintf(xs)) <= s.half[q][slot];
-        if (dy == 0.f) L = fminf(L, xs), R = fmaxf(R, xs);
-    }
-    return close;
 }
 
 // Rows [row0, row0 + rows) of the cell of every slot, eight at a time; adds each cell's totals.  Returns true (in all eight lanes) if
@@ -442,9 +564,9 @@ __device__ __forceinline__ bool grid_rows(const GridArgs& a, const GridWarpSmem&
     {
         const int i = base + corner, j = row0 + i;
         bool close  = false;
+        float L = 0.f, R = 0.f;
         if (i < rows)
         {
-            float L, R;
             close = grid_crossings(s, slot, j, L, R);
             if (!close)
             {
@@ -456,6 +578,17 @@ __device__ __forceinline__ bool grid_rows(const GridArgs& a, const GridWarpSmem&
             }
         }
         unsigned todo = __ballot_sync(0xffffffffu, close);
+        if (__popc(todo) >= kGridExactLanes)
+        {
+            double rs = 0.0;
+            int rh    = 0;
+            if (close && grid_exact_lane(a, s, slot, j, L, R, rs, rh))
+            {
+                close = false;
+                if (rh > 0) refuse |= grid_cancels(rs, grid_prefix(a, s.rect[slot].y + j)[a.w]), sum += rs, hits += rh;
+            }
+            todo = __ballot_sync(0xffffffffu, close);
+        }
         while (todo)
         {
             const int from = __ffs(todo) - 1;
@@ -541,32 +674,18 @@ __device__ __forceinline__ GridPlane grid_plane(const GridArgs& a, const Camera&
     return p;
 }
 
-// True if no cell of the group is drawn (false for anything that is not a number).
-__device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridPlane* planes, int group)
+// True if the cell is not drawn (false for anything that is not a number).
+__device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridPlane* planes, int c)
 {
-    float lo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, hi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    bool number     = true;
-    const auto take = [&](int j, float b, float e)
-    {
-        lo[j] = fminf(lo[j], fminf(b, e)), hi[j] = fmaxf(hi[j], fmaxf(b, e));
-        number &= fabsf(e) < 1e30f;
-    };
-    const int c0 = group * kGridGroup;
-    if (c0 + kGridGroup <= a.n_cells && (((uintptr_t)a.bb_min | (uintptr_t)a.bb_len) & 15) == 0)
-    {
-        // the group's four boxes are three 16-byte words of either array (the lanes' groups lie far apart: a load per number would
-        // be 32 accesses each)
-        const float4* m = reinterpret_cast<const float4*>(a.bb_min) + 3 * (size_t)group;
-        const float4* s = reinterpret_cast<const float4*>(a.bb_len) + 3 * (size_t)group;
-        const float4 m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2), s0 = __ldg(s), s1 = __ldg(s + 1), s2 = __ldg(s + 2);
-        take(0, m0.x, m0.x + s0.x), take(1, m0.y, m0.y + s0.y), take(2, m0.z, m0.z + s0.z), take(0, m0.w, m0.w + s0.w);
-        take(1, m1.x, m1.x + s1.x), take(2, m1.y, m1.y + s1.y), take(0, m1.z, m1.z + s1.z), take(1, m1.w, m1.w + s1.w);
-        take(2, m2.x, m2.x + s2.x), take(0, m2.y, m2.y + s2.y), take(1, m2.z, m2.z + s2.z), take(2, m2.w, m2.w + s2.w);
-    }
-    else
-        for (int c = c0; c < min(c0 + kGridGroup, a.n_cells); ++c)
+    float centre[3], half[3];
+    bool number = true;
 #pragma unroll
-            for (int j = 0; j < 3; ++j) take(j, a.bb_min[3 * c + j], a.bb_min[3 * c + j] + a.bb_len[3 * c + j]);
+    for (int j = 0; j < 3; ++j)
+    {
+        const float b = __ldg(a.bb_min + 3 * (size_t)c + j), e = b + __ldg(a.bb_len + 3 * (size_t)c + j);
+        centre[j] = 0.5f * b + 0.5f * e, half[j] = fabsf(0.5f * e - 0.5f * b);
+        number &= fabsf(e) < 1e30f;
+    }
     bool out = false;
 #pragma unroll
     for (int k = 0; k < kGridPlanes; ++k)
@@ -576,112 +695,118 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
 #pragma unroll
         for (int j = 0; j < 3; ++j)
         {
-            const float centre = 0.5f * lo[j] + 0.5f * hi[j], half = 0.5f * hi[j] - 0.5f * lo[j], reach = fabsf(p.w[j]) * half;
-            v += p.w[j] * centre + reach, size += fabsf(p.w[j] * centre) + reach;
+            const float reach = fabsf(p.w[j]) * half[j], at = p.w[j] * centre[j];
+            v += at + reach, size += fabsf(at) + reach;
         }
         out |= v < -1e-5f * size;
     }
     return number && out;
 }
 
-// First kernel: one warp per group of four cells.  kCull: a warp's next 32 groups are looked at first, a lane each; groups that lie
-// altogether out of sight are left out before their corners are projected, which costs about 200 instructions per group.
-// Cells with many rows (next to the camera a cell covers 10^5 pixels) and large rectangles in the per-pixel form are cut into
-// chunks that go to a queue, so that the second kernel can spread them over all SMs.  If the queue is full the warp does the
-// whole cell itself.
+// First kernel (kChunks = false): a warp takes `each` groups of four cells at a time, leaves out those that lie out of sight and prepares the others, a
+// lane per cell, as soon as it has 32 of them; what is left of these is drawn in groups of four, eight lanes per cell.  Cells with many rows
+// (next to the camera a cell covers 10^5 pixels) and large rectangles in the per-pixel form are cut into chunks that go to a queue,
+// so that the second kernel (kChunks = true) can spread them over all SMs.  If the queue is full the warp does the whole cell itself.
 //
-// Looking ahead wants groups to look at: with few per warp it saves less than the half-spaces and the second reading of the boxes cost,
-// unless the image is so small that there is little but the projection.  The whole call without and with it, camera on an orbit inside
-// the grid: 1920x1080 64^3 cells (9 groups a warp) 406 to 535 and 397 to 544 us (three cameras), 96^3 556 to 737 and 510 to 705, 128^3 941
-// to 1096 and 825 to 1006; 640x480 48^3 (4) 213 to 268 and 211 to 270, 56^3 (6) 167 to 208 and 154 to 205, 96^3 311 to 445 and 278 to
-// 412; 160x120 48^3 60 to 84 and 57 to 79, 40^3 (2) no difference.  All cells in sight: 64^3 186 and 189, 128^3 903 and 901, 48^3 at
-// 640x480 71 and 73.  (With a load per number instead of 16 bytes at a time all of that was 5 % slower than without looking.)
-constexpr int kGridCullGroups = 6, kGridCullGroupsSmall = 3, kGridCullCells = 4;  // groups per warp; in images of no more than a
-                                                                                  // pixel per kGridCullCells cells
-template <bool kCull>
+// Bound by instruction issue: at 128^3 cells and 1920x1080 80 us go into looking at and preparing the cells, 160 into the groups' segments and
+// what surrounds them, 270 into the rows, 50 to 100 into pixels tested one by one.  The whole call, before and after: 128^3 cells at 1920x1080 946 -> 631 us,
+// 117^3 at 373x249 274 -> 222, 112^3 at 160x120 171 -> 127, 47^3 at 369x277 149 -> 87, 58^3 at 308x173 74 -> 70 (before: preparation with eight
+// lanes per cell, a band kappa times as wide along all edges, chunks of 32 rows, an even stride, which gave a warp the same part of an axis of a power
+// of two of cells again and again).  Handing the groups out by an atomic counter as warps come for them: 890 us without the rows alone.
+template <bool kChunks>
 __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
-                                                                     int2* queue, int* queue_count)
+                                                                               int2* queue, int* queue_count, int each)
 {
     __shared__ Camera s_cam;
     __shared__ GridWarpSmem s_warp[kGridWarps];
+    __shared__ GridPlane s_planes[kGridPlanes];
+    int n = a.n_cells;
+    if (kChunks)
+    {
+        // reservations past the capacity were never written: those cells were done by the first kernel
+        n = min(*queue_count, kGridQueueCap);
+        if (n == 0) return;
+        each = min(32 / kGridGroup, max(1, n / ((int)gridDim.x * kGridWarps * kGridGroup)));
+    }
     if (threadIdx.x == 0) s_cam = load_camera(f, a.view);
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    GridWarpSmem& s    = s_warp[warp];
-    const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
-    const int n_groups = (a.n_cells + kGridGroup - 1) / kGridGroup, stride = gridDim.x * kGridWarps;
-    __shared__ GridPlane s_planes[kCull ? kGridPlanes : 1];
-    if (kCull)
+    if (!kChunks)
     {
         if (threadIdx.x < kGridPlanes) s_planes[threadIdx.x] = grid_plane(a, s_cam, threadIdx.x);
         __syncthreads();
     }
-    unsigned todo = 0;  // groups first + k stride still to do (bit k)
-    int first = blockIdx.x * kGridWarps + warp - 32 * stride;
-    for (;;)
-    {
-        if (todo == 0)
-        {
-            first += 32 * stride;
-            if (first >= n_groups) break;
-            const int mine = first + lane * stride;
-            todo = __ballot_sync(0xffffffffu, mine < n_groups && (!kCull || s_cam.has_dist || !grid_out_of_sight(a, s_planes, mine)));
-            continue;
-        }
-        const int group = first + (__ffs(todo) - 1) * stride;
-        todo &= todo - 1;
-        const int c         = group * kGridGroup + (lane >> 3);
-        const GridCell cell = grid_prepare(f, a, s_cam, s, c < a.n_cells ? c : -1, no_rows);
-        if (!__any_sync(0xffffffffu, cell.total > 0)) continue;
-        bool here = cell.total > 0;  // this warp does the cell itself
-        const long long units = cell.by_rows ? cell.y_size : cell.total;
-        const int unit        = cell.by_rows ? kGridRowChunk : kGridChunk;
-        const int n_chunks    = (int)((units + unit - 1) / unit);
-        unsigned large        = __ballot_sync(0xffffffffu, (lane & 7) == 0 && units > unit);
-        while (large)
-        {
-            const int from = __ffs(large) - 1;
-            large &= large - 1;
-            const int chunks = __shfl_sync(0xffffffffu, n_chunks, from);
-            int at = 0;
-            if (lane == 0) at = atomicAdd(queue_count, chunks);
-            at = __shfl_sync(0xffffffffu, at, 0);
-            // no room for all chunks: whatever part of the reservation lies inside the queue is marked unused
-            const bool fits = at + chunks <= kGridQueueCap;
-            const int ci    = group * kGridGroup + (from >> 3);
-            for (int k = lane; k < chunks && at + k < kGridQueueCap; k += 32) queue[at + k] = fits ? make_int2(ci, k) : make_int2(-1, 0);
-            if (fits && (lane >> 3) == (from >> 3)) here = false;
-        }
-        const bool refused  = grid_rows(a, s, 0, here && cell.by_rows ? cell.y_size : 0, c);
-        const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && here && (!cell.by_rows || refused));
-        grid_pixels(a, s, cell, c, slow, 0, cell.total);
-    }
-}
-
-// Second kernel: one warp per four queued (cell, chunk of rows or pixels).
-__global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_chunk_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
-                                                                           const int2* queue, const int* queue_count)
-{
-    __shared__ Camera s_cam;
-    __shared__ GridWarpSmem s_warp[kGridWarps];
-    if (threadIdx.x == 0) s_cam = load_camera(f, a.view);
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     GridWarpSmem& s    = s_warp[warp];
     const bool no_rows = s_cam.has_dist || *a.no_rows != 0;
-    // reservations past the capacity were never written: those cells were done by the first kernel
-    const int n = min(*queue_count, kGridQueueCap);
-    for (int e = blockIdx.x * kGridWarps + warp; e * kGridGroup < n; e += gridDim.x * kGridWarps)
+    // A warp's groups lie far apart, because cells of much work lie next to one another; the stride is odd (one warp stays idle), because
+    // grids tend to have a power of two of cells along an axis, and an even one would give a warp the same part of that axis again and again.
+    const long long stride = max(1, (int)gridDim.x * kGridWarps - 1);
+    int waiting            = 0;  // in s.todo, whole groups
+    for (long long first = blockIdx.x * kGridWarps + warp;; first += each * stride)
     {
-        const int mine = e * kGridGroup + (lane >> 3);
-        const int2 q   = mine < n ? queue[mine] : make_int2(-1, 0);
-        const GridCell cell = grid_prepare(f, a, s_cam, s, q.x, no_rows);
-        const int row0      = q.y * kGridRowChunk;
-        const bool refused  = grid_rows(a, s, row0, cell.by_rows ? min(kGridRowChunk, cell.y_size - row0) : 0, q.x);
-        const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && cell.total > 0 && (!cell.by_rows || refused));
-        const int unit      = cell.by_rows ? kGridRowChunk * cell.x_size : kGridChunk;  // pixels of a chunk
-        const long long first = (long long)q.y * unit;
-        grid_pixels(a, s, cell, q.x, slow, first, min(first + unit, cell.total));
+        if (blockIdx.x * kGridWarps + warp < stride && first * kGridGroup < n)
+        {
+            const long long at = (first + lane / kGridGroup * stride) * kGridGroup + lane % kGridGroup;
+            int2 q             = make_int2(-1, 0);
+            if (lane < each * kGridGroup && at < n) q = kChunks ? queue[at] : make_int2((int)at, 0);
+            if (!kChunks && q.x >= 0 && !s_cam.has_dist && grid_out_of_sight(a, s_planes, q.x)) q.x = -1;
+            unsigned kept = __ballot_sync(0xffffffffu, q.x >= 0);
+            kept |= kept >> 1 & 0x55555555u, kept |= kept >> 2 & 0x11111111u;  // bit 0 of a group: one of its four
+            kept = (kept & 0x11111111u) * 15u;
+            if (kept >> lane & 1) s.todo[waiting + __popc(kept & ((1u << lane) - 1u))] = q;
+            waiting += __popc(kept);
+            __syncwarp();
+            if (waiting < 32) continue;
+        }
+        if (waiting == 0) break;
+        int2 mine = make_int2(-1, 0);
+        if (lane < waiting) mine = s.todo[lane];
+        const int2 later = s.todo[lane + 32];
+        __syncwarp();
+        if (lane + 32 < waiting) s.todo[lane] = later;
+        waiting = max(waiting - 32, 0);
+        const GridCell prepared = grid_prepare(f, a, s_cam, s, mine.x, no_rows);
+        unsigned todo           = __ballot_sync(0xffffffffu, prepared.total() > 0);
+        while (todo)
+        {
+            const int group = (__ffs(todo) - 1) & -kGridGroup, from = group + (lane >> 3);  // the lane that prepared the slot's cell
+            todo &= ~(15u << group);
+            const GridCell cell = grid_cell_of(prepared, from);
+            const int c = __shfl_sync(0xffffffffu, mine.x, from), chunk = __shfl_sync(0xffffffffu, mine.y, from);
+            grid_segments(s, cell, from);
+            if constexpr (kChunks)
+            {
+                const int row0        = chunk * kGridRowChunk;
+                const bool refused    = grid_rows(a, s, row0, cell.by_rows ? min(kGridRowChunk, cell.y_size - row0) : 0, c);
+                const unsigned slow   = __ballot_sync(0xffffffffu, (lane & 7) == 0 && cell.total() > 0 && (!cell.by_rows || refused));
+                const int size        = cell.by_rows ? kGridRowChunk * cell.x_size : kGridChunk;  // pixels of a chunk
+                const long long begin = (long long)chunk * size;
+                grid_pixels(a, s, cell, c, slow, begin, min(begin + size, cell.total()));
+            }
+            else
+            {
+                bool here = cell.total() > 0;  // this warp does the cell itself
+                const int parts = cell.by_rows ? cell.y_size : (int)cell.total();
+                unsigned large  = __ballot_sync(0xffffffffu, (lane & 7) == 0 && parts > (cell.by_rows ? kGridRowChunk : kGridChunk));
+                while (large)
+                {
+                    const int head = __ffs(large) - 1;
+                    large &= large - 1;
+                    const int n_chunks = cell.by_rows ? (parts - 1) / kGridRowChunk + 1 : (parts - 1) / kGridChunk + 1;
+                    const int chunks = __shfl_sync(0xffffffffu, n_chunks, head), ci = __shfl_sync(0xffffffffu, c, head);
+                    int at = 0;
+                    if (lane == 0) at = atomicAdd(queue_count, chunks);
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    // no room for all chunks: whatever part of the reservation lies inside the queue is marked unused
+                    const bool fits = at + chunks <= kGridQueueCap;
+                    for (int k = lane; k < chunks && at + k < kGridQueueCap; k += 32) queue[at + k] = fits ? make_int2(ci, k) : make_int2(-1, 0);
+                    if (fits && (lane >> 3) == (head >> 3)) here = false;
+                }
+                const bool refused  = grid_rows(a, s, 0, here && cell.by_rows ? cell.y_size : 0, c);
+                const unsigned slow = __ballot_sync(0xffffffffu, (lane & 7) == 0 && here && (!cell.by_rows || refused));
+                grid_pixels(a, s, cell, c, slow, 0, cell.total());
+            }
+        }
     }
 }
 

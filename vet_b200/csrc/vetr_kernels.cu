@@ -3593,16 +3593,16 @@ extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vet
             ctx->grid_queue_count = reinterpret_cast<int*>(ctx->grid_queue + kGridQueueCap);
         }
         a.prefix = grid_prefix(ctx, (long long)view->h * (view->w + 1)), a.no_rows = ctx->grid_queue_count + 1;
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, sizeof(int), ctx->stream));
-        VETR_CUDA(ctx, cudaMemsetAsync(a.no_rows, a.prefix ? 0 : 1, sizeof(int), ctx->stream));
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, 2 * sizeof(int), ctx->stream));
+        if (!a.prefix) VETR_CUDA(ctx, cudaMemsetAsync(a.no_rows, 1, sizeof(int), ctx->stream));
         ctx->launches += 2 + (a.prefix != nullptr);
         if (a.prefix) grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
-        const int groups = (n_cells + kGridGroup - 1) / kGridGroup;
-        const int ctas   = std::min((groups + kGridWarps - 1) / kGridWarps, ctx->sm_count * 12);
-        const bool small = n_cells / kGridCullCells >= (long long)view->w * view->h;
-        const bool cull  = groups / (small ? kGridCullGroupsSmall : kGridCullGroups) >= ctas * kGridWarps;
-        (cull ? grid_loss_kernel<true> : grid_loss_kernel<false>)<<<ctas, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
-        grid_loss_chunk_kernel<<<ctx->sm_count * 16, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count);
+        const int resident = ctx->sm_count * kGridCtas;
+        const int groups = (int)((n_cells + (long long)kGridGroup - 1) / kGridGroup);
+        const int each   = std::min(32 / kGridGroup, std::max(1, groups / (resident * kGridWarps)));
+        const int ctas   = std::min((groups + kGridWarps - 1) / kGridWarps, resident);
+        grid_loss_kernel<false><<<ctas, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count, each);
+        grid_loss_kernel<true><<<resident, 32 * kGridWarps, 0, ctx->stream>>>(f, a, ctx->grid_queue, ctx->grid_queue_count, 0);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
