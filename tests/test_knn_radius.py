@@ -155,3 +155,28 @@ def test_gpu_dense_sheet_and_outliers(axis):
     xyz = np.concatenate([sheet, rng.uniform(-1, 1, size=(300, 3)).astype(np.float32) * np.float32(1.5)])
     for k in (1, 4, 8, 16):
         assert np.array_equal(_gpu(xyz, k), O.knn_radius(xyz, k)), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 5, 31, 257, 3001])
+@pytest.mark.parametrize("stride", [3, 4])
+def test_gpu_rows_of_three_and_four(n, stride):
+    """Rows of four floats are read with one 16-byte access, rows of three one by one; a coordinate that is not finite is refused
+    wherever it stands."""
+    from vet_b200 import _lib
+    from vet_b200.render import Rasterizer
+
+    rng = np.random.default_rng(n)
+    p = rng.standard_normal((n, stride)).astype(np.float32)
+    rast = Rasterizer(0)
+    pos = torch.from_numpy(p).cuda()
+    assert np.array_equal(rast.knn_radius(pos, 4).cpu().numpy(), O.knn_radius(np.ascontiguousarray(p[:, :3]), 4))
+    for row in {0, n // 2, n - 1}:
+        for column in range(3):
+            for value in (float("nan"), float("inf"), -float("inf")):
+                bad = pos.clone()
+                bad[row, column] = value
+                with pytest.raises(_lib.VetrError) as ei:
+                    rast.knn_radius(bad, 4)
+                assert ei.value.status == _lib.E_INVALID_ARG
+    rast.close()

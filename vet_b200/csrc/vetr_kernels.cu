@@ -3745,7 +3745,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     {
         cudaFree(ctx->knn_sorted), cudaFree(ctx->knn_point_cell), cudaFree(ctx->knn_queue);
         ctx->knn_sorted = nullptr, ctx->knn_point_cell = nullptr, ctx->knn_queue = nullptr, ctx->knn_cap_points = 0;
-        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_sorted, (size_t)n * sizeof(float4)));
+        VETR_CUDA(ctx, cudaMalloc(&ctx->knn_sorted, ((size_t)n + kKnnSortedPad) * sizeof(float4)));
         VETR_CUDA(ctx, cudaMalloc(&ctx->knn_point_cell, (size_t)n * sizeof(int)));
         VETR_CUDA(ctx, cudaMalloc(&ctx->knn_queue, (size_t)n * sizeof(int)));
         ctx->knn_cap_points = n;
@@ -3760,7 +3760,8 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     unsigned keys[6];
     VETR_CUDA(ctx, cudaMemcpyAsync(d_bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
     const int sweep = std::min((n + 255) / 256, ctx->sm_count * 8);
-    knn_bounds_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, d_bounds);
+    const bool four = position_stride == 4 && ((uintptr_t)position & 15) == 0;
+    (four ? knn_bounds_kernel<true> : knn_bounds_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, d_bounds);
     VETR_CUDA(ctx, cudaMemcpyAsync(keys, d_bounds, sizeof(keys), cudaMemcpyDeviceToHost, st));
     VETR_CUDA(ctx, cudaStreamSynchronize(st));
     float lo[3], hi[3], ext = 0.f, maxabs = 0.f;
@@ -3812,8 +3813,8 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
         VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
         VETR_CUDA(ctx, cudaMemsetAsync(d_occ, 0, sizeof(unsigned long long), st));
-        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
-        knn_occupied_kernel<<<(int)std::min<long long>((cells + 255) / 256, ctx->sm_count * 16), 256, 0, st>>>(ctx->knn_cells + kKnnCellsPad, cells, d_occ);
+        (four ? knn_count_kernel<true> : knn_count_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
+        knn_occupied_kernel<<<(int)std::min<long long>((cells + 1023) / 1024, ctx->sm_count * 8), 256, 0, st>>>(ctx->knn_cells + kKnnCellsPad, cells, d_occ);
         unsigned long long occupied = 0;
         VETR_CUDA(ctx, cudaMemcpyAsync(&occupied, d_occ, sizeof(occupied), cudaMemcpyDeviceToHost, st));
         VETR_CUDA(ctx, cudaStreamSynchronize(st));
@@ -3843,13 +3844,13 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     if (!counted)
     {
         VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
-        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
+        (four ? knn_count_kernel<true> : knn_count_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
         ctx->launches += 1;
     }
     knn_tile_sums_kernel<true><<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums);
     knn_spine_kernel<<<1, 1024, 0, st>>>(ctx->knn_tile_sums, n_tiles);
     knn_apply_kernel<true><<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums, cursor);
-    knn_scatter_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, cursor, ctx->knn_sorted);
+    (four ? knn_scatter_kernel<true> : knn_scatter_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, cursor, ctx->knn_sorted);
 
     // search
     KnnSearch a;

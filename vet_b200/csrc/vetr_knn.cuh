@@ -19,6 +19,7 @@ namespace vetr
 constexpr int kKnnMaxK       = 16;
 constexpr int kKnnScanTile   = 4096;       // cells per thread block of the scan (256 threads x 16)
 constexpr int kKnnCellsPad   = 4;          // zeros in front of the per-cell array (the first cell begins at slot 0), a whole 16 bytes
+constexpr int kKnnSortedPad    = 3;        // entries behind the sorted points, read with the last of them and not used
 constexpr long long kKnnMaxCells = 1ll << 26;  // 64 Mi cells: 16384 scan tiles, one spine block
 
 struct KnnGrid
@@ -46,33 +47,60 @@ __host__ __device__ inline float knn_unkey(unsigned k)
 #endif
 }
 
-// bounds[0..2] = min keys (initialised to 0xffffffff), bounds[3..5] = max keys (initialised to 0)
+// A point's coordinates; kFour: rows of four floats, 16-byte aligned.
+template <bool kFour>
+__device__ __forceinline__ float3 knn_load(const float* __restrict__ pos, int stride, int i)
+{
+    if (kFour)
+    {
+        const float4 p = __ldg(reinterpret_cast<const float4*>(pos) + i);
+        return make_float3(p.x, p.y, p.z);
+    }
+    const float* p = pos + (size_t)i * stride;
+    return make_float3(p[0], p[1], p[2]);
+}
+
+// bounds[0..2] = min keys (initialised to 0xffffffff), bounds[3..5] = max keys (initialised to 0; all ones if a coordinate is not finite:
+// the keys alone are not enough, nvcc 12.9 turns their maxima into maxima of floats, which pass over a NaN).  One atomic per
+// block and value: with one per warp the six addresses took longer than the points.
+template <bool kFour>
 __global__ void __launch_bounds__(256) knn_bounds_kernel(const float* __restrict__ pos, int stride, int n, unsigned* bounds)
 {
+    __shared__ unsigned s_part[8][6];
     unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
+    bool finite          = true;
+    const long long step = gridDim.x * 256;
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i < n; i += 4 * step)
     {
-        const float* p = pos + (size_t)i * stride;
+        float3 p[4];  // requested together; behind the last point the first of them once more
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int u = 0; u < 4; ++u) p[u] = knn_load<kFour>(pos, stride, (int)(i + u * step < n ? i + u * step : i));
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
         {
-            const unsigned k = knn_key(p[a]);
-            lo[a] = min(lo[a], k), hi[a] = max(hi[a], k);
+            const unsigned k[3] = {knn_key(p[u].x), knn_key(p[u].y), knn_key(p[u].z)};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) lo[a] = min(lo[a], k[a]), hi[a] = max(hi[a], k[a]);
+            finite &= fabsf(p[u].x) < CUDART_INF_F && fabsf(p[u].y) < CUDART_INF_F && fabsf(p[u].z) < CUDART_INF_F;
         }
     }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
     {
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-        if ((threadIdx.x & 31) == 0)
-        {
-            atomicMin(bounds + a, lo[a]);
-            atomicMax(bounds + 3 + a, hi[a]);
-        }
+        if (!finite) hi[a] = 0xffffffffu;
+        lo[a] = __reduce_min_sync(0xffffffffu, lo[a]), hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+        if (lane == 0) s_part[warp][a] = lo[a], s_part[warp][3 + a] = hi[a];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6)
+    {
+        unsigned v = s_part[0][threadIdx.x];
+        for (int w = 1; w < 8; ++w) v = threadIdx.x < 3 ? min(v, s_part[w][threadIdx.x]) : max(v, s_part[w][threadIdx.x]);
+        if (threadIdx.x < 3)
+            atomicMin(bounds + threadIdx.x, v);
+        else
+            atomicMax(bounds + threadIdx.x, v);
     }
 }
 
@@ -91,26 +119,47 @@ __device__ __forceinline__ int knn_cell_of(const KnnGrid& g, float x, float y, f
 }
 
 // counts[cell] += 1 for every point; point_cell[i] = its cell.
+template <bool kFour>
 __global__ void __launch_bounds__(256) knn_count_kernel(const float* __restrict__ pos, int stride, int n, const __grid_constant__ KnnGrid g,
                                                         int* counts, int* point_cell)
 {
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
+    const long long step = gridDim.x * 256;
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i < n; i += 4 * step)
     {
-        const float* p = pos + (size_t)i * stride;
-        int cx, cy, cz;
-        const int c = knn_cell_of(g, p[0], p[1], p[2], cx, cy, cz);
-        if (point_cell) point_cell[i] = c;
-        atomicAdd(counts + c, 1);
+        float3 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p[u] = knn_load<kFour>(pos, stride, (int)(i + u * step < n ? i + u * step : i));
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+        {
+            if (i + u * step >= n) break;
+            int cx, cy, cz;
+            const int c = knn_cell_of(g, p[u].x, p[u].y, p[u].z, cx, cy, cz);
+            point_cell[i + u * step] = c;
+            atomicAdd(counts + c, 1);
+        }
     }
 }
 
-// Number of non-empty cells (the cell size is chosen from the points per occupied cell).
+// Number of non-empty cells (the cell size is chosen from the points per occupied cell).  counts: 16-byte aligned.
 __global__ void __launch_bounds__(256) knn_occupied_kernel(const int* __restrict__ counts, long long n_cells, unsigned long long* occupied)
 {
     int mine = 0;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n_cells; i += (long long)gridDim.x * 256) mine += counts[i] > 0;
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(occupied, (unsigned long long)mine);
+    for (long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4; i < n_cells; i += (long long)gridDim.x * 1024)
+    {
+        const int4 c = scan_load<true>(counts, i, n_cells);
+        mine += (c.x > 0) + (c.y > 0) + (c.z > 0) + (c.w > 0);
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    __shared__ int s_part[8];
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        unsigned long long sum = 0;
+        for (int w = 0; w < 8; ++w) sum += s_part[w];
+        if (sum) atomicAdd(occupied, sum);
+    }
 }
 
 // Exclusive scan of the cell counts in three kernels: sums of tiles, scan of the tile sums by one block, scan inside the tiles.
@@ -200,14 +249,25 @@ __global__ void __launch_bounds__(256) knn_apply_kernel(const int* counts, long 
 
 // Counting sort, last step: sorted[slot] = (x, y, z, index bits); cursor[cell] starts at the cell's first slot and ends
 // at its last + 1, the first slot of the next cell.
+template <bool kFour>
 __global__ void __launch_bounds__(256) knn_scatter_kernel(const float* __restrict__ pos, int stride, int n, const int* __restrict__ point_cell,
                                                           int* cursor, float4* sorted)
 {
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
+    const long long step = gridDim.x * 256;
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i < n; i += 4 * step)
     {
-        const float* p = pos + (size_t)i * stride;
-        const int slot = atomicAdd(cursor + point_cell[i], 1);
-        sorted[slot]   = make_float4(p[0], p[1], p[2], __int_as_float(i));
+        // four points of a thread together (no faster than one by one, 56 us for 3.8 M points: points of a cell follow each other, and so do
+        // their atomics)
+        int slot[4];
+        float3 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) slot[u] = i + u * step < n ? point_cell[i + u * step] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (slot[u] >= 0) slot[u] = atomicAdd(cursor + slot[u], 1), p[u] = knn_load<kFour>(pos, stride, (int)(i + u * step));
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (slot[u] >= 0) sorted[slot[u]] = make_float4(p[u].x, p[u].y, p[u].z, __int_as_float((int)(i + u * step)));
     }
 }
 
@@ -242,14 +302,15 @@ __device__ __forceinline__ void knn_insert(float (&best)[KMAX], float d)
 template <int KMAX>
 __device__ __forceinline__ void knn_scan_slots(const KnnSearch& a, int b, int e, float x, float y, float z, float (&best)[KMAX])
 {
-    // four candidates at a time: their loads are in flight together, and one comparison passes over most groups
+    // Four candidates at a time: their loads are in flight together, and one comparison passes over most groups.  (Candidates closer than
+    // the k-th put by in shared memory and inserted together, because lanes rarely meet one at the same time: 575 -> 744 us.)
     for (int j = b; j < e; j += 4)
     {
         float d[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
         {
-            const float4 q = __ldg(a.sorted + min(j + k, e - 1));
+            const float4 q = __ldg(a.sorted + j + k);  // there are kKnnSortedPad entries behind the last
             const float dx = x - q.x, dy = y - q.y, dz = z - q.z;
             d[k]           = j + k < e ? dx * dx + dy * dy + dz * dz : CUDART_INF_F;
         }
@@ -289,8 +350,9 @@ __device__ __forceinline__ float knn_gap2(const KnnSearch& a, float d)
 // First pass: one thread per point (in cell order, so that a warp's points share their cells), the cube of 3^3 cells.  The
 // point's own cell comes first: in a dense cell it holds neighbours closer than the cell's faces, and the other cells, nearest
 // first, are passed over where they lie beyond the k-th distance found so far (a later candidate would have to be smaller, so
-// the result is the same).  Bound by instruction issue, 79 % of the slots with ten of 32 lanes.  4 M points of a planar scene with
-// 5 % outliers, k = 4: 969 -> 769 us (before: all 27 cells, row by row from one corner).
+// the result is the same).  Bound by instruction issue, 82 % of the slots with ten of 32 lanes.  4 M points of a planar scene with
+// 5 % outliers, k = 4: 969 us with all 27 cells, row by row from one corner, 769 with all lanes going through the rows that any of them
+// needs, 575 like this.
 template <int KMAX>
 __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ KnnSearch a)
 {
@@ -307,13 +369,27 @@ __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ K
     const float ylo = knn_gap2(a, p.y - (g.oy + (float)cy * g.cell)), yhi = knn_gap2(a, (g.oy + (float)(cy + 1) * g.cell) - p.y);
     const float zlo = knn_gap2(a, p.z - (g.oz + (float)cz * g.cell)), zhi = knn_gap2(a, (g.oz + (float)(cz + 1) * g.cell) - p.z);
     knn_scan_slots<KMAX>(a, a.first[own], a.first[own + 1], p.x, p.y, p.z, best);
-    // steps 0, 1: the neighbours along x; 2..9: the other rows of three cells, those that share a face with the own row first
+    // Steps 0, 1: the neighbours along x; 2..9: the other rows of three cells, those that share a face with the own row first.  Each lane
+    // goes through the steps that it needs and not through all of the warp's: with the own cell done these are two or three of ten.
+    const bool y0 = cy > 0, y1 = cy < g.ny - 1, z0 = cz > 0, z1 = cz < g.nz - 1;
+    const float k0 = best[KMAX - 1];
+    unsigned rest  = 0;
+    if (cx > 0 && xlo < k0) rest |= 1u << 0;
+    if (cx < g.nx - 1 && xhi < k0) rest |= 1u << 1;
+    if (y0 && ylo < k0) rest |= 1u << 2;
+    if (y1 && yhi < k0) rest |= 1u << 3;
+    if (z0 && zlo < k0) rest |= 1u << 4;
+    if (z1 && zhi < k0) rest |= 1u << 5;
+    if (y0 && z0 && ylo + zlo < k0) rest |= 1u << 6;
+    if (y1 && z0 && yhi + zlo < k0) rest |= 1u << 7;
+    if (y0 && z1 && ylo + zhi < k0) rest |= 1u << 8;
+    if (y1 && z1 && yhi + zhi < k0) rest |= 1u << 9;
 #pragma unroll 1
-    for (int t = 0; t < 10; ++t)
+    while (rest)
     {
+        const int t = __ffs(rest) - 1;
+        rest &= rest - 1;
         const int dy = (int)(0x88585u >> (2 * t) & 3) - 1, dz = (int)(0xa0855u >> (2 * t) & 3) - 1;  // two bits a step
-        const int y = cy + dy, z = cz + dz;
-        if ((unsigned)y >= (unsigned)g.ny || (unsigned)z >= (unsigned)g.nz) continue;
         const float gap = (dy < 0 ? ylo : dy > 0 ? yhi : 0.f) + (dz < 0 ? zlo : dz > 0 ? zhi : 0.f);
         const float kth = best[KMAX - 1];
         if (!(gap < kth)) continue;
@@ -329,7 +405,7 @@ __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ K
             if (!right) continue;
             c0 = c1;
         }
-        const int row = (z * g.ny + y) * g.nx;
+        const int row = ((cz + dz) * g.ny + cy + dy) * g.nx;
         knn_scan_slots<KMAX>(a, a.first[row + c0], a.first[row + c1 + 1], p.x, p.y, p.z, best);
     }
     if (knn_done(best[KMAX - 1], knn_margin(a, p.x, p.y, p.z, cx, cy, cz, 1)))
@@ -343,6 +419,10 @@ __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ K
 // slots, or two (left and right of the cube already visited), and rows or their ends that lie beyond the k-th distance known so
 // far are left out.  The ranges of 32 rows are then laid end to end and every lane takes every 32nd candidate of them.
 // After each stage the stopping rule is applied to the cube's faces.
+//
+// From stage to stage: 2, 4, 8, ... until there are k candidates, then the cube that holds the k-th of them.  4 M points of a planar
+// scene with 5 % outliers, k = 4: 553 us with the stages 2, 4, 6, 9, 13, ..., row coordinates by division and a k-th distance formed by shuffles
+// for every 32 rows, 470 like this; a first stage of 3 instead of 2 is 12 us faster there and slower with 30 to 200 k points (the whole call by 3 %).
 //
 // Where the cube of an isolated point meets a dense surface, a few rows hold hundreds of candidates: with a lane scanning
 // the whole of its row the others waited for it.  4 M points of a planar scene with 5 % outliers, k = 4: 1054 -> 557 us.
@@ -363,18 +443,20 @@ __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ Kn
         for (int j = 0; j < KMAX; ++j) best[j] = (lane == 0 && j < a.dummies) ? -CUDART_INF_F : CUDART_INF_F;
         float kth       = CUDART_INF_F;  // k-th smallest of all lanes' candidates so far
         const int r_max = max(max(max(cx, g.nx - 1 - cx), max(cy, g.ny - 1 - cy)), max(cz, g.nz - 1 - cz));
-        int r_prev = -1;  // half-width of the cube already visited (-1: nothing yet)
-        for (int r = min(2, max(r_max, 1));; r = min(r + max(r / 2, 2), max(r_max, 1)))  // 2, 4, 6, 9, 13, ...
+        bool closer = false;  // the lane has a new candidate since kth was formed
+        int r_prev  = -1;     // half-width of the cube already visited (-1: nothing yet)
+        for (int r = min(2, max(r_max, 1));;)
         {
             const int ylo = max(cy - r, 0), yhi = min(cy + r, g.ny - 1), zlo = max(cz - r, 0), zhi = min(cz + r, g.nz - 1);
             const int wz = zhi - zlo + 1, rows = (yhi - ylo + 1) * wz;  // <= ny nz <= 2^26
-            for (int base = 0; base < rows; base += 32)
+            const int dy = 32 / wz, dz = 32 % wz;                       // from one of the lane's rows to its next
+            int y = ylo + lane / wz, z = zlo + lane % wz;
+            for (int base = 0; base < rows; base += 32, y += dy, z += dz)
             {
+                if (z > zhi) z -= wz, ++y;
                 int b0 = 0, n0 = 0, b1 = 0, n1 = 0;  // the lane's row: its one or two ranges of slots
-                const int t = base + lane;
-                if (t < rows)
+                if (base + lane < rows)
                 {
-                    const int y = ylo + t / wz, z = zlo + t % wz;
                     float gap = 0.f;
                     if (y != cy) gap += knn_gap2(a, y < cy ? p.y - (g.oy + (float)(y + 1) * g.cell) : (g.oy + (float)y * g.cell) - p.y);
                     if (z != cz) gap += knn_gap2(a, z < cz ? p.z - (g.oz + (float)(z + 1) * g.cell) : (g.oz + (float)z * g.cell) - p.z);
@@ -414,19 +496,22 @@ __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ Kn
                         const float4 q = __ldg(a.sorted + (at < n_left ? left + at : right + at - n_left));
                         const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
                         const float d  = dx * dx + dy * dy + dz * dz;
-                        if (d < best[KMAX - 1]) knn_insert<KMAX>(best, d);
+                        if (d < best[KMAX - 1] && d < kth) knn_insert<KMAX>(best, d), closer = true;
                     }
                 }
-                // the k-th smallest of all lanes: k times, take the smallest head off its list (of a copy)
+                // the k-th smallest of all lanes: k times, take the smallest head off its list (of a copy).  Squares of distances order
+                // like their bits, and the one -inf of a lane's head comes before them.
+                if (!__any_sync(kAll, closer)) continue;
+                closer = false;
                 float rest[KMAX];
 #pragma unroll
                 for (int j = 0; j < KMAX; ++j) rest[j] = best[j];
 #pragma unroll 1
                 for (int j = 0; j < KMAX; ++j)
                 {
-                    kth = rest[0];
-                    for (int o = 16; o > 0; o >>= 1) kth = fminf(kth, __shfl_xor_sync(kAll, kth, o));
-                    const unsigned holders = __ballot_sync(kAll, rest[0] == kth);
+                    const int head         = __reduce_min_sync(kAll, __float_as_int(rest[0]));
+                    const unsigned holders = __ballot_sync(kAll, __float_as_int(rest[0]) == head);
+                    kth                    = __int_as_float(head);
                     if (lane == __ffs(holders) - 1)
                     {
 #pragma unroll
@@ -440,7 +525,10 @@ __global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ Kn
                 if (lane == 0) a.radius[(size_t)__float_as_int(p.w) * a.radius_stride] = sqrtf(kth);
                 break;
             }
-            r_prev = r;
+            // as far as the k-th distance reaches, or twice as far while there are not k candidates
+            r_prev     = r;
+            const int next = kth < CUDART_INF_F ? (int)fminf(ceilf((sqrtf(kth) + a.slack) * g.inv_cell), 1e6f) : 2 * r;
+            r          = min(max(next, r + 1), max(r_max, 1));
         }
     }
 }
