@@ -6,7 +6,7 @@ import pytest
 from oracle import oracle as O
 from tests import util
 from vet_b200 import scenes
-from vet_b200.render import default_params
+from vet_b200.render import default_params, level_sizes
 
 pytestmark = pytest.mark.gpu
 
@@ -545,3 +545,45 @@ def test_launch_count_of_an_empty_cloud():
     rast.backward_raw([torch.ones_like(c) for c in out["color"]], want_points=False)
     assert rast.launch_count() - before == 2 + 1 + 1  # gradients cleared, background summed
     rast.close()
+
+
+# ---- kernels that are set up while the one before them ends
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_steps_follow_one_another(rasterizer, mode):
+    """Steps that follow one another on the stream, each with inputs that were written just before it, give what the same steps give with
+    the device waited for between all calls: no kernel starts on data that the one before it still works on."""
+    import torch
+
+    sc = scenes.config_planar(20_000, 200, 120, 125.0, n_views=2, seed=5)
+    pos, index, tex, conf, bg, poses, intr = (torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device) for a in (
+        sc.position, sc.index, sc.texture, sc.confidence, sc.background, sc.poses, sc.intrinsics))
+    prm = default_params(render_mode=mode, num_layers=4, num_channels=tex.shape[0])
+    loss = torch.zeros((), device=rasterizer.device)
+    given = [torch.randn(2, tex.shape[0], h, w, device=rasterizer.device) for w, h in level_sizes(200, 120, 4)]
+
+    def steps(wait):
+        p, t, q, results = pos.clone(), tex.clone(), poses.clone(), []
+        for k in range(12):
+            p[:, :3] += 0.01 * (-1) ** k
+            q[:, 4] += 0.02
+            t.mul_(0.9)
+            wait()
+            out = rasterizer.forward(p, index, t, conf, bg, q, intr, sc.views, prm)
+            wait()
+            targets = [torch.zeros_like(c) for c in out["color"]]
+            grads = [torch.empty_like(c) for c in out["color"]]
+            rasterizer.l1_loss_grad(out["color"], targets, grads, loss)
+            wait()
+            raw = rasterizer.backward_raw(given)  # (grads holds signs, which may differ where an image is next to nothing)
+            wait()
+            g = rasterizer.finalize(raw)
+            results.append([c.clone() for c in out["color"]] + [loss.clone(), g["texture"].clone(), g["points"].clone(), g["pose"].clone()])
+            wait()
+        torch.cuda.synchronize()
+        return results
+
+    for a, b in zip(steps(torch.cuda.synchronize), steps(lambda: None)):
+        for x, y in zip(a, b):  # the order of fp32 sums is not fixed
+            assert torch.allclose(x, y, rtol=1e-4, atol=1e-5 * float(x.abs().max()))

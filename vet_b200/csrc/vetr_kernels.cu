@@ -47,6 +47,15 @@
 
 namespace vetr
 {
+// First statement of every kernel that launch() starts, and of those in between: the next kernel on the stream may be set up on SMs that have room as soon
+// as all blocks of this one run, and this one goes on when the kernel before it has ended and its writes are to be seen.  Nothing is
+// read or written before; because every kernel waits like this, the end of one is the end of all before it.
+__device__ __forceinline__ void begin_kernel()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #ifndef VETR_ITEM_THREADS
 #    define VETR_ITEM_THREADS 128
 #endif
@@ -220,6 +229,7 @@ constexpr int kCollectThreads = 128, kCollectCtas = 12;
 template <bool kCollect, int kPts>
 __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCollect ? kCollectCtas : 5) project_kernel(const __grid_constant__ Frame f)
 {
+    begin_kernel();
     constexpr int kThreadsHere = kCollect ? kCollectThreads : kProjThreads;
     __shared__ Camera s_cam;
     const int b     = blockIdx.y;
@@ -516,6 +526,7 @@ template <bool kVec>
 __global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restrict__ counts, long long n, long long* tile_sums, int* status,
                                                              long long capacity, int* item_start, unsigned* ticket)
 {
+    begin_kernel();
     __shared__ long long s_sum[8];
     __shared__ int s_max[8];
     const long long base = (long long)blockIdx.x * kScanTile;
@@ -554,6 +565,7 @@ __global__ void __launch_bounds__(256) scan_apply_kernel(const int* __restrict__
                                                          int* __restrict__ ends, const int* __restrict__ status,
                                                          int* __restrict__ item_start)
 {
+    begin_kernel();
     __shared__ int s_warp[32];
     const long long base = (long long)blockIdx.x * kScanTile;
     int4 c[4];
@@ -907,6 +919,7 @@ struct BlendSmem
 __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const __grid_constant__ Frame f,
                                                                           const __grid_constant__ OutPtrs out)
 {
+    begin_kernel();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlendSmem& s = *reinterpret_cast<BlendSmem*>(smem_raw);
     const int tid     = threadIdx.x;
@@ -1103,6 +1116,7 @@ __device__ __forceinline__ float transmittance_chain(const float* alpha, float* 
 __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ OutPtrs out)
 {
+    begin_kernel();
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LongBlendSmem& s = *reinterpret_cast<LongBlendSmem*>(smem_raw);
@@ -1518,6 +1532,7 @@ __device__ __forceinline__ float4 pack_pixel(const Frame& f, const BackPtrs& bp,
 }
 __global__ void __launch_bounds__(256) pack_images_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int view, l, o;
     if (r < f.Prm * f.n_views) pack_pixel(f, bp, r, view, l, o);
@@ -1842,6 +1857,7 @@ template <bool kFuzzy, bool kBilinear>
 __global__ void __launch_bounds__(kThreads, kBackCtas) backward_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     static_assert(!(kFuzzy && kBilinear), "mode 2 and mode 3 exclude each other");
     using Smem = typename BackSmemOf<kFuzzy, kBilinear>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1935,6 +1951,7 @@ template <bool kBilinear>
 __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_constant__ Frame f,
                                                                  const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BackSmemSuffix& s = *reinterpret_cast<BackSmemSuffix*>(smem_raw);
@@ -2081,6 +2098,7 @@ template <int kMin, int kMax>
 __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     if (f.status[2] <= kMin) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FuzzyLongSmem<kMax>& s = *reinterpret_cast<FuzzyLongSmem<kMax>*>(smem_raw);
@@ -2163,6 +2181,7 @@ template <int kCam, bool kBilinear>
 __global__ void __launch_bounds__(kProjThreads, kCam == 2 || kBilinear ? 3 : 4)
     point_backward_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp, int tiles)
 {
+    begin_kernel();
     extern __shared__ __align__(16) float4 s_gp[];  // [tiles][kProjThreads], every thread its own column
     __shared__ Camera s_cam[VETR_MAX_VIEWS];
     __shared__ double s_red[kProjThreads / 32][kCamValues];
@@ -2317,6 +2336,7 @@ __device__ __forceinline__ float4 load_grad_planar(const Frame& f, const BackPtr
 // Start of a call: no depth, empty accumulators, status.
 __global__ void __launch_bounds__(256) fuzzy_dt_clear_kernel(const __grid_constant__ Frame f)
 {
+    begin_kernel();
     const long long g = (long long)blockIdx.x * 256 + threadIdx.x;
     if (g < f.PT)
     {
@@ -2331,6 +2351,7 @@ __global__ void __launch_bounds__(256) fuzzy_dt_clear_kernel(const __grid_consta
 template <int kPass>
 __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_point_kernel(const __grid_constant__ Frame f)
 {
+    begin_kernel();
     __shared__ Camera s_cam;
     const int b = blockIdx.y;
     if (threadIdx.x == 0) s_cam = load_camera(f, b);
@@ -2376,6 +2397,7 @@ __global__ void __launch_bounds__(kProjThreads) fuzzy_dt_point_kernel(const __gr
 // CombineAndFill (PointRenderer.cu:24-52) + CreateMask + depth output, one thread per pixel of the pixel space.
 __global__ void __launch_bounds__(256) fuzzy_dt_combine_kernel(const __grid_constant__ Frame f, const __grid_constant__ OutPtrs out)
 {
+    begin_kernel();
     __shared__ int s_sum[8], s_max[8];
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int n_acc = 0;
@@ -2431,6 +2453,7 @@ __device__ __forceinline__ void fuzzy_dt_background_sum(const Frame& f, const Ba
 __global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_constant__ Frame f,
                                                                    const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < f.PT; g += (long long)gridDim.x * blockDim.x)
         if (f.counts[g] == 0)
@@ -2444,6 +2467,7 @@ __global__ void __launch_bounds__(256) fuzzy_dt_background_kernel(const __grid_c
 }
 __global__ void __launch_bounds__(256) fuzzy_dt_pack_kernel(const __grid_constant__ Frame f, const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     const long long total = f.Prm * f.n_views;
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < total; r += (long long)gridDim.x * blockDim.x)
@@ -2466,6 +2490,7 @@ template <int kCam>  // as in point_backward_kernel
 __global__ void __launch_bounds__(kProjThreads, 4) fuzzy_dt_backward_kernel(const __grid_constant__ Frame f,
                                                                          const __grid_constant__ BackPtrs bp)
 {
+    begin_kernel();
     constexpr bool kIntr = kCam == 2;
     __shared__ Camera s_cam;
     __shared__ double s_red[kProjThreads / 32][kCamValues];
@@ -2586,6 +2611,7 @@ __device__ __forceinline__ void normalize_row(T* g, const float* count, int i, i
 
 __global__ void __launch_bounds__(256) finalize_kernel(const __grid_constant__ FinalizeArgs a)
 {
+    begin_kernel();
     const unsigned b = blockIdx.x;
     if (b < a.desc_end)
     {
@@ -2626,6 +2652,7 @@ struct ZeroArgs
 
 __global__ void __launch_bounds__(256) zero_buffers_kernel(const __grid_constant__ ZeroArgs a)
 {
+    begin_kernel();
     const long long total = a.end[a.n - 1];
     for (long long u = (long long)blockIdx.x * 256 + threadIdx.x; u < total; u += (long long)gridDim.x * 256)
     {
@@ -2882,6 +2909,7 @@ struct L1Args
 
 __global__ void __launch_bounds__(256) l1_loss_grad_kernel(const __grid_constant__ L1Args a)
 {
+    begin_kernel();
     __shared__ float s_part[8];
     const long long total  = a.end[a.levels - 1];
     const long long stride = (long long)gridDim.x * blockDim.x * 4;
@@ -2996,6 +3024,27 @@ struct PassScope
         }
     }
 };
+
+// Launches a kernel that begins with begin_kernel().  overlap: its blocks may be set up while the kernel before it on the stream ends, which hides
+// the way from one kernel to the next.  100 k points at 512x512 101 -> 85 us, a smallest batch 85 -> 82, 3 M points at 1920x1080
+// forward only 344 -> 335, mode 2 with 1 M points 459 -> 440, mode 0 with 2 M points and two views 388 -> 374, mode 3 with 3 M points and two views
+// the same.  Not where
+// - the kernel is one of the item kernels (sort + blend, backward, their long lists), whose blocks take every n-th item: set up early they
+//   come to lie next to each other on the SMs that are free first, and so do the items of much work (mode 3 at 1280x720 428 -> 450 us);
+// - there is much to do (20 M points, eight views 18120 -> 18440 us, 8 M points and four views the same): nothing to be gained.
+constexpr long long kOverlapPoints = 1 << 24;            // points times views, elements
+constexpr long long kOverlapUnits  = 3 * kOverlapPoints;  // 16-byte units of zeros: a point's gradients are 2.25 of them
+template <typename... Parameters, typename... Arguments>
+static void launch(bool overlap, void (*kernel)(Parameters...), dim3 grid, int block, size_t smem, cudaStream_t stream, const Arguments&... arguments)
+{
+    cudaLaunchConfig_t config = {};
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.gridDim = grid, config.blockDim = dim3(block), config.dynamicSmemBytes = smem, config.stream = stream;
+    config.attrs = &attribute, config.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&config, kernel, arguments...);
+}
 
 #define VETR_CUDA(ctx, call)                      \
     do                                            \
@@ -3239,11 +3288,11 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
 // The two kernels of the scan.  *ticket and status[0..3] are zero on the stream before it (a ticket that is not would have the sums of
 // the tiles scanned too early).
 static void launch_scan(const int* counts, long long n, long long capacity, long long* tile_sums, unsigned* ticket, int n_tiles, int* ends,
-                        int* status, int* items, cudaStream_t st)
+                        int* status, int* items, cudaStream_t st, bool overlap)
 {
     const bool vec = (((uintptr_t)counts | (uintptr_t)ends) & 15) == 0;
-    (vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, status, capacity, items, ticket);
-    (vec ? scan_apply_kernel<true> : scan_apply_kernel<false>)<<<n_tiles, 256, 0, st>>>(counts, n, tile_sums, ends, status, items);
+    launch(overlap, vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>, n_tiles, 256, 0, st, counts, n, tile_sums, status, capacity, items, ticket);
+    launch(overlap, vec ? scan_apply_kernel<true> : scan_apply_kernel<false>, n_tiles, 256, 0, st, counts, n, tile_sums, ends, status, items);
 }
 
 // Launches zero_buffers_kernel on the context's stream; `bytes` are multiples of 4, as are the addresses.
@@ -3262,7 +3311,7 @@ static int zero_buffers(vetr_ctx* ctx, void* const* buffers, const int64_t* byte
     }
     if (a.n == 0) return VETR_OK;
     ctx->launches += 1;
-    zero_buffers_kernel<<<(unsigned)std::min<long long>((total + 255) / 256, ctx->sm_count * 32ll), 256, 0, ctx->stream>>>(a);
+    launch(total <= kOverlapUnits, zero_buffers_kernel, (unsigned)std::min<long long>((total + 255) / 256, ctx->sm_count * 32ll), 256, 0, ctx->stream, a);
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }
@@ -3297,24 +3346,25 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         if (out_mask) out.mask[l] = out_mask[l];
         if (out_depth) out.depth[l] = out_depth[l];
     }
-    cudaStream_t st = ctx->stream;
+    cudaStream_t st    = ctx->stream;
+    const bool overlap = (long long)f.n * n_views <= kOverlapPoints;
     if (f.mode == VETR_MODE_FUZZY_DT)
     {
         if (f.capacity < f.PT) return VETR_E_INVALID_ARG;  // the fragment buffer holds one accumulator record per pixel
         const int ctas = (f.n + kProjThreads - 1) / kProjThreads;
         {
             PassScope t(ctx, VETR_T_COUNT, 1 + (ctas > 0));
-            fuzzy_dt_clear_kernel<<<(unsigned)((f.PT + 255) / 256), 256, 0, st>>>(f);
-            if (ctas > 0) fuzzy_dt_point_kernel<0><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f);
+            launch(overlap, fuzzy_dt_clear_kernel, (unsigned)((f.PT + 255) / 256), 256, 0, st, f);
+            if (ctas > 0) launch(overlap, fuzzy_dt_point_kernel<0>, dim3(ctas, n_views), kProjThreads, 0, st, f);
         }
         if (ctas > 0)
         {
             PassScope t(ctx, VETR_T_COLLECT, 1);
-            fuzzy_dt_point_kernel<1><<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f);
+            launch(overlap, fuzzy_dt_point_kernel<1>, dim3(ctas, n_views), kProjThreads, 0, st, f);
         }
         {
             PassScope t(ctx, VETR_T_SORT_BLEND, 1);
-            fuzzy_dt_combine_kernel<<<(unsigned)((f.PT + 255) / 256), 256, 0, st>>>(f, out);
+            launch(overlap, fuzzy_dt_combine_kernel, (unsigned)((f.PT + 255) / 256), 256, 0, st, f, out);
         }
         VETR_CUDA(ctx, cudaGetLastError());
         return VETR_OK;
@@ -3329,18 +3379,18 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     if (point_ctas > 0)
     {
         PassScope t(ctx, VETR_T_COUNT, 1);
-        project_kernel<false, kPointsPerThread><<<dim3(point_ctas, n_views), kProjThreads, 0, st>>>(f);
+        launch(overlap, project_kernel<false, kPointsPerThread>, dim3(point_ctas, n_views), kProjThreads, 0, st, f);
     }
     const int n_tiles = (int)((f.PT + kScanTile - 1) / kScanTile);
     {
         PassScope t(ctx, VETR_T_SCAN, 2);
-        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, st);
+        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, st, overlap);
     }
     if (point_ctas > 0)
     {
         PassScope t(ctx, VETR_T_COLLECT, 1);
         const int ctas = (f.n + kCollectThreads * kCollectPoints - 1) / (kCollectThreads * kCollectPoints);
-        project_kernel<true, kCollectPoints><<<dim3(ctas, n_views), kCollectThreads, 0, st>>>(f);
+        launch(overlap, project_kernel<true, kCollectPoints>, dim3(ctas, n_views), kCollectThreads, 0, st, f);
     }
     {
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
@@ -3392,7 +3442,8 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
     bp.g_desc = (float4*)g_desc, bp.g_conf = g_conf, bp.g_points = (float4*)g_points, bp.g_background = g_background;
     bp.g_pose = g_pose, bp.g_pose_count = g_pose_count, bp.g_intr = g_intr, bp.g_intr_count = g_intr_count;
     if (!f.need_point_grad && f.mode != VETR_MODE_BILINEAR_BLEND && f.mode != VETR_MODE_FUZZY_DT) bp.g_points = nullptr;
-    f.dropout = dropout;
+    f.dropout          = dropout;
+    const bool overlap = (long long)f.n * n_views <= kOverlapPoints;
     if (f.mode == VETR_MODE_FUZZY_DT)
     {
         if (!(phases & VETR_BACKWARD_FRAGMENTS)) return VETR_OK;  // mode 0 has one phase
@@ -3404,13 +3455,13 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         PassScope t(ctx, VETR_T_BACKWARD, 1 + (ctas > 0));
         cudaStream_t st = ctx->stream;
         if (f.img4)
-            fuzzy_dt_pack_kernel<<<ctx->sm_count * 16, 256, 0, st>>>(f, bp);
+            launch(overlap, fuzzy_dt_pack_kernel, ctx->sm_count * 16, 256, 0, st, f, bp);
         else
-            fuzzy_dt_background_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(f, bp);
+            launch(overlap, fuzzy_dt_background_kernel, ctx->sm_count * 4, 256, 0, st, f, bp);
         if (ctas > 0)
         {
             const auto kernel = g_intr ? fuzzy_dt_backward_kernel<2> : g_pose ? fuzzy_dt_backward_kernel<1> : fuzzy_dt_backward_kernel<0>;
-            kernel<<<dim3(ctas, n_views), kProjThreads, 0, st>>>(f, bp);
+            launch(overlap, kernel, dim3(ctas, n_views), kProjThreads, 0, st, f, bp);
         }
         VETR_CUDA(ctx, cudaGetLastError());
         return VETR_OK;
@@ -3428,7 +3479,7 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
     {
         PassScope t(ctx, VETR_T_BACKWARD, f.mode == VETR_MODE_FUZZY_BLEND ? 4 : 3);
         cudaStream_t st = ctx->stream;
-        pack_images_kernel<<<(unsigned)((f.Prm * n_views + 255) / 256), 256, 0, st>>>(f, bp);
+        launch(overlap, pack_images_kernel, (unsigned)((f.Prm * n_views + 255) / 256), 256, 0, st, f, bp);
         if (f.mode == VETR_MODE_FUZZY_BLEND)
         {
             const int grid = ctx->sm_count * ctx->fuzzy_ctas_per_sm;
@@ -3458,7 +3509,7 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         const size_t smem = (size_t)tiles * kProjThreads * sizeof(float4);
         const auto kernel = bilinear ? (g_intr ? point_backward_kernel<2, true> : g_pose ? point_backward_kernel<1, true> : point_backward_kernel<0, true>)
                                      : (g_intr ? point_backward_kernel<2, false> : g_pose ? point_backward_kernel<1, false> : point_backward_kernel<0, false>);
-        kernel<<<ctas, kProjThreads, smem, ctx->stream>>>(f, bp, tiles);
+        launch(overlap, kernel, ctas, kProjThreads, smem, ctx->stream, f, bp, tiles);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
@@ -3482,7 +3533,7 @@ extern "C" int vetr_finalize_gradients(vetr_ctx* ctx, int channels, int n_tex, c
     a.pose_end   = a.points_end + blocks(g_pose && g_pose_count, n_img);
     const unsigned grid = a.pose_end + blocks(g_intr && g_intr_count, n_cam);
     PassScope t(ctx, VETR_T_FINALIZE, grid > 0);
-    if (grid > 0) finalize_kernel<<<grid, 256, 0, st>>>(a);
+    if (grid > 0) launch((long long)n + n_tex <= kOverlapPoints, finalize_kernel, grid, 256, 0, st, a);
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }
@@ -3913,7 +3964,7 @@ static void gather_arrays(vetr_ctx* ctx, Kernel kernel, int n, int n_kept, const
     memset(&g, 0, sizeof(g));
     g.new_index = new_index, g.n = n, g.n_kept = n_kept;
     long long total   = 0;
-    const auto launch = [&]()
+    const auto flush = [&]()
     {
         if (g.arrays == 0) return;
         const int blocks = (int)(((long long)n + kGatherBlock - 1) / kGatherBlock);
@@ -3928,13 +3979,13 @@ static void gather_arrays(vetr_ctx* ctx, Kernel kernel, int n, int n_kept, const
         const long long units     = (long long)a.rows * units_of(a.width);
         if (units == 0) continue;
         // a launch when the table is full, and where one more array would leave the counter's range
-        if (g.arrays == kGatherArrays || total + units > (long long)std::numeric_limits<Total>::max()) launch();
+        if (g.arrays == kGatherArrays || total + units > (long long)std::numeric_limits<Total>::max()) flush();
         total += units;
         g.src[g.arrays] = (const uint32_t*)a.src, g.dst[g.arrays] = (uint32_t*)a.dst;
         g.end[g.arrays] = (Total)total, g.width[g.arrays] = a.width;
         ++g.arrays;
     }
-    launch();
+    flush();
 }
 
 extern "C" int vetr_gather_points(vetr_ctx* ctx, int n, int n_kept, const int32_t* new_index, const vetr_point_array* arrays, int n_arrays)
@@ -3977,7 +4028,7 @@ extern "C" int vetr_l1_loss_grad(vetr_ctx* ctx, int num_levels, const float* con
     VETR_CUDA(ctx, cudaSetDevice(ctx->device));
     VETR_CUDA(ctx, cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
     ctx->launches += 1;
-    l1_loss_grad_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(a);
+    launch(run <= kOverlapPoints, l1_loss_grad_kernel, ctx->sm_count * 8, 256, 0, ctx->stream, a);
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
 }
@@ -4057,7 +4108,7 @@ extern "C" int vetr_scan_counts_static(int device, void* cuda_stream, const int3
     // the status words are accumulated into (longest list is an atomic maximum): start them at zero
     if (cudaMemsetAsync(status, 0, 4 * sizeof(int), st) != cudaSuccess) return VETR_E_CUDA;
     if (cudaMemsetAsync(tile_sums + kStaticScanTiles, 0, sizeof(long long), st) != cudaSuccess) return VETR_E_CUDA;
-    launch_scan(counts, n_pixels, capacity, tile_sums, reinterpret_cast<unsigned*>(tile_sums + kStaticScanTiles), (int)n_tiles, ends, status, items, st);
+    launch_scan(counts, n_pixels, capacity, tile_sums, reinterpret_cast<unsigned*>(tile_sums + kStaticScanTiles), (int)n_tiles, ends, status, items, st, false);
     return cudaGetLastError() == cudaSuccess ? VETR_OK : VETR_E_CUDA;
 }
 
