@@ -56,6 +56,15 @@ __device__ __forceinline__ void begin_kernel()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// First statement of a kernel that has nothing to do with what the kernel before it does, only with what was there when that one started (it
+// was launched in the plain way, or is such a kernel itself): it starts on the SMs that the other one's blocks have left, and ends
+// after it, so that a kernel behind it may take the end of both for granted.
+struct BesidePrevious
+{
+    __device__ __forceinline__ BesidePrevious() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+    __device__ __forceinline__ ~BesidePrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+};
+
 #ifndef VETR_ITEM_THREADS
 #    define VETR_ITEM_THREADS 128
 #endif
@@ -1018,7 +1027,8 @@ __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const 
     }
 }
 
-// Lists longer than kLongList: one CTA per list.  Up to kLongSortMax fragments the keys are merge-sorted in shared memory
+// Lists longer than kLongList: one CTA per list, beside the end of sort_blend_kernel, whose CTAs take the same share of the items but not the same
+// time (the two together: 3 M points, one 1920x1080 view, 190 -> 171 us; mode 3, 3 M x 2 views, 1230 -> 1130).  Up to kLongSortMax fragments the keys are merge-sorted in shared memory
 // and the records follow, half a record at a time (the reference's <= 4096 bucket is a CTA-wide shared-memory sort as well,
 // AlphaListSort.cu:601-703); longer lists are sorted in global memory.  The fold runs in blocks of kFoldCap fragments.
 //
@@ -1125,7 +1135,7 @@ __device__ __forceinline__ float transmittance_chain(const float* alpha, float* 
 __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ OutPtrs out)
 {
-    begin_kernel();
+    const BesidePrevious beside;
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LongBlendSmem& s = *reinterpret_cast<LongBlendSmem*>(smem_raw);
@@ -1950,7 +1960,7 @@ __global__ void __launch_bounds__(kThreads, kBackCtas) backward_kernel(const __g
     reduce_background(f, bp, s, bg_acc, p0_acc);
 }
 
-// Lists longer than kLongList: one CTA per list, blocks of kCap fragments, a forward sweep that records the
+// Lists longer than kLongList, beside the end of backward_kernel: one CTA per list, blocks of kCap fragments, a forward sweep that records the
 // transmittance at every block start and a backward sweep over the blocks that carries the suffix sum.  One thread runs the
 // two chains of a list (transmittance: a multiplication per fragment; suffix sum: an addition); the division and the
 // products that hang on them are left to all threads.  Bound by those chains, hence as many lists in flight as fit an SM:
@@ -1960,7 +1970,7 @@ template <bool kBilinear>
 __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_constant__ Frame f,
                                                                  const __grid_constant__ BackPtrs bp)
 {
-    begin_kernel();
+    const BesidePrevious beside;
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BackSmemSuffix& s = *reinterpret_cast<BackSmemSuffix*>(smem_raw);
@@ -2079,7 +2089,7 @@ __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_co
 }
 
 // Mode 2, lists longer than kLongList: one CTA per list with the whole list staged (the group structure does not split
-// into blocks).  Lists beyond kFuzzyLongMax are skipped and flagged in the status word (the reference itself sorts only
+// into blocks), beside the end of backward_kernel (mode 2, 1 M points, 801x603: the whole call 431 -> 373 us).  Lists beyond kFuzzyLongMax are skipped and flagged in the status word (the reference itself sorts only
 // the first 4096 fragments of a list, AlphaListSort.cu:289-290, so its result for longer lists is not defined either).
 //
 // Launched twice: lists of up to kFuzzyMidMax fragments, eight of which fit an SM, and the longer ones, one per SM.  Two steps of a
@@ -2107,7 +2117,7 @@ template <int kMin, int kMax>
 __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ BackPtrs bp)
 {
-    begin_kernel();
+    const BesidePrevious beside;
     if (f.status[2] <= kMin) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FuzzyLongSmem<kMax>& s = *reinterpret_cast<FuzzyLongSmem<kMax>*>(smem_raw);
@@ -3405,7 +3415,7 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
         const int grid = ctx->sm_count * ctx->blend_ctas_per_sm;
         sort_blend_kernel<<<grid, kThreads, sizeof(BlendSmem), st>>>(f, out);
-        sort_blend_long_kernel<<<ctx->sm_count * ctx->blend_long_ctas_per_sm, kLongThreads, sizeof(LongBlendSmem), st>>>(f, out);
+        launch(true, sort_blend_long_kernel, ctx->sm_count * ctx->blend_long_ctas_per_sm, kLongThreads, sizeof(LongBlendSmem), st, f, out);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
@@ -3493,20 +3503,20 @@ extern "C" int vetr_backward_phase(vetr_ctx* ctx, const vetr_params* params, con
         {
             const int grid = ctx->sm_count * ctx->fuzzy_ctas_per_sm;
             backward_kernel<true, false><<<grid, kThreads, sizeof(BackSmemFuzzy), st>>>(f, bp);
-            backward_fuzzy_long_kernel<kLongList, kFuzzyMidMax><<<ctx->sm_count * ctx->fuzzy_mid_ctas_per_sm, kThreads, sizeof(FuzzyLongSmem<kFuzzyMidMax>), st>>>(f, bp);
-            backward_fuzzy_long_kernel<kFuzzyMidMax, kFuzzyLongMax><<<ctx->sm_count, kThreads, sizeof(FuzzyLongSmem<kFuzzyLongMax>), st>>>(f, bp);
+            launch(true, backward_fuzzy_long_kernel<kLongList, kFuzzyMidMax>, ctx->sm_count * ctx->fuzzy_mid_ctas_per_sm, kThreads, sizeof(FuzzyLongSmem<kFuzzyMidMax>), st, f, bp);
+            launch(true, backward_fuzzy_long_kernel<kFuzzyMidMax, kFuzzyLongMax>, ctx->sm_count, kThreads, sizeof(FuzzyLongSmem<kFuzzyLongMax>), st, f, bp);
         }
         else if (bilinear)
         {
             const int grid = ctx->sm_count * ctx->bilinear_ctas_per_sm;
             backward_kernel<false, true><<<grid, kThreads, sizeof(BackSmemSuffix), st>>>(f, bp);
-            backward_long_kernel<true><<<ctx->sm_count * ctx->bilinear_long_ctas_per_sm, kThreads, sizeof(BackSmemSuffix), st>>>(f, bp);
+            launch(true, backward_long_kernel<true>, ctx->sm_count * ctx->bilinear_long_ctas_per_sm, kThreads, sizeof(BackSmemSuffix), st, f, bp);
         }
         else
         {
             const int grid = ctx->sm_count * ctx->back_ctas_per_sm;
             backward_kernel<false, false><<<grid, kThreads, sizeof(BackSmem), st>>>(f, bp);
-            backward_long_kernel<false><<<ctx->sm_count * ctx->back_long_ctas_per_sm, kThreads, sizeof(BackSmemSuffix), st>>>(f, bp);
+            launch(true, backward_long_kernel<false>, ctx->sm_count * ctx->back_long_ctas_per_sm, kThreads, sizeof(BackSmemSuffix), st, f, bp);
         }
     }
     if ((phases & VETR_BACKWARD_POINTS) && point_pass && f.n > 0)
