@@ -170,6 +170,31 @@ def test_sizes_of_any_tensor(recorded, kind):
         host.l1_loss_grad(1, [np.zeros(4)], image, image, image[0])
 
 
+@pytest.mark.parametrize("kind", [lambda t: t, _Array, lambda t: t.as_subclass(_SubTensor), torch.nn.Parameter])
+@pytest.mark.parametrize("mode, w, h, layers, views", [(0, 40, 32, 4, 2), (1, 321, 200, 5, 8), (3, 5, 3, 2, 1), (1, 4, 4, 1, 3)])
+def test_scene(kind, mode, w, h, layers, views):
+    """Parameters, addresses, numbers of rows and the library's sizes in one call, whatever kind of tensor they come from."""
+    params = default_params(render_mode=mode, num_layers=layers)
+    position, index, texture, confidence = torch.zeros(33, 4), torch.zeros(33), torch.zeros(3, 35), torch.zeros(35)
+    background, poses, intrinsics = torch.zeros(3), torch.zeros(5, 8).double(), torch.zeros(2, 13)
+    tensors = (position, index, texture, confidence, background, poses, intrinsics)
+    s, want = L.Scene(), L.Params()
+    n, levels, pixels, capacity = L.host().scene(C.addressof(s), params, w, h, views, *[kind(t) for t in tensors])
+    L.host().params(C.addressof(want), params, 3)
+    assert bytes(s.params) == bytes(want) and s.params.num_channels == 3
+    assert (n, levels, pixels) == (33, layers, L.lib().vetr_pyramid_pixels(w, h, layers))
+    assert capacity == L.lib().vetr_list_capacity(33, views, w, h, C.byref(want))
+    assert (s.cloud.position, s.cloud.index, s.cloud.n) == (position.data_ptr(), index.data_ptr(), 33)
+    assert (s.texture.texture, s.texture.confidence, s.texture.background) == (texture.data_ptr(), confidence.data_ptr(), background.data_ptr())
+    assert s.texture.n_tex == 35 and (s.cameras.poses_se3, s.cameras.n_img) == (poses.data_ptr(), 5)
+    assert (s.cameras.intrinsics, s.cameras.n_cam) == (intrinsics.data_ptr(), 2)
+    assert L.host().scene(C.addressof(s), params, 0, h, views, *tensors)[2:] == (-1, -1)
+    with pytest.raises(KeyError):
+        L.host().scene(C.addressof(s), {}, w, h, views, *tensors)
+    with pytest.raises(TypeError):
+        L.host().scene(C.addressof(s), params, w, h, views, 1.0, *tensors[1:])
+
+
 def test_whole_numbers_are_cut_to_32_bits():
     params = default_params(debug_max_list_length=2**70 + 5, viewer_only=True)
     want, got = L.Params(**{k: params[k] for k, _ in L.Params._fields_}), L.Params()

@@ -49,6 +49,10 @@ class Cameras(C.Structure):
     _fields_ = [("poses_se3", C.c_void_p), ("intrinsics", C.c_void_p), ("n_img", C.c_int32), ("n_cam", C.c_int32)]
 
 
+class Scene(C.Structure):  # filled by the native host side in one call
+    _fields_ = [("params", Params), ("cloud", Cloud), ("texture", Texture), ("cameras", Cameras)]
+
+
 class Lists(C.Structure):
     _fields_ = [("counts", C.c_void_p), ("ends", C.c_void_p), ("frags", C.c_void_p), ("capacity", C.c_int64),
                 ("status", C.c_void_p), ("items", C.c_void_p), ("items_capacity", C.c_int64),
@@ -168,6 +172,8 @@ def host():
         from . import _host
 
         names = ("vetr_forward", "vetr_backward_phase", "vetr_finalize_gradients", "vetr_l1_loss_grad", "vetr_zero_buffers")
-        _host.bind(*[C.cast(getattr(lib(), n), C.c_void_p).value for n in names])
+        address = lambda n: C.cast(getattr(lib(), n), C.c_void_p).value  # noqa: E731
+        _host.bind(*[address(n) for n in names])
+        _host.bind_sizes(address("vetr_pyramid_pixels"), address("vetr_list_capacity"))
         _bound = _host
     return _bound

@@ -53,7 +53,7 @@ def build_host(force: bool = False) -> str:
     cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-D_GLIBCXX_USE_CXX11_ABI=" + str(int(torch._C._GLIBCXX_USE_CXX11_ABI))]
     for inc in ce.include_paths("cuda") + [sysconfig.get_paths()["include"]]:
         cmd += ["-isystem", inc]
-    cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+    cmd += HOST_SOURCES + ["-o", HOST_PATH, "-L" + torch_lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
                            "-Wl,-rpath," + torch_lib]
     # up to date: newer than its sources, made by this command with this torch and this interpreter
     made_by, made_by_path = "\n".join([torch.__version__, sys.version] + [c.replace(_HERE, ".") for c in cmd]), HOST_PATH + ".made_by"

@@ -5,9 +5,11 @@
 //
 // Why: a training batch of a small scene is bound by the host.  5 k points, two views 96x64, camera gradients: a pass takes
 // 173 to 181 us with these steps in Python (64 us of it on the device), 84 to 89 us like this; 100 k points at 512x512 158 to
-// 164 and 105 to 112 us (several GPUs; both times include a scan that became 3 us faster meanwhile).
+// 164 and 105 to 112 us (several GPUs; both times include a scan that became 3 us faster meanwhile).  The first again, 81 -> 73 us: parameters, addresses
+// and sizes of a call in one step (scene), and output tensors without the dispatcher's way to at::empty (17 of them, 0.9 us each before).
 #include <Python.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
 #include <torch/csrc/Exceptions.h>
@@ -26,6 +28,8 @@ decltype(&vetr_backward_phase) p_backward_phase         = nullptr;
 decltype(&vetr_finalize_gradients) p_finalize_gradients = nullptr;
 decltype(&vetr_l1_loss_grad) p_l1_loss_grad             = nullptr;
 decltype(&vetr_zero_buffers) p_zero_buffers             = nullptr;
+decltype(&vetr_pyramid_pixels) p_pyramid_pixels         = nullptr;
+decltype(&vetr_list_capacity) p_list_capacity           = nullptr;
 
 void require(bool ok, const char* what)
 {
@@ -91,13 +95,14 @@ long long numel(PyObject* o)
     if (const at::Tensor* t = plain_tensor(o)) return t->numel();
     return integer(held(PyObject_CallNoArgs(attribute(o, "numel").get())).get());
 }
-int rows(PyObject* o)  // of a tensor, or 0 for None
+int extent(PyObject* o, int dimension)  // of a tensor, or 0 for None
 {
     if (o == Py_None) return 0;
-    if (const at::Tensor* t = plain_tensor(o)) return (int)t->size(0);
+    if (const at::Tensor* t = plain_tensor(o)) return (int)t->size(dimension);
     THPObjectPtr shape = attribute(o, "shape");
-    return (int)integer(held(PySequence_GetItem(shape.get(), 0)).get());
+    return (int)integer(held(PySequence_GetItem(shape.get(), dimension)).get());
 }
+int rows(PyObject* o) { return extent(o, 0); }
 template <typename T>
 T* data(PyObject* o)  // a tensor, or None
 {
@@ -107,6 +112,12 @@ at::TensorOptions on(PyObject* device, at::ScalarType type = at::kFloat)
 {
     if (!THPDevice_Check(device)) throw torch::TypeError("expected a device");
     return at::TensorOptions().dtype(type).device(reinterpret_cast<THPDevice*>(device)->device);
+}
+// at::empty, without the dispatcher's way to it where the device is CUDA.
+at::Tensor fresh(at::IntArrayRef size, const at::TensorOptions& opt)
+{
+    if (!opt.device().is_cuda()) return at::empty(size, opt);
+    return at::Tensor(at::detail::empty_cuda(size, c10::typeMetaToScalarType(opt.dtype()), opt.device(), std::nullopt));
 }
 PyObject* wrap(at::Tensor t) { return held(THPVariable_Wrap(std::move(t))).release(); }
 
@@ -157,6 +168,15 @@ PyObject* bind(const Call& c)
     Py_RETURN_NONE;
 }
 
+// bind_sizes(pyramid_pixels, list_capacity): the same
+PyObject* bind_sizes(const Call& c)
+{
+    c.expect(2);
+    p_pyramid_pixels = reinterpret_cast<decltype(p_pyramid_pixels)>(integer(c[0]));
+    p_list_capacity  = reinterpret_cast<decltype(p_list_capacity)>(integer(c[1]));
+    Py_RETURN_NONE;
+}
+
 // current_stream(device index) -> address of torch's current stream on that device
 PyObject* current_stream(const Call& c)
 {
@@ -184,24 +204,22 @@ PyObject* images(const Call& c)
         }
         PyTuple_SET_ITEM(out.get(), kind, held(PyList_New(levels)).release());
         for (int64_t l = 0; l < levels; ++l)
-            PyList_SET_ITEM(PyTuple_GET_ITEM(out.get(), kind), l, wrap(at::empty({B, kind == 0 ? C : 1, h >> l, w >> l}, opt)));
+            PyList_SET_ITEM(PyTuple_GET_ITEM(out.get(), kind), l, wrap(fresh({B, kind == 0 ? C : 1, h >> l, w >> l}, opt)));
     }
     return out.release();
 }
 
-// params(address of vetr_params, dict, channels): every field from the dict's entry of that name, but the channel count
-PyObject* params(const Call& c)
+// Every field from the dict's entry of that name, but the channel count.
+void read_params(vetr_params& p, PyObject* dict, int32_t channels)
 {
-    c.expect(3);
-    vetr_params& p = *address<vetr_params>(c[0]);
     const auto get = [&](const char* name)
     {
         THPObjectPtr key = held(PyUnicode_InternFromString(name));
-        return held(PyObject_GetItem(c[1], key.get()));
+        return held(PyObject_GetItem(dict, key.get()));
     };
     const auto i = [&](const char* name) { return whole(get(name).get()); };
     const auto f = [&](const char* name) { return real(get(name).get()); };
-    p.render_mode = i("render_mode"), p.num_layers = i("num_layers"), i("num_channels"), p.num_channels = (int32_t)integer(c[2]);
+    p.render_mode = i("render_mode"), p.num_layers = i("num_layers"), i("num_channels"), p.num_channels = channels;
     p.drop_out_points_by_radius = i("drop_out_points_by_radius"), p.drop_out_radius_threshold = f("drop_out_radius_threshold");
     p.dist_cutoff = f("dist_cutoff"), p.use_environment_map = i("use_environment_map"), p.viewer_only = i("viewer_only");
     p.stability_cutoff_value = f("stability_cutoff_value"), p.debug_max_list_length = i("debug_max_list_length");
@@ -209,7 +227,40 @@ PyObject* params(const Call& c)
     p.distortion_gradient_factor = f("distortion_gradient_factor"), p.output_background_mask_value = f("output_background_mask_value");
     p.background_alpha_to_point0 = i("background_alpha_to_point0"), p.keep_sorted_lists = i("keep_sorted_lists");
     p.depth_accept_blend = f("depth_accept_blend"), p.depth_accept = f("depth_accept"), p.ghost_gradients = i("ghost_gradients");
+}
+
+// params(address of vetr_params, dict, channels)
+PyObject* params(const Call& c)
+{
+    c.expect(3);
+    read_params(*address<vetr_params>(c[0]), c[1], (int32_t)integer(c[2]));
     Py_RETURN_NONE;
+}
+
+struct Scene  // _lib.Scene
+{
+    vetr_params params;
+    vetr_cloud cloud;
+    vetr_texture texture;
+    vetr_cameras cameras;
+};
+
+// scene(address of Scene, dict of parameters, w, h, views, position, index, texture, confidence, background, poses, intrinsics) -> (points,
+// levels, pixels of a view, capacity of the lists of that many views); the last two -1 where the library refuses the sizes
+PyObject* scene(const Call& c)
+{
+    c.expect(12);
+    Scene& s = *address<Scene>(c[0]);
+    read_params(s.params, c[1], extent(c[7], 0));
+    const int w = (int)integer(c[2]), h = (int)integer(c[3]), views = (int)integer(c[4]);
+    s.cloud.position = static_cast<const float*>(storage(c[5])), s.cloud.index = static_cast<const int32_t*>(storage(c[6])), s.cloud.n = rows(c[5]);
+    s.texture.texture = static_cast<const float*>(storage(c[7])), s.texture.confidence = static_cast<const float*>(storage(c[8]));
+    s.texture.background = static_cast<const float*>(storage(c[9])), s.texture.n_tex = extent(c[7], 1);
+    s.cameras.poses_se3 = static_cast<const double*>(storage(c[10])), s.cameras.intrinsics = static_cast<const float*>(storage(c[11]));
+    s.cameras.n_img = rows(c[10]), s.cameras.n_cam = rows(c[11]);
+    const long long pixels = p_pyramid_pixels(w, h, s.params.num_layers);
+    const long long capacity = pixels > 0 ? p_list_capacity(s.cloud.n, views, w, h, &s.params) : -1;
+    return held(Py_BuildValue("iiLL", s.cloud.n, s.params.num_layers, pixels, capacity)).release();
 }
 
 // views(address of an array of vetr_view, sequence of vet_b200.scenes.View)
@@ -286,10 +337,10 @@ PyObject* gradients(const Call& c)
     const auto n_tex = integer(c[3]);
     std::vector<at::Tensor> t;
     t.reserve(8);
-    t.push_back(at::empty({n_tex, 4}, f32)), t.push_back(at::empty({n_tex}, f32)), t.push_back(at::empty({integer(c[4])}, f32));
-    if (c[2] != Py_None) t.push_back(at::empty({integer(c[2]), 4}, f32));
-    if (c[5] != Py_None) t.push_back(at::empty({integer(c[5]), 6}, on(c[1], at::kDouble))), t.push_back(at::empty({integer(c[5])}, f32));
-    if (c[6] != Py_None) t.push_back(at::empty({integer(c[6]), 13}, f32)), t.push_back(at::empty({integer(c[6])}, f32));
+    t.push_back(fresh({n_tex, 4}, f32)), t.push_back(fresh({n_tex}, f32)), t.push_back(fresh({integer(c[4])}, f32));
+    if (c[2] != Py_None) t.push_back(fresh({integer(c[2]), 4}, f32));
+    if (c[5] != Py_None) t.push_back(fresh({integer(c[5]), 6}, on(c[1], at::kDouble))), t.push_back(fresh({integer(c[5])}, f32));
+    if (c[6] != Py_None) t.push_back(fresh({integer(c[6]), 13}, f32)), t.push_back(fresh({integer(c[6])}, f32));
     void* p[8];
     int64_t bytes[8];
     for (size_t k = 0; k < t.size(); ++k) p[k] = t[k].data_ptr(), bytes[k] = (int64_t)t[k].nbytes();
@@ -329,7 +380,7 @@ PyObject* finalize(const Call& c)
     c.expect(9);
     vetr_ctx* ctx   = address<vetr_ctx>(c[0]);
     const int C     = (int)integer(c[2]), n_tex = rows(c[3]);
-    at::Tensor out  = at::empty({C, n_tex}, on(c[1]));
+    at::Tensor out  = fresh({C, n_tex}, on(c[1]));
     const int n = rows(c[4]), n_img = rows(c[5]), n_cam = rows(c[7]);
     const float* desc       = data<const float>(c[3]);
     float *texture          = static_cast<float*>(out.data_ptr()), *points = data<float>(c[4]), *intr = data<float>(c[7]);
@@ -366,7 +417,7 @@ PyObject* l1_loss_grad(const Call& c)
     {#name, (PyCFunction)(void*)(+[](PyObject*, PyObject* const* args, Py_ssize_t n) { return guarded(name, args, n); }), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {VETR_METHOD(bind),     VETR_METHOD(current_stream), VETR_METHOD(images),    VETR_METHOD(params),
                          VETR_METHOD(views),    VETR_METHOD(forward),        VETR_METHOD(gradients), VETR_METHOD(backward),
-                         VETR_METHOD(finalize), VETR_METHOD(l1_loss_grad),   {nullptr, nullptr, 0, nullptr}};
+                         VETR_METHOD(finalize), VETR_METHOD(l1_loss_grad),   VETR_METHOD(bind_sizes), VETR_METHOD(scene), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 }  // namespace
 

@@ -152,34 +152,38 @@ class Rasterizer:
     def forward(self, position, index, texture, confidence, background, poses, intrinsics, views, params: dict,
                 dropout=None, capacity: Optional[int] = None, want_weight=True, want_mask=False, want_depth=False):
         """Returns dict(color=[L x [B,C,h,w]], weight=..., mask=..., depth=...).  Keeps what backward() needs."""
-        lib, host = L.lib(), L.host()
+        host = L.host()
         self._sync_stream()
-        prm = L.Params()
-        host.params(C.addressof(prm), params, texture.shape[0])
-        B, Cn, Ln = len(views), texture.shape[0], prm.num_layers
-        w, h = views[0].w, views[0].h
-        sizes = level_sizes(w, h, Ln)
-        P = int(lib.vetr_pyramid_pixels(w, h, Ln))
+        B, w, h = len(views), views[0].w, views[0].h
+        s = L.Scene()
+        n, Ln, P, room = host.scene(C.addressof(s), params, w, h, min(B, L.MAX_VIEWS), position, index, texture, confidence, background, poses,
+                                    intrinsics)
         if P <= 0:
             raise L.VetrError(L.E_INVALID_ARG, "vetr_pyramid_pixels")
-        color, weight, mask, depth = host.images(self.device, B, Cn, w, h, Ln, want_weight, want_mask, want_depth)
-        cloud = L.Cloud(position.data_ptr(), index.data_ptr(), position.shape[0])
-        tex = L.Texture(texture.data_ptr(), confidence.data_ptr(), background.data_ptr(), texture.shape[1])
-        cams = L.Cameras(poses.data_ptr(), intrinsics.data_ptr(), poses.shape[0], intrinsics.shape[0])
-        groups = []
+        prm, cloud, tex, cams = s.params, s.cloud, s.texture, s.cameras
+        color, weight, mask, depth = host.images(self.device, B, prm.num_channels, w, h, Ln, want_weight, want_mask, want_depth)
+        masks = prm.render_mode == 3 or (prm.render_mode in (1, 2) and prm.need_point_gradient)
+        groups, frames = [], []
         for gi, b0 in enumerate(range(0, B, L.MAX_VIEWS)):
             b1 = min(B, b0 + L.MAX_VIEWS)
             nb = b1 - b0
-            cap = capacity if capacity is not None else int(lib.vetr_list_capacity(position.shape[0], nb, w, h, C.byref(prm)))
+            if capacity is not None:
+                cap = capacity
+            else:
+                cap = room if b0 == 0 else int(L.lib().vetr_list_capacity(n, nb, w, h, C.byref(prm)))
             lists = self._lists(gi, P * nb, cap, exact=capacity is not None)
-            if prm.render_mode == 3 or (prm.render_mode in (1, 2) and prm.need_point_gradient):
-                lists.ensure_level_mask(nb * position.shape[0])
-            varr = self._views(views[b0:b1])
-            rc = host.forward(self._address, C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams),
-                              C.addressof(varr), nb, b0, dropout, C.addressof(lists.c), Ln, color, weight, mask, depth)
-            self._check(rc, "vetr_forward")
+            if masks:
+                lists.ensure_level_mask(nb * n)
+            varr = self._views(views if nb == B else views[b0:b1])
+            # what vetr_forward and vetr_backward_phase are given in common
+            frame = (self._address, C.addressof(prm), C.addressof(cloud), C.addressof(tex), C.addressof(cams), C.addressof(varr), nb, b0, dropout,
+                     C.addressof(lists.c), Ln)
+            rc = host.forward(*frame, color, weight, mask, depth)
+            if rc:
+                self._check(rc, "vetr_forward")
             groups.append((b0, b1, lists, varr))
-        self._saved = dict(prm=prm, cloud=cloud, tex=tex, cams=cams, groups=groups, color=color, P=P, sizes=sizes,
+            frames.append(frame[1:])
+        self._saved = dict(prm=prm, cloud=cloud, tex=tex, cams=cams, groups=groups, frames=frames, color=color, P=P, sizes=level_sizes(w, h, Ln),
                            tensors=(position, index, texture, confidence, background, poses, intrinsics, dropout))
         return dict(color=color, weight=weight, mask=mask, depth=depth)
 
@@ -223,7 +227,7 @@ class Rasterizer:
         self._sync_stream()
         ctx = self._address
         position, index, texture = s["tensors"][0], s["tensors"][1], s["tensors"][2]
-        poses, intrinsics, dropout = s["tensors"][5], s["tensors"][6], s["tensors"][7]
+        poses, intrinsics = s["tensors"][5], s["tensors"][6]
         n, n_tex, Cn = position.shape[0], texture.shape[1], texture.shape[0]
         g = accum
         if g is None:
@@ -235,17 +239,16 @@ class Rasterizer:
                 self._check(bufs, "vetr_zero_buffers")
             g = dict(zip(names, bufs))
         grad_color = [x.contiguous() for x in grad_color]
-        for (b0, b1, lists, varr) in s["groups"]:
+        gradients = (g["desc"], g["conf"], g.get("points"), g["background"], g.get("pose"), g.get("pose_count"), g.get("intrinsics"),
+                     g.get("intrinsics_count"), phases | L.BACKWARD_PIXEL_SCRATCH if phases & L.BACKWARD_FRAGMENTS else phases)
+        for (b0, b1, lists, _), frame in zip(s["groups"], s["frames"]):
             lists.ensure_pixel_scratch()
             if lists.level_mask is not None:  # 2 floats per (view, level, point), 4 (one per bilinear corner) in mode 3
                 per = 4 if s["prm"].render_mode == 3 else 2
                 lists.ensure_point_grad((b1 - b0) * s["prm"].num_layers * n * per)
-            rc = host.backward(ctx, C.addressof(s["prm"]), C.addressof(s["cloud"]), C.addressof(s["tex"]), C.addressof(s["cams"]),
-                               C.addressof(varr), b1 - b0, b0, dropout, C.addressof(lists.c), s["prm"].num_layers, s["color"], grad_color,
-                               g["desc"], g["conf"], g.get("points"), g["background"], g.get("pose"), g.get("pose_count"),
-                               g.get("intrinsics"), g.get("intrinsics_count"),
-                               phases | L.BACKWARD_PIXEL_SCRATCH if phases & L.BACKWARD_FRAGMENTS else phases)
-            self._check(rc, "vetr_backward_phase")
+            rc = host.backward(ctx, *frame, s["color"], grad_color, *gradients)
+            if rc:
+                self._check(rc, "vetr_backward_phase")
         return g
 
     def finalize(self, g: dict):
