@@ -184,6 +184,9 @@ __device__ __forceinline__ void store_record(const Frame& f, int slot, unsigned 
 }
 __device__ __forceinline__ void load_record(const Frame& f, int slot, uint4& h, uint4& d) { load_sector(f.recs + 2 * (size_t)slot, h, d); }
 __device__ __forceinline__ unsigned long long record_key(uint4 h) { return ((unsigned long long)h.y << 32) | h.x; }
+// A key as a positive fp64 number, which orders as the key does (depths are finite, so none is a NaN): one comparison instead of two.
+// Ranking with 8 M points x 4 views: sort_blend_kernel 918 -> 901 us; mode 3, 3 M x 2 views 1023 -> 995.
+__device__ __forceinline__ double ordered(unsigned long long key) { return __longlong_as_double((long long)key); }
 __device__ __forceinline__ float4 as_float4(uint4 v)
 {
     return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
@@ -977,7 +980,7 @@ __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const 
             const int ss = s.seg_end[a], se = s.seg_end[a + 1];
             const unsigned long long key = s.key[i];
             int rank = 0;
-            for (int k = ss; k < se; ++k) rank += s.key[k] < key;
+            for (int k = ss; k < se; ++k) rank += ordered(s.key[k]) < ordered(key);
             s.perm[ss + rank] = (unsigned short)i;
             // the sorted lists go back for the backward pass (all of the item's records are in shared memory by now)
             if (f.keep_sorted) store_record(f, f0 + ss + rank, key, s.alpha[i], s.tex[i], s.desc[i]);
@@ -1070,7 +1073,7 @@ __device__ void sort_long_list_shared(const Frame& f, LongBlendSmem& ls, int fir
         const int r0 = i & ~31, m = min(32, n - r0);
         const unsigned long long key = ls.key[0][i];
         int rank = 0;
-        for (int k = 0; k < m; ++k) rank += ls.key[0][r0 + k] < key;
+        for (int k = 0; k < m; ++k) rank += ordered(ls.key[0][r0 + k]) < ordered(key);
         ls.key[1][r0 + rank] = key;
         ls.idx[1][r0 + rank] = (unsigned short)i;
     }
