@@ -125,7 +125,8 @@ typedef struct vetr_lists
     int32_t*  status;   /* [4] device words: {total fragments F, overflow flag, longest list, number of work items} */
     int32_t*  items;    /* [items_capacity] work-item table written by the scan: first pixel of every run of pixels that
                            one thread block of the blend / backward kernels processes (balanced by fragments) */
-    int64_t   items_capacity; /* >= vetr_item_table_entries(capacity, n_views*P) */
+    int64_t   items_capacity; /* >= vetr_item_table_entries(capacity, n_views*P), whose last entry is never a pixel's: the
+                                 forward pass counts the items there that it has handed out */
     uint8_t*  level_mask;  /* [n_views*n] written by vetr_forward when not NULL: bit l set = the point has a fragment on
                               pyramid level l of that view */
     float*    point_grad;  /* 16-byte aligned scratch of vetr_backward, indexed by (view, level, point): modes 1 and 2

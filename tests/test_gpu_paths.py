@@ -6,7 +6,7 @@ import pytest
 from oracle import oracle as O
 from tests import util
 from vet_b200 import scenes
-from vet_b200.render import default_params, level_sizes
+from vet_b200.render import default_params, level_sizes, scene_to_device
 
 pytestmark = pytest.mark.gpu
 
@@ -587,3 +587,33 @@ def test_steps_follow_one_another(rasterizer, mode):
     for a, b in zip(steps(torch.cuda.synchronize), steps(lambda: None)):
         for x, y in zip(a, b):  # the order of fp32 sums is not fixed
             assert torch.allclose(x, y, rtol=1e-4, atol=1e-5 * float(x.abs().max()))
+
+
+# ---- items of sort + blend from a counter, long lists first
+
+
+@pytest.mark.parametrize("mode, n", [(1, 270_000), (2, 270_000), (3, 70_000)])
+def test_large_batches_are_their_halves(rasterizer, mode, n):
+    """Eight views of a cloud that reach the number of fragments from which on long lists go first and items come from a counter, against the same
+    views four at a time, below it: the same lists in the same order, the same images bit for bit."""
+    import torch
+
+    sc = scenes.config_planar(n, 160, 96, 100.0, n_views=8, seed=6)
+    tensors = scene_to_device(sc, rasterizer.device)
+    params = default_params(render_mode=mode, num_layers=3, drop_out_points_by_radius=0)
+    whole = rasterizer.forward(*tensors, sc.views, params)
+    fragments, longest = rasterizer.fragment_count()
+    assert longest > 256  # some are left to the kernel for long lists
+    lists = [rasterizer.lists_of(view, level) for view in range(8) for level in range(3)]
+    seen = 0
+    for first in (0, 4):
+        half = rasterizer.forward(*tensors, sc.views[first:first + 4], params)
+        seen += rasterizer.fragment_count()[0]
+        for key in ("color", "weight"):
+            for a, b in zip(whole[key], half[key]):
+                assert torch.equal(a[first:first + 4], b)
+        for view in range(4):
+            for level in range(3):
+                for a, b in zip(lists[3 * (first + view) + level], rasterizer.lists_of(view, level)):
+                    assert torch.equal(a, b)
+    assert seen == fragments

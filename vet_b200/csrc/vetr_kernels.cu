@@ -64,6 +64,10 @@ struct BesidePrevious
     __device__ __forceinline__ BesidePrevious() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
     __device__ __forceinline__ ~BesidePrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 };
+struct BeginKernel
+{
+    __device__ __forceinline__ BeginKernel() { begin_kernel(); }
+};
 
 #ifndef VETR_ITEM_THREADS
 #    define VETR_ITEM_THREADS 128
@@ -138,6 +142,7 @@ struct Frame  // kernel parameter block (travels by value; no global or __consta
     long long capacity;
     int* status;      // {F, overflow, longest, number of work items}
     int* item_start;  // [n_items + 1]
+    int* next_item;   // counts the items handed out; the last entry of the caller's table, which is never one of the above
     unsigned char* level_mask;  // [n_views * n]: levels of the view on which the point has a fragment (written by collect)
     float2* point_grad;         // [(view * L + level) * n + point]: image-space gradient of that fragment (backward scratch)
     float4* img4;               // [PT] forward image, channels interleaved, indexed like counts[] (backward scratch)
@@ -482,7 +487,7 @@ __device__ __forceinline__ bool last_block(unsigned* ticket)
 }
 
 // One block: exclusive scan of the tile sums in place; writes F, the overflow flag and the number of work items.
-__device__ void scan_spine(long long* tile_sums, int n_tiles, long long n_pixels, long long capacity, int* status, int* item_start)
+__device__ void scan_spine(long long* tile_sums, int n_tiles, long long n_pixels, long long capacity, int* status, int* item_start, int* next_item)
 {
     constexpr int kEach = 8;  // consecutive tiles per thread
     __shared__ long long s_warp[8];
@@ -530,13 +535,14 @@ __device__ void scan_spine(long long* tile_sums, int n_tiles, long long n_pixels
         const int items      = overflow ? 0 : (int)((work + kQuantum - 1) / kQuantum);
         status[3]            = items;
         item_start[items]    = (int)n_pixels;  // sentinel
+        *next_item           = 0;
     }
 }
 
 // Sums of the tiles; the last block to finish scans them (a launch of its own for that cost a small scene as much as the tiles).
 template <bool kVec>
 __global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restrict__ counts, long long n, long long* tile_sums, int* status,
-                                                             long long capacity, int* item_start, unsigned* ticket)
+                                                             long long capacity, int* item_start, int* next_item, unsigned* ticket)
 {
     begin_kernel();
     __shared__ long long s_sum[8];
@@ -564,7 +570,7 @@ __global__ void __launch_bounds__(256) scan_tile_sums_kernel(const int* __restri
         tile_sums[blockIdx.x] = sum;
         if (mx > 0) atomicMax(status + 2, mx);
     }
-    if (last_block(ticket)) scan_spine(tile_sums, (int)gridDim.x, n, capacity, status, item_start);
+    if (last_block(ticket)) scan_spine(tile_sums, (int)gridDim.x, n, capacity, status, item_start, next_item);
 }
 
 // Writes the exclusive offsets and cuts the pixel space into work items: with work(p) = end(p) + kPixelWork*(p+1)
@@ -781,6 +787,52 @@ struct ItemStream
     }
 };
 
+// The same for items from a counter behind every CTA's first three: thread 0 asks for an item before the one in front of it is looked up in the
+// table.  A CTA that has come late, or has items of much work, takes fewer.
+struct ItemQueue
+{
+    struct Smem
+    {
+        int id[2];  // item whose table entry is read next; in turn, because nobody waits for those who read it
+    };
+    Smem& s;
+    int item, n_items, turn;          // item: in thread 0, the next but one
+    int next_lo, next_hi;             // range of the item after the one whose ends are in flight; behind the last item 0, -1
+    int lo, hi, before, first, last;  // item in flight: pixels [lo, hi), list ends of lo - 1, lo and hi - 1
+    __device__ __forceinline__ void range(const Frame& f, int i)
+    {
+        next_lo = 0, next_hi = -1;
+        if (i < n_items) next_lo = f.item_start[i], next_hi = f.item_start[i + 1];
+    }
+    __device__ __forceinline__ void ends(const Frame& f)
+    {
+        lo = next_lo, hi = next_hi;
+        before = first = last = 0;
+        if (lo < hi) before = list_end(f, lo - 1), first = f.ends[lo], last = f.ends[hi - 1];
+    }
+    __device__ __forceinline__ ItemQueue(const Frame& f, Smem& smem) : s(smem), item(blockIdx.x + 2 * (int)gridDim.x), n_items(f.status[3]), turn(0)
+    {
+        range(f, blockIdx.x);
+        ends(f);
+        range(f, blockIdx.x + gridDim.x);
+    }
+    // As ItemStream's, but all threads call it together, and every warp has left the previous item when it returns.
+    __device__ __forceinline__ bool next(const Frame& f, int& p0, int& np, int& f0, int& nf)
+    {
+        if (threadIdx.x == 0) s.id[turn] = item;
+        __syncthreads();
+        if (hi < 0) return false;
+        const int skip = lo < hi && first - before > kLongList ? 1 : 0;
+        p0 = lo + skip, np = hi - p0;
+        f0 = skip ? first : before, nf = last - f0;
+        ends(f);
+        range(f, s.id[turn]);
+        turn ^= 1;
+        if (threadIdx.x == 0) item = atomicAdd(f.next_item, 1) + 3 * (int)gridDim.x;
+        return true;
+    }
+};
+
 // Work items whose first pixel holds a long list, for the kernels that take one such list per CTA.  Testing an item costs
 // four dependent loads (two table entries, two list ends), and only a few items in a thousand qualify, so the threads of
 // a CTA test one item each and the CTA then works through the hits: next() is called by all threads and returns the same
@@ -932,10 +984,14 @@ struct BlendSmem
 // of 3 M points forward only 44, 47, 13, 12 of 182.  Records go back from the slot that they arrived in, by the thread that has just ranked
 // them, which reads shared memory without conflicts and spares a phase, and the fold asks for its operands one fragment ahead (slot, then
 // contents: two dependent reads): 1017 -> 916 us, 183 -> 166; mode 3, 3 M points x 2 views 1083 -> 989.
+//
+// kQueue: beside sort_blend_long_kernel, which has started before it, with the items from a counter, because blocks come to run as those of the other
+// kernel leave room (see kQueueFragments).
+template <bool kQueue>
 __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const __grid_constant__ Frame f,
                                                                           const __grid_constant__ OutPtrs out)
 {
-    begin_kernel();
+    const std::conditional_t<kQueue, BesidePrevious, BeginKernel> begin;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlendSmem& s = *reinterpret_cast<BlendSmem*>(smem_raw);
     const int tid     = threadIdx.x;
@@ -944,12 +1000,19 @@ __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const 
     if (tid == 0) s.seg.n_long[0] = s.seg.n_long[1] = 0;
     int parity = 0;
 
-    ItemStream items(f);
+    __shared__ ItemQueue::Smem s_items;
+    auto items = [&]
+    {
+        if constexpr (kQueue)
+            return ItemQueue(f, s_items);
+        else
+            return ItemStream(f);
+    }();
     int lo, np, f0, nf;
     while (items.next(f, lo, np, f0, nf))
     {
         if (np <= 0) continue;
-        __syncthreads();  // every warp has left the previous item
+        if (!kQueue) __syncthreads();  // every warp has left the previous item
         parity ^= 1;
         if (tid == 0) s.seg.n_long[parity ^ 1] = 0;
         // the thread's first record is requested before the per-pixel set-up, each further one before the previous is stored
@@ -1135,10 +1198,11 @@ __device__ __forceinline__ float transmittance_chain(const float* alpha, float* 
     return T;
 }
 
+template <bool kFirst>  // started before sort_blend_kernel, or beside its end
 __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ OutPtrs out)
 {
-    const BesidePrevious beside;
+    const std::conditional_t<kFirst, BeginKernel, BesidePrevious> begin;
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LongBlendSmem& s = *reinterpret_cast<LongBlendSmem*>(smem_raw);
@@ -3179,8 +3243,10 @@ extern "C" int vetr_create(vetr_ctx** out, int device, void* cuda_stream)
         if (e == cudaSuccess && ctas_per_sm) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, kernel, threads, smem);
         if (ctas_per_sm && *ctas_per_sm < 1) *ctas_per_sm = 1;
     };
-    prepare(sort_blend_kernel, kThreads, sizeof(BlendSmem), &ctx->blend_ctas_per_sm);
-    prepare(sort_blend_long_kernel, kLongThreads, sizeof(LongBlendSmem), &ctx->blend_long_ctas_per_sm);
+    prepare(sort_blend_kernel<false>, kThreads, sizeof(BlendSmem), &ctx->blend_ctas_per_sm);
+    prepare(sort_blend_kernel<true>, kThreads, sizeof(BlendSmem), nullptr);
+    prepare(sort_blend_long_kernel<false>, kLongThreads, sizeof(LongBlendSmem), &ctx->blend_long_ctas_per_sm);
+    prepare(sort_blend_long_kernel<true>, kLongThreads, sizeof(LongBlendSmem), nullptr);
     prepare(backward_kernel<false, false>, kThreads, sizeof(BackSmem), &ctx->back_ctas_per_sm);
     prepare(backward_kernel<false, true>, kThreads, sizeof(BackSmemSuffix), &ctx->bilinear_ctas_per_sm);
     prepare(backward_kernel<true, false>, kThreads, sizeof(BackSmemFuzzy), &ctx->fuzzy_ctas_per_sm);
@@ -3300,6 +3366,7 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
     int rc = ensure_scratch(ctx, n_tiles);
     if (rc != VETR_OK) return rc;
     f.item_start = lists->items;
+    f.next_item  = lists->items + (lists->items_capacity - 1);
     f.level_mask = lists->level_mask;
     f.point_grad = (float2*)lists->point_grad;
     f.img4       = (float4*)lists->pixel_scratch;
@@ -3310,10 +3377,10 @@ static int fill_frame(vetr_ctx* ctx, Frame& f, const vetr_params* p, const vetr_
 // The two kernels of the scan.  *ticket and status[0..3] are zero on the stream before it (a ticket that is not would have the sums of
 // the tiles scanned too early).
 static void launch_scan(const int* counts, long long n, long long capacity, long long* tile_sums, unsigned* ticket, int n_tiles, int* ends,
-                        int* status, int* items, cudaStream_t st, bool overlap)
+                        int* status, int* items, int* next_item, cudaStream_t st, bool overlap)
 {
     const bool vec = (((uintptr_t)counts | (uintptr_t)ends) & 15) == 0;
-    launch(overlap, vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>, n_tiles, 256, 0, st, counts, n, tile_sums, status, capacity, items, ticket);
+    launch(overlap, vec ? scan_tile_sums_kernel<true> : scan_tile_sums_kernel<false>, n_tiles, 256, 0, st, counts, n, tile_sums, status, capacity, items, next_item, ticket);
     launch(overlap, vec ? scan_apply_kernel<true> : scan_apply_kernel<false>, n_tiles, 256, 0, st, counts, n, tile_sums, ends, status, items);
 }
 
@@ -3347,6 +3414,11 @@ extern "C" int vetr_zero_buffers(vetr_ctx* ctx, void* const* buffers, const int6
     return zero_buffers(ctx, buffers, bytes, n);
 }
 
+// Fragments per level, at most, from which on the long lists go first, with sort_blend_kernel beside them from the start and its items handed out by a
+// counter.  3 M points forward only 297 -> 292 us, 8 M points and four views 3855 -> 3806, 20 M and eight 17410 -> 17290, mode 3 with 1 M
+// points 394 -> 381 and with 3 M and two views 2933 -> 2840; below it the late blocks and the counter cost more: 99 k points in mode 1 46 -> 47,
+// 39 k in mode 3 58 -> 72, 114 k 122 -> 131, mode 2 with 1 M points the same.
+constexpr long long kQueueFragments = 1 << 21;
 extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr_cloud* cloud, const vetr_texture* texture,
                             const vetr_cameras* cameras, const vetr_view* views, int n_views, const float* dropout,
                             const vetr_lists* lists, float* const* out_color, float* const* out_weight,
@@ -3406,7 +3478,7 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     const int n_tiles = (int)((f.PT + kScanTile - 1) / kScanTile);
     {
         PassScope t(ctx, VETR_T_SCAN, 2);
-        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, st, overlap);
+        launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, f.next_item, st, overlap);
     }
     if (point_ctas > 0)
     {
@@ -3417,8 +3489,17 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     {
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
         const int grid = ctx->sm_count * ctx->blend_ctas_per_sm;
-        sort_blend_kernel<<<grid, kThreads, sizeof(BlendSmem), st>>>(f, out);
-        launch(true, sort_blend_long_kernel, ctx->sm_count * ctx->blend_long_ctas_per_sm, kLongThreads, sizeof(LongBlendSmem), st, f, out);
+        const int long_grid = ctx->sm_count * ctx->blend_long_ctas_per_sm;
+        if ((long long)f.n * n_views * (f.mode == VETR_MODE_BILINEAR_BLEND ? 4 : 1) >= kQueueFragments)
+        {
+            sort_blend_long_kernel<true><<<long_grid, kLongThreads, sizeof(LongBlendSmem), st>>>(f, out);
+            launch(true, sort_blend_kernel<true>, grid, kThreads, sizeof(BlendSmem), st, f, out);
+        }
+        else
+        {
+            sort_blend_kernel<false><<<grid, kThreads, sizeof(BlendSmem), st>>>(f, out);
+            launch(true, sort_blend_long_kernel<false>, long_grid, kLongThreads, sizeof(LongBlendSmem), st, f, out);
+        }
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
@@ -4130,7 +4211,7 @@ extern "C" int vetr_scan_counts_static(int device, void* cuda_stream, const int3
     // the status words are accumulated into (longest list is an atomic maximum): start them at zero
     if (cudaMemsetAsync(status, 0, 4 * sizeof(int), st) != cudaSuccess) return VETR_E_CUDA;
     if (cudaMemsetAsync(tile_sums + kStaticScanTiles, 0, sizeof(long long), st) != cudaSuccess) return VETR_E_CUDA;
-    launch_scan(counts, n_pixels, capacity, tile_sums, reinterpret_cast<unsigned*>(tile_sums + kStaticScanTiles), (int)n_tiles, ends, status, items, st, false);
+    launch_scan(counts, n_pixels, capacity, tile_sums, reinterpret_cast<unsigned*>(tile_sums + kStaticScanTiles), (int)n_tiles, ends, status, items, items + (items_capacity - 1), st, false);
     return cudaGetLastError() == cudaSuccess ? VETR_OK : VETR_E_CUDA;
 }
 
