@@ -617,3 +617,9 @@ def test_large_batches_are_their_halves(rasterizer, mode, n):
                 for a, b in zip(lists[3 * (first + view) + level], rasterizer.lists_of(view, level)):
                     assert torch.equal(a, b)
     assert seen == fragments
+
+
+@pytest.mark.parametrize("mode, n", [(1, 1_048_577), (3, 262_145)])
+def test_points_per_thread_same_lists(rasterizer, mode, n):
+    """Eight views at which a thread counts and collects several points, against four at a time at which it takes one."""
+    test_large_batches_are_their_halves(rasterizer, mode, n)

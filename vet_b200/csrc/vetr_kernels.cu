@@ -96,11 +96,6 @@ constexpr int kCap        = kQuantum + kLongList;   // fragments staged per item
 constexpr int kBlendCtas  = VETR_BLEND_CTAS;        // resident CTAs per SM the item kernels are compiled for; 8 is also what
 constexpr int kBackCtas   = VETR_BACK_CTAS;         // fits the shared memory of sort_blend_kernel
 constexpr int kProjThreads     = 256;
-#ifndef VETR_COLLECT_POINTS
-#    define VETR_COLLECT_POINTS 2
-#endif
-constexpr int kPointsPerThread = 4;                      // count pass
-constexpr int kCollectPoints   = VETR_COLLECT_POINTS;    // collection pass (its slots and payload live in registers)
 static_assert(kQuantum % kPixelWork == 0, "an item of kQuantum work units holds at most kQuantum / kPixelWork pixels");
 static_assert(kMaxPixels <= kThreads, "one thread per pixel of an item");
 static_assert(kMaxPixels <= 256, "seg_of is a byte");
@@ -228,7 +223,7 @@ __device__ __forceinline__ Camera load_camera(const Frame& f, int b)
 // ---------------------------------------------------------------------------------------------------------
 // Pass 1 and 3: projection + counting / collection.  kPts points per thread.  Modes 1 and 2 run in three sweeps over
 // the thread's points so that independent memory operations are in flight together: (1) project and find the pixel of
-// every (point, level), (2) issue ALL count reductions / slot reservations, (3) load the payload and store the records.
+// every (point, level), (2) load the payload and issue ALL count reductions / slot reservations, (3) store the records.
 // (The slot reservation is an atomic with a return value: with one in flight per thread the kernel waits on it.)
 
 __device__ __forceinline__ bool point_is_live(const Frame& f, int b, int pid)
@@ -238,13 +233,36 @@ __device__ __forceinline__ bool point_is_live(const Frame& f, int b, int pid)
     return true;
 }
 
-// The collection waits for its atomics (55 % of the issue slots), so it wants warps: blocks of 128 threads, twelve per SM (40
-// registers).  8 M points x 4 views: 648 us (656 with the positions requested behind the camera); six, seven or eight blocks of
-// 256: 671, 664, 664, fourteen of 128: 659, twenty-four of 64: 653, five of 256: 725.  The count pass is bound by instruction
-// issue (89 %) and stays at 256 threads: 320 us, six blocks 319, twelve of 128 341.
-constexpr int kCollectThreads = 128, kCollectCtas = 12;
-template <bool kCollect, int kPts>
-__global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCollect ? kCollectCtas : 5) project_kernel(const __grid_constant__ Frame f)
+// Few points: one point per thread, because a pass that does not fill the chip lasts as long as one thread's chain of points.  Many:
+// several, which share the block's camera and keep more memory operations in flight per warp.  Mode 3 has kernels of its own; its
+// loop over levels and corners shared the registers of modes 1 and 2 (and theirs its).  us, modes 1 and 2 / mode 3, on a planar
+// cloud and (in brackets) a cube's surface at 1920 x 1080:
+//                        several per thread             one per thread
+//   count    100 k       7.3 (7.5)  / 10.8 (11.5)       4.4 (4.8)  /  8.4 (10.3)
+//            2 M         26.6 (26.4) / 63.5 (51.1)      26.9 (26.1) / 57.7 (42.9)
+//            2 M x 4     89.4 (87.3) / 222 (184)        96.0 (93.3)
+//   collect  100 k       15.4 (18.4) / 45.5 (50.8)      10.8 (12.5) / 25.0 (30.4)
+//            1 M x 4     133 (91)   / 512 (283)         133 (89)   / 508 (291)
+//            2 M x 4     247 (158)  / 914 (417)         250 (147)  / 919 (448)
+//            4 M x 4     448 (232)  / 1534 (550)        452 (252)  / 1545 (631)
+// The collection waits for its atomics (55 % of the issue slots), so it wants warps, blocks of 128 threads, and the payload asked
+// for ahead of the atomics instead of after them.  8 M points x 4 views, modes 1 and 2, two points per thread: twelve blocks per SM
+// (40 registers) 614 us, ten 621, nine 621; the payload after the slots 647 (eight to fourteen blocks, or blocks of 64 and 256:
+// 653 to 725).  One point per thread at 1 M points: sixteen blocks (32 registers) 80 us, thirteen 83, seven of 256 threads 85,
+// two points 85.
+// The count pass is bound by instruction issue (89 %) and stays at 256 threads: 320 us, six blocks 319, twelve of 128 341.  Mode 3
+// counts two points per thread with six blocks: 4 M x 4 of the cube 232 us, four points 268, with four blocks 287.
+constexpr int kCollectThreads = 128;
+constexpr long long kCollectPairs = 1 << 23;          // points times views from which on a thread collects two points, modes 1, 2
+constexpr long long kCollectPairsBilinear = 1 << 21;  // and mode 3
+constexpr long long kCountSeveral = 1 << 21;          // and from which on it counts several
+constexpr int count_points(bool bilinear) { return bilinear ? 2 : 4; }
+constexpr int project_ctas(bool collect, int points, bool bilinear)
+{
+    return collect ? (points > 1 ? 12 : bilinear ? 10 : 16) : bilinear ? 6 : 5;
+}
+template <bool kCollect, int kPts, bool kBilinear>
+__global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, project_ctas(kCollect, kPts, kBilinear)) project_kernel(const __grid_constant__ Frame f)
 {
     begin_kernel();
     constexpr int kThreadsHere = kCollect ? kCollectThreads : kProjThreads;
@@ -259,13 +277,16 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCo
         const int pid = first + it * kThreadsHere;
         pos[it]       = pid < f.n ? __ldg(f.position + pid) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    int tex[kPts];
+    if (kCollect)
+#pragma unroll
+        for (int it = 0; it < kPts; ++it) tex[it] = first + it * kThreadsHere < f.n ? __ldg(f.index + first + it * kThreadsHere) : 0;
     if (threadIdx.x == 0) s_cam = load_camera(f, b);
     __syncthreads();
     const Camera& cam   = s_cam;
     const int vbase     = b * (int)f.P;
-    const bool bilinear = f.mode == VETR_MODE_BILINEAR_BLEND;
 
-    if (!bilinear)
+    if constexpr (!kBilinear)
     {
         int g[kPts][VETR_MAX_LAYERS];  // pixel of (point, level) in the global pixel space, then its record slot; -1 = none
         unsigned zbits[kPts];
@@ -307,13 +328,28 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCo
         }
         else
         {
-#pragma unroll
-            for (int it = 0; it < kPts; ++it)
-#pragma unroll
-                for (int l = 0; l < VETR_MAX_LAYERS; ++l)
-                    if (g[it][l] >= 0) g[it][l] = atomicAdd(f.ends + g[it][l], 1);
         // what the blend needs of the point travels next to every key (coalesced loads here, one per point, instead of
-        // a dependent gather per fragment later)
+        // a dependent gather per fragment later); asked for ahead of the slots, so that the two waits overlap
+        float conf[kPts];
+        float4 desc[kPts];
+#pragma unroll
+        for (int it = 0; it < kPts; ++it)
+        {
+            bool any = false;
+#pragma unroll
+            for (int l = 0; l < VETR_MAX_LAYERS; ++l) any |= g[it][l] >= 0;
+            if (!any) continue;
+            conf[it]   = __ldg(f.confidence + tex[it]);
+            desc[it].x = __ldg(f.texture + tex[it]);
+            desc[it].y = __ldg(f.texture + (size_t)f.n_tex + tex[it]);
+            desc[it].z = __ldg(f.texture + 2 * (size_t)f.n_tex + tex[it]);
+            desc[it].w = f.C > 3 ? __ldg(f.texture + 3 * (size_t)f.n_tex + tex[it]) : 0.f;
+        }
+#pragma unroll
+        for (int it = 0; it < kPts; ++it)
+#pragma unroll
+            for (int l = 0; l < VETR_MAX_LAYERS; ++l)
+                if (g[it][l] >= 0) g[it][l] = atomicAdd(f.ends + g[it][l], 1);
 #pragma unroll
         for (int it = 0; it < kPts; ++it)
         {
@@ -324,17 +360,10 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCo
             for (int l = 0; l < VETR_MAX_LAYERS; ++l) bits |= g[it][l] >= 0 ? 1u << l : 0u;
             if (f.level_mask) f.level_mask[(size_t)b * f.n + pid] = (unsigned char)bits;
             if (!bits) continue;
-            const int tex   = __ldg(f.index + pid);
-            const float conf = __ldg(f.confidence + tex);
-            float4 desc;
-            desc.x = __ldg(f.texture + tex);
-            desc.y = __ldg(f.texture + (size_t)f.n_tex + tex);
-            desc.z = __ldg(f.texture + 2 * (size_t)f.n_tex + tex);
-            desc.w = f.C > 3 ? __ldg(f.texture + 3 * (size_t)f.n_tex + tex) : 0.f;
             const unsigned long long key = ((unsigned long long)zbits[it] << 32) | (unsigned)pid;
 #pragma unroll
             for (int l = 0; l < VETR_MAX_LAYERS; ++l)
-                if (g[it][l] >= 0 && (long long)g[it][l] < f.capacity) store_record(f, g[it][l], key, conf, tex, desc);
+                if (g[it][l] >= 0 && (long long)g[it][l] < f.capacity) store_record(f, g[it][l], key, conf[it], tex[it], desc[it]);
         }
         }
         return;
@@ -359,17 +388,15 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCo
         float2 ip     = pr.ip;
         float radius  = pr.radius_px;
         const unsigned long long key = ((unsigned long long)__float_as_uint(pr.z) << 32) | (unsigned)pid;
-        int tex      = 0;
         float conf   = 0.f;
         float4 desc  = make_float4(0.f, 0.f, 0.f, 0.f);
         if (kCollect && !(f.drop_by_radius && radius < f.radius_threshold))
         {
-            tex    = __ldg(f.index + pid);
-            conf   = __ldg(f.confidence + tex);
-            desc.x = __ldg(f.texture + tex);
-            desc.y = __ldg(f.texture + (size_t)f.n_tex + tex);
-            desc.z = __ldg(f.texture + 2 * (size_t)f.n_tex + tex);
-            desc.w = f.C > 3 ? __ldg(f.texture + 3 * (size_t)f.n_tex + tex) : 0.f;
+            conf   = __ldg(f.confidence + tex[it]);
+            desc.x = __ldg(f.texture + tex[it]);
+            desc.y = __ldg(f.texture + (size_t)f.n_tex + tex[it]);
+            desc.z = __ldg(f.texture + 2 * (size_t)f.n_tex + tex[it]);
+            desc.w = f.C > 3 ? __ldg(f.texture + 3 * (size_t)f.n_tex + tex[it]) : 0.f;
         }
 #pragma unroll 1
         for (int l = 0; l < f.L; ++l, radius *= 0.5f, ip.x *= 0.5f, ip.y *= 0.5f)
@@ -401,7 +428,7 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, kCo
                     level_bits |= 1u << l;
                     if ((long long)slot[cidx] < f.capacity)
                         store_record(f, slot[cidx], key, blending_fac(ip, cidx, nullptr, nullptr) * conf,  // RenderForward.cu:1619
-                                     tex | (cidx << kCornerShift), desc);
+                                     tex[it] | (cidx << kCornerShift), desc);
                 }
             }
         }
@@ -3469,22 +3496,29 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
         rc = zero_buffers(ctx, buffers, bytes, 3);
         if (rc != VETR_OK) return rc;
     }
-    const int point_ctas = (f.n + kProjThreads * kPointsPerThread - 1) / (kProjThreads * kPointsPerThread);
-    if (point_ctas > 0)
+    const bool bilinear = f.mode == VETR_MODE_BILINEAR_BLEND;
+    if (f.n > 0)
     {
         PassScope t(ctx, VETR_T_COUNT, 1);
-        launch(overlap, project_kernel<false, kPointsPerThread>, dim3(point_ctas, n_views), kProjThreads, 0, st, f);
+        const bool one    = (long long)f.n * n_views < kCountSeveral;
+        const int per     = kProjThreads * (one ? 1 : count_points(bilinear));
+        const auto kernel = bilinear ? (one ? project_kernel<false, 1, true> : project_kernel<false, count_points(true), true>)
+                                     : (one ? project_kernel<false, 1, false> : project_kernel<false, count_points(false), false>);
+        launch(overlap, kernel, dim3((f.n + per - 1) / per, n_views), kProjThreads, 0, st, f);
     }
     const int n_tiles = (int)((f.PT + kScanTile - 1) / kScanTile);
     {
         PassScope t(ctx, VETR_T_SCAN, 2);
         launch_scan(f.counts, f.PT, f.capacity, ctx->tile_sums, reinterpret_cast<unsigned*>(ctx->tile_sums + ctx->tile_cap), n_tiles, f.ends, f.status, f.item_start, f.next_item, st, overlap);
     }
-    if (point_ctas > 0)
+    if (f.n > 0)
     {
         PassScope t(ctx, VETR_T_COLLECT, 1);
-        const int ctas = (f.n + kCollectThreads * kCollectPoints - 1) / (kCollectThreads * kCollectPoints);
-        launch(overlap, project_kernel<true, kCollectPoints>, dim3(ctas, n_views), kCollectThreads, 0, st, f);
+        const bool one    = (long long)f.n * n_views < (bilinear ? kCollectPairsBilinear : kCollectPairs);
+        const int per     = kCollectThreads * (one ? 1 : 2);
+        const auto kernel = bilinear ? (one ? project_kernel<true, 1, true> : project_kernel<true, 2, true>)
+                                     : (one ? project_kernel<true, 1, false> : project_kernel<true, 2, false>);
+        launch(overlap, kernel, dim3((f.n + per - 1) / per, n_views), kCollectThreads, 0, st, f);
     }
     {
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
