@@ -314,6 +314,26 @@ def test_gpu_envmap_on_either_side_of_flat_slices(S):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("R, S, C", [(6, 4, 4), (6, 8, 3), (20, 5, 1), (36, 3, 4), (180, 4, 4), (180, 6, 3)])
+def test_gpu_envmap_gradient_runs_of_all_lengths(R, S, C):
+    """From coarse textures, where a warp's lanes all fall into one texel, to fine ones, where none shares its texel; image sizes that
+    leave the last warp partly empty, pixels that are left out, and spheres that rays miss."""
+    sc = util.env_scene(n_views=2, w=157, h=43, f=110.0)
+    rng = np.random.default_rng(R + S)
+    env = util.env_map(rng, S=S, R=R, C=C, inner_radius=1.0)
+    weight = util.env_weights(rng, sc, 2)
+    grad_out = [rng.standard_normal((2, C, 43 >> l, 157 >> l)).astype(np.float32) for l in range(2)]
+    # equal texels: a sample's value does not depend on where inside the texture it lies
+    env.color[:] = rng.normal(size=(C, S, 1, 1))
+    env.density[:] = rng.normal(size=(S, 1, 1))
+    rgd, rgc, md, mc = O.envmap_backward(sc, sc.views, 2, env, weight, grad_out, flags=O.ENV_NOT_AT_POINTS)
+    _, gd, gc = util.env_gpu_run(sc, env, 2, weight, O.ENV_NOT_AT_POINTS, grad_out)
+    assert np.abs(rgc).max() > 0
+    assert np.all(np.abs(gd - rgd) <= util.env_grad_tolerance(md, env))
+    assert np.all(np.abs(gc - rgc) <= util.env_grad_tolerance(mc, env))
+
+
+@pytest.mark.gpu
 def test_gpu_envmap_of_a_very_tall_image():
     """2^24 rows, the most whose numbers are exact in fp32: a pixel's row is formed from an estimate that is off by two there.  A small
     focal length and a centre near the last rows make neighbouring rows differ."""

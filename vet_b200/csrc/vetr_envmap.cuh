@@ -13,13 +13,14 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "vetr_math.cuh"
 
 namespace vetr
 {
 constexpr int kEnvMaxSpheres = 8;  // MAX_NUM_SPHERES, EnvironmentMap.cu:91
-constexpr int kEnvThreads    = 256;
+constexpr int kEnvThreads    = 256, kEnvBackThreads = 128;
 
 struct EnvView
 {
@@ -316,28 +317,32 @@ __global__ void __launch_bounds__(kEnvThreads) envmap_forward_kernel(const __gri
 // scattered to its corners.  Neighbouring pixels of a row fall into the same texel (a level-0 row of 1920
 // pixels crosses a few hundred texels), so before the atomics the lanes of a warp that share a base texel, in runs of
 // consecutive lanes, are summed with a segmented shuffle reduction and the run's first lane issues one atomic per corner and
-// value.  (Ending the reduction at the warp's longest run, five values side by side, was measured slower: 843 -> 955 us with
-// four spheres, 1890 -> 2390 us with eight, at eight corners per sample.)
+// value.  Five steps, or three where no run of the warp is longer than eight lanes.  More such forms lose: with all of 0 to 5, or
+// 5, 3 and 2, the loop's instructions are too many (1280 x 720 x 2, three spheres of 200 x 200: five 322 us, 5 and 3 337, 5, 3 and 2
+// 344, all 377; 1920 x 1080, four of 1024 x 1024: 574, 533, 538, 572).
 //
-// kMaxSpheres is 4 or 8: what the sweeps keep per sphere lives in registers, so the usual map of up to four spheres does not
-// pay for eight, and has room for the texel coordinates (asin, atan2, two square roots) of the first sweep; with eight they
-// are formed anew.  1920x1080, four levels, one view: four spheres of 1024 x 1024 708 us (902 with eight corners per sample),
-// five of 512 x 512 1064 (1112), eight of 1024 x 1024 2140 us (2295).
+// What the first sweep keeps per sphere lies in shared memory, so that both loops over spheres stay loops: unrolled, with the
+// state in registers, the kernel was several times the size, with three blocks of 256 per SM, and with eight spheres formed the
+// texel coordinates twice.  Blocks of 128 threads, nine per SM (55 registers): with four blocks of 256 a medium-sized
+// image leaves a last wave nearly empty (480 x 270 x 2, three spheres: 125 us, unrolled 112, now 110); ten per SM spill.
+// kMaxSpheres is kEnvFlatSpheres or eight.  1920x1080, four levels, one view: four spheres of 1024 x 1024 707 -> 538 us, two
+// of them 347 -> 272, five of 512 x 512 1072 -> 629, eight of 1024 x 1024 2160 -> 1457.
 #ifndef VETR_ENV_BACK_CTAS
-#    define VETR_ENV_BACK_CTAS 3
+#    define VETR_ENV_BACK_CTAS 9
 #endif
-template <int kMaxSpheres>  // a map of up to four spheres is flat; one of five goes with the larger ones
-__global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backward_kernel(const __grid_constant__ EnvArgs a)
+template <int kMaxSpheres>
+__global__ void __launch_bounds__(kEnvBackThreads, VETR_ENV_BACK_CTAS) envmap_backward_kernel(const __grid_constant__ EnvArgs a)
 {
     __shared__ EnvCam s_cam[VETR_MAX_VIEWS];
+    __shared__ float kept[kMaxSpheres][5][kEnvBackThreads];  // a thread's own: alpha, D, T, texel coordinates
     if (threadIdx.x < a.n_views) s_cam[threadIdx.x] = load_env_cam(a, threadIdx.x);
     __syncthreads();
     constexpr bool kFlat  = kMaxSpheres <= kEnvFlatSpheres;
     constexpr int kN      = EnvCorners<kFlat>::N;
-    const long long plane = (long long)a.S * a.R * a.R, slice = kFlat ? (long long)a.R * a.R : 0;
+    const int plane = a.S * a.R * a.R, slice = kFlat ? a.R * a.R : 0;  // below 2^31; all channels' planes need not be
     const int lane = threadIdx.x & 31;
     const int span = (a.lend[a.L - 1] + 31) / 32 * 32;  // whole warps stay in the loop together
-    for (int idx = blockIdx.x * kEnvThreads + threadIdx.x; idx < span; idx += gridDim.x * kEnvThreads)
+    for (int idx = blockIdx.x * kEnvBackThreads + threadIdx.x; idx < span; idx += gridDim.x * kEnvBackThreads)
     {
         EnvPixelId p;
         bool active = env_locate(a, idx, p);
@@ -358,32 +363,29 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                 if (ch < a.C) G[ch] = g[ch * per_view];
             ray = env_ray(s_cam[p.b], a.lw[p.l], a.lh[p.l], a.scale[p.l], p.x, p.y);
         }
-        constexpr bool kKeep = kMaxSpheres <= 4;
-        float alpha[kMaxSpheres], dot[kMaxSpheres], Tin[kMaxSpheres], ix[kKeep ? kMaxSpheres : 1], iy[kKeep ? kMaxSpheres : 1];
         unsigned hits     = 0;  // bit s: the ray hits sphere s
         unsigned negative = 0;  // bit 4 s + ch: the raw colour sample is negative (S <= 8, C <= 4)
         unsigned zero     = 0;  // the raw colour sample is exactly zero (abs has no gradient there)
         float T = env_start_T(wgt, a.flags);
-#pragma unroll
-        for (int s = 0; s < kMaxSpheres; ++s)
+        if (active)
         {
-            alpha[s] = 0.f, dot[s] = 0.f, Tin[s] = T;
-            float x = 0.f, y = 0.f;
-            if (s < a.S && active)
+#pragma unroll 1
+            for (int s = 0; s < a.S; ++s)
             {
+                float x, y;
                 if (env_coordinates(a, ray, s, x, y))
                 {
                     hits |= 1u << s;
                     EnvCorners<kFlat> c;
                     env_corners<kFlat>(a, x, y, s, c);
-                    alpha[s] = 1.f;
-                    if (s != a.S - 1) alpha[s] = 1.f / (1.f + expf(-env_fetch<kFlat>(a.density + s * slice, c)));
+                    float alpha = 1.f;
+                    if (s != a.S - 1) alpha = 1.f / (1.f + expf(-env_fetch<kFlat>(a.density + s * slice, c)));
                     float d = 0.f;
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch)
                         if (ch < a.C)
                         {
-                            float col = env_fetch<kFlat>(a.color + ch * plane + s * slice, c);
+                            float col = env_fetch<kFlat>(a.color + ((long long)ch * plane + s * slice), c);
                             if (a.non_subzero)
                             {
                                 if (col < 0.f) negative |= 1u << (4 * s + ch);
@@ -392,34 +394,32 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
                             }
                             d += col * G[ch];
                         }
-                    dot[s] = d;
+                    kept[s][0][threadIdx.x] = alpha, kept[s][1][threadIdx.x] = d, kept[s][2][threadIdx.x] = T;
+                    kept[s][3][threadIdx.x] = x, kept[s][4][threadIdx.x] = y;
+                    T = (1.f - alpha) * T;
                 }
-                if (kKeep) ix[kKeep ? s : 0] = x, iy[kKeep ? s : 0] = y;
-                T = (1.f - alpha[s]) * T;
             }
         }
         float rest = 0.f;
-#pragma unroll
-        for (int s = kMaxSpheres - 1; s >= 0; --s)
+#pragma unroll 1
+        for (int s = a.S - 1; s >= 0; --s)
         {
-            if (s >= a.S) continue;  // uniform over the grid
-            const float g_alpha = Tin[s] * (dot[s] - rest);
-            rest                = alpha[s] * dot[s] + (1.f - alpha[s]) * rest;
             const bool live = hits >> s & 1;
             EnvCorners<kFlat> c;
             float gv[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // gradient of the density sample, then of the colour samples
             int key = -1 - lane;                      // never equal between lanes
             if (live)
             {
-                float x = kKeep ? ix[kKeep ? s : 0] : 0.f, y = kKeep ? iy[kKeep ? s : 0] : 0.f;
-                if (!kKeep) env_coordinates(a, ray, s, x, y);
-                key   = env_corners<kFlat>(a, x, y, s, c, key);
-                gv[0] = s == a.S - 1 ? 0.f : g_alpha * (alpha[s] * (1.f - alpha[s]));  // alpha is the sigmoid
+                const float alpha = kept[s][0][threadIdx.x], dot = kept[s][1][threadIdx.x], Tin = kept[s][2][threadIdx.x];
+                const float g_alpha = Tin * (dot - rest);
+                rest                = alpha * dot + (1.f - alpha) * rest;
+                key   = env_corners<kFlat>(a, kept[s][3][threadIdx.x], kept[s][4][threadIdx.x], s, c, key);
+                gv[0] = s == a.S - 1 ? 0.f : g_alpha * (alpha * (1.f - alpha));  // alpha is the sigmoid
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch)
                     if (ch < a.C)
                     {
-                        float v = Tin[s] * alpha[s] * G[ch];
+                        float v = Tin * alpha * G[ch];
                         if (negative >> (4 * s + ch) & 1) v = -v;
                         if (zero >> (4 * s + ch) & 1) v = 0.f;
                         gv[1 + ch] = v;
@@ -434,35 +434,36 @@ __global__ void __launch_bounds__(kEnvThreads, VETR_ENV_BACK_CTAS) envmap_backwa
             const int prev       = __shfl_up_sync(0xffffffffu, key, 1);
             const bool head      = lane == 0 || key != prev;
             const unsigned heads = __ballot_sync(0xffffffffu, head);
-            const int seg        = __popc(heads & (0xffffffffu >> (31 - lane)));
-            unsigned same = 0;  // bit k: lane + 2^k belongs to this lane's run
-#pragma unroll
-            for (int k = 0; k < 5; ++k)
+            const unsigned later = heads >> lane >> 1;  // lanes behind this one that begin a run
+            const int behind     = later ? __ffs(later) - 1 : 31 - lane;  // lanes behind this one in its run
+            const auto scatter   = [&](auto steps)
             {
-                const int other = __shfl_down_sync(0xffffffffu, seg, 1 << k);
-                if (lane + (1 << k) < 32 && other == seg) same |= 1u << k;
-            }
 #pragma unroll
-            for (int q = 0; q < kN; ++q)
-            {
-                // a corner no lane of the warp uses (the empty z slice of a sample that sits on a slice)
-                if (!kFlat && !__any_sync(0xffffffffu, c.w[q] != 0.f)) continue;
-#pragma unroll
-                for (int v = 0; v < 5; ++v)
+                for (int q = 0; q < kN; ++q)
                 {
-                    if (v > a.C) continue;
-                    if (v == 0 && s == a.S - 1) continue;  // the last sphere's alpha is a constant
-                    float x = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
+                    // a corner no lane of the warp uses (the empty z slice of a sample that sits on a slice)
+                    if (!kFlat && !__any_sync(0xffffffffu, c.w[q] != 0.f)) continue;
 #pragma unroll
-                    for (int k = 0; k < 5; ++k)
+                    for (int v = 0; v < 5; ++v)
                     {
-                        const float y = __shfl_down_sync(0xffffffffu, x, 1 << k);
-                        if (same >> k & 1) x += y;
+                        if (v > a.C) continue;
+                        if (v == 0 && s == a.S - 1) continue;  // the last sphere's alpha is a constant
+                        float x = c.off[q] >= 0 ? c.w[q] * gv[v] : 0.f;
+#pragma unroll
+                        for (int k = 0; k < decltype(steps)::value; ++k)
+                        {
+                            const float y = __shfl_down_sync(0xffffffffu, x, 1 << k);
+                            if (behind >= 1 << k) x += y;
+                        }
+                        if (head && c.off[q] >= 0 && x != 0.f)
+                            atomicAdd((v == 0 ? a.g_density : a.g_color + (long long)(v - 1) * plane) + (s * slice + c.off[q]), x);
                     }
-                    if (head && c.off[q] >= 0 && x != 0.f)
-                        atomicAdd((v == 0 ? a.g_density : a.g_color + (v - 1) * plane) + s * slice + c.off[q], x);
                 }
-            }
+            };
+            if (__any_sync(0xffffffffu, behind >= 8))
+                scatter(std::integral_constant<int, 5>{});
+            else
+                scatter(std::integral_constant<int, 3>{});
         }
     }
 }

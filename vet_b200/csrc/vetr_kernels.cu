@@ -3904,11 +3904,11 @@ extern "C" int vetr_envmap_backward(vetr_ctx* ctx, const vetr_cameras* cams, con
         }
         a.g_density = g_density, a.g_color = g_color;
         ctx->launches += 1;
-        const int grid = std::min((a.lend[num_layers - 1] + kEnvThreads - 1) / kEnvThreads, ctx->sm_count * 32);
-        if (a.S <= 4)
-            envmap_backward_kernel<4><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
+        const int grid = std::min((a.lend[num_layers - 1] + kEnvBackThreads - 1) / kEnvBackThreads, ctx->sm_count * 72);
+        if (a.S <= kEnvFlatSpheres)
+            envmap_backward_kernel<kEnvFlatSpheres><<<grid, kEnvBackThreads, 0, ctx->stream>>>(a);
         else
-            envmap_backward_kernel<kEnvMaxSpheres><<<grid, kEnvThreads, 0, ctx->stream>>>(a);
+            envmap_backward_kernel<kEnvMaxSpheres><<<grid, kEnvBackThreads, 0, ctx->stream>>>(a);
     }
     VETR_CUDA(ctx, cudaGetLastError());
     return VETR_OK;
