@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, pro
 #pragma unroll
                 for (int l = 0; l < VETR_MAX_LAYERS; ++l)
                     if (g[it][l] >= 0) atomicAdd(f.counts + g[it][l], 1);
-            return;
         }
         else
         {
@@ -366,9 +365,8 @@ __global__ void __launch_bounds__(kCollect ? kCollectThreads : kProjThreads, pro
                 if (g[it][l] >= 0 && (long long)g[it][l] < f.capacity) store_record(f, g[it][l], key, conf[it], tex[it], desc[it]);
         }
         }
-        return;
     }
-
+    else
     // mode 3: every (point, level) touches the four pixels around its position.  The record's descriptor index carries
     // the corner (0..3) in its two top bits: the backward pass files a fragment's result under (point, level, corner).
 #pragma unroll
