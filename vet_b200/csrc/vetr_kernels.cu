@@ -3259,9 +3259,7 @@ extern "C" int vetr_create(vetr_ctx** out, int device, void* cuda_stream)
     ctx->device = device;
     ctx->stream = (cudaStream_t)cuda_stream;
     cudaError_t e = cudaSetDevice(device);
-    cudaDeviceProp prop;
-    if (e == cudaSuccess) e = cudaGetDeviceProperties(&prop, device);
-    if (e == cudaSuccess) ctx->sm_count = prop.multiProcessorCount;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
     const auto prepare = [&e](auto kernel, int threads, size_t smem, int* ctas_per_sm)
     {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
