@@ -19,9 +19,9 @@
 //   project_kernel<count>    stream positions, strict-fp32 projection, per-level pixel, one reduction per fragment
 //   scan_*                   exclusive scan of counts -> ends, total F, longest list, work-item table, in two kernels (the last block
 //                            of the first scans the sums of the tiles)
-//   project_kernel<collect>  re-project, reserve all slots of a thread's points, then store the 32-byte records
+//   project_kernel<collect>  re-project, request the payload, reserve all slots of a thread's points, store the 32-byte records
 //   sort_blend_kernel        per work item: stage records in shared memory, rank-sort each list by (depth, index),
-//                            write the sorted records back, blend front to back, write all outputs (+ _long variant)
+//                            write every record to its sorted place, blend front to back, write all outputs (+ _long variant)
 //   pack_images_kernel       channel-interleaved copies of the forward image and its gradient
 //   backward_kernel          per work item: stream sorted records, image-space gradient of each fragment (parked for
 //                            the per-point pass), O(n) transmittance / suffix sweeps per pixel, vector reductions of
@@ -30,7 +30,7 @@
 //                            written once, camera gradients reduced per CTA and view (mode 3: confidence gradient too)
 //   fuzzy_dt_*               mode 0 (no lists): depth pre-pass, splat, combine, per-point backward
 //   exchange_finalize_kernel multi-GPU: sum over ranks + epilogue over NVLink peer memory (plain or multicast)
-//   grid_row_sums / grid_loss (+ _chunk)   error-grid rasterisation (four cells per warp, a lane per pixel row)
+//   grid_row_sums / grid_loss (cells, chunks)   error-grid rasterisation (a lane prepares a cell, then lanes own pixel rows)
 //   zero_buffers / finalize / apply_tangent   zero fill, epilogue, pose update
 #include <cuda_runtime.h>
 #include <stdint.h>
