@@ -3914,7 +3914,7 @@ template <int KMAX>
 static void knn_launch_search(vetr_ctx* ctx, const KnnSearch& a)
 {
     knn_near_kernel<KMAX><<<(a.n + 127) / 128, 128, 0, ctx->stream>>>(a);
-    knn_far_kernel<KMAX><<<ctx->sm_count * 8, 128, 0, ctx->stream>>>(a);
+    knn_far_kernel<KMAX><<<ctx->sm_count * kKnnFarCtas, 128, 0, ctx->stream>>>(a);
 }
 
 extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int position_stride, int n, int k, float* radius, int radius_stride)

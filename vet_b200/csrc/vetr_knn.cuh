@@ -426,8 +426,14 @@ __global__ void __launch_bounds__(128) knn_near_kernel(const __grid_constant__ K
 //
 // Where the cube of an isolated point meets a dense surface, a few rows hold hundreds of candidates: with a lane scanning
 // the whole of its row the others waited for it.  4 M points of a planar scene with 5 % outliers, k = 4: 1054 -> 557 us.
+//
+// Points next to each other in the queue lie next to each other and cost alike, from a few rows to thousands, so the blocks are many more than
+// fit at once and the SMs take them as they come free: 8 / 32 / 64 / 128 / 256 blocks per SM 474 / 442 / 425 / 426 / 433 us there (8 M points 769 /
+// 727 / 687 / 668 / 681; 30 k points 16 us, 21 with 256).  Ten blocks per SM at a time (48 registers, 12 bytes spilled) instead of nine: 408 (658);
+// twelve lose: 506.  For more than four neighbours the compiler's own choice is faster (200 k points, k = 8: 91 us).
+constexpr int kKnnFarCtas = 64;
 template <int KMAX>
-__global__ void __launch_bounds__(128) knn_far_kernel(const __grid_constant__ KnnSearch a)
+__global__ void __launch_bounds__(128, KMAX <= 5 ? 10 : 0) knn_far_kernel(const __grid_constant__ KnnSearch a)
 {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane   = threadIdx.x & 31;
