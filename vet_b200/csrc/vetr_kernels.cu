@@ -3442,6 +3442,20 @@ extern "C" int vetr_zero_buffers(vetr_ctx* ctx, void* const* buffers, const int6
 // points 394 -> 381 and with 3 M and two views 2933 -> 2840; below it the late blocks and the counter cost more: 99 k points in mode 1 46 -> 47,
 // 39 k in mode 3 58 -> 72, 114 k 122 -> 131, mode 2 with 1 M points the same.
 constexpr long long kQueueFragments = 1 << 21;
+
+// Blocks of sort_blend_kernel.  As many as are resident leave the SMs finishing at different times, however evenly the items are cut:
+// neighbouring items lie on the same stretch of the image.  Four times as many are taken by the SMs as they come free, at the price of a first
+// item that nothing was requested ahead for, so each block should still have one or more.  How many items there are is known only on
+// the device; the pixels alone give at least `items`.  us with 1 / 2 / 4 / 8 / 16 times the resident blocks, items per resident block in front:
+//   2.3 (100 k points, 512 x 512) 12.3 / 11.5 / 13.3 / 14.1 / 24.0      4.2 (mode 2, 1 M points, 801 x 603) 72.8 / 65.4 / 57.4 / 61.4 / 62.3
+//   18 (3 M points, 1920 x 1080) 163 / 157 / 144 / 149 / 161            27 (8 M points x 4 views) 860 / 859 / 857 / 859 / 867
+// (The backward kernel gains as well, mode 2 170 -> 125, but adds each block's share of the terms that all pixels send to one address:
+// with more blocks their fp32 sum left its bound.)
+static int blend_blocks(long long pixels, int resident)
+{
+    const long long items = pixels * kPixelWork / kQuantum;
+    return items < 3ll * resident ? resident : 4 * resident;
+}
 extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr_cloud* cloud, const vetr_texture* texture,
                             const vetr_cameras* cameras, const vetr_view* views, int n_views, const float* dropout,
                             const vetr_lists* lists, float* const* out_color, float* const* out_weight,
@@ -3518,7 +3532,7 @@ extern "C" int vetr_forward(vetr_ctx* ctx, const vetr_params* params, const vetr
     }
     {
         PassScope t(ctx, VETR_T_SORT_BLEND, 2);
-        const int grid = ctx->sm_count * ctx->blend_ctas_per_sm;
+        const int grid = blend_blocks(f.PT, ctx->sm_count * ctx->blend_ctas_per_sm);
         const int long_grid = ctx->sm_count * ctx->blend_long_ctas_per_sm;
         if ((long long)f.n * n_views * (f.mode == VETR_MODE_BILINEAR_BLEND ? 4 : 1) >= kQueueFragments)
         {
