@@ -436,6 +436,49 @@ def test_grid_loss_rows_and_corners(rasterizer, n):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+# Rotation of the camera, box, principal row: of the boxes with the outermost corner on a whole row (one in ten thousand of them) some for which
+# the fp32 middles and halves of the segments that meet at the corner, as they are rounded, leave the row out.
+_CORNERS_ON_ROWS = [
+    ((0.30658183, 0.36946553, 0.5665552, -0.66971487), (4.2802687, -0.24014834, 1.4477539), (2.1629434, 1.3006504, 1.2766961), 350.27316),
+    ((0.07821663, -0.5740086, -0.34341568, 0.7392307), (3.5538538, 1.9203218, -1.1163687), (1.498105, 1.3347545, 0.76249063), 349.79883),
+    ((-0.22463317, -0.9429001, 0.18938075, 0.15688913), (-0.5152078, -3.4728684, -4.5743327), (1.0238084, 1.3970141, 1.3433175), 349.5322),
+    ((-0.22463317, -0.9429001, 0.18938075, 0.15688913), (-0.6212897, -4.195308, -6.3612576), (1.0719604, 2.115874, 1.9900571), 349.7246),
+    ((-0.7046612, -0.5607396, -0.15494646, 0.40622082), (3.4207447, -2.508509, -7.8716316), (2.3550122, 2.3201106, 3.090605), 350.05362),
+    ((0.7350364, -0.5994996, 0.31396294, 0.041821703), (1.9027438, -1.8412875, -3.2669928), (1.125605, 1.089446, 1.4549216), 349.70297),
+    ((-0.2781702, 0.555939, 0.44323123, -0.6458322), (3.2008967, 2.9440315, 1.6696035), (1.8064176, 2.9341648, 1.5898691), 349.9827),
+    ((-0.42319033, 0.78361243, 0.22142796, 0.39727974), (-5.389095, 0.34001753, -5.5709224), (2.9694746, 1.5295297, 1.505763), 349.54324),
+    ((-0.8119283, -0.18111958, 0.3197237, 0.4535911), (-2.4465358, -5.170887, -5.085798), (2.266861, 1.5348879, 2.192551), 350.13196),
+    ((-0.5533877, 0.038533997, 0.70032746, 0.44924226), (-4.645606, -1.2301524, 1.5215195), (2.0896008, 1.491314, 0.97503215), 349.83658),
+    ((0.79685336, -0.52456146, 0.21881467, 0.20489049), (2.2056577, -1.0097961, -2.7729173), (2.0048594, 0.9074665, 1.3701627), 350.31216),
+    ((-0.62642443, 0.5759482, -0.31922892, 0.41709593), (-1.5578544, -6.227739, -1.2585564), (2.7273932, 2.3098223, 1.7034277), 350.2481),
+    ((0.7696578, -0.5616687, 0.3031369, -0.01622326), (2.23646, -4.3709273, -4.1443353), (2.1590297, 1.5269341, 3.0312054), 350.3346),
+    ((-0.5932387, -0.104229875, 0.67960924, 0.4187305), (-5.274751, -2.8566115, 0.8076543), (3.3586922, 1.9716004, 2.1268368), 350.19293),
+]
+
+
+def test_grid_loss_outermost_corner_on_a_row(rasterizer):
+    """Boxes of 270 to 700 pixels whose leftmost or rightmost corner alone lies on a whole row: the run of that row ends at the corner
+    and not at an inner segment (47 to 274 pixels less).  Coverage is exact."""
+    import torch
+
+    w, h = 1400, 700
+    sc = scenes.config_planar(64, w, h, 700.0, n_views=1, seed=3)
+    loss = np.random.default_rng(5).standard_normal((3, h, w)).astype(np.float32)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    on = t(loss)
+    for quaternion, bb_min, bb_len, row in _CORNERS_ON_ROWS:
+        sc.poses = np.array([quaternion + (0, 0, 0, 0)], np.float32).astype(np.float64)
+        sc.intrinsics[:] = 0
+        sc.intrinsics[0, :4] = 700.0, 700.0, 700.0, row
+        box = [np.array([a], np.float32) for a in (bb_min, bb_len)]
+        ref_v, ref_c = O.grid_loss(sc, sc.views[0], *box, loss)
+        value, count = torch.zeros(1, device=rasterizer.device), torch.zeros(1, dtype=torch.int32, device=rasterizer.device)
+        rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(box[0]), t(box[1]), on, value, count)
+        assert ref_c[0] > 10_000
+        np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
+        np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
+
+
 # ---- mode 0 without camera gradients: the pixels of all levels are looked up together
 
 

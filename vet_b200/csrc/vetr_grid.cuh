@@ -154,7 +154,7 @@ struct GridWarpSmem
 {
     float2 corner[8][33];                   // projected corners of up to 32 cells, a lane's cell per column
     float2 pp[kGridGroup][8];               // those of the group in work
-    float4 seg[kGridSegments][kGridGroup];   // {x at row 0, dx/dy, middle row, half the rows}, relative to the rectangle's first pixel
+    float4 seg[kGridSegments][kGridGroup];   // {x at row 0, dx/dy, middle row, half the rows (rounded up)}, relative to the rectangle's first pixel
     float2 band[kGridSegments][kGridGroup];  // {half-width of the band along the row, half the rows with what the band adds to them}
     int4 rect[kGridGroup];                   // first column, first row, columns, rows
     int2 spot[kGridGroup][8];                // {row, column} of the pixel next to a corner, row -1 if it is far enough away
@@ -432,6 +432,12 @@ struct GridCell
 // a quarter pixel are refused) and at least 7 rho: a pixel above or below a segment of |k| <= 4 that is nearest to a point inside it is at
 // most sqrt(17) rho away from its end, so that only flatter segments have to be followed beyond their ends.  (All of the edges' bands
 // as wide as the corners' want 3 % of the rows tested pixel by pixel, a sixth of the whole call.)
+// A row crosses a segment if it is no farther from the segment's middle row than half its rows.  Middle, half and distance are rounded, by less
+// than 1.8e-7 E together, so 2.4e-7 E are added to the half: without them a corner on a whole row can lie outside every segment that meets
+// there, and the run then ends at an inner one.  A row that is let in without crossing lies within 4.2e-7 E of the segment's end.  With
+// |k| <= 4 its extended crossing is off the end by less than 4 of these and the crossing's own 2e-6 E, inside the corner's band (7e-6 E and
+// more); with a steeper k by less than 4.2e-7 E |k| and 4e-7 E |k|, inside the 1.25e-6 E |k| by which the segment's band is longer.  So any
+// pixel that such a crossing adds to the run is tested.
 // All this takes the projected corners as they are, whatever rounding went into them.  Cells whose corners' bands would be wider than a
 // quarter pixel, or with a triangle as thin as a few units in the last place of a pixel coordinate, take the per-pixel form.
 __device__ __forceinline__ GridCell grid_prepare(const Frame& f, const GridArgs& a, const Camera& cam, GridWarpSmem& s, int c, bool no_rows)
@@ -529,13 +535,14 @@ __device__ __forceinline__ void grid_segments(GridWarpSmem& s, const GridCell& c
             p.x -= bx, p.y -= by, q.x -= bx, q.y -= by;
             const float dx = q.x - p.x, dy = q.y - p.y, rho = cell.rho;
             const bool flat = dy < 1e-3f;  // as good as horizontal: the band covers the whole segment
-            const float k_  = flat ? 0.f : dx / dy, rows = 0.5f * dy, steep = fabsf(k_);
-            s.seg[k][slot]  = make_float4(flat ? p.x + 0.5f * dx : __fmaf_rn(-k_, p.y, p.x), k_, p.y + rows, rows);
+            const float k_  = flat ? 0.f : dx / dy, middle = 0.5f * dy, steep = fabsf(k_);
+            const float rows = middle + 0.24f * rho;  // half the rows, and what the roundings can take from them
+            s.seg[k][slot]  = make_float4(flat ? p.x + 0.5f * dx : __fmaf_rn(-k_, p.y, p.x), k_, p.y + middle, rows);
             const bool beyond = flat || steep > 4.f;  // followed beyond its ends: by rho in height, the last term of its reach along the row
             // (which is also for the rounding of the crossing where the reach is cut: 1.2e-7 E |dx/dy|)
             float half = flat ? 0.5f * fabsf(dx) + 4.f * rho : fminf(rho * (1.f + steep), fabsf(dx) + 2.f * rho);
             if (beyond) half += 1.25f * rho * steep;
-            s.band[k][slot] = make_float2(half, beyond ? rows + rho : rows);
+            s.band[k][slot] = make_float2(half, beyond ? middle + rho : rows);
         }
         const float2 c = s.pp[slot][corner];
         const float x = rintf(c.x), y = rintf(c.y);
