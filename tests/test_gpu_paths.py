@@ -479,6 +479,28 @@ def test_grid_loss_outermost_corner_on_a_row(rasterizer):
         np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
+def test_grid_loss_more_chunks_than_an_int(rasterizer):
+    """Boxes without depth (per-pixel form) over the whole of a large view, so many that the chunks asked for would pass 2^31: those that
+    find no room in the queue are counted like the others."""
+    import torch
+
+    w, h, n = 1920, 1080, 74_000
+    chunks = (w - 65) * (h - 65) // 64  # of a box, at least: the rectangle leaves out 32 pixels on either side
+    assert n * chunks > 2 ** 31
+    sc = scenes.config_planar(64, w, h, 1000.0, n_views=1, seed=3)
+    sc.poses = np.array([[0, 0, 0, 1, 0, 0, 0, 0]], np.float64)
+    sc.intrinsics[0, :4] = 1000.0, 1000.0, 960.0, 540.0
+    box = np.array([[-2.0, -2.0, 1.0]], np.float32), np.array([[4.0, 4.0, 0.0]], np.float32)
+    loss = np.ones((1, h, w), np.float32)
+    _, ref_c = O.grid_loss(sc, sc.views[0], *box, loss)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
+    value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(np.tile(box[0], (n, 1))), t(np.tile(box[1], (n, 1))), t(loss), value, count)
+    assert ref_c[0] >= 64 * chunks
+    np.testing.assert_array_equal(count.cpu().numpy(), np.full(n, ref_c[0]))
+    np.testing.assert_array_equal(value.cpu().numpy(), np.full(n, ref_c[0], np.float32))  # whole numbers below 2^24
+
+
 # ---- mode 0 without camera gradients: the pixels of all levels are looked up together
 
 

@@ -722,7 +722,7 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
 // of two of cells again and again).  Handing the groups out by an atomic counter as warps come for them: 890 us without the rows alone.
 template <bool kChunks>
 __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(const __grid_constant__ Frame f, const __grid_constant__ GridArgs a,
-                                                                               int2* queue, int* queue_count, int each)
+                                                                               int2* queue, unsigned long long* queue_count, int each)
 {
     __shared__ Camera s_cam;
     __shared__ GridWarpSmem s_warp[kGridWarps];
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
     if (kChunks)
     {
         // reservations past the capacity were never written: those cells were done by the first kernel
-        n = min(*queue_count, kGridQueueCap);
+        n = (int)min(*queue_count, (unsigned long long)kGridQueueCap);
         if (n == 0) return;
         each = min(32 / kGridGroup, max(1, n / ((int)gridDim.x * kGridWarps * kGridGroup)));
     }
@@ -801,8 +801,9 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
                     large &= large - 1;
                     const int n_chunks = cell.by_rows ? (parts - 1) / kGridRowChunk + 1 : (parts - 1) / kGridChunk + 1;
                     const int chunks = __shfl_sync(0xffffffffu, n_chunks, head), ci = __shfl_sync(0xffffffffu, c, head);
-                    int at = 0;
-                    if (lane == 0) at = atomicAdd(queue_count, chunks);
+                    // (in 64 bits: the counter adds up what finds no room as well, and 2^31 cells of 2^31 pixels are not 2^63 chunks)
+                    unsigned long long at = 0;
+                    if (lane == 0) at = atomicAdd(queue_count, (unsigned long long)chunks);
                     at = __shfl_sync(0xffffffffu, at, 0);
                     // no room for all chunks: whatever part of the reservation lies inside the queue is marked unused
                     const bool fits = at + chunks <= kGridQueueCap;
