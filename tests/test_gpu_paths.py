@@ -479,26 +479,32 @@ def test_grid_loss_outermost_corner_on_a_row(rasterizer):
         np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
-def test_grid_loss_more_chunks_than_an_int(rasterizer):
-    """Boxes without depth (per-pixel form) over the whole of a large view, so many that the chunks asked for would pass 2^31: those that
-    find no room in the queue are counted like the others."""
+@pytest.mark.parametrize("n, w, h, distorted", [(30, 1920, 1080, False), (4000, 1920, 1080, False), (20_000, 1920, 1080, False),
+                                                (30, 1920, 1080, True), (30, 640, 480, True), (30, 333, 251, True)])
+def test_grid_loss_chunks_of_the_per_pixel_form(rasterizer, n, w, h, distorted):
+    """Boxes without depth (per-pixel form) of a few to 1.8 million pixels, around the sizes from which on a cell's chunks are larger; few of them, so many
+    that all chunks are of the largest size, and more than the queue has room for.  A distorted camera in images of the three sizes that
+    its chunks go by.  Coverage is exact."""
     import torch
 
-    w, h, n = 1920, 1080, 74_000
-    chunks = (w - 65) * (h - 65) // 64  # of a box, at least: the rectangle leaves out 32 pixels on either side
-    assert n * chunks > 2 ** 31
     sc = scenes.config_planar(64, w, h, 1000.0, n_views=1, seed=3)
     sc.poses = np.array([[0, 0, 0, 1, 0, 0, 0, 0]], np.float64)
-    sc.intrinsics[0, :4] = 1000.0, 1000.0, 960.0, 540.0
-    box = np.array([[-2.0, -2.0, 1.0]], np.float32), np.array([[4.0, 4.0, 0.0]], np.float32)
+    sc.intrinsics[0, :4] = 1000.0, 1000.0, w / 2, h / 2
+    if distorted:
+        sc.intrinsics[0, 5:] = (0.05, -0.02, 0.001, 0.01, 0.0, 0.0, 0.001, -0.002)
+    size = np.array([(3, 3), (8, 8), (9, 8), (64, 9), (256, 255), (256, 256), (257, 256), (256, 257), (512, 256), (513, 256), (512, 257), (512, 512),
+                     (513, 513), (700, 700), (1800, 1000)], np.float32)
+    bb_len = np.concatenate([size / 1000, np.zeros((len(size), 1))], 1).astype(np.float32)
+    bb_min = np.tile(np.array([[(90.3 - w / 2) / 1000, (60.3 - h / 2) / 1000, 1.0]], np.float32), (len(size), 1))
     loss = np.ones((1, h, w), np.float32)
-    _, ref_c = O.grid_loss(sc, sc.views[0], *box, loss)
+    _, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
+    assert ref_c.min() > 0 and n * ref_c.mean() / 512 > {30: 0, 4000: 2 ** 18, 20_000: 2 ** 22}[n]
+    which = np.arange(n) % len(size)
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
     value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
-    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(np.tile(box[0], (n, 1))), t(np.tile(box[1], (n, 1))), t(loss), value, count)
-    assert ref_c[0] >= 64 * chunks
-    np.testing.assert_array_equal(count.cpu().numpy(), np.full(n, ref_c[0]))
-    np.testing.assert_array_equal(value.cpu().numpy(), np.full(n, ref_c[0], np.float32))  # whole numbers below 2^24
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min[which]), t(bb_len[which]), t(loss), value, count)
+    np.testing.assert_array_equal(count.cpu().numpy(), ref_c[which])
+    np.testing.assert_array_equal(value.cpu().numpy(), ref_c[which].astype(np.float32))  # whole numbers below 2^24
 
 
 # ---- mode 0 without camera gradients: the pixels of all levels are looked up together

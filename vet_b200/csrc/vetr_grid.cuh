@@ -71,13 +71,18 @@ __device__ __forceinline__ float grid_pixel_loss(const GridArgs& a, int x, int y
 
 constexpr int kGridWarps    = 4;
 constexpr int kGridGroup    = 4;                // cells a warp takes together: eight lanes each
-constexpr int kGridChunk      = 64;             // pixels of a rectangle one warp walks in the per-pixel form (256: a warp with four such chunks
-                                                // ends late, 128^3 cells at 1920x1080 681 instead of 631 us; 512: 50 us more)
-constexpr int kGridRowChunk   = 64;             // rows of a queued chunk; cells of up to that many rows are not queued (32: 702 instead of 655 us,
+constexpr int kGridRowBits    = 6;              // 64 rows of a queued chunk; cells of up to that many rows are not queued (32: 702 instead of 655 us,
                                                 // 35^3 cells at 160x120 45 instead of 37; 128: 835 instead of 805)
+constexpr int kGridRowChunk   = 1 << kGridRowBits;
+constexpr int kGridChunkBits  = 6;              // 64 pixels of a rectangle, at least, that one warp walks in the per-pixel form
 constexpr int kGridExactLanes = 6;              // rows of a warp with pixels to be tested from which on their own lanes test them (2 to 6 the same;
                                                 // never: 1089 instead of 958 us with the bands as wide as they were then)
 constexpr int kGridQueueCap = 4 * 1024 * 1024;  // (cell, chunk) pairs handed to the second kernel
+// Sizes of the per-pixel form's chunks, 64 << 0 to kGridCoarsest pixels: see grid_coarse.
+constexpr int kGridCoarsest   = 3;
+constexpr int kGridCoarseFrom = kGridQueueCap / 16;  // chunks in the queue
+constexpr int kGridVast       = 1 << 16;        // pixels of a cell
+constexpr int kGridMarkAt     = 28;             // bit of a chunk's number from which on the shift stands (an image has no more than 2^31 / 64 chunks)
 constexpr int kGridSegments = 18;               // 12 edges, then 6 face diagonals
 constexpr int kGridCtas     = 6;                // resident CTAs per SM the kernels are compiled for (5: the same, 8: 10 % slower)
 
@@ -160,6 +165,7 @@ struct GridWarpSmem
     int2 spot[kGridGroup][8];                // {row, column} of the pixel next to a corner, row -1 if it is far enough away
     int spots[kGridGroup];                   // not 0: there are some
     int2 todo[64];                          // {cell, chunk} to be prepared
+    int queued;                             // chunks in the queue when the warp looked last
 };
 
 // Corner order of the reference: (0,0,0) (1,0,0) (0,1,0) (0,0,1) (1,1,0) (1,0,1) (0,1,1) (1,1,1).
@@ -710,6 +716,25 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
     return number && out;
 }
 
+// A chunk of the per-pixel form holds 64 << grid_coarse(...) pixels.  Few cells in that form: small ones, because the warps with the last chunks of
+// 512 end late (128^3 cells at 1920x1080 without distortion 706 instead of 600 us).  But a chunk costs its cell's segments and additions to the cell's
+// two words anew, a third of the time with 64 pixels, and 64 of them fill the queue with 268 million pixels, after which a warp is left alone with
+// its cell.  So they are larger
+// - where no cell goes by rows, by the size of the image.  Eight distortion coefficients, 64 pixels / 256 / 512: 128^3 cells at 1920x1080 64 / 7.0 / 6.8 ms,
+//   64^3 4.1 / 3.4 / 3.3, 16^3 1.01 / 0.88 / 0.80, 96^3 at 1237x823 3.2 / 2.6 / 2.5, 48^3 at 960x540 0.76 / 0.68 / 0.75, 32^3 at 640x480
+//   0.32 / 0.30 / 0.36, 16^3 at 320x240 0.08 / 0.11 / 0.18, 128^3 at 160x120 0.38 / 0.47 / 0.45;
+// - from kGridCoarseFrom chunks on.  Without distortion, 4e6 units from the origin, 64 pixels / 512 / like this: 128^3 71 / 13.9 / 14.0 ms, 64^3 2.5 /
+//   2.1 / 2.3 (from four times as many on: 2.5);
+// - in vast cells, by the pixels of all of them so far.  Flat boxes, always 64 / like this: four over the whole view 396 / 180 us, 300 of them
+//   112 / 6.4 ms, 20 of 700x700 pixels 290 / 210 us, one 87 / 85.
+__device__ __forceinline__ int grid_coarse(const GridArgs& a, bool no_rows, int queued)
+{
+    if (queued >= kGridCoarseFrom) return kGridCoarsest;
+    const int pixels = a.w * a.h;
+    return !no_rows || pixels < 1 << 17 ? 0 : pixels < 1 << 20 ? 2 : kGridCoarsest;
+}
+__device__ __forceinline__ int grid_coarse_vast(unsigned long long pixels) { return min(64 - __clzll((long long)(pixels >> 20)), kGridCoarsest); }
+
 // First kernel (kChunks = false): a warp takes `each` groups of four cells at a time, leaves out those that lie out of sight and prepares the others, a
 // lane per cell, as soon as it has 32 of them; what is left of these is drawn in groups of four, eight lanes per cell.  Cells with many rows
 // (next to the camera a cell covers 10^5 pixels) and large rectangles in the per-pixel form are cut into chunks that go to a queue,
@@ -749,6 +774,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
     // grids tend to have a power of two of cells along an axis, and an even one would give a warp the same part of that axis again and again.
     const long long stride = max(1, (int)gridDim.x * kGridWarps - 1);
     int waiting            = 0;  // in s.todo, whole groups
+    if (lane == 0) s.queued = 0;
     for (long long first = blockIdx.x * kGridWarps + warp;; first += each * stride)
     {
         if (blockIdx.x * kGridWarps + warp < stride && first * kGridGroup < n)
@@ -779,14 +805,14 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
             const int group = (__ffs(todo) - 1) & -kGridGroup, from = group + (lane >> 3);  // the lane that prepared the slot's cell
             todo &= ~(15u << group);
             const GridCell cell = grid_cell_of(prepared, from);
-            const int c = __shfl_sync(0xffffffffu, mine.x, from), chunk = __shfl_sync(0xffffffffu, mine.y, from);
+            const int c = __shfl_sync(0xffffffffu, mine.x, from), part = __shfl_sync(0xffffffffu, mine.y, from);
             grid_segments(s, cell, from);
             if constexpr (kChunks)
             {
-                const int row0        = chunk * kGridRowChunk;
+                const int chunk       = part & ((1 << kGridMarkAt) - 1), row0 = chunk * kGridRowChunk;
                 const bool refused    = grid_rows(a, s, row0, cell.by_rows ? min(kGridRowChunk, cell.y_size - row0) : 0, c);
                 const unsigned slow   = __ballot_sync(0xffffffffu, (lane & 7) == 0 && cell.total() > 0 && (!cell.by_rows || refused));
-                const int size        = cell.by_rows ? kGridRowChunk * cell.x_size : kGridChunk;  // pixels of a chunk
+                const int size        = cell.by_rows ? kGridRowChunk * cell.x_size : 1 << (kGridChunkBits + (part >> kGridMarkAt));  // pixels of a chunk
                 const long long begin = (long long)chunk * size;
                 grid_pixels(a, s, cell, c, slow, begin, min(begin + size, cell.total()));
             }
@@ -794,20 +820,31 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
             {
                 bool here = cell.total() > 0;  // this warp does the cell itself
                 const int parts = cell.by_rows ? cell.y_size : (int)cell.total();
-                unsigned large  = __ballot_sync(0xffffffffu, (lane & 7) == 0 && parts > (cell.by_rows ? kGridRowChunk : kGridChunk));
+                int coarse      = cell.by_rows ? 0 : grid_coarse(a, no_rows, s.queued);
+                const bool vast = (lane & 7) == 0 && !cell.by_rows && parts > kGridVast;
+                if (__any_sync(0xffffffffu, vast))
+                {
+                    const int mine = __reduce_add_sync(0xffffffffu, vast ? min(parts, 1 << 28) : 0);
+                    unsigned long long all = 0;
+                    if (lane == 0) all = atomicAdd(queue_count + 2, (unsigned long long)mine);
+                    all = __shfl_sync(0xffffffffu, all, 0) + mine;
+                    if (vast) coarse = max(coarse, grid_coarse_vast(all));
+                }
+                const int n_chunks = ((parts - 1) >> (cell.by_rows ? kGridRowBits : kGridChunkBits + coarse)) + 1;
+                unsigned large     = __ballot_sync(0xffffffffu, (lane & 7) == 0 && n_chunks > 1);
                 while (large)
                 {
                     const int head = __ffs(large) - 1;
                     large &= large - 1;
-                    const int n_chunks = cell.by_rows ? (parts - 1) / kGridRowChunk + 1 : (parts - 1) / kGridChunk + 1;
                     const int chunks = __shfl_sync(0xffffffffu, n_chunks, head), ci = __shfl_sync(0xffffffffu, c, head);
+                    const int mark   = __shfl_sync(0xffffffffu, coarse, head) << kGridMarkAt;
                     // (in 64 bits: the counter adds up what finds no room as well, and 2^31 cells of 2^31 pixels are not 2^63 chunks)
                     unsigned long long at = 0;
-                    if (lane == 0) at = atomicAdd(queue_count, (unsigned long long)chunks);
+                    if (lane == 0) at = atomicAdd(queue_count, (unsigned long long)chunks), s.queued = (int)min(at, (unsigned long long)kGridQueueCap);
                     at = __shfl_sync(0xffffffffu, at, 0);
                     // no room for all chunks: whatever part of the reservation lies inside the queue is marked unused
                     const bool fits = at + chunks <= kGridQueueCap;
-                    for (int k = lane; k < chunks && at + k < kGridQueueCap; k += 32) queue[at + k] = fits ? make_int2(ci, k) : make_int2(-1, 0);
+                    for (int k = lane; k < chunks && at + k < kGridQueueCap; k += 32) queue[at + k] = fits ? make_int2(ci, k | mark) : make_int2(-1, 0);
                     if (fits && (lane >> 3) == (head >> 3)) here = false;
                 }
                 const bool refused  = grid_rows(a, s, 0, here && cell.by_rows ? cell.y_size : 0, c);

@@ -3091,7 +3091,7 @@ struct vetr_ctx
     long long* tile_sums = nullptr;  // scan scratch
     long long tile_cap   = 0;
     int2* grid_queue     = nullptr;  // (cell, chunk) queue of vetr_grid_loss, allocated by its first call
-    unsigned long long* grid_queue_count = nullptr;  // {queue length, no cell by rows}
+    unsigned long long* grid_queue_count = nullptr;  // {queue length, no cell by rows, pixels of vast cells}
     // running sums of the loss image's rows: the last one is in use, the ones before it were outgrown and stay until the context
     // goes, because a recorded graph may still write to them (each at least twice the one before: together no more than the last)
     double* grid_prefix[32] = {};
@@ -3791,7 +3791,7 @@ extern "C" int vetr_grid_loss(vetr_ctx* ctx, const vetr_cameras* cams, const vet
             ctx->grid_queue_count = reinterpret_cast<unsigned long long*>(ctx->grid_queue + kGridQueueCap);
         }
         a.prefix = grid_prefix(ctx, (long long)view->h * (view->w + 1)), a.no_rows = reinterpret_cast<int*>(ctx->grid_queue_count + 1);
-        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        VETR_CUDA(ctx, cudaMemsetAsync(ctx->grid_queue_count, 0, 3 * sizeof(unsigned long long), ctx->stream));
         if (!a.prefix) VETR_CUDA(ctx, cudaMemsetAsync(a.no_rows, 1, sizeof(int), ctx->stream));
         ctx->launches += 2 + (a.prefix != nullptr);
         if (a.prefix) grid_row_sums_kernel<<<view->h, 256, 0, ctx->stream>>>(a);
