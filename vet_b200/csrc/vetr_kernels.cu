@@ -58,11 +58,25 @@ __device__ __forceinline__ void begin_kernel()
 
 // First statement of a kernel that has nothing to do with what the kernel before it does, only with what was there when that one started (it
 // was launched in the plain way, or is such a kernel itself): it starts on the SMs that the other one's blocks have left, and ends
-// after it, so that a kernel behind it may take the end of both for granted.
+// after it, so that a kernel behind it may take the end of both for granted.  For that one block has to wait, the first; the others give their room back,
+// to blocks of either kernel that want it.  The next kernel may be set up when the first block has waited: earlier, its blocks come to lie next to
+// each other on the SMs that are free first (mode 3, 35 k points x 4 views 385x385 184 -> 201 us), unless it starts beside the same kernel.
+// All blocks waiting / like this, us: 3 M points in a 1920x1080 frame and in it one list of 3000 780 / 745, 50 of 2000 630 / 597, 600 of 1000 786 / 756
+// (three quarters of sort_blend_kernel<true>'s blocks came after the longest list); training, mode 2, 1 M points and 300 lists of 600
+// 901 / 840, 60 k points x 8 views 200x150 415 / 352 (the second of the two kernels for long lists came after the first); no long lists the same.
+template <bool kMoreBeside = false>  // the next kernel starts beside the previous one as well
 struct BesidePrevious
 {
-    __device__ __forceinline__ BesidePrevious() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-    __device__ __forceinline__ ~BesidePrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+    __device__ __forceinline__ BesidePrevious()
+    {
+        if (kMoreBeside) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    __device__ __forceinline__ ~BesidePrevious()
+    {
+        if (blockIdx.x != 0) return;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (!kMoreBeside) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
 };
 struct BeginKernel
 {
@@ -813,7 +827,7 @@ struct ItemStream
 };
 
 // The same for items from a counter behind every CTA's first three: thread 0 asks for an item before the one in front of it is looked up in the
-// table.  A CTA that has come late, or has items of much work, takes fewer.
+// table.  A CTA that has come late, or has items of much work, takes fewer of those.
 struct ItemQueue
 {
     struct Smem
@@ -1016,7 +1030,7 @@ template <bool kQueue>
 __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const __grid_constant__ Frame f,
                                                                           const __grid_constant__ OutPtrs out)
 {
-    const std::conditional_t<kQueue, BesidePrevious, BeginKernel> begin;
+    const std::conditional_t<kQueue, BesidePrevious<>, BeginKernel> begin;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BlendSmem& s = *reinterpret_cast<BlendSmem*>(smem_raw);
     const int tid     = threadIdx.x;
@@ -1227,7 +1241,7 @@ template <bool kFirst>  // started before sort_blend_kernel, or beside its end
 __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ OutPtrs out)
 {
-    const std::conditional_t<kFirst, BeginKernel, BesidePrevious> begin;
+    const std::conditional_t<kFirst, BeginKernel, BesidePrevious<>> begin;
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     LongBlendSmem& s = *reinterpret_cast<LongBlendSmem*>(smem_raw);
@@ -2062,7 +2076,7 @@ template <bool kBilinear>
 __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_constant__ Frame f,
                                                                  const __grid_constant__ BackPtrs bp)
 {
-    const BesidePrevious beside;
+    const BesidePrevious<> beside;
     if (f.status[2] <= kLongList) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BackSmemSuffix& s = *reinterpret_cast<BackSmemSuffix*>(smem_raw);
@@ -2209,7 +2223,7 @@ template <int kMin, int kMax>
 __global__ void __launch_bounds__(kThreads) backward_fuzzy_long_kernel(const __grid_constant__ Frame f,
                                                                        const __grid_constant__ BackPtrs bp)
 {
-    const BesidePrevious beside;
+    const BesidePrevious<kMin == kLongList> beside;
     if (f.status[2] <= kMin) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FuzzyLongSmem<kMax>& s = *reinterpret_cast<FuzzyLongSmem<kMax>*>(smem_raw);
