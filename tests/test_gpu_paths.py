@@ -149,7 +149,16 @@ def test_grid_loss_recorded(rasterizer):
 
 @pytest.mark.parametrize("mode, opacity", [(1, 0.005), (3, 0.005), (3, 0.1), (2, 0.005)])
 def test_long_list_lengths(rasterizer, mode, opacity):
-    lengths = (1, 255, 256, 257, 319, 511, 513, 767, 768, 769, 1023, 1024, 1025, 1537, 2047, 2048, 2049)
+    _check_lists(rasterizer, mode, opacity, (1, 255, 256, 257, 319, 511, 513, 767, 768, 769, 1023, 1024, 1025, 1537, 2047, 2048, 2049))
+
+
+@pytest.mark.parametrize("mode", [1, 3])
+def test_long_list_runs(rasterizer, mode):
+    """Lists of several runs of 2048 fragments, the last run of one fragment, of almost all and in between."""
+    _check_lists(rasterizer, mode, 0.002, (4095, 4096, 4097, 6144, 7000, 8191, 8193, 10241))
+
+
+def _check_lists(rasterizer, mode, opacity, lengths):
     w, h, f = 64, 48, 50.0
     n = sum(lengths)
     sc = scenes.tiny_scene(n=n, w=w, h=h, n_views=1, seed=9)

@@ -709,37 +709,6 @@ __device__ __forceinline__ int row_major_index(const Frame& f, const PixInfo& px
 
 __device__ __forceinline__ int list_end(const Frame& f, int g) { return g < 0 ? 0 : f.ends[g]; }
 
-// In-place ascending sort of a list (keys with their payload) in global memory by the whole CTA, for lists longer
-// than kLongList.  Sorting network with all comparators pointing the same way, so that positions >= n behave as
-// +infinity without padding.
-__device__ void sort_long_list(const Frame& f, int first, int n)
-{
-    uint4* recs = f.recs + 2 * (size_t)first;
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int k = 2; k <= n2; k <<= 1)
-    {
-        for (int j = k >> 1; j > 0; j >>= 1)
-        {
-            for (int i = threadIdx.x; i < n2; i += blockDim.x)
-            {
-                int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-                if (partner > i && partner < n)
-                {
-                    uint4 a = recs[2 * i], b = recs[2 * partner];
-                    if (record_key(a) > record_key(b))
-                    {
-                        recs[2 * i] = b, recs[2 * partner] = a;
-                        uint4 da = recs[2 * i + 1], db = recs[2 * partner + 1];
-                        recs[2 * i + 1] = db, recs[2 * partner + 1] = da;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
 // Which list a staged fragment belongs to.  The thread that owns a pixel writes its index over the pixel's slots when
 // the list is short; the few long lists of an item are recorded separately and matched by range.  (A binary search
 // per fragment costs more instructions than everything else the sort does for it.)
@@ -1135,7 +1104,7 @@ __global__ void __launch_bounds__(kThreads, kBlendCtas) sort_blend_kernel(const 
 // Lists longer than kLongList: one CTA per list, beside the end of sort_blend_kernel, whose CTAs take the same share of the items but not the same
 // time (the two together: 3 M points, one 1920x1080 view, 190 -> 171 us; mode 3, 3 M x 2 views, 1230 -> 1130).  Up to kLongSortMax fragments the keys are merge-sorted in shared memory
 // and the records follow, half a record at a time (the reference's <= 4096 bucket is a CTA-wide shared-memory sort as well,
-// AlphaListSort.cu:601-703); longer lists are sorted in global memory.  The fold runs in blocks of kFoldCap fragments.
+// AlphaListSort.cu:601-703); runs of that many of a longer list are merged in global memory.  The fold runs in blocks of kFoldCap fragments.
 //
 // Bound by latency: the fold of a list is one chain.  So as much as possible is taken out of it - a lane forms the
 // transmittances (one multiplication per fragment), four more the channels (one fused multiply-add per fragment), both on
@@ -1212,6 +1181,39 @@ __device__ void sort_long_list_shared(const Frame& f, LongBlendSmem& ls, int fir
     }
 }
 
+// Any list: runs of kLongSortMax like that, then in global memory by the whole CTA.  Sorting network with all comparators pointing the same
+// way, so that positions >= n behave as +infinity without padding.  One list of 20 000 among 300 k points, one 1920x1080 frame: the network alone 4.99 ms,
+// started beside sort_blend_kernel 5.25 (of 200 000: 64.2, 68.5; most likely the L1 that the kernel before leaves it is smaller), with runs 2.71 (44.2); of
+// 3000 700 -> 280 us; 100 lists of 3000 among 3 M points 2695 -> 892 us.
+__device__ void sort_long_list(const Frame& f, LongBlendSmem& ls, int first, int n)
+{
+    for (int run = 0; run < n; run += kLongSortMax) sort_long_list_shared(f, ls, first + run, min(kLongSortMax, n - run));
+    uint4* recs = f.recs + 2 * (size_t)first;
+    int n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    for (int k = 2 * kLongSortMax; k <= n2; k <<= 1)
+    {
+        for (int j = k >> 1; j > 0; j >>= 1)
+        {
+            for (int i = threadIdx.x; i < n2; i += blockDim.x)
+            {
+                int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
+                if (partner > i && partner < n)
+                {
+                    uint4 a = recs[2 * i], b = recs[2 * partner];
+                    if (record_key(a) > record_key(b))
+                    {
+                        recs[2 * i] = b, recs[2 * partner] = a;
+                        uint4 da = recs[2 * i + 1], db = recs[2 * partner + 1];
+                        recs[2 * i + 1] = db, recs[2 * partner + 1] = da;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // Transmittances of m fragments of one list by one thread: trans[i] in front of fragment i, returns the one behind the last.
 // alpha[m .. next multiple of four) is 0, which leaves the product as it is.  kStop: `m` becomes the number of fragments up
 // to the one that takes the transmittance below 0.001 (mode 3 ends a list there).
@@ -1259,10 +1261,7 @@ __global__ void __launch_bounds__(kLongThreads) sort_blend_long_kernel(const __g
         const int e0 = list_end(f, lo - 1);
         const int n  = f.ends[lo] - e0;
         __syncthreads();
-        if (n <= kLongSortMax)
-            sort_long_list_shared(f, s, e0, n);
-        else
-            sort_long_list(f, e0, n);
+        sort_long_list(f, s, e0, n);
         int cnt = n;
         if (f.dbg_max_len > 0) cnt = min(cnt, f.dbg_max_len);
         if (tid == 0)
