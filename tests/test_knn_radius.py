@@ -161,8 +161,7 @@ def test_gpu_dense_sheet_and_outliers(axis):
 @pytest.mark.parametrize("n", [1, 5, 31, 257, 3001])
 @pytest.mark.parametrize("stride", [3, 4])
 def test_gpu_rows_of_three_and_four(n, stride):
-    """Rows of four floats are read with one 16-byte access, rows of three one by one; a coordinate that is not finite is refused
-    wherever it stands."""
+    """Rows of four and of three floats; a coordinate that is not finite is refused wherever it stands."""
     from vet_b200 import _lib
     from vet_b200.render import Rasterizer
 

@@ -3971,8 +3971,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     unsigned keys[6];
     VETR_CUDA(ctx, cudaMemcpyAsync(d_bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
     const int sweep = std::min((n + 255) / 256, ctx->sm_count * 8);
-    const bool four = position_stride == 4 && ((uintptr_t)position & 15) == 0;
-    (four ? knn_bounds_kernel<true> : knn_bounds_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, d_bounds);
+    knn_bounds_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, d_bounds);
     VETR_CUDA(ctx, cudaMemcpyAsync(keys, d_bounds, sizeof(keys), cudaMemcpyDeviceToHost, st));
     VETR_CUDA(ctx, cudaStreamSynchronize(st));
     float lo[3], hi[3], ext = 0.f, maxabs = 0.f;
@@ -4024,7 +4023,7 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
         g.cell = cell, g.inv_cell = 1.f / cell, g.nx = d[0], g.ny = d[1], g.nz = d[2];
         VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
         VETR_CUDA(ctx, cudaMemsetAsync(d_occ, 0, sizeof(unsigned long long), st));
-        (four ? knn_count_kernel<true> : knn_count_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
         knn_occupied_kernel<<<(int)std::min<long long>((cells + 1023) / 1024, ctx->sm_count * 8), 256, 0, st>>>(ctx->knn_cells + kKnnCellsPad, cells, d_occ);
         unsigned long long occupied = 0;
         VETR_CUDA(ctx, cudaMemcpyAsync(&occupied, d_occ, sizeof(occupied), cudaMemcpyDeviceToHost, st));
@@ -4055,13 +4054,13 @@ extern "C" int vetr_knn_radius(vetr_ctx* ctx, const float* position, int positio
     if (!counted)
     {
         VETR_CUDA(ctx, cudaMemsetAsync(ctx->knn_cells, 0, (size_t)(cells + kKnnCellsPad) * sizeof(int), st));
-        (four ? knn_count_kernel<true> : knn_count_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
+        knn_count_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, g, ctx->knn_cells + kKnnCellsPad, ctx->knn_point_cell);
         ctx->launches += 1;
     }
     knn_tile_sums_kernel<true><<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums);
     knn_spine_kernel<<<1, 1024, 0, st>>>(ctx->knn_tile_sums, n_tiles);
     knn_apply_kernel<true><<<n_tiles, 256, 0, st>>>(cursor, cells, ctx->knn_tile_sums, cursor);
-    (four ? knn_scatter_kernel<true> : knn_scatter_kernel<false>)<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, cursor, ctx->knn_sorted);
+    knn_scatter_kernel<<<sweep, 256, 0, st>>>(position, position_stride, n, ctx->knn_point_cell, cursor, ctx->knn_sorted);
 
     // search
     KnnSearch a;
