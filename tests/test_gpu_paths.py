@@ -392,13 +392,12 @@ def test_grid_loss_cells_around_the_edges_of_the_view(rasterizer, crop):
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
 
-@pytest.mark.parametrize("shift", [0, 1])
-@pytest.mark.parametrize("n, w, h", [(6 * 28416 - 4, 321, 243), (6 * 28416, 321, 243), (6 * 28416 + 3, 321, 243), (1_000_001, 321, 243),
-                                     (3 * 28416 - 4, 147, 143), (3 * 28416 + 1, 147, 143), (3 * 28416, 149, 143)])
-def test_grid_loss_many_cells(rasterizer, n, w, h, shift):
-    """Cell numbers around and above those from which on groups are looked at first on 148 SMs (six groups of four for each of 7104
-    warps, three in an image of few pixels): small and large boxes around the camera and the border of the image; coverage is
-    exact.  shift = 1: boxes that start 12 bytes behind a 16-byte boundary."""
+@pytest.mark.parametrize("w, h", [(321, 243), (147, 143)])
+@pytest.mark.parametrize("n", [4 * 3551 - 1, 4 * 3551 + 1, 8 * 3552 - 4, 8 * 3552 + 1, 32 * 3552 - 4, 32 * 3552 + 1, 1_000_001])
+def test_grid_loss_many_cells(rasterizer, n, w, h):
+    """Cell numbers around those at which a warp of 148 SMs goes about its cells in another way: more groups of four than the stride from one of its
+    groups to the next (3551), from twice to eight times as many as there are warps (two groups, eight groups at a time).  Small and large boxes around
+    the camera and the border of the image; coverage is exact."""
     import torch
 
     sc = scenes.config_planar(64, w, h, 200.0, n_views=1, seed=3)
@@ -410,11 +409,9 @@ def test_grid_loss_many_cells(rasterizer, n, w, h, shift):
     loss = rng.standard_normal((3, h, w)).astype(np.float32)
     ref_v, ref_c = O.grid_loss(sc, sc.views[0], bb_min, bb_len, loss)
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rasterizer.device)  # noqa: E731
-    boxes = [t(np.concatenate([np.zeros((shift, 3), np.float32), a]))[shift:] for a in (bb_min, bb_len)]
-    assert all(a.data_ptr() % 16 == 12 * shift and a.is_contiguous() for a in boxes)
     value, count = torch.zeros(n, device=rasterizer.device), torch.zeros(n, dtype=torch.int32, device=rasterizer.device)
-    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], *boxes, t(loss), value, count)
-    assert (ref_c > 0).sum() > 1000 and (ref_c == 0).sum() > 10_000
+    rasterizer.grid_loss(t(sc.poses), t(sc.intrinsics), sc.views[0], t(bb_min), t(bb_len), t(loss), value, count)
+    assert (ref_c > 0).sum() > n // 100 and (ref_c == 0).sum() > n // 2
     np.testing.assert_array_equal(count.cpu().numpy(), ref_c)
     np.testing.assert_allclose(value.cpu().numpy(), ref_v, rtol=1e-5, atol=0)
 
@@ -699,7 +696,8 @@ def test_large_batches_are_their_halves(rasterizer, mode, n):
     assert seen == fragments
 
 
-@pytest.mark.parametrize("mode, n", [(1, 1_048_577), (3, 262_145)])
+@pytest.mark.parametrize("mode, n", [(1, 262_145), (1, 1_048_577), (3, 262_145)])
 def test_points_per_thread_same_lists(rasterizer, mode, n):
-    """Eight views at which a thread counts and collects several points, against four at a time at which it takes one."""
+    """Eight views against four at a time, just above the points times views from which on a thread takes several points: mode 1 in counting, mode 1 in
+    collecting (both count several), mode 3 in both."""
     test_large_batches_are_their_halves(rasterizer, mode, n)
