@@ -2197,13 +2197,11 @@ __global__ void __launch_bounds__(kThreads) backward_long_kernel(const __grid_co
 // into blocks), beside the end of backward_kernel (mode 2, 1 M points, 801x603: the whole call 431 -> 373 us).  Lists beyond kFuzzyLongMax are skipped and flagged in the status word (the reference itself sorts only
 // the first 4096 fragments of a list, AlphaListSort.cu:289-290, so its result for longer lists is not defined either).
 //
-// Launched twice: lists of up to kFuzzyMidMax fragments, eight of which fit an SM, and the longer ones, one per SM.  Two steps of a
-// list are one thread's chain each (fuzzy_groups, fuzzy_suffix), so a launch with few lists takes as long as the longest of them: 1 M
-// points, 801x603, 61 us with the line anywhere from 512 to 4096 (one launch for all).  With lists on both sides of the line the
-// two launches follow each other, so that no line is the best one everywhere.  Both launches, without a drop-out radius, line at
-// 512 / 1024 / 2048 / 4096: 60 k points, 8 views 200x150 (174 lists up to 851) 284 / 166 / 176 / 175 us; 200 k, one view (188 up to
-// 1024, 11 up to 2252) 459 / 547 / 633 / 361; 400 k, 4 views 400x300 (1256 and 16 up to 1496) 956 / 616 / 527 / 686; 1 M, 8 views
-// 801x603 (3731 and 50 up to 2041) 2101 / 1524 / 837 / 1353.
+// Launched twice, beside backward_kernel and each other: lists of up to kFuzzyMidMax fragments, eight of which fit an SM, and the longer ones, one per
+// SM.  Two steps of a list are one thread's chain each (fuzzy_groups, fuzzy_suffix), so a launch with few lists takes as long as the longest of them.
+// A training step without a drop-out radius, us, line at 512 / 1024 / 2048 / 4095: 60 k points, 8 views 200x150 (longest list 578) 364 / 353 / 430 /
+// 440; 200 k, one view (1256) 448 / 410 / 397 / 447; 400 k, 4 views 400x300 (1110) 948 / 833 / 986 / 1091; 1 M, 8 views 801x603 (1545) 3250 / 2853 /
+// 3010 / 3397; with the radius, 1 M, one view (179), no difference.
 constexpr int kFuzzyLongMax = 4096;  // what the reference sorts of a list (AlphaListSort.cu:289-290)
 constexpr int kFuzzyMidMax  = 1024;
 template <int kMax>
@@ -3149,12 +3147,13 @@ struct PassScope
     }
 };
 
-// Launches a kernel that begins with begin_kernel().  overlap: its blocks may be set up while the kernel before it on the stream ends, which hides
-// the way from one kernel to the next.  100 k points at 512x512 101 -> 85 us, a smallest batch 85 -> 82, 3 M points at 1920x1080
+// Launches a kernel that waits for the one before it on the stream: begin_kernel() at the start or, where it has nothing to do with what that one does,
+// BesidePrevious at the end (always with overlap).  overlap: its blocks may be set up while the kernel before it ends, which hides
+// the way from one kernel to the next.  Waiting at the start, 100 k points at 512x512 101 -> 85 us, a smallest batch 85 -> 82, 3 M points at 1920x1080
 // forward only 344 -> 335, mode 2 with 1 M points 459 -> 440, mode 0 with 2 M points and two views 388 -> 374, mode 3 with 3 M points and two views
 // the same.  Not where
-// - the kernel is one of the item kernels (sort + blend, backward, their long lists), whose blocks take every n-th item: set up early they
-//   come to lie next to each other on the SMs that are free first, and so do the items of much work (mode 3 at 1280x720 428 -> 450 us);
+// - the kernel is an item kernel (sort + blend, backward, the long lists that go first) and waits at its start: its blocks take every n-th item, and set
+//   up early they come to lie next to each other on the SMs that are free first, and so do the items of much work (mode 3 at 1280x720 428 -> 450 us);
 // - there is much to do (20 M points, eight views 18120 -> 18440 us, 8 M points and four views the same): nothing to be gained.
 constexpr long long kOverlapPoints = 1 << 24;            // points times views, elements
 constexpr long long kOverlapUnits  = 3 * kOverlapPoints;  // 16-byte units of zeros: a point's gradients are 2.25 of them
