@@ -47,9 +47,9 @@
 
 namespace vetr
 {
-// First statement of every kernel that launch() starts, and of those in between: the next kernel on the stream may be set up on SMs that have room as soon
-// as all blocks of this one run, and this one goes on when the kernel before it has ended and its writes are to be seen.  Nothing is
-// read or written before; because every kernel waits like this, the end of one is the end of all before it.
+// First statement of the kernels that launch() starts (but those that wait at their end, below), and of those in between: the next kernel on the stream
+// may be set up on SMs that have room as soon as all blocks of this one run, and this one goes on when the kernel before it has ended and its writes
+// are to be seen.  Nothing is read or written before; because every kernel waits, the end of one is the end of all before it.
 __device__ __forceinline__ void begin_kernel()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
