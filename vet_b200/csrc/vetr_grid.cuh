@@ -824,10 +824,10 @@ __global__ void __launch_bounds__(32 * kGridWarps, kGridCtas) grid_loss_kernel(c
                 const bool vast = (lane & 7) == 0 && !cell.by_rows && parts > kGridVast;
                 if (__any_sync(0xffffffffu, vast))
                 {
-                    const int mine = __reduce_add_sync(0xffffffffu, vast ? min(parts, 1 << 28) : 0);
+                    const int pixels = __reduce_add_sync(0xffffffffu, vast ? min(parts, 1 << 28) : 0);
                     unsigned long long all = 0;
-                    if (lane == 0) all = atomicAdd(queue_count + 2, (unsigned long long)mine);
-                    all = __shfl_sync(0xffffffffu, all, 0) + mine;
+                    if (lane == 0) all = atomicAdd(queue_count + 2, (unsigned long long)pixels);
+                    all = __shfl_sync(0xffffffffu, all, 0) + pixels;
                     if (vast) coarse = max(coarse, grid_coarse_vast(all));
                 }
                 const int n_chunks = ((parts - 1) >> (cell.by_rows ? kGridRowBits : kGridChunkBits + coarse)) + 1;
