@@ -80,7 +80,7 @@ constexpr int kGridExactLanes = 6;              // rows of a warp with pixels to
 constexpr int kGridQueueCap = 4 * 1024 * 1024;  // (cell, chunk) pairs handed to the second kernel
 // Sizes of the per-pixel form's chunks, 64 << 0 to kGridCoarsest pixels: see grid_coarse.
 constexpr int kGridCoarsest   = 3;
-constexpr int kGridCoarseFrom = kGridQueueCap / 16;  // chunks in the queue
+constexpr int kGridCoarseFrom = kGridQueueCap / 8;  // chunks in the queue
 constexpr int kGridVast       = 1 << 16;        // pixels of a cell
 constexpr int kGridMarkAt     = 28;             // bit of a chunk's number from which on the shift stands (an image has no more than 2^31 / 64 chunks)
 constexpr int kGridSegments = 18;               // 12 edges, then 6 face diagonals
@@ -723,17 +723,22 @@ __device__ __forceinline__ bool grid_out_of_sight(const GridArgs& a, const GridP
 // - where no cell goes by rows, by the size of the image.  Eight distortion coefficients, 64 pixels / 256 / 512: 128^3 cells at 1920x1080 64 / 7.0 / 6.8 ms,
 //   64^3 4.1 / 3.4 / 3.3, 16^3 1.01 / 0.88 / 0.80, 96^3 at 1237x823 3.2 / 2.6 / 2.5, 48^3 at 960x540 0.76 / 0.68 / 0.75, 32^3 at 640x480
 //   0.32 / 0.30 / 0.36, 16^3 at 320x240 0.08 / 0.11 / 0.18, 128^3 at 160x120 0.38 / 0.47 / 0.45;
-// - from kGridCoarseFrom chunks on.  Without distortion, 4e6 units from the origin, 64 pixels / 512 / like this: 128^3 71 / 13.9 / 14.0 ms, 64^3 2.5 /
-//   2.1 / 2.3 (from four times as many on: 2.5);
-// - in vast cells, by the pixels of all of them so far.  Flat boxes, always 64 / like this: four over the whole view 396 / 180 us, 300 of them
-//   112 / 6.4 ms, 20 of 700x700 pixels 290 / 210 us, one 87 / 85.
+// - from kGridCoarseFrom chunks on.  Without distortion, 4e6 units from the origin, 64 pixels / 512 / like this: 128^3 71 / 13.9 / 14.1 ms, 64^3 2.45 /
+//   2.1 / 2.43.  Views near a face of the grid, where 30 million pixels are in that form, stay below it: half of that line 1051 -> 1233 us;
+// - in vast cells, by the pixels of all of them so far.  Flat boxes, always 64 / like this: four over the whole view 396 / 185 us, 300 of them
+//   112 / 6.5 ms, 20 of 700x700 pixels 290 / 200 us, one 90 / 86.  Up to 512 pixels only where there are 33 million, because the few of a
+//   grid among cells by rows are the last to end (200 views of 128^3 cells, against always 64: 0.996 of the time on average and 1.02 at most; with
+//   512 from four million on 1.17 at most).
 __device__ __forceinline__ int grid_coarse(const GridArgs& a, bool no_rows, int queued)
 {
     if (queued >= kGridCoarseFrom) return kGridCoarsest;
     const int pixels = a.w * a.h;
     return !no_rows || pixels < 1 << 17 ? 0 : pixels < 1 << 20 ? 2 : kGridCoarsest;
 }
-__device__ __forceinline__ int grid_coarse_vast(unsigned long long pixels) { return min(64 - __clzll((long long)(pixels >> 20)), kGridCoarsest); }
+__device__ __forceinline__ int grid_coarse_vast(unsigned long long pixels)
+{
+    return pixels >= 1ull << 25 ? kGridCoarsest : min(64 - __clzll((long long)(pixels >> 20)), 2);
+}
 
 // First kernel (kChunks = false): a warp takes `each` groups of four cells at a time, leaves out those that lie out of sight and prepares the others, a
 // lane per cell, as soon as it has 32 of them; what is left of these is drawn in groups of four, eight lanes per cell.  Cells with many rows
